@@ -116,9 +116,9 @@ PSOCI_API psoci_status psoci_get_determinants(const psoci_ctx *ctx, uint64_t *al
  * psoci_save_hamiltonian and psoci_sigma_mixed_noalloc answer PSOCI_ERR_STATE. */
 PSOCI_API psoci_status psoci_build_hamiltonian(psoci_ctx *ctx, psoci_hmode mode, int64_t *nnz);
 /* Counters and phase times of the last psoci_build_hamiltonian.  Times are CUDA-event
- * intervals on the library stream, in milliseconds; the evaluation time covers the final
- * attempt only (an undersized value slab makes the build evaluate twice).  The reference
- * reports its build time through PsociTimer; there is no direct counterpart. */
+ * intervals on the library stream, in milliseconds: screen; evaluate (coupling tables, diagonal
+ * blocks and the count of each row's elements); rows (offsets); assemble (the elements written).
+ * The reference reports its build time through PsociTimer; there is no direct counterpart. */
 typedef struct {
   int64_t candidates;    /* configuration pairs the screen tested one by one (ordered): all   */
                          /* pairs within two excitations (all-pairs screen), or those left  */
@@ -127,20 +127,21 @@ typedef struct {
   int64_t segments;      /* warp work items (<= 32 neighbours of one row configuration)      */
   int64_t nnz;           /* stored elements, both triangles                                  */
   int64_t nnz_lower;     /* the reference's lower-triangle count, (nnz + N) / 2              */
-  int64_t slab_slots;    /* value-slab slots taken by the evaluation                         */
-  int evaluations;       /* 1, or 2 after a slab overflow                                    */
-  int fast;              /* 1: lower blocks evaluated once and mirrored; 0: generic path      */
+  int64_t slab_slots;    /* 0 (the build has no value slab)                                  */
+  int evaluations;       /* 1                                                                */
+  int fast;              /* 1: elements from coupling tables (at most 10 open shells);       */
+                         /* 0: generic path                                                  */
   int lookup_screen;     /* 1: neighbours found by table lookup; 0: all-pairs test            */
-  int eval_launches;     /* fast path: 2 masks and elements launched apart, 1 one launch;    */
-                         /* 0 otherwise                                                     */
+  int eval_launches;     /* fast path: 2 pair integrals in a launch of their own, 1 in the   */
+                         /* element launches; 0 otherwise                                    */
   double screen_ms, evaluate_ms, rows_ms, assemble_ms, total_ms;
 } psoci_build_info;
 PSOCI_API psoci_status psoci_build_stats(const psoci_ctx *ctx, psoci_build_info *info);
-/* The fast build evaluates its elements in two launches (the determinant-connectivity masks,
- * 8 bytes per (pair, row SEF), then the elements) when those masks fit in a quarter of the
- * free device memory, else in one launch.  launches = 1 asks for the one-launch form (less
- * memory, slower), 0 for the automatic choice (the default).  The stored matrix is the same
- * bit for bit either way.  No counterpart in the reference (a GPU scheduling choice). */
+/* The fast build evaluates the integrals of every configuration pair in a launch of their own and
+ * lists them (16 bytes a pair) when the list takes at most a quarter of the device memory at
+ * hand; otherwise the element launches evaluate them themselves.  launches = 1 asks for the
+ * latter (less memory, slower), 0 for the automatic choice (the default).  The stored matrix is
+ * the same bit for bit either way.  No counterpart in the reference (a GPU scheduling choice). */
 PSOCI_API psoci_status psoci_set_eval_launches(psoci_ctx *ctx, int launches);
 
 /* Replaces PsociHamiltonian::generateSOCIblocks (PsociHamiltonian.C:401-558) for a batch of

@@ -37,7 +37,7 @@ def main(argv=None):
     ap.add_argument("--gradient", action="store_true", help="energy gradients of the roots")
     ap.add_argument("--direct", action="store_true", help="direct mode: no stored elements")
     ap.add_argument("--eval-launches", type=int, default=0, choices=(0, 1),
-                    help="1: the H build's element evaluation in one launch (default 0: two when they fit)")
+                    help="1: the H build's pair integrals in the element launches (default 0: listed by their own when they fit)")
     ap.add_argument("--max-subspace", type=int, default=48)
     ap.add_argument("--device", type=int, default=0)
     ap.add_argument("--verbose", type=int, default=0)

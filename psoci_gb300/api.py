@@ -353,7 +353,8 @@ class Context:
         return ch.value, [float(x) for x in t]
 
     def set_eval_launches(self, launches: int):
-        """1: evaluate the H build's elements in one launch; 0: automatic (two when they fit)."""
+        """1: the H build's pair integrals evaluated in the element launches; 0: automatic (listed
+        by a launch of their own when the list fits)."""
         self._check(self.lib.psoci_set_eval_launches(self.ctx, launches), "set_eval_launches")
 
     def set_sigma_variant(self, v: int):

@@ -13,24 +13,20 @@
 // Storage.  The reference keeps the lower triangle and runs a symmetric product.  On one
 // GPU the full matrix in CSR streams twice the bytes but needs no scattered atomics in
 // sigma, so both triangles are stored.  Every off-diagonal element is the reference's
-// lower-triangle value: only the blocks (I, J <= I) are evaluated, as the reference does,
-// and the upper half of the matrix is their mirror image.  Rows are written in ascending
-// column order, deterministically:
+// lower-triangle value: a block (I, J > I) is the block (J, I) in the reference's roles,
+// transposed.  Rows are written in ascending column order, deterministically:
 //
-//   1. screen:   per configuration, the sorted list of configurations within two
-//                excitations (XOR + popcount on occupancy bit-planes), then the blocks
-//                that the integrals alone make zero are dropped;
-//   2. segments: the lower neighbours (J <= I) of each row configuration in groups of <= 32,
-//                one warp each;
-//   3. evaluate: each warp marks the SEF elements that determinant connectivity allows and
-//                evaluates them; kept values go to slab slots, per (pair, row SEF) a mask of
-//                kept columns (fast path, <= 32 determinants per configuration);
-//   4. rows:     full row lengths = lower counts + the mirrored columns of upper neighbours;
-//   5. assemble: columns and values in order, the FP32 copy and the diagonal.
+//   1. screen:  per configuration, the sorted list of configurations within two
+//               excitations (XOR + popcount on occupancy bit-planes), then the blocks
+//               that the integrals alone make zero are dropped;
+//   2. tables:  every pair's coupling table (blocktab.cuh) and integrals;
+//   3. count:   the kept elements of each row, from the tables;
+//   4. offsets: a scan of the counts;
+//   5. fill:    columns and values in order, the FP32 copy.
+// The diagonal blocks are evaluated determinant by determinant before the count.
 //
-// Configurations with more than 32 determinants (7-11 open shells) take the generic path:
-// every block (I, J) of the full neighbour list is evaluated in a count pass and again in
-// a fill pass (a block with J > I as the reference's block (J, I), transposed).
+// Spaces with 11 open shells take the generic path instead: every block of the full neighbour
+// list is evaluated determinant by determinant in a count pass and again in a fill pass.
 //
 // Floating point follows the reference's operation order; this file is compiled with
 // --fmad=false so products and sums round as the reference's do.
@@ -42,6 +38,7 @@
 #include <queue>
 #include <vector>
 
+#include "blocktab.cuh"
 #include "psoci_internal.cuh"
 
 namespace {
@@ -85,7 +82,6 @@ struct Params {
   // screen
   const int64_t *nbroff;
   int32_t *nbr;
-  int64_t nbr_len;         // entries of nbr
   // segments
   int64_t nseg;
   const int32_t *seg_cfg;
@@ -93,17 +89,6 @@ struct Params {
   const int32_t *seg_n;
   const int64_t *seg_rowoff;
   int64_t *seg_cnt;        // count pass output / fill pass row offsets (local)
-  // single-pass fast build over the lower pairs (J <= I): kept values are appended to slab
-  // slots; per (pair, row SEF) a mask of kept columns and the pair's offset in the slot
-  const int64_t *segoff;   // first segment of each configuration
-  const int64_t *nlow;     // neighbours J <= I
-  const int64_t *pr_off;   // first (pair, row) mask of each configuration
-  uint64_t *prm;           // bits 0-15: kept column SEFs t; bits 16-63: slab position of the first
-                           // of them (the pair's values in the row run follow one another)
-  unsigned long long *slab_counter;
-  int64_t slab_cap;
-  double *slab_val;
-  uint64_t *cg;            // connectivity masks C[r] per (pair, row SEF), as prm (two-launch evaluation)
   const int64_t *rowptr;
   int32_t *col;
   double *val;
@@ -675,24 +660,23 @@ __global__ void k_screen_offsets(int nconf, int nsplit, const int64_t *cnt, int6
   tot[i] = run;
 }
 
-// per configuration: number of segments and segment-row slots over its first nlen[i]
-// neighbours (all of them when nlen is null)
-__global__ void k_seg_counts(int nconf, const int64_t *nbroff, const int64_t *nlen, const int64_t *sefoff,
-                             int64_t *nseg_i, int64_t *nrow_i) {
+// per configuration: number of segments and segment-row slots over its neighbours
+__global__ void k_seg_counts(int nconf, const int64_t *nbroff, const int64_t *sefoff, int64_t *nseg_i,
+                             int64_t *nrow_i) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nconf) return;
-  int64_t nn = nlen ? nlen[i] : nbroff[i + 1] - nbroff[i];
+  int64_t nn = nbroff[i + 1] - nbroff[i];
   int64_t ns = (nn + PSOCI_SEG - 1) / PSOCI_SEG;
   nseg_i[i] = ns;
   nrow_i[i] = ns * (sefoff[i + 1] - sefoff[i]);
 }
 
-__global__ void k_seg_init(int nconf, const int64_t *nbroff, const int64_t *nlen, const int64_t *sefoff,
-                           const int64_t *segoff, const int64_t *rowslot, int32_t *seg_cfg, int64_t *seg_k0,
+__global__ void k_seg_init(int nconf, const int64_t *nbroff, const int64_t *sefoff, const int64_t *segoff,
+                           const int64_t *rowslot, int32_t *seg_cfg, int64_t *seg_k0,
                            int32_t *seg_n, int64_t *seg_rowoff) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nconf) return;
-  int64_t nn = nlen ? nlen[i] : nbroff[i + 1] - nbroff[i];
+  int64_t nn = nbroff[i + 1] - nbroff[i];
   int64_t s0 = segoff[i], ns = segoff[i + 1] - s0;
   int64_t nsef = sefoff[i + 1] - sefoff[i];
   for (int64_t s = 0; s < ns; ++s) {
@@ -702,21 +686,6 @@ __global__ void k_seg_init(int nconf, const int64_t *nbroff, const int64_t *nlen
     seg_n[s0 + s] = (int32_t)(left < PSOCI_SEG ? left : PSOCI_SEG);
     seg_rowoff[s0 + s] = rowslot[i] + s * nsef;
   }
-}
-
-// per configuration: nlow = neighbours J <= i (the lists are sorted ascending) and the
-// number of (lower pair, row SEF) mask slots, nlow * nsef_i
-__global__ void k_lower_counts(int nconf, const int64_t *nbroff, const int32_t *nbr, const int64_t *sefoff,
-                               int64_t *nlow, int64_t *prrows) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nconf) return;
-  int64_t lo = nbroff[i], hi = nbroff[i + 1];
-  while (lo < hi) {  // first entry > i
-    int64_t mid = (lo + hi) >> 1;
-    if (nbr[mid] <= (int32_t)i) lo = mid + 1; else hi = mid;
-  }
-  nlow[i] = lo - nbroff[i];
-  prrows[i] = nlow[i] * (sefoff[i + 1] - sefoff[i]);
 }
 
 // per configuration: exclusive scan over its segments of the per-row counts (in place),
@@ -1066,33 +1035,20 @@ __device__ __forceinline__ double det_elem(const double *eri, const PairInfo &pi
   return (ncount & 1) ? -v : v;
 }
 
-// Where sef_elem finds the determinants of A: the global tables, or a copy of A's own
-// determinants in shared memory (rows indexed from A's first determinant).
-struct RowDets {
-  const uint64_t *al, *be;
-  const uint8_t *ph, *na;
-};
-
-// SEF element (a, b) of the reference block (A, B): ciout / transformCDCt.  conn bit
-// (x << 1 | y) says whether determinant x of SEF a and determinant y of SEF b can couple;
-// a determinant element that cannot is exactly zero and is not evaluated (adding the zero
-// it would return leaves every partial sum unchanged).  The determinant elements are
+// SEF element (a, b) of the reference block (A, B): ciout / transformCDCt.  The determinant elements are
 // added in the reference's order: t = d00 + mB d01, u = d10 + mB d11, r (r t) + mA r (r u).
 template <int W>
-__device__ double sef_elem(const Params &PP, const PairInfo &pi, const double *Kd, int a, int b,
-                           unsigned conn = 0xFu, const RowDets *rowA = nullptr) {
+__device__ double sef_elem(const Params &PP, const PairInfo &pi, const double *Kd, int a, int b) {
   if (pi.kind == K_NONE) return 0.0;
   const bool odd = PP.nelec & 1;
   const bool oa = !odd && pi.nopenA != 0, ob = !odd && pi.nopenB != 0;
   const int64_t a0 = odd ? a : (oa ? 2 * a : 0), b0 = pi.detB + (odd ? b : (ob ? 2 * b : 0));
-  if (!ob) conn &= 0x5u;
-  if (!oa) conn &= 0x3u;
+  const unsigned conn = (ob ? 0xFu : 0x5u) & (oa ? 0xFu : 0x3u);  // determinant pairs there are: bit x << 1 | y
   DetBits<W> A[2] = {}, B[2] = {};
 #pragma unroll
   for (int x = 0; x < 2; ++x) {
     if (x == 1 && !oa) break;
-    if (rowA) load_det<W>(A[x], rowA->al, rowA->be, rowA->ph, rowA->na, a0 + x);
-    else load_det<W>(A[x], PP.alpha, PP.beta, PP.phase, PP.nalpha, pi.detA + a0 + x);
+    load_det<W>(A[x], PP.alpha, PP.beta, PP.phase, PP.nalpha, pi.detA + a0 + x);
   }
 #pragma unroll
   for (int y = 0; y < 2; ++y) {
@@ -1249,762 +1205,601 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32) k_hbuild(Params P) {
 }
 
 // ------------------------------------------------------------------------------------
-// Fast segment kernel for configurations of at most 32 determinants (<= 6 open shells with
-// an even electron count, <= 5 with an odd one; at most 16 SEFs).  A SEF block is sparse:
-// a determinant couples only to determinants within two spin-orbital substitutions with
-// the same spin projection (one substitution, any spin, for spin-orbit pairs).  Each lane
-// owns one neighbour J and first marks, per row SEF r of I, the column SEFs t whose
-// determinants pass that test; only marked elements are then evaluated, with the same
-// element function (and operation order) as the generic kernel.  An unmarked element is
-// a combination of zero determinant elements and therefore exactly zero.
+// Elements from coupling tables (blocktab.cuh), for configurations of at most TAB_MAXOPEN open
+// shells.  k_pair_slots gives every pair of the neighbour lists its table (and its integrals);
+// k_elems then walks each configuration's list, 32 pairs at a time, and
+//   MODE 0  counts the kept elements of its rows,
+//   MODE 1  writes them, columns ascending, at the rows' places,
+//   MODE 2  multiplies them with X (direct mode), MODE 3 with X in FP32.
+// Both triangles are evaluated: an element costs so little that reading its pair twice is cheaper
+// than mirroring it.  mrcisd_6e8o_v48 (2.18 million SEFs, 1.25e9 elements): pair slots, tables and
+// diagonal 10.7 ms, count 6.9 ms, fill 17.5 ms (12.5 GB of CSR: 1.9 ms at the copy rate), where
+// evaluating the lower triangle determinant by determinant, counting its mirror image and
+// assembling the rows took 98 + 7 + 27 ms; 31,650 SEFs with up to 8 open shells: 14.6 -> 2.1 ms.
 // ------------------------------------------------------------------------------------
-constexpr int FAST_MAXDET = 32;
-constexpr int FAST_MAXSEF = 16;
-constexpr int FAST_MAXOPEN = 6;  // 2^(6-1) = 32 determinants
-constexpr int SLAB_CHUNK = 4096; // slab slots a warp takes at a time
-constexpr int FAST_ROWS = 4;     // rows of a configuration evaluated together
-constexpr int FAST_MAXK = 1 + FAST_MAXOPEN * (FAST_MAXOPEN - 1) / 2;  // diagonal list, <= 6 open shells
-
-__device__ __forceinline__ bool tbit(const uint64_t *x, int p) { return (x[p >> 6] >> (p & 63)) & 1ull; }
-
 template <int W>
-struct FastSmem {
-  PairInfo pi[PSOCI_SEG];
-  double K[FAST_MAXK];
-  uint64_t ra[FAST_MAXDET * W], rb[FAST_MAXDET * W];
-  uint8_t rna[FAST_MAXDET], rph[FAST_MAXDET];
-  // phase 2, per row of a group: connectivity of the marked elements of each slot (see
-  // below; the marked columns are its four 16-bit quarters or-ed), their exclusive prefix,
-  // kept columns of each neighbour
-  uint64_t cm[FAST_ROWS][PSOCI_SEG];
-  int16_t pre[FAST_ROWS][PSOCI_SEG];
-  uint32_t keep[FAST_ROWS][PSOCI_SEG];
-  int8_t perm[PSOCI_SEG];  // evaluation order: slot -> neighbour lane, grouped by pair kind
-};
-
-// DIRECT (direct mode): segments over the full neighbour lists; instead of storing the kept
-// elements, Y[row, 0:kvec] += element * X[column, 0:kvec], added atomically per row.
-// PH: 0 both phases in one launch; 2 phase 2 alone, from the connectivity masks that
-// k_hbuild_masks stored in P.cg (each launch then runs a smaller body).
-template <int W, int DIRECT = 0, int PH = 0>
-__global__ void __launch_bounds__(WARPS_PER_CTA * 32) k_hbuild_fast(Params P) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  FastSmem<W> *ws = reinterpret_cast<FastSmem<W> *>(smem_raw) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const bool odd = P.nelec & 1;
-  unsigned long long cursor = 0, chunk_end = 0;  // this warp's slab chunk
-  for (int64_t s = warp; s < P.nseg; s += nwarps) {
-    const int I = P.seg_cfg[s];
-    const int64_t k0 = P.seg_k0[s];
-    const int n = P.seg_n[s];
-    const int nsefI = (int)(P.sefoff[I + 1] - P.sefoff[I]);
-    const int64_t d0I = P.detoff[I];
-    const int ndI = (int)(P.detoff[I + 1] - d0I);
-    const int nopI = P.nopen[I];
-    if (lane < n) pair_setup<W>(P, I, P.nbr[k0 + lane], ws->pi[lane], ws->K);
-    for (int d = lane; d < ndI; d += 32) {
+__global__ void k_cfg_rec(Params P, CfgRec<W> *__restrict__ out) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P.nconf; i += (int64_t)gridDim.x * blockDim.x) {
+    CfgRec<W> r;
 #pragma unroll
-      for (int w = 0; w < W; ++w) {
-        ws->ra[d * W + w] = P.alpha[(d0I + d) * W + w];
-        ws->rb[d * W + w] = P.beta[(d0I + d) * W + w];
-      }
-      ws->rna[d] = P.nalpha[d0I + d];
-      ws->rph[d] = P.phase[d0I + d];
-    }
-    __syncwarp();
-    // phase 1: connectivity masks C[r] for this lane's neighbour, bit-parallel over the
-    // row determinants.  With m_a the alpha pattern of row det a on I's open shells, a column
-    // det b (alpha ab, beta bb) differs from a in
-    //   c(a) = F + #{p in x : p not in m_a} + #{p in y : p in m_a}
-    // spin-orbitals of b, where x, y are b's alpha / beta patterns on I's open shells and F
-    // counts b's electrons in orbitals empty in I.  Non-spin-orbit pairs need c(a) <= 2 and
-    // equal alpha counts, spin-orbit pairs c(a) <= 1 (the tests det_elem starts with).  The sets
-    // {a : p in m_a} and {a : |m_a| = k} are warp ballots; c(a) is kept as a saturating
-    // bit-sliced counter over all row dets at once.
-    uint32_t Ap[FAST_MAXOPEN], Nk[FAST_MAXOPEN + 1];
-    int sI[FAST_MAXOPEN];
-    uint64_t occI[W];
-    if (PH != 2) {
-      uint64_t SI[W];
-#pragma unroll
-      for (int w = 0; w < W; ++w) {
-        occI[w] = P.e1[(int64_t)I * W + w];
-        SI[w] = occI[w] & ~P.e2[(int64_t)I * W + w];
-      }
-      // open shells of I, ascending (fixed-size loops keep these arrays in registers)
-#pragma unroll
-      for (int p = 0; p < FAST_MAXOPEN; ++p) {
-        sI[p] = lowest_bit<W>(SI);
-        bool done = false;
-#pragma unroll
-        for (int w = 0; w < W; ++w)
-          if (!done && SI[w]) { SI[w] &= SI[w] - 1; done = true; }
-      }
-      uint32_t ma = 0u;
-      if (lane < ndI)
-#pragma unroll
-        for (int p = 0; p < FAST_MAXOPEN; ++p)
-          if (p < nopI) ma |= (uint32_t)tbit(&ws->ra[lane * W], sI[p]) << p;
-#pragma unroll
-      for (int p = 0; p < FAST_MAXOPEN; ++p) Ap[p] = __ballot_sync(0xffffffffu, (lane < ndI) && ((ma >> p) & 1u));
-#pragma unroll
-      for (int k = 0; k <= FAST_MAXOPEN; ++k) Nk[k] = __ballot_sync(0xffffffffu, (lane < ndI) && __popc(ma) == k);
-    }
-    const int ndblI = P.nelec - nopI;  // electrons in I's doubly occupied orbitals
-    // C[r]: for row SEF r and column SEF t, bit t + 16 (x << 1 | y) says that determinant x
-    // of SEF r and determinant y of SEF t can couple; the SEF element is marked when any can.
-    uint64_t C[FAST_MAXSEF];
-    for (int r = 0; r < FAST_MAXSEF; ++r) C[r] = 0ull;
-    if (PH != 2 && lane < n) {
-      const PairInfo &pi = ws->pi[lane];
-      if (pi.kind != K_NONE) {
-        const bool so = (pi.kind == K_SO);
-        const int64_t d0J = pi.swap ? pi.detA : pi.detB;
-        const int nopJ = pi.swap ? pi.nopenA : pi.nopenB;
-        const int ndJ = 1 << (nopJ > 1 ? nopJ - 1 : 0);
-        const int thr = so ? 1 : 2;
-        const uint32_t rows_valid = (ndI >= 32) ? 0xffffffffu : ((1u << ndI) - 1u);
-        for (int b = 0; b < ndJ; ++b) {
-          uint64_t ja[W], jb[W];
-#pragma unroll
-          for (int w = 0; w < W; ++w) { ja[w] = __ldg(P.alpha + (d0J + b) * W + w); jb[w] = __ldg(P.beta + (d0J + b) * W + w); }
-          int F = 0;
-#pragma unroll
-          for (int w = 0; w < W; ++w) F += __popcll(ja[w] & ~occI[w]) + __popcll(jb[w] & ~occI[w]);
-          if (F > thr) continue;
-          uint32_t ok = 0u;
-          {
-            // saturating counter over the row dets: S0 (c'=0), S1, S2, S3 (>= 3)
-            uint32_t S0 = 0xffffffffu, S1 = 0u, S2 = 0u;
-#pragma unroll
-            for (int p = 0; p < FAST_MAXOPEN; ++p) {
-              if (p >= nopI) break;
-              const bool xa = bit_w<W>(ja, sI[p]), yb = bit_w<W>(jb, sI[p]);
-              if (xa) {  // mismatch where row det has beta on p
-                const uint32_t T = ~Ap[p];
-                S2 = (S2 & ~T) | (S1 & T);
-                S1 = (S1 & ~T) | (S0 & T);
-                S0 &= ~T;
-              }
-              if (yb) {  // mismatch where row det has alpha on p
-                const uint32_t T = Ap[p];
-                S2 = (S2 & ~T) | (S1 & T);
-                S1 = (S1 & ~T) | (S0 & T);
-                S0 &= ~T;
-              }
-            }
-            ok = (thr - F >= 2) ? (S0 | S1 | S2) : (thr - F == 1) ? (S0 | S1) : S0;
-          }
-          int na = 0;
-#pragma unroll
-          for (int w = 0; w < W; ++w) na += __popcll(ja[w]);
-          const int need = na - (ndblI / 2);  // alpha open shells a row det needs for equal counts
-          ok &= rows_valid;
-          if (!so) {
-            uint32_t nk = 0u;
-#pragma unroll
-            for (int k = 0; k <= FAST_MAXOPEN; ++k)
-              if (k == need) nk = Nk[k];
-            ok &= (need >= 0 && need <= nopI) ? nk : 0u;
-          }
-          const int t = odd ? b : (nopJ ? (b >> 1) : 0);
-          const int y = (!odd && nopJ) ? (b & 1) : 0;
-          while (ok) {
-            const int a = __ffs(ok) - 1;
-            ok &= ok - 1;
-            const int x = (!odd && nopI) ? (a & 1) : 0;
-            C[odd ? a : (nopI ? (a >> 1) : 0)] |= 1ull << (t + 16 * ((x << 1) | y));
-          }
-        }
-      }
-    }
-    const int64_t prbase = DIRECT ? 0 : P.pr_off[I] + (k0 - P.nbroff[I]) * nsefI;
-    // phase 2, FAST_ROWS rows at a time (one row in the direct modes, whose sums are per
-    // row): the marked elements of the group's rows, in (row, neighbour, column) order, are
-    // numbered e = 0..T-1 and lane e % 32 evaluates element e, so the lanes share the work
-    // whatever the spread of marks over the neighbours and rows (a row holds about one
-    // warp's worth of marks: taken alone, its last pass would run on few lanes).  Kept values
-    // are compacted in the same order, so each row's values form one run in ascending column
-    // order and the runs of a group follow one another.  Each warp takes slab space in chunks
-    // and advances through a chunk by the kept count of each group.
-    const RowDets rowA = {ws->ra, ws->rb, ws->rph, ws->rna};  // I's determinants (A = I)
-    // evaluation order of the neighbours: grouped by pair kind (doubles, singles, spin-orbit,
-    // diagonal), ascending within a kind, so that neighbouring lanes mostly run the same
-    // branch of the element code.  Values of a row are stored in this order; each pair's
-    // offset in its row run goes to prm, which is all the assembly needs.
-    {
-      const int kd = (lane < n) ? ws->pi[lane].kind : -1;
-      const int key = (kd == K_DOUBLE) ? 0 : (kd == K_SINGLE) ? 1 : (kd == K_SO) ? 2 : (kd == K_DIAG) ? 3
-                                                                                         : (kd == K_NONE) ? 4 : 5;
-      int rank = 0, base = 0;
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const unsigned m = __ballot_sync(0xffffffffu, key == k);
-        if (key == k) rank = base + __popc(m & ((1u << lane) - 1u));
-        base += __popc(m);
-      }
-      ws->perm[rank] = (int8_t)lane;
-      __syncwarp();
-    }
-    const int src = ws->perm[lane];  // the neighbour lane at evaluation slot `lane`
-    constexpr int R = DIRECT ? 1 : FAST_ROWS;
-    for (int r0 = 0; r0 < nsefI; r0 += R) {
-      const int nr = min(R, nsefI - r0);
-      // per row g of the group: marked columns of each slot, their exclusive prefix counted
-      // from the group's first element, and rs[g], the row's first element
-      int T = 0, rs[R];
-#pragma unroll
-      for (int g = 0; g < R; ++g) {
-        rs[g] = T;
-        if (g < nr) {
-          const uint64_t cr = (PH == 2) ? ((src < n) ? __ldg(P.cg + prbase + (int64_t)src * nsefI + r0 + g) : 0ull)
-                                        : __shfl_sync(0xffffffffu, (lane < n) ? C[r0 + g] : 0ull, src);
-          const uint32_t mr = (uint32_t)((cr | (cr >> 16) | (cr >> 32) | (cr >> 48)) & 0xffffull);
-          const int cm = __popc(mr);
-          int inclm = cm;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, inclm, o);
-            if (lane >= o) inclm += v;
-          }
-          ws->pre[g][lane] = (int16_t)(T + inclm - cm);
-          ws->cm[g][lane] = cr;
-          ws->keep[g][lane] = 0u;
-          T += __shfl_sync(0xffffffffu, inclm, 31);
-        }
-      }
-      if (!DIRECT && cursor + T > chunk_end) {  // room for every marked element of the group
-        const unsigned long long len = (unsigned long long)max(T, SLAB_CHUNK);
-        unsigned long long b = 0;
-        if (lane == 0) b = atomicAdd(P.slab_counter, len);
-        cursor = __shfl_sync(0xffffffffu, b, 0);
-        chunk_end = cursor + len;
-      }
-      double acc[8];
-      float accs[8], accc[8];  // DIRECT == 2: compensated FP32 sums of FP32 products
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { acc[q] = 0.0; accs[q] = 0.f; accc[q] = 0.f; }
-      const unsigned long long base = cursor;
-      // chunks beyond the slab capacity are counted but not written; the host sees the
-      // final counter, enlarges the slab and evaluates again
-      const bool fits = (int64_t)chunk_end <= P.slab_cap;
-      __syncwarp();
-      int kc = 0;
-      for (int e0 = 0; e0 < T; e0 += 32) {
-        const int e = e0 + lane;
-        bool keep = false;
-        double v = 0.0;
-        if (e < T) {
-          int g = 0;  // the row of element e: last row whose first element is <= e
-#pragma unroll
-          for (int k = 1; k < R; ++k) g += (rs[k] <= e);
-          const int r = r0 + g;
-          int o = 0;  // the slot owning element e: last slot whose prefix is <= e
-#pragma unroll
-          for (int step = 16; step > 0; step >>= 1)
-            if (ws->pre[g][o + step] <= e) o += step;
-          const uint64_t cw = ws->cm[g][o];
-          uint32_t m = (uint32_t)((cw | (cw >> 16) | (cw >> 32) | (cw >> 48)) & 0xffffull);
-          for (int q = e - ws->pre[g][o]; q > 0; --q) m &= m - 1;
-          const int t = __ffs(m) - 1;
-          const int pl = ws->perm[o];  // its neighbour lane
-          const PairInfo &pi = ws->pi[pl];
-          // reference roles: the lower half of a diagonal block, block (J, I) for J > I
-          const bool diag_blk = (pi.kind == K_DIAG);
-          const bool flip = diag_blk ? (t > r) : (pi.swap != 0);
-          const uint64_t co = cw >> t;
-          unsigned conn = (unsigned)((co & 1ull) | ((co >> 15) & 2ull) | ((co >> 30) & 4ull) | ((co >> 45) & 8ull));
-          // a diagonal block is symmetric: the transposed element swaps the determinant roles
-          if (flip) conn = (conn & 9u) | ((conn & 2u) << 1) | ((conn & 4u) >> 1);
-          // A's determinants come from shared memory when A = I (every lower pair; a pair
-          // J > I of the direct mode has A = J, read from the tables)
-          v = sef_elem<W>(P, pi, ws->K, flip ? t : r, flip ? r : t, conn, (DIRECT && pi.swap) ? nullptr : &rowA);
-          keep = (fabs(v) >= PSOCI_MIN_VALUE) || (diag_blk && t == r);
-          if (DIRECT) {
-            if (DIRECT == 2 && keep) {
-              const float vf = (float)v;
-              const float4 *xr = reinterpret_cast<const float4 *>(P.dx32 + (pi.colbase + t) * 8);
-              const float4 xa = __ldg(xr), xb = __ldg(xr + 1);
-              const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-#pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                // Kahan: the rounding error of each addition is carried in accc and fed back
-                const float yv = __fsub_rn(__fmul_rn(vf, xv[q]), accc[q]);
-                const float tt = __fadd_rn(accs[q], yv);
-                accc[q] = __fsub_rn(__fsub_rn(tt, accs[q]), yv);
-                accs[q] = tt;
-              }
-            } else if (keep) {
-              const double *xr = P.dx + (pi.colbase + t) * P.ldx;
-#pragma unroll
-              for (int q = 0; q < 8; ++q)
-                if (q < P.kvec) acc[q] = fma(v, xr[q], acc[q]);
-            }
-          } else if (keep) {
-            atomicOr(&ws->keep[g][pl], 1u << t);
-          }
-        }
-        if (!DIRECT) {
-          const unsigned kb = __ballot_sync(0xffffffffu, keep);
-          if (keep && fits) P.slab_val[(int64_t)base + kc + __popc(kb & ((1u << lane) - 1u))] = v;
-          kc += __popc(kb);
-        }
-      }
-      if (DIRECT) {  // one row per group
-        if (DIRECT == 2) {
-#pragma unroll
-          for (int q = 0; q < 8; ++q) acc[q] = (double)accs[q] - (double)accc[q];
-        }
-        const double tot = reduce_scatter8_f64(acc, lane);
-        const int q = lane >> 2;
-        if ((lane & 3) == 0 && q < P.kvec && tot != 0.0) atomicAdd(P.dy + (P.sefoff[I] + r0) * P.ldy + q, tot);
-        __syncwarp();
-        continue;
-      }
-      __syncwarp();
-      // per row of the group: its kept count, its run's place in the slab, and each pair's
-      // offset in the run (kept columns before it, in the evaluation order)
-      unsigned long long run = base;
-      for (int g = 0; g < nr; ++g) {
-        const uint32_t keepm = (lane < n) ? ws->keep[g][lane] : 0u;
-        const int cs = __popc(__shfl_sync(0xffffffffu, keepm, src));
-        int incl = cs;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += v;
-        }
-        const int kg = __shfl_sync(0xffffffffu, incl, 31);
-        ws->pre[g][src] = (int16_t)(incl - cs);  // the element loop is done with pre
-        __syncwarp();
-        if (lane == 0) P.seg_cnt[P.seg_rowoff[s] + r0 + g] = kg;
-        if (lane < n)
-          P.prm[prbase + (int64_t)lane * nsefI + r0 + g] =
-              (uint64_t)keepm | ((uint64_t)(run + (unsigned long long)ws->pre[g][lane]) << 16);
-        run += (unsigned long long)kg;
-      }
-      cursor += (unsigned long long)kc;
-      __syncwarp();
-    }
-    __syncwarp();
+    for (int w = 0; w < W; ++w) { r.e1[w] = P.e1[i * W + w]; r.e2[w] = P.e2[i * W + w]; }
+    const int js = P.jsym[i];
+    r.sef = (uint32_t)P.sefoff[i];
+    r.flags = (uint32_t)P.nopen[i] | ((uint32_t)(P.phase[P.detoff[i]] & 1) << 4) |
+              ((uint32_t)(psoci_det_class(P.nelec & 1, js, P.ksym) & 1) << 5) | ((uint32_t)(js & 1) << 6) |
+              ((uint32_t)(P.sefoff[i + 1] - P.sefoff[i]) << 16);
+    r.jsym = js;
+    r.pad = 0u;
+    out[i] = r;
   }
 }
 
-// Connectivity masks of the lower pairs for the two-launch evaluation: for every (pair, row
-// SEF r) the word C[r] of k_hbuild_fast's phase 1 (bit t + 16 (x << 1 | y): determinant x of
-// row SEF r and determinant y of column SEF t can couple), stored in P.cg at the pair's prm
-// index.  Pair kinds come from the excitation level and the symmetries alone, without the
-// integrals: a pair whose integrals vanish is marked all the same, and its elements then
-// evaluate to exactly zero and are not kept.  The work items, (neighbour, column SEF t), are
-// spread evenly over the lanes; an item tests t's one or two column determinants against all
-// row determinants at once (the bit-sliced counter of k_hbuild_fast) and ors the result into
-// the neighbour's words in shared memory.
-constexpr int MASK_WARPS = 8;
-struct MaskSmem {
-  uint64_t C[PSOCI_SEG][FAST_MAXSEF];
-  int64_t d0J[PSOCI_SEG];
-  int8_t nopJ[PSOCI_SEG], so[PSOCI_SEG];
-  int16_t ipre[PSOCI_SEG];
-};
+__device__ __forceinline__ bool is_zero(double v) { return ((uint64_t)__double_as_longlong(v) << 1) == 0ull; }
 
+// Integrals of a pair in the reference's roles, times its sign.  Singles: v0 and, for the
+// X[t] that the element kernels gather themselves, ie | je << 8 | sign bit in v1.  False when
+// they make the whole block zero (the reference's skips).
 template <int W>
-__global__ void __launch_bounds__(MASK_WARPS * 32) k_hbuild_masks(Params P) {
-  __shared__ MaskSmem smem_masks[MASK_WARPS];
-  MaskSmem &ws = smem_masks[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const bool odd = P.nelec & 1;
-  for (int64_t s = warp; s < P.nseg; s += nwarps) {
-    const int I = P.seg_cfg[s];
-    const int64_t k0 = P.seg_k0[s];
-    const int n = P.seg_n[s];
-    const int nsefI = (int)(P.sefoff[I + 1] - P.sefoff[I]);
-    const int64_t d0I = P.detoff[I];
-    const int ndI = (int)(P.detoff[I + 1] - d0I);
-    const int nopI = P.nopen[I];
-    uint64_t occI[W], dblI[W];
+__device__ __forceinline__ bool pair_values(const Params &P, const CfgRec<W> &A, const CfgRec<W> &B,
+                                            const PairShape &s, double &v0, double &v1) {
+  v0 = v1 = 0.0;
+  bool any = false;
+  if (s.kind == K_DOUBLE) {  // processDoubleExcitation (PsociHamiltonian.C:180-184)
+    v0 = g2(P, s.ex0, s.jy0, s.ex1, s.jy1);
+    v1 = g2(P, s.ex0, s.jy1, s.ex1, s.jy0);
+    any = !(is_zero(v0) && is_zero(v1));
+  } else if (s.kind == K_SO) {  // PsociHamiltonian.C:223-237: +-SO/2, sign flip if jex > iex
+    v0 = g1(P, s.ex0, s.jy0);
+    any = !is_zero(v0);
+    v0 = flip_sign(v0 * 0.5, s.jy0 > s.ex0 ? 0x80000000u : 0u);
+  } else if (s.kind == K_SINGLE) {  // PsociHamiltonian.C:239-258
+    const int ie = s.ex0, je = s.jy0;
+    double v = g1(P, ie, je) - g2(P, ie, je, ie, ie);
 #pragma unroll
-    for (int w = 0; w < W; ++w) { occI[w] = P.e1[(int64_t)I * W + w]; dblI[w] = P.e2[(int64_t)I * W + w]; }
-    // this lane's neighbour J <= I: diagonal, single (spin-orbit when the symmetries differ)
-    // or double by the excitation level I -> J
-    int nit = 0;
-    if (lane < n) {
-      const int J = P.nbr[k0 + lane];
-      int ni = 0;
-#pragma unroll
-      for (int w = 0; w < W; ++w)
-        ni += __popcll(occI[w] & ~P.e1[(int64_t)J * W + w]) + __popcll(dblI[w] & ~P.e2[(int64_t)J * W + w]);
-      const bool diag = (J == I);
-      ws.so[lane] = (int8_t)(!diag && ni == 1 && P.jsym[I] != P.jsym[J]);
-      ws.d0J[lane] = P.detoff[J];
-      ws.nopJ[lane] = (int8_t)P.nopen[J];
-      nit = (diag || ni == 1 || ni == 2) ? (int)(P.sefoff[J + 1] - P.sefoff[J]) : 0;
-    }
-    for (int q = lane; q < PSOCI_SEG * FAST_MAXSEF; q += 32) (&ws.C[0][0])[q] = 0ull;
-    int incl = nit;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    ws.ipre[lane] = (int16_t)(incl - nit);
-    const int NIT = __shfl_sync(0xffffffffu, incl, 31);
-    // I's open shells and, over the row determinants, the ballots of the counter
-    uint32_t Ap[FAST_MAXOPEN], Nk[FAST_MAXOPEN + 1];
-    int sI[FAST_MAXOPEN];
-    {
-      uint64_t SI[W];
-#pragma unroll
-      for (int w = 0; w < W; ++w) SI[w] = occI[w] & ~dblI[w];
-#pragma unroll
-      for (int p = 0; p < FAST_MAXOPEN; ++p) {
-        sI[p] = lowest_bit<W>(SI);
-        bool done = false;
-#pragma unroll
-        for (int w = 0; w < W; ++w)
-          if (!done && SI[w]) { SI[w] &= SI[w] - 1; done = true; }
-      }
-      uint32_t ma = 0u;
-      if (lane < ndI) {
-        uint64_t ra[W];
-#pragma unroll
-        for (int w = 0; w < W; ++w) ra[w] = P.alpha[(d0I + lane) * W + w];
-#pragma unroll
-        for (int p = 0; p < FAST_MAXOPEN; ++p)
-          if (p < nopI) ma |= (uint32_t)bit_w<W>(ra, sI[p]) << p;
-      }
-#pragma unroll
-      for (int p = 0; p < FAST_MAXOPEN; ++p) Ap[p] = __ballot_sync(0xffffffffu, (lane < ndI) && ((ma >> p) & 1u));
-#pragma unroll
-      for (int k = 0; k <= FAST_MAXOPEN; ++k) Nk[k] = __ballot_sync(0xffffffffu, (lane < ndI) && __popc(ma) == k);
-    }
-    const int ndblI = P.nelec - nopI;
-    const uint32_t rows_valid = (ndI >= 32) ? 0xffffffffu : ((1u << ndI) - 1u);
-    __syncwarp();
-    for (int i0 = 0; i0 < NIT; i0 += 32) {
-      const int it = i0 + lane;
-      if (it >= NIT) break;
-      int p = 0;  // the neighbour owning item it: last lane whose first item is <= it
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1)
-        if (ws.ipre[p + step] <= it) p += step;
-      const int t = it - ws.ipre[p];
-      const bool so = ws.so[p] != 0;
-      const int nopJ = ws.nopJ[p];
-      const int thr = so ? 1 : 2;
-      // column SEF t: determinant t (odd electron count), 2t and 2t + 1 (even, open shells)
-      // or the configuration's one determinant
-      const bool two = !odd && nopJ;
-      const int64_t b0 = ws.d0J[p] + (two ? 2 * t : t);
-      uint32_t okv[2] = {0u, 0u};
-#pragma unroll
-      for (int y = 0; y < 2; ++y) {
-        if (y == 1 && !two) break;
-        uint64_t ja[W], jb[W];
-#pragma unroll
-        for (int w = 0; w < W; ++w) { ja[w] = __ldg(P.alpha + (b0 + y) * W + w); jb[w] = __ldg(P.beta + (b0 + y) * W + w); }
-        int F = 0;
-#pragma unroll
-        for (int w = 0; w < W; ++w) F += __popcll(ja[w] & ~occI[w]) + __popcll(jb[w] & ~occI[w]);
-        if (F > thr) continue;
-        // saturating counter over the row dets: S0 (c'=0), S1, S2, S3 (>= 3)
-        uint32_t S0 = 0xffffffffu, S1 = 0u, S2 = 0u;
-#pragma unroll
-        for (int q = 0; q < FAST_MAXOPEN; ++q) {
-          if (q >= nopI) break;
-          const bool xa = bit_w<W>(ja, sI[q]), yb = bit_w<W>(jb, sI[q]);
-          if (xa) {  // mismatch where row det has beta on q
-            const uint32_t T = ~Ap[q];
-            S2 = (S2 & ~T) | (S1 & T);
-            S1 = (S1 & ~T) | (S0 & T);
-            S0 &= ~T;
-          }
-          if (yb) {  // mismatch where row det has alpha on q
-            const uint32_t T = Ap[q];
-            S2 = (S2 & ~T) | (S1 & T);
-            S1 = (S1 & ~T) | (S0 & T);
-            S0 &= ~T;
-          }
-        }
-        uint32_t ok = (thr - F >= 2) ? (S0 | S1 | S2) : (thr - F == 1) ? (S0 | S1) : S0;
-        ok &= rows_valid;
-        if (!so) {
-          int na = 0;
-#pragma unroll
-          for (int w = 0; w < W; ++w) na += __popcll(ja[w]);
-          const int need = na - (ndblI / 2);  // alpha open shells a row det needs for equal counts
-          uint32_t nk = 0u;
-#pragma unroll
-          for (int k = 0; k <= FAST_MAXOPEN; ++k)
-            if (k == need) nk = Nk[k];
-          ok &= (need >= 0 && need <= nopI) ? nk : 0u;
-        }
-        okv[y] = ok;
-      }
-      if (odd) {  // row SEF r = row det r, column SEF t = column det t
-        uint32_t rows = okv[0];
-        while (rows) {
-          const int r = __ffs(rows) - 1;
-          rows &= rows - 1;
-          atomicOr(reinterpret_cast<unsigned long long *>(&ws.C[p][r]), 1ull << t);
-        }
-      } else {  // row SEF r holds row dets 2r (x = 0) and 2r + 1 (x = 1)
-        uint32_t rows = (okv[0] | okv[1]);
-        rows = (rows | (rows >> 1)) & 0x55555555u;
-        while (rows) {
-          const int a = __ffs(rows) - 1;  // 2r
-          rows &= rows - 1;
-          const uint64_t wd = ((uint64_t)((okv[0] >> a) & 1u) << t) | ((uint64_t)((okv[1] >> a) & 1u) << (t + 16)) |
-                              ((uint64_t)((okv[0] >> (a + 1)) & 1u) << (t + 32)) |
-                              ((uint64_t)((okv[1] >> (a + 1)) & 1u) << (t + 48));
-          atomicOr(reinterpret_cast<unsigned long long *>(&ws.C[p][a >> 1]), (unsigned long long)wd);
-        }
+    for (int w = 0; w < W; ++w) {
+      uint64_t o = A.e1[w];
+      while (o) {
+        const int b = __ffsll((long long)o) - 1, p = 64 * w + b;
+        o &= o - 1;
+        const double buf = g2(P, ie, je, p, p);
+        v += buf;
+        const bool dA = (A.e2[w] >> b) & 1ull;
+        if (dA) v += buf;
+        if (dA && ((B.e2[w] >> b) & 1ull)) v -= g2(P, ie, p, p, je);
       }
     }
-    __syncwarp();
-    // the words at the pairs' prm positions (pair-major, then row)
-    const int64_t prbase = P.pr_off[I] + (k0 - P.nbroff[I]) * nsefI;
-    for (int q = lane; q < n * nsefI; q += 32) P.cg[prbase + q] = ws.C[q / nsefI][q % nsefI];
-    __syncwarp();
+    v0 = v;
+    any = !is_zero(v);
+    v1 = __longlong_as_double((long long)((uint32_t)ie | ((uint32_t)je << 8) | s.sign));
   }
+  v0 = flip_sign(v0, s.sign);
+  if (s.kind != K_SINGLE) v1 = flip_sign(v1, s.sign);
+  return any;
 }
 
-// Full rows from the lower pairs.  Row r of configuration I holds, in ascending column order,
-// the kept entries of its lower pairs (J <= I, evaluated above; the diagonal block in full)
-// and, for every neighbour J > I, column r of the lower block (J, I): the entries whose
-// mask bit r is set in the (J, I) pair's rows t.  mk[k] is the position of I in J's list.
-//
-// One warp per configuration: row lengths, and I's position in each upper neighbour's list.
-constexpr int NBR_SKIP = 16;  // one skip-table entry per 16 neighbour-list entries
-
-// skip[q] = nbr[16 q]: the first entry of every 64-byte block of the neighbour lists
-__global__ void k_nbr_skip(int64_t nq, const int32_t *__restrict__ nbr, int32_t *__restrict__ skip) {
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nq; q += (int64_t)gridDim.x * blockDim.x)
-    skip[q] = nbr[q * NBR_SKIP];
-}
-
-__global__ void k_mirror_count(Params P, const int32_t *__restrict__ skip, int64_t *row_nnz, int32_t *mk, int *err) {
+// Slot of every pair (ordered; one warp a configuration, lanes over its list), and with VALS
+// its integrals.  drop: pairs whose integrals make the block zero get TAB_NONE.
+template <int W, bool VALS>
+__global__ void __launch_bounds__(256) k_pair_slots(Params P, const CfgRec<W> *__restrict__ cfg,
+                                                    const int64_t *__restrict__ nbroff, const int32_t *__restrict__ nbr,
+                                                    uint64_t *keys, uint32_t mask, int *err, uint32_t *__restrict__ slot,
+                                                    double2 *__restrict__ vals) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t I = warp; I < P.nconf; I += nwarps) {
-    const int64_t b0 = P.nbroff[I], nl = P.nlow[I], nn = P.nbroff[I + 1] - b0;
-    const int nsefI = (int)(P.sefoff[I + 1] - P.sefoff[I]);
-    int64_t low = 0;
-    if (lane < nsefI)
-      for (int64_t sg = P.segoff[I]; sg < P.segoff[I + 1]; ++sg) low += P.seg_cnt[P.seg_rowoff[sg] + lane];
-    int up[FAST_MAXSEF];
+    const CfgRec<W> a = cfg[I];
+    const int64_t e = nbroff[I + 1];
+    for (int64_t q = nbroff[I] + lane; q < e; q += 32) {
+      const int J = nbr[q];
+      uint32_t sl = TAB_NONE;
+      double v0 = 0.0, v1 = 0.0;
+      if (J == (int)I) {
+        sl = TAB_DIAG;
+      } else {
+        const CfgRec<W> b = cfg[J];
+        const bool up = J > (int)I;  // block (J, I): A = J, rows are B's SEFs
+        CfgRec<W> A, B;
 #pragma unroll
-    for (int r = 0; r < FAST_MAXSEF; ++r) up[r] = 0;
-    for (int64_t k = nl + lane; k < nn; k += 32) {
-      const int J = P.nbr[b0 + k];
-      const int64_t jb = P.nbroff[J], je = jb + P.nlow[J];
-      // I in J's lower list [jb, je) (ascending): the last 16-entry block starting inside
-      // the list whose first entry is <= I, by binary search over the skip table (small
-      // enough to stay in L2), then a scan of that block (64 bytes)
-      int64_t qa = jb / NBR_SKIP, qb = (je - 1) / NBR_SKIP;  // blocks qa + 1 .. qb start inside
-      while (qa < qb) {
-        const int64_t mid = (qa + qb + 1) >> 1;
-        if (__ldg(skip + mid) <= (int32_t)I) qa = mid; else qb = mid - 1;
-      }
-      int64_t lo = -1;
-      const int64_t b16 = qa * NBR_SKIP;
-      if (b16 + NBR_SKIP <= P.nbr_len) {  // the block as four 16-byte loads, compared in registers
-        const int4 *blk = reinterpret_cast<const int4 *>(P.nbr + b16);
-        int4 v[NBR_SKIP / 4];
-#pragma unroll
-        for (int u = 0; u < NBR_SKIP / 4; ++u) v[u] = __ldg(blk + u);
-#pragma unroll
-        for (int u = 0; u < NBR_SKIP / 4; ++u) {
-          const int64_t p = b16 + 4 * u;
-          if (v[u].x == (int32_t)I && p >= jb && p < je) lo = p;
-          if (v[u].y == (int32_t)I && p + 1 >= jb && p + 1 < je) lo = p + 1;
-          if (v[u].z == (int32_t)I && p + 2 >= jb && p + 2 < je) lo = p + 2;
-          if (v[u].w == (int32_t)I && p + 3 >= jb && p + 3 < je) lo = p + 3;
+        for (int w = 0; w < W; ++w) {
+          A.e1[w] = up ? b.e1[w] : a.e1[w]; A.e2[w] = up ? b.e2[w] : a.e2[w];
+          B.e1[w] = up ? a.e1[w] : b.e1[w]; B.e2[w] = up ? a.e2[w] : b.e2[w];
         }
-      } else {  // the last, partial block of the lists
-        for (int64_t p = max(jb, b16); p < je && p < b16 + NBR_SKIP; ++p)
-          if (P.nbr[p] == (int32_t)I) lo = p;
+        A.flags = up ? b.flags : a.flags; A.jsym = up ? b.jsym : a.jsym;
+        B.flags = up ? a.flags : b.flags; B.jsym = up ? a.jsym : b.jsym;
+        const PairShape s = pair_shape<W>(A, B);
+        bool any = s.kind != K_NONE;
+        if (VALS && any) any = pair_values<W>(P, A, B, s, v0, v1);
+        if (any) {
+          sl = tab_insert(keys, mask, pair_key<W>(A, B, s.kind, up), err);
+          if (sl != TAB_NONE) sl |= s.sign;
+        }
       }
-      if (lo < 0) {
-        atomicExch(err, 1);
-        mk[b0 + k] = -1;
-        continue;
-      }
-      mk[b0 + k] = (int32_t)(lo - jb);
-      const int nsefJ = (int)(P.sefoff[J + 1] - P.sefoff[J]);
-      const uint64_t *pm = P.prm + P.pr_off[J] + (lo - jb) * nsefJ;
-      for (int t = 0; t < nsefJ; ++t) {
-        const uint32_t m = (uint32_t)pm[t];
-#pragma unroll
-        for (int r = 0; r < FAST_MAXSEF; ++r) up[r] += (int)((m >> r) & 1u);
-      }
+      slot[q] = sl;
+      if (VALS) vals[q] = make_double2(v0, v1);
     }
-    int mine = 0;
-#pragma unroll
-    for (int r = 0; r < FAST_MAXSEF; ++r) {
-      int v = up[r];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == r) mine = v;
-    }
-    if (lane < nsefI) row_nnz[P.sefoff[I] + lane] = low + mine;
   }
 }
 
-// One warp per configuration: columns, values (and the FP32 copy and the diagonal) of its
-// rows; lane r carries the write position of row r.  Entries are spread over the lanes one
-// per lane (e = lane, lane + 32, ...), so consecutive lanes write consecutive positions:
-// the lane that owns entry e is found by binary search over the per-pair offsets.
-constexpr int ASM_THREADS = 256;
-__global__ void __launch_bounds__(ASM_THREADS) k_assemble(Params P, const int32_t *mk) {
-  __shared__ int s_off[ASM_THREADS / 32][33];     // per lane: first entry of the lane in the row
-  __shared__ int s_soff[ASM_THREADS / 32][32];    // lower part: per row, its first entry in the segment
-  __shared__ uint32_t s_msk[ASM_THREADS / 32][32];  // per lane: columns t of the run, as bits
-  __shared__ int32_t s_J[ASM_THREADS / 32][32];
-  __shared__ int64_t s_col[ASM_THREADS / 32][32];
-  __shared__ uint64_t s_mm[ASM_THREADS / 32][32][FAST_MAXSEF];  // mask words (prm)
-  __shared__ int16_t s_ro[ASM_THREADS / 32][FAST_MAXSEF][32];  // lower part: per row, first entry of each slot
-  __shared__ int64_t s_dst[ASM_THREADS / 32][FAST_MAXSEF];      // lower part: per row, its write position
+// Diagonal blocks: D[(sef r) * ldd + t], the lower half as the reference computes it and its
+// mirror image, and the diagonal.  One warp a configuration: the diagonal's integral sums with
+// their loads spread over the lanes and added in the reference's order, then lanes over the
+// elements.
+constexpr int DG_WARPS = 4;
+template <int W>
+__global__ void __launch_bounds__(DG_WARPS * 32) k_diag_blocks(Params P, int ldd, double *__restrict__ D,
+                                                               double *__restrict__ diag) {
+  __shared__ PairInfo spi[DG_WARPS];
+  __shared__ double sK[DG_WARPS][MAXK];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  PairInfo &pi = spi[wib];
+  double *Kd = sK[wib];
   for (int64_t I = warp; I < P.nconf; I += nwarps) {
+    uint64_t o1[W], o2[W], so[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      o1[w] = P.e1[I * W + w];
+      o2[w] = P.e2[I * W + w];
+      so[w] = o1[w] & ~o2[w];
+    }
+    // the p-th lowest set bit of x, or -1
+    auto nth = [](const uint64_t(&x)[W], int p) {
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        uint64_t u = x[w];
+        const int c = __popcll(u);
+        if (p < c) {
+          for (; p > 0; --p) u &= u - 1;
+          return 64 * w + __ffsll((long long)u) - 1;
+        }
+        p -= c;
+      }
+      return -1;
+    };
+    const int nop = popc_w<W>(so), nocc = popc_w<W>(o1);
+    // exchange of the open-shell pairs (a > b), in diag_det_elem's order
+    for (int mm = lane; mm < nop * (nop - 1) / 2; mm += 32) {
+      int a = 1, q = mm;
+      while (q >= a) { q -= a; ++a; }
+      const int oa = nth(so, a), ob = nth(so, q);
+      Kd[1 + mm] = g2(P, oa, ob, ob, oa);
+    }
+    // processDiagExcitation (PsociHamiltonian.C:306-388): per occupied ib its own term, then
+    // its pairs jb < ib ascending
+    double v = 0.0;
+    for (int i = 0; i < nocc; ++i) {
+      const int ib = nth(o1, i), occi = 1 + (int)bit_w<W>(o2, ib);
+      for (int j0 = -1; j0 < i; j0 += 32) {
+        const int j = j0 + lane;
+        double x = 0.0;
+        if (j < 0) {
+          x = occi == 1 ? g1(P, ib, ib) : 2.0 * g1(P, ib, ib) + g2(P, ib, ib, ib, ib);
+        } else if (j < i) {
+          const int jb = nth(o1, j), ninj = occi * (1 + (int)bit_w<W>(o2, jb));
+          if (ninj == 1) x = g2(P, ib, ib, jb, jb);
+          else {
+            double buf = 2.0 * g2(P, ib, ib, jb, jb);
+            buf -= g2(P, ib, jb, ib, jb);
+            x = ninj == 2 ? buf : 2.0 * buf;
+          }
+        }
+        const int m = min(32, i - j0);
+        for (int l = 0; l < m; ++l) v += __shfl_sync(0xffffffffu, x, l);
+      }
+    }
     const int64_t row0 = P.sefoff[I];
-    const int nsefI = (int)(P.sefoff[I + 1] - row0);
-    const int64_t b0 = P.nbroff[I], nl = P.nlow[I], nn = P.nbroff[I + 1] - b0;
-    int64_t mypos = (lane < nsefI) ? P.rowptr[row0 + lane] : 0;
-    // lower pairs, segment by segment: the run of (segment, row r) is contiguous in the slab
-    // and in row r, in the same order.  The segment's runs and mask words are loaded first;
-    // then its entries, all rows together, are numbered in (row, neighbour, column) order
-    // and spread evenly over the lanes.
-    for (int64_t sg = P.segoff[I]; sg < P.segoff[I + 1]; ++sg) {
-      const int64_t k0 = P.seg_k0[sg];
-      const int ns = P.seg_n[sg];
-      if (lane < ns) {
-        const int J = P.nbr[k0 + lane];
-        s_J[wib][lane] = J;
-        s_col[wib][lane] = P.sefoff[J];
+    const int nsef = (int)(P.sefoff[I + 1] - row0);
+    if (lane == 0) {
+      Kd[0] = v;
+      pi.kind = K_DIAG;
+      pi.swap = 0;
+      pi.detA = pi.detB = P.detoff[I];
+      pi.colbase = row0;
+      pi.nsefJ = nsef;
+      pi.iex0 = pi.jex0 = -1;
+      pi.nopenA = pi.nopenB = nop;
+      pi.jsA = pi.jsB = P.jsym[I];
+      pi.v0 = v;
+      pi.v1 = 0.0;
+#pragma unroll
+      for (int w = 0; w < W; ++w) pi.SA[w] = so[w];
+    }
+    __syncwarp();
+    for (int e = lane; e < nsef * nsef; e += 32) {
+      const int r = e / nsef, t = e - r * nsef;
+      if (t > r) continue;
+      const double x = sef_elem<W>(P, pi, Kd, r, t);
+      D[(row0 + r) * ldd + t] = x;
+      if (t != r) D[(row0 + t) * ldd + r] = x;
+      else diag[row0 + r] = x;
+    }
+    __syncwarp();
+  }
+}
+
+// Rounding to FP32 on the integer pipe (round to nearest even; values outside FP32's normal
+// range by the conversion instruction, which shares the narrow FP64 pipe).
+__device__ __forceinline__ float f32_of(double v) {
+  const uint32_t hi = (uint32_t)__double2hiint(v);
+  const uint64_t a = ((uint64_t)(hi & 0x7fffffffu) << 32) | (uint32_t)__double2loint(v);
+  const uint64_t r = (a + 0x0fffffffull + ((a >> 29) & 1ull)) >> 29;  // 11 exponent bits, 23 mantissa bits
+  const uint64_t f = r - (896ull << 23);
+  if (f - 0x00800000ull >= 0x7f000000ull) return (float)v;
+  return __uint_as_float((uint32_t)f | (hi & 0x80000000u));
+}
+// |v| >= PSOCI_MIN_VALUE (not NaN) by its bits, word by word: masking the sign of the 64-bit
+// pattern compiles to an FP64 absolute value
+__device__ __forceinline__ bool kept_value(double v) {
+  const uint64_t a = ((uint64_t)((uint32_t)__double2hiint(v) & 0x7fffffffu) << 32) | (uint32_t)__double2loint(v);
+  constexpr uint64_t lo = 0x3e45798ee2308c3aull, inf = 0x7ff0000000000000ull;  // the bits of 1e-8
+  return a - lo <= inf - lo;
+}
+
+// Per warp, followed by X (ms doubles a pair) and, MODE 0 and 1, an int32 a row (count, write
+// position from the configuration's first), MODE 2 and 3 four times eight doubles a row (its
+// products).  The pairs that have elements, in order.
+struct ElemWarp {
+  uint2 run[PSOCI_SEG];        // runs of elements: first entry less first element, pair
+  uint4 pair[PSOCI_SEG];       // info, first column, offset of the row indices from the entries
+  double F[PSOCI_SEG][4];      // the pair's scaled integrals v0, v1, v0 - v1 (singles: v0, its orbitals)
+  float F32[PSOCI_SEG][4];     // and in FP32
+};
+// in the info of ElemWarp::pair, in place of the number of entries: diagonal block, elements that are sums
+// (tab_sum_value), forms above the threshold
+constexpr uint32_t EL_DIAG = 1u, EL_SUMS = 2u;
+constexpr int EL_KEPT = 4;
+
+// Warps a block: their configurations differ in size by up to 256 times, and a block holds its
+// shared memory and registers until its last warp ends (8 warps: 31% of the SM's warps active)
+constexpr int EL_WARPS = 2;
+
+template <int W>
+struct ElemArgs {
+  const CfgRec<W> *cfg;
+  const uint32_t *slot;
+  const double2 *vals;       // VALS: the pairs' integrals
+  const uint4 *hdr;
+  const uint32_t *pool;
+  const double *D;           // diagonal blocks
+  int ldd, ms;               // SEFs / open shells of the largest configuration
+  int64_t *row_nnz;          // MODE 0
+  unsigned long long *segments;
+  int warp_bytes;
+};
+
+// One warp per configuration.  Per chunk of 32 pairs the lanes load a pair each (table header,
+// integrals; the singles' exchange integrals spread over all lanes), then the pairs' entries are
+// laid end to end and lane e % 32 takes element e.  A table lists a row's columns ascending, so
+// the elements of one row come in the order in which the matrix holds them: an element's place
+// is its row's write position plus the elements of that row on lower lanes.
+//   Pair by pair the entries are read coalesced and a pair's kind is uniform over most warps;
+// laid out row by row instead (so that the stores coalesce) the bookkeeping of the (row, pair)
+// runs took 3,500 instructions a chunk and the kernel 30.5 ms at mrcisd_6e8o_v48 (MODE 1).
+// MODE 1 takes four rows of all 32 pairs at a time, so that a warp's elements still fall into few
+// runs of the matrix.
+// GB300's FP64 pipe takes a warp instruction every 16 clocks an SM, so a double's or spin-orbit
+// pair's three values, and their FP32 copies, are formed once a pair, and an element takes one
+// with its sign; signs and the threshold are integer operations.
+//   MODE 0 reads elements only of singles and two-term forms; a double or spin-orbit pair adds
+// the row counts of the forms that pass the threshold.  VALS: integrals read from the pair list
+// instead of evaluated here (the list takes 16 bytes a pair; without room for it the kernel
+// gathers them itself, to the same values).  SMALL: no configuration of more than 16 SEFs.
+template <int W, int MODE, bool VALS, bool SMALL>
+__global__ void __launch_bounds__(EL_WARPS * 32) k_elems(Params P, ElemArgs<W> E) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ElemWarp &ws = *reinterpret_cast<ElemWarp *>(smem_raw + (size_t)(threadIdx.x >> 5) * E.warp_bytes);
+  double *X = reinterpret_cast<double *>(&ws + 1);
+  int *pos = reinterpret_cast<int *>(X + E.ms * PSOCI_SEG);
+  double *yacc = reinterpret_cast<double *>(pos);
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u, le = lt | (1u << lane);
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t I = warp; I < P.nconf; I += nwarps) {
+    const CfgRec<W> a = E.cfg[I];
+    const int nsefI = (int)(a.flags >> 16) & 0x1ff, lgI = __ffs(nsefI) - 1;  // a power of two
+    const int64_t row0 = a.sef, b0 = P.nbroff[I], b1 = P.nbroff[I + 1];
+    const int64_t first = MODE == 1 ? P.rowptr[row0] : 0;
+    if (MODE < 2)
+      for (int r = lane; r < nsefI; r += 32) pos[r] = MODE == 0 ? 0 : (int)(P.rowptr[row0 + r] - first);
+    else
+      for (int r = lane; r < nsefI * 32; r += 32) yacc[r] = 0.0;
+    int32_t *col0 = MODE == 1 ? P.col + first : nullptr;
+    double *val0 = MODE == 1 ? P.val + first : nullptr;
+    float *val320 = (MODE == 1 && P.val32) ? P.val32 + first : nullptr;
+    // MODE 0: this lane's row counts, 16 bits a row (cnt[q]: rows q, q + 4, q + 8, q + 12), added to
+    // pos before they can carry
+    uint64_t cnt[4] = {0ull, 0ull, 0ull, 0ull};
+    auto add_counts = [&]() {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint64_t lo = cnt[q] & 0x0000ffff0000ffffull, hi = (cnt[q] >> 16) & 0x0000ffff0000ffffull;
+        cnt[q] = 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          lo += __shfl_xor_sync(FULL, lo, o);
+          hi += __shfl_xor_sync(FULL, hi, o);
+        }
+        if (lane == 0) {
+          if (q < nsefI) pos[q] += (int)(uint32_t)lo;
+          if (q + 8 < nsefI) pos[q + 8] += (int)(lo >> 32);
+          if (q + 4 < nsefI) pos[q + 4] += (int)(uint32_t)hi;
+          if (q + 12 < nsefI) pos[q + 12] += (int)(hi >> 32);
+        }
       }
-      // mask words of (neighbour o, row r): contiguous in prm, pair-major
-      const uint64_t *pm = P.prm + P.pr_off[I] + (k0 - b0) * nsefI;
-      for (int q = lane; q < ns * nsefI; q += 32) s_mm[wib][q / nsefI][q % nsefI] = pm[q];
-      // row r (lane r): its entry count and its first entry in the segment
-      int cnt = 0;
-      if (lane < nsefI) {
-        cnt = (int)P.seg_cnt[P.seg_rowoff[sg] + lane];
-        s_dst[wib][lane] = mypos;
+      __syncwarp();
+    };
+    for (int64_t k0 = b0; k0 < b1; k0 += 32) {
+      const int n = (int)min((int64_t)32, b1 - k0);
+      __syncwarp();
+      if (MODE == 0 && ((k0 - b0) & (4096 * 32 - 1)) == 4095 * 32) add_counts();
+      // this lane's pair
+      uint32_t sl = TAB_NONE;
+      int J = 0;
+      if (lane < n) {
+        J = P.nbr[k0 + lane];
+        sl = E.slot[k0 + lane];
       }
-      int rincl = cnt;
+      bool single = false, two = false;
+      int c = 0;           // its elements
+      uint4 pr = make_uint4(0u, 0u, 0u, 0u);
+      double v0 = 0.0, v1 = 0.0, f0 = 0.0, f1 = 0.0, f2 = 0.0;
+      uint64_t sa[W], rows = 0ull;  // open shells of A; entries of each row, 4 bits a row
+      uint32_t ent0 = 0u;           // first entry
+      if (sl == TAB_DIAG) {
+        c = nsefI * nsefI;
+        pr.x = EL_DIAG;
+        pr.y = (uint32_t)row0;
+      } else if (sl != TAB_NONE) {
+        const uint4 h = __ldg(E.hdr + 2 * (size_t)(sl & ~TAB_SIGN));
+        single = ((h.y >> TAB_KIND) & 7u) == K_SINGLE;
+#pragma unroll
+        for (int w = 0; w < W; ++w) sa[w] = a.e1[w] & ~a.e2[w];
+        if (VALS) {
+          const double2 v = __ldg(E.vals + k0 + lane);
+          v0 = v.x;
+          v1 = v.y;
+          if (MODE != 0) pr.y = __ldg(&E.cfg[J].sef);
+          if (single && J > (int)I) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) sa[w] = __ldg(&E.cfg[J].e1[w]) & ~__ldg(&E.cfg[J].e2[w]);
+          }
+        } else {
+          const CfgRec<W> b = E.cfg[J];
+          const bool up = J > (int)I;
+          CfgRec<W> A, B;
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            A.e1[w] = up ? b.e1[w] : a.e1[w]; A.e2[w] = up ? b.e2[w] : a.e2[w];
+            B.e1[w] = up ? a.e1[w] : b.e1[w]; B.e2[w] = up ? a.e2[w] : b.e2[w];
+            sa[w] = A.e1[w] & ~A.e2[w];
+          }
+          A.flags = up ? b.flags : a.flags; A.jsym = up ? b.jsym : a.jsym;
+          B.flags = up ? a.flags : b.flags; B.jsym = up ? a.jsym : b.jsym;
+          const PairShape s = pair_shape<W>(A, B);
+          pair_values<W>(P, A, B, s, v0, v1);
+          pr.y = b.sef;
+        }
+        c = (int)(h.y & TAB_ENTRIES);
+        ent0 = h.x;
+        rows = (uint64_t)h.z | ((uint64_t)h.w << 32);
+        pr.z = 3u * h.x + 4u * (uint32_t)c;  // row indices: a byte each, after the entries
+        pr.x = h.y & ((3u << TAB_FACTORS) | (7u << TAB_KIND));
+        if (single) {
+          pr.x |= EL_SUMS;
+        } else {
+          const uint32_t forms = (h.y >> TAB_FORMS) & 0xfffu;
+          f0 = tab_scale(v0, h.y);
+          if (forms & ~1u) {  // more than v0 in use
+            f1 = tab_scale(v1, h.y);
+            f2 = tab_scale(v0 - v1, h.y);
+          }
+          const uint32_t keep = (kept_value(f0) ? 1u : 0u) | (kept_value(f1) ? 2u : 0u) | (kept_value(f2) ? 4u : 0u);
+          pr.x |= keep << EL_KEPT;
+          two = (forms >> 3) != 0u;
+          if (two) pr.x |= EL_SUMS;
+          if (MODE == 0 && !two && !(h.y & TAB_NOCOUNTS)) {
+            c = 0;
+            const uint4 h2 = __ldg(E.hdr + 2 * (size_t)(sl & ~TAB_SIGN) + 1);
+            const uint64_t m = 0x000f000f000f000full;
+            const uint64_t n1 = (uint64_t)h2.x | ((uint64_t)h2.y << 32), n2 = (uint64_t)h2.z | ((uint64_t)h2.w << 32);
+            const uint64_t nib = ((keep & 1u) ? rows - n1 - n2 : 0ull) + ((keep & 2u) ? n1 : 0ull) + ((keep & 4u) ? n2 : 0ull);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) cnt[q] += (nib >> (4 * q)) & m;
+          }
+        }
+      }
+      const unsigned nz = __ballot_sync(FULL, c > 0);
+      const int me = __popc(nz & lt);  // this pair among those with elements
+      if (c > 0) {
+        ws.pair[me] = pr;
+        ws.F[me][0] = single ? v0 : f0;
+        ws.F[me][1] = single ? v1 : f1;
+        ws.F[me][2] = f2;
+        if (MODE == 1) *reinterpret_cast<float4 *>(ws.F32[me]) = make_float4((float)f0, (float)f1, (float)f2, 0.f);
+        if (single) {
+#pragma unroll
+          for (int w = 0; w < W; ++w) X[me * E.ms + w] = __longlong_as_double((long long)sa[w]);
+        } else if (two) {
+          X[me * E.ms] = v0;
+          X[me * E.ms + 1] = v1;
+        }
+      }
+      // exchange integrals of the singles: lane = (single, open shell)
+      unsigned sm = __ballot_sync(FULL, single && c > 0);
+      __syncwarp();
+      while (sm) {
+        const int per = 32 / E.ms, g = lane / E.ms, t = lane - g * E.ms;
+        unsigned m = sm;
+        for (int q = 0; q < g && m; ++q) m &= m - 1;
+        const int p = m ? __popc(nz & ((m & (~m + 1u)) - 1u)) : 0;
+        double x = 0.0;
+        bool have = false;
+        if (g < per && m) {
+          const uint64_t meta = (uint64_t)__double_as_longlong(ws.F[p][1]);
+          const int ie = (int)(meta & 0xffu), je = (int)((meta >> 8) & 0xffu);
+          int tt = t, o = -1;
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            uint64_t u = (uint64_t)__double_as_longlong(X[p * E.ms + w]);
+            const int cc = __popcll(u);
+            if (o < 0) {
+              if (tt < cc) {
+                for (; tt > 0; --tt) u &= u - 1;
+                o = 64 * w + __ffsll((long long)u) - 1;
+              } else {
+                tt -= cc;
+              }
+            }
+          }
+          if (o >= 0) {
+            have = true;
+            x = g2(P, ie, o, o, je);
+            x = flip_sign(x, (uint32_t)meta & TAB_SIGN);
+          }
+        }
+        __syncwarp();
+        if (have) X[p * E.ms + t] = x;
+        for (int q = 0; q < per && sm; ++q) sm &= sm - 1;
+        __syncwarp();
+      }
+      const int ng = (MODE == 1 && SMALL && nsefI > 4) ? nsefI >> 2 : 1;
+      for (int g = 0; g < ng; ++g) {
+      int cg = c;  // this lane's elements in the rows of the group
+      if (ng > 1) {
+        const uint32_t x = (uint32_t)(rows >> (16 * g)) & 0xffffu, y = (x & 0x0f0fu) + ((x >> 4) & 0x0f0fu);
+        cg = (pr.x & EL_DIAG) ? 4 * nsefI : (int)((y + (y >> 8)) & 0xffu);
+      }
+      int T = cg;  // elements up to and with this pair's
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, rincl, o);
-        if (lane >= o) rincl += v;
+        const int u = __shfl_up_sync(FULL, T, o);
+        if (lane >= o) T += u;
       }
-      const int T = __shfl_sync(0xffffffffu, rincl, 31);
-      s_soff[wib][lane] = rincl - cnt;
+      const int st = T - cg;
+      T = __shfl_sync(FULL, T, 31);
+      const unsigned nzg = __ballot_sync(FULL, cg > 0);
+      if (cg > 0) ws.run[__popc(nzg & lt)] = make_uint2(ent0 - (uint32_t)st, (uint32_t)me);
+      ent0 += (uint32_t)cg;
       __syncwarp();
-      // per row, the first entry of each neighbour: the row takes the pairs in neighbour
-      // order; the slab run holds them in the evaluation order, each where its prm word says
-      for (int r = 0; r < nsefI; ++r) {
-        const int cl = (lane < ns) ? __popc(s_mm[wib][lane][r] & 0xffffu) : 0;
-        int incl = cl;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += v;
-        }
-        s_ro[wib][r][lane] = (int16_t)(incl - cl);
-      }
-      __syncwarp();
-      for (int e = lane; e < T; e += 32) {
-        int r = 0;  // the row of entry e: last row whose first entry is <= e
-#pragma unroll
-        for (int st = 8; st > 0; st >>= 1)
-          if (r + st < nsefI && s_soff[wib][r + st] <= e) r += st;
-        const int el = e - s_soff[wib][r];
-        int o = 0;  // its neighbour: last slot whose first entry in the row is <= el
-#pragma unroll
-        for (int st = 16; st > 0; st >>= 1)
-          if (o + st < 32 && s_ro[wib][r][o + st] <= el) o += st;
-        const uint64_t w = s_mm[wib][o][r];
-        const int k = el - s_ro[wib][r][o];
-        uint32_t m = (uint32_t)w & 0xffffu;
-        for (int q = k; q > 0; --q) m &= m - 1;
-        const int t = __ffs(m) - 1;
-        const double v = P.slab_val[(int64_t)(w >> 16) + k];
-        const int64_t dst = s_dst[wib][r] + el;
-        P.col[dst] = (int32_t)(s_col[wib][o] + t);
-        P.val[dst] = v;
-        if (P.val32) P.val32[dst] = (float)v;
-        if (s_J[wib][o] == (int)I && t == r) P.diag[row0 + r] = v;
-      }
-      __syncwarp();
-      mypos += cnt;
-    }
-    // upper neighbours, 32 at a time: column r of their lower block (J, I)
-    for (int64_t kc = nl; kc < nn; kc += 32) {
-      const int64_t k = kc + lane;
-      uint32_t mm[FAST_MAXSEF];  // kept-column masks of the block's rows t
-#pragma unroll
-      for (int t = 0; t < FAST_MAXSEF; ++t) mm[t] = 0u;
-      int64_t colJ = 0;
-      if (k < nn) {
-        const int J = P.nbr[b0 + k];
-        const int kk = mk[b0 + k];
-        if (kk >= 0) {
-          const int nsefJ = (int)(P.sefoff[J + 1] - P.sefoff[J]);
-          colJ = P.sefoff[J];
-          const uint64_t *pm = P.prm + P.pr_off[J] + (int64_t)kk * nsefJ;
-#pragma unroll
-          for (int t = 0; t < FAST_MAXSEF; ++t)
-            if (t < nsefJ) {
-              const uint64_t w = pm[t];
-              s_mm[wib][lane][t] = w;
-              mm[t] = (uint32_t)w & 0xffffu;
+      int started = 0;
+      for (int e0 = 0; e0 < T; e0 += 32) {
+        const int e = e0 + lane;
+        // runs starting in this pass, and with them this element's run
+        const unsigned bw = __reduce_or_sync(FULL, (cg > 0 && (unsigned)(st - e0) < 32u) ? 1u << ((st - e0) & 31) : 0u);
+        bool keep = false;
+        double v = 0.0;
+        float v32 = 0.f;
+        int r = 0;
+        uint32_t col = 0u;
+        if (e < T) {
+          const uint2 run = ws.run[started + __popc(bw & le) - 1];
+          const int p = (int)run.y;
+          const uint4 q = ws.pair[p];
+          const uint32_t at = run.x + (uint32_t)e;
+          if (q.x & EL_DIAG) {
+            const int b = (int)at, t = b & (nsefI - 1);
+            r = b >> lgI;
+            v = __ldg(E.D + (row0 + r) * E.ldd + t);
+            v32 = f32_of(v);
+            keep = t == r || kept_value(v);
+            col = q.y + (uint32_t)t;
+          } else {
+            const uint32_t ent = __ldg(E.pool + at);
+            const int f = (int)(ent >> 8) & 15;
+            col = q.y + (ent & 0xffu);
+            r = (int)(ent >> 12) & 0xff;
+            if ((q.x & EL_SUMS) && (f > 2 || ((q.x >> TAB_KIND) & 7u) == K_SINGLE)) {
+              v = tab_sum_value(ent, q.x, ws.F[p][0], X + p * E.ms);
+              v32 = f32_of(v);
+              keep = kept_value(v);
+              if (((q.x >> TAB_KIND) & 7u) == K_SINGLE)
+                r = __ldg(reinterpret_cast<const uint8_t *>(E.pool) + (size_t)(q.z + at));
+            } else {
+              v = flip_sign(ws.F[p][f], ent & 0x80000000u);
+              if (MODE == 1) v32 = __int_as_float(__float_as_int(ws.F32[p][f]) ^ (int)(ent & 0x80000000u));
+              keep = (q.x >> (EL_KEPT + f)) & 1u;
             }
+          }
         }
-      }
-      s_col[wib][lane] = colJ;
-      for (int r = 0; r < nsefI; ++r) {
-        uint32_t cm = 0u;  // columns t of this lane's block whose row t keeps column r
+        started += __popc(bw);
+        if (MODE < 2) {
+          unsigned same = __ballot_sync(FULL, keep);  // the kept elements of this one's row
 #pragma unroll
-        for (int t = 0; t < FAST_MAXSEF; ++t) cm |= ((mm[t] >> r) & 1u) << t;
-        const int cnt = __popc(cm);
-        int incl = cnt;
+          for (int b = 0; b < (SMALL ? (MODE == 1 ? 2 : 4) : 8); ++b) {
+            const unsigned B = __ballot_sync(FULL, (r >> b) & 1);
+            same &= ((r >> b) & 1) ? B : ~B;
+          }
+          int at = 0;
+          if (keep) at = pos[r] + __popc(same & lt);
+          if (MODE == 1 && keep) {
+            col0[(uint32_t)at] = (int32_t)col;
+            val0[(uint32_t)at] = v;
+            if (val320) val320[(uint32_t)at] = v32;
+          }
+          __syncwarp();
+          if (keep && (same & ~le) == 0u) pos[r] = at + 1;
+          __syncwarp();
+        } else {
+          // lanes = (element slot, vector); a slot has its own sums of each row
+          const int s4 = lane >> 3, q = lane & 7;
+          if (!keep) col = 0xffffffffu;
+          const int m = min(32, T - e0);
+          double *ya = yacc + (s4 * nsefI) * 8 + q;
+          for (int x0 = 0; x0 < m; x0 += 16) {
+            double vv[4], xx[4];
+            int rr[4];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += v;
+            for (int u = 0; u < 4; ++u) {
+              const int l = x0 + 4 * u + s4;
+              vv[u] = __shfl_sync(FULL, v, l);
+              rr[u] = __shfl_sync(FULL, r, l);
+              const uint32_t cc = __shfl_sync(FULL, col, l);
+              const bool ok = cc != 0xffffffffu && q < P.kvec;
+              if (!ok) vv[u] = 0.0;
+              if (MODE == 2) xx[u] = ok ? __ldg(P.dx + (int64_t)cc * P.ldx + q) : 0.0;
+              else xx[u] = __hiloint2double(0, __float_as_int(ok ? __ldg(P.dx32 + (int64_t)cc * 8 + q) : 0.f));
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              if (MODE == 2) {
+                double *y = ya + rr[u] * 8;
+                *y = fma(vv[u], xx[u], *y);
+              } else {
+                // FP32 product, Kahan sum: the rounding error of each addition is carried in .y
+                float2 *y = reinterpret_cast<float2 *>(ya + rr[u] * 8);
+                const float2 sc = *y;
+                const float pr32 = __fmul_rn(f32_of(vv[u]), __int_as_float(__double2loint(xx[u])));
+                const float yv = __fsub_rn(pr32, sc.y), tt = __fadd_rn(sc.x, yv);
+                *y = make_float2(tt, __fsub_rn(__fsub_rn(tt, sc.x), yv));
+              }
+            }
+          }
         }
-        const int tot = __shfl_sync(0xffffffffu, incl, 31);
-        const int64_t dst = __shfl_sync(0xffffffffu, mypos, r);
-        s_off[wib][lane] = incl - cnt;
-        s_msk[wib][lane] = cm;
-        __syncwarp();
-        const uint32_t below = (1u << r) - 1u;
-        for (int e = lane; e < tot; e += 32) {
-          int o = 0;
-#pragma unroll
-          for (int st = 16; st > 0; st >>= 1)
-            if (o + st < 32 && s_off[wib][o + st] <= e) o += st;
-          uint32_t m = s_msk[wib][o];
-          for (int q = e - s_off[wib][o]; q > 0; --q) m &= m - 1;
-          const int t = __ffs(m) - 1;
-          const uint64_t wt = s_mm[wib][o][t];
-          const double v = P.slab_val[(int64_t)(wt >> 16) + __popc((uint32_t)wt & below)];
-          P.col[dst + e] = (int32_t)(s_col[wib][o] + t);
-          P.val[dst + e] = v;
-          if (P.val32) P.val32[dst + e] = (float)v;
-        }
-        __syncwarp();
-        if (lane == r) mypos += tot;
       }
       __syncwarp();
+      }
     }
+    __syncwarp();
+    if (MODE == 0) {
+      add_counts();
+      for (int r = lane; r < nsefI; r += 32) E.row_nnz[row0 + r] = pos[r];
+      if (lane == 0) atomicAdd(E.segments, (unsigned long long)((b1 - b0 + 31) / 32));
+    }
+    if (MODE >= 2)
+      for (int r = lane; r < nsefI * 8; r += 32) {
+        double y[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          y[u] = yacc[u * nsefI * 8 + r];
+          if (MODE == 3) y[u] = (double)__int_as_float(__double2loint(y[u])) - (double)__int_as_float(__double2hiint(y[u]));
+        }
+        if ((r & 7) < P.kvec) P.dy[(row0 + (r >> 3)) * P.ldy + (r & 7)] = (y[0] + y[1]) + (y[2] + y[3]);
+      }
+    __syncwarp();
   }
 }
 
@@ -2257,6 +2052,159 @@ psoci_status screen_pairs(psoci_ctx *c, const Params &P0, const double *prune_on
 #undef TRYC
 }
 
+// A coupling table set and what its kernels read beside it (freed by free()).
+template <int W>
+struct TabSet {
+  BlockTab t;
+  CfgRec<W> *cfg = nullptr;
+  uint32_t *slot = nullptr;   // [npairs]
+  double2 *vals = nullptr;    // [npairs] or null
+  double *D = nullptr;        // diagonal blocks, ldd columns
+  int ldd = 0;
+  void free() {
+    psoci_free(t.keys); psoci_free(t.hdr); psoci_free(t.pool); psoci_free(t.counter);
+    psoci_free(cfg); psoci_free(slot); psoci_free(vals); psoci_free(D);
+  }
+};
+
+// Whether a space goes by coupling tables: every configuration within TAB_MAXOPEN open shells
+// and room for the diagonal blocks (N rows of the largest configuration's SEFs).
+bool tab_usable(const psoci_ctx *c, bool want_diag) {
+  if (c->max_ndet > TAB_MAXDET) return false;
+  if (!want_diag) return true;
+  size_t freeb = 0, totb = 0;
+  if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess) return false;
+  return (double)c->nsef_total * c->max_nsef * 8.0 <= 0.25 * ((double)freeb + (double)c->pool_bytes);
+}
+
+int max_open_of(const psoci_ctx *c) {
+  int no = 1;
+  while (no < PSOCI_MAX_OPEN && (1 << (no - 1)) < c->max_ndet) ++no;
+  return no;
+}
+
+// Slots (and with vals the integrals) of the npairs pairs of the lists and the tables they
+// need.  ok = false: the patterns do not fit the tables and nothing is left allocated; the
+// generic kernels take the space.
+template <int W>
+psoci_status tab_prepare(psoci_ctx *c, const Params &P, const int64_t *nbroff, const int32_t *nbr, int64_t npairs,
+                         bool vals, TabSet<W> &S, bool &ok) {
+  cudaStream_t st = c->stream;
+  const int n = c->nconf;
+  psoci_status s = PSOCI_OK;
+  ok = false;
+  const int wblocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n * 32 + 255) / 256, 1 << 20));
+  if ((s = psoci_alloc(c, &S.cfg, n)) || (s = psoci_alloc(c, &S.slot, npairs)) ||
+      (vals && (s = psoci_alloc(c, &S.vals, npairs))) || (s = psoci_alloc(c, &S.t.counter, 2))) {
+    S.free();
+    return s;
+  }
+  S.t.err = reinterpret_cast<int *>(S.t.counter + 1);
+  cudaError_t e = cudaSuccess;
+  psoci_note_launch();
+  k_cfg_rec<W><<<(int)std::min<int64_t>((n + 255) / 256, 152 * 16), 256, 0, st>>>(P, S.cfg);
+  // 2^18 key slots hold every space measured (up to 6 * 10^4 patterns); a full table grows
+  int64_t slots = 1 << 14, cap = std::max<int64_t>(c->tab_words_hint + c->tab_words_hint / 8, 1 << 20);
+  while (slots < 4 * npairs && slots < (1 << 18)) slots <<= 1;
+  for (int attempt = 0; attempt < 6 && e == cudaSuccess; ++attempt) {
+    if ((s = psoci_alloc(c, &S.t.keys, slots)) || (s = psoci_alloc(c, &S.t.hdr, 2 * slots)) ||
+        (s = psoci_alloc(c, &S.t.pool, cap))) {
+      S.free();
+      return s;
+    }
+    S.t.slots = slots;
+    S.t.cap = cap;
+    e = cudaMemsetAsync(S.t.keys, 0, sizeof(uint64_t) * slots, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S.t.counter, 0, 2 * sizeof(unsigned long long), st);
+    if (e != cudaSuccess) break;
+    psoci_note_launch();
+    if (vals)
+      k_pair_slots<W, true><<<wblocks, 256, 0, st>>>(P, S.cfg, nbroff, nbr, S.t.keys, (uint32_t)(slots - 1), S.t.err,
+                                                     S.slot, S.vals);
+    else
+      k_pair_slots<W, false><<<wblocks, 256, 0, st>>>(P, S.cfg, nbroff, nbr, S.t.keys, (uint32_t)(slots - 1), S.t.err,
+                                                      S.slot, nullptr);
+    const TabBuildArgs B = {S.t.keys, slots, c->d_tmpl, c->d_tmpl_off, c->nelec, c->ksym & 1,
+                            S.t.hdr, S.t.pool, S.t.counter, cap, S.t.err};
+    psoci_note_launch();
+    k_tab_build<<<(unsigned)((slots / 32 + TABB_WARPS - 1) / TABB_WARPS), TABB_WARPS * 32, 0, st>>>(B);
+    if ((e = cudaGetLastError()) != cudaSuccess) break;
+    unsigned long long back[2] = {0, 0};  // words used; error bits
+    e = cudaMemcpyAsync(back, S.t.counter, sizeof(back), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) break;
+    const int err = (int)(uint32_t)back[1];
+    c->tab_words_hint = (int64_t)back[0];
+    if (err & 2) break;  // a pattern outside the tables' form
+    if (!(err & 1) && (int64_t)back[0] <= cap) {
+      ok = true;
+      break;
+    }
+    if (err & 1) slots <<= 2;
+    cap = std::max(cap, (int64_t)back[0] + (int64_t)back[0] / 8);
+    if (slots > ((int64_t)1 << 24) || cap > ((int64_t)1 << 30)) break;
+  }
+  if (e != cudaSuccess) {
+    S.free();
+    return psoci_cuda_fail(c, e, "coupling tables");
+  }
+  if (!ok) S.free();
+  return PSOCI_OK;
+}
+
+// The diagonal blocks and the diagonal of H.
+template <int W>
+psoci_status tab_diagonal(psoci_ctx *c, const Params &P, TabSet<W> &S, double *diag) {
+  psoci_status s;
+  S.ldd = c->max_nsef;
+  if ((s = psoci_alloc(c, &S.D, (size_t)c->nsef_total * S.ldd))) return s;
+  psoci_note_launch();
+  k_diag_blocks<W><<<(unsigned)std::min<int64_t>((c->nconf + DG_WARPS - 1) / DG_WARPS, 1 << 20), DG_WARPS * 32, 0,
+                     c->stream>>>(P, S.ldd, S.D, diag);
+  PSOCI_CUDA(c, cudaGetLastError());
+  return PSOCI_OK;
+}
+
+// One launch of k_elems: EL_WARPS warps a block, one where two do not fit.
+template <int W, int MODE, bool VALS, bool SMALL>
+psoci_status elems_launch_as(psoci_ctx *c, const Params &P, ElemArgs<W> &E) {
+  const size_t per = (sizeof(ElemWarp) + (size_t)E.ms * PSOCI_SEG * 8 + (size_t)E.ldd * (MODE < 2 ? 4 : 256) + 15) & ~(size_t)15;
+  E.warp_bytes = (int)per;
+  const int warps = per * EL_WARPS <= (size_t)200 * 1024 ? EL_WARPS : 1;
+  const size_t smem = per * warps;
+  auto k = k_elems<W, MODE, VALS, SMALL>;
+  PSOCI_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PSOCI_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  psoci_note_launch();
+  k<<<(unsigned)std::min<int64_t>((c->nconf + warps - 1) / warps, 1 << 20), warps * 32, smem, c->stream>>>(P, E);
+  PSOCI_CUDA(c, cudaGetLastError());
+  return PSOCI_OK;
+}
+template <int W, int MODE, bool VALS>
+psoci_status elems_launch(psoci_ctx *c, const Params &P, ElemArgs<W> &E) {
+  return E.ldd <= 16 ? elems_launch_as<W, MODE, VALS, true>(c, P, E) : elems_launch_as<W, MODE, VALS, false>(c, P, E);
+}
+
+template <int W>
+ElemArgs<W> elem_args(const psoci_ctx *c, const TabSet<W> &S) {
+  ElemArgs<W> E = {};
+  E.cfg = S.cfg; E.slot = S.slot; E.vals = S.vals; E.hdr = S.t.hdr; E.pool = S.t.pool; E.D = S.D;
+  E.ldd = S.ldd;
+  E.ms = std::max(2, max_open_of(c));  // X also holds a two-word mask, or two integrals
+  return E;
+}
+
+// What a direct-mode build keeps of its tables (psoci_ctx::dir_tabs).
+struct DirTabs {
+  TabSet<1> s1;
+  TabSet<2> s2;
+};
+template <int W>
+TabSet<W> &dir_set(DirTabs *d) {
+  if constexpr (W == 1) return d->s1;
+  else return d->s2;
+}
+
 template <int W>
 psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
   cudaStream_t st = c->stream;
@@ -2269,34 +2217,16 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
   P.one = c->d_one; P.eri = c->d_eri;
 
   psoci_status s;
-  int64_t *d_cnt = nullptr, *d_nbroff = nullptr, *d_nseg = nullptr, *d_nrow = nullptr, *d_segoff = nullptr,
-          *d_rowslot = nullptr, *d_segk0 = nullptr, *d_segrow = nullptr, *d_segcnt = nullptr, *d_rownnz = nullptr;
+  int64_t *d_nbroff = nullptr, *d_nseg = nullptr, *d_nrow = nullptr, *d_segoff = nullptr, *d_rowslot = nullptr,
+          *d_segk0 = nullptr, *d_segrow = nullptr, *d_segcnt = nullptr, *d_rownnz = nullptr;
   int32_t *d_nbr = nullptr, *d_segcfg = nullptr, *d_segn = nullptr;
-  int64_t *d_soff = nullptr, *d_tot = nullptr, *d_candoff = nullptr;
-  int64_t *d_nlow = nullptr, *d_prrows = nullptr, *d_proff = nullptr;
-  int32_t *d_cand = nullptr, *d_mk = nullptr, *d_skip = nullptr;
-  int64_t *d_gcnt = nullptr, *d_goff = nullptr;
-  uint32_t *d_glist = nullptr;
-  uint64_t *d_prm = nullptr;
-  uint64_t *d_cg = nullptr;
-  int *d_err = nullptr;
-  unsigned long long *d_counter = nullptr;
-  double *d_slabval = nullptr;
-  int32_t *d_jslab = nullptr;
-  int64_t *d_jstart = nullptr;
-  int2 *d_tpairs = nullptr;
-  uint32_t *d_dkept = nullptr;
+  TabSet<W> T;
   cudaEvent_t ev[6] = {};
   auto cleanup = [&]() {
     for (auto &e : ev)
       if (e) cudaEventDestroy(e);
-    psoci_free(d_soff); psoci_free(d_tot); psoci_free(d_counter);
-    psoci_free(d_candoff); psoci_free(d_cand); psoci_free(d_skip);
-    psoci_free(d_nlow); psoci_free(d_prrows); psoci_free(d_proff); psoci_free(d_mk); psoci_free(d_prm); psoci_free(d_cg);
-    psoci_free(d_err); psoci_free(d_slabval); psoci_free(d_jslab); psoci_free(d_jstart);
-    psoci_free(d_tpairs); psoci_free(d_dkept);
-    psoci_free(d_gcnt); psoci_free(d_goff); psoci_free(d_glist);
-    psoci_free(d_cnt); psoci_free(d_nbroff); psoci_free(d_nseg); psoci_free(d_nrow); psoci_free(d_segoff);
+    T.free();
+    psoci_free(d_nbroff); psoci_free(d_nseg); psoci_free(d_nrow); psoci_free(d_segoff);
     psoci_free(d_rowslot); psoci_free(d_segk0); psoci_free(d_segrow); psoci_free(d_segcnt); psoci_free(d_rownnz);
     psoci_free(d_nbr); psoci_free(d_segcfg); psoci_free(d_segn);
   };
@@ -2335,169 +2265,114 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
   TRYC(cudaEventRecord(ev[1], st));
   auto t_b = tnow();
 
-  // fast path: only the lower pairs (J <= I) are evaluated; the rest are mirrored
+  // coupling tables for configurations of at most TAB_MAXOPEN open shells; the generic kernels
+  // for others, and for patterns the tables do not hold
   const bool direct = (mode == PSOCI_HMODE_DIRECT);
-  const bool fast = !direct && c->max_ndet <= FAST_MAXDET;
-  int64_t nprm = 0;
-  bool split = false;  // fast path: masks and elements in two launches
+  const int64_t N = c->nsef_total;
+  bool fast = tab_usable(c, true), vals = false;
   if (fast) {
-    TRY(psoci_alloc(c, &d_nlow, n + 1));
-    TRY(psoci_alloc(c, &d_prrows, n + 1));
-    TRY(psoci_alloc(c, &d_proff, n + 1));
-    psoci_note_launch();
-    k_lower_counts<<<(n + 255) / 256, 256, 0, st>>>(n, d_nbroff, d_nbr, c->d_sefoff, d_nlow, d_prrows);
-    TRYC(cudaGetLastError());
-    TRY(psoci_scan_i64(c, d_prrows, d_proff, n, &nprm));
-    TRY(psoci_alloc(c, &d_prm, nprm));
-    P.nlow = d_nlow; P.pr_off = d_proff; P.prm = d_prm;
+    // the pairs' integrals in a list (16 bytes a pair) when it takes at most a quarter of the
+    // memory there is, evaluated in each element launch otherwise
+    size_t freeb = 0, totb = 0;
+    TRYC(cudaMemGetInfo(&freeb, &totb));
+    vals = !direct && c->eval_launches != 1 && (double)npairs * 16.0 <= 0.25 * ((double)freeb + (double)c->pool_bytes);
+    TRYC(cudaEventRecord(ev[2], st));
+    TRY(tab_prepare<W>(c, P, d_nbroff, d_nbr, npairs, vals, T, fast));
   }
+  auto t_c = tnow();
 
-  // 2. segments
-  TRY(psoci_alloc(c, &d_nseg, n + 1));
-  TRY(psoci_alloc(c, &d_nrow, n + 1));
-  TRY(psoci_alloc(c, &d_segoff, n + 1));
-  TRY(psoci_alloc(c, &d_rowslot, n + 1));
-  psoci_note_launch();
-  k_seg_counts<<<(n + 255) / 256, 256, 0, st>>>(n, d_nbroff, d_nlow, c->d_sefoff, d_nseg, d_nrow);
-  TRYC(cudaGetLastError());
+  // 2. segments of the generic kernels (<= 32 neighbours of a configuration, one warp each)
   int64_t nseg = 0, nslots = 0;
-  TRY(psoci_scan_i64(c, d_nseg, d_segoff, n, &nseg));
-  TRY(psoci_scan_i64(c, d_nrow, d_rowslot, n, &nslots));
-  TRY(psoci_alloc(c, &d_segcfg, nseg));
-  TRY(psoci_alloc(c, &d_segk0, nseg));
-  TRY(psoci_alloc(c, &d_segn, nseg));
-  TRY(psoci_alloc(c, &d_segrow, nseg));
-  TRY(psoci_alloc(c, &d_segcnt, nslots));
-  psoci_note_launch();
-  k_seg_init<<<(n + 255) / 256, 256, 0, st>>>(n, d_nbroff, d_nlow, c->d_sefoff, d_segoff, d_rowslot, d_segcfg, d_segk0,
-                                              d_segn, d_segrow);
-  TRYC(cudaGetLastError());
+  if (!fast) {
+    TRY(psoci_alloc(c, &d_nseg, n + 1));
+    TRY(psoci_alloc(c, &d_nrow, n + 1));
+    TRY(psoci_alloc(c, &d_segoff, n + 1));
+    TRY(psoci_alloc(c, &d_rowslot, n + 1));
+    psoci_note_launch();
+    k_seg_counts<<<(n + 255) / 256, 256, 0, st>>>(n, d_nbroff, c->d_sefoff, d_nseg, d_nrow);
+    TRYC(cudaGetLastError());
+    TRY(psoci_scan_i64(c, d_nseg, d_segoff, n, &nseg));
+    TRY(psoci_scan_i64(c, d_nrow, d_rowslot, n, &nslots));
+    TRY(psoci_alloc(c, &d_segcfg, nseg));
+    TRY(psoci_alloc(c, &d_segk0, nseg));
+    TRY(psoci_alloc(c, &d_segn, nseg));
+    TRY(psoci_alloc(c, &d_segrow, nseg));
+    TRY(psoci_alloc(c, &d_segcnt, nslots));
+    psoci_note_launch();
+    k_seg_init<<<(n + 255) / 256, 256, 0, st>>>(n, d_nbroff, c->d_sefoff, d_segoff, d_rowslot, d_segcfg, d_segk0,
+                                                d_segn, d_segrow);
+    TRYC(cudaGetLastError());
+    P.nseg = nseg; P.seg_cfg = d_segcfg; P.seg_k0 = d_segk0; P.seg_n = d_segn; P.seg_rowoff = d_segrow;
+    P.seg_cnt = d_segcnt;
+  }
   c->nseg = nseg;
-  P.nseg = nseg; P.seg_cfg = d_segcfg; P.seg_k0 = d_segk0; P.seg_n = d_segn; P.seg_rowoff = d_segrow;
-  P.seg_cnt = d_segcnt; P.segoff = d_segoff;
 
   // 3. evaluate
-  int hb_blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nseg + WARPS_PER_CTA - 1) / WARPS_PER_CTA, 152 * 16));
-  const int64_t N = c->nsef_total;
-  int64_t nnz = 0, slab_used = 0;
-  int evaluations = 0;
-  auto t_c = tnow();
+  const int hb_blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nseg + WARPS_PER_CTA - 1) / WARPS_PER_CTA, 152 * 16));
+  int64_t nnz = 0;
   auto t_d = t_c, t_e = t_c;
   if (direct) {
     // direct mode: the diagonal now, the other elements in every sigma; the neighbour lists
-    // and segments move to the context
+    // and tables (or segments) move to the context
     TRY(psoci_alloc(c, &c->d_diag, N));
     P.diag = c->d_diag;
-    const size_t smem = sizeof(WarpSmem) * WARPS_PER_CTA;
-    TRYC(cudaFuncSetAttribute(k_hbuild<W, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    TRYC(cudaEventRecord(ev[2], st));
-    psoci_note_launch();
-    k_hbuild<W, 3><<<hb_blocks, WARPS_PER_CTA * 32, smem, st>>>(P);
-    TRYC(cudaGetLastError());
+    if (fast) {
+      TRY(tab_diagonal<W>(c, P, T, c->d_diag));
+      c->nseg = nseg = (npairs + PSOCI_SEG - 1) / PSOCI_SEG;
+    } else {
+      const size_t smem = sizeof(WarpSmem) * WARPS_PER_CTA;
+      TRYC(cudaFuncSetAttribute(k_hbuild<W, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      TRYC(cudaEventRecord(ev[2], st));
+      psoci_note_launch();
+      k_hbuild<W, 3><<<hb_blocks, WARPS_PER_CTA * 32, smem, st>>>(P);
+      TRYC(cudaGetLastError());
+    }
     TRYC(cudaEventRecord(ev[3], st));
     TRYC(cudaEventRecord(ev[4], st));
     TRYC(cudaEventRecord(ev[5], st));
     TRYC(cudaStreamSynchronize(st));
     c->dir_nbroff = d_nbroff; d_nbroff = nullptr;
     c->dir_nbr = d_nbr; d_nbr = nullptr;
-    c->dir_segcfg = d_segcfg; d_segcfg = nullptr;
-    c->dir_segk0 = d_segk0; d_segk0 = nullptr;
-    c->dir_segn = d_segn; d_segn = nullptr;
+    if (fast) {
+      DirTabs *d = new DirTabs();
+      dir_set<W>(d) = T;
+      T = TabSet<W>();
+      c->dir_tabs = d;
+    } else {
+      c->dir_segcfg = d_segcfg; d_segcfg = nullptr;
+      c->dir_segk0 = d_segk0; d_segk0 = nullptr;
+      c->dir_segn = d_segn; d_segn = nullptr;
+    }
     c->direct = true;
   } else if (fast) {
-    // 3. evaluate the lower pairs once: kept values go to slab slots, masks to prm
-    const size_t smem = sizeof(FastSmem<W>) * WARPS_PER_CTA;
-    TRYC(cudaFuncSetAttribute(k_hbuild_fast<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // two launches when the masks fit (8 bytes per (pair, row SEF), a quarter of the free
-    // memory at most): the connectivity masks (k_hbuild_masks), then the elements from them;
-    // otherwise both phases in one launch
-    size_t freeb = 0, totb = 0;
-    TRYC(cudaMemGetInfo(&freeb, &totb));
-    split = c->eval_launches != 1 && (double)nprm * 8.0 <= 0.25 * (double)freeb;
-    if (split) {
-      TRYC(cudaFuncSetAttribute(k_hbuild_fast<W, 0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      TRY(psoci_alloc(c, &d_cg, nprm));
-      P.cg = d_cg;
-    }
-    TRY(psoci_alloc(c, &d_counter, 1));
-    TRYC(cudaMemGetInfo(&freeb, &totb));
-    // slots hold the kept elements of the lower pairs plus the unused tails of the warps'
-    // chunks; first guess from the pair count (observed up to 7 kept elements per lower
-    // pair; (npairs + nconf) / 2 lower pairs) or from the previous build of the same space;
-    // an overflow is detected by the kernel's counter and the evaluation repeats with the
-    // exact size
-    const int64_t tails = (int64_t)hb_blocks * WARPS_PER_CTA * SLAB_CHUNK;
-    int64_t cap = std::max<int64_t>(4 * npairs + 4 * (int64_t)n, c->slab_hint) + tails;
-    cap = std::min<int64_t>((int64_t)(freeb * 0.5) / 8, cap);
-    int64_t nlower = 0;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-      auto t_al = std::chrono::steady_clock::now();
-      TRY(psoci_alloc(c, &d_slabval, cap));
-      if (c->verbose)
-        fprintf(stderr, "psoci: H build slab allocation %.4f s (%lld slots)\n",
-                std::chrono::duration<double>(std::chrono::steady_clock::now() - t_al).count(), (long long)cap);
-      TRYC(cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), st));
-      P.slab_counter = d_counter; P.slab_cap = cap; P.slab_val = d_slabval;
-      TRYC(cudaEventRecord(ev[2], st));
-      if (split && attempt == 0) {
-        const int mblocks = (int)std::max<int64_t>(1, std::min<int64_t>((nseg + MASK_WARPS - 1) / MASK_WARPS, 152 * 8));
-        psoci_note_launch();
-        k_hbuild_masks<W><<<mblocks, MASK_WARPS * 32, 0, st>>>(P);
-        TRYC(cudaGetLastError());
-      }
-      psoci_note_launch();
-      if (split) k_hbuild_fast<W, 0, 2><<<hb_blocks, WARPS_PER_CTA * 32, smem, st>>>(P);
-      else k_hbuild_fast<W><<<hb_blocks, WARPS_PER_CTA * 32, smem, st>>>(P);
-      TRYC(cudaGetLastError());
-      TRYC(cudaEventRecord(ev[3], st));
-      ++evaluations;
-      unsigned long long used = 0;
-      TRYC(cudaMemcpyAsync(&used, d_counter, sizeof(used), cudaMemcpyDeviceToHost, st));
-      TRYC(cudaStreamSynchronize(st));
-      nlower = (int64_t)used;
-      if (c->verbose)
-        fprintf(stderr, "psoci: H build slab %lld of %lld slots used\n", (long long)nlower, (long long)cap);
-      if (nlower <= cap) break;
-      psoci_free(d_slabval);
-      cap = nlower + tails;  // chunk tails differ from run to run
-      if (attempt == 1) TRY(psoci_fail(c, PSOCI_ERR_NOMEM, "H build: element slab overflow"));
-    }
-    psoci_free(d_cg);  // the masks are done with
-    t_d = tnow();
-    // 4. full row lengths (lower counts + mirrored columns) and offsets
+    TRY(psoci_alloc(c, &c->d_diag, N));
+    TRY(tab_diagonal<W>(c, P, T, c->d_diag));
     TRY(psoci_alloc(c, &d_rownnz, N + 1));
-    TRY(psoci_alloc(c, &d_mk, npairs));
-    TRY(psoci_alloc(c, &d_err, 1));
-    TRYC(cudaMemsetAsync(d_err, 0, sizeof(int), st));
-    const int cfg_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n * 32 + 255) / 256, 152 * 32));
-    const int64_t nq = (npairs + NBR_SKIP - 1) / NBR_SKIP;
-    P.nbr_len = npairs;
-    TRY(psoci_alloc(c, &d_skip, nq));
-    psoci_note_launch();
-    k_nbr_skip<<<(int)std::min<int64_t>((nq + 255) / 256, 152 * 16), 256, 0, st>>>(nq, d_nbr, d_skip);
-    TRYC(cudaGetLastError());
-    psoci_note_launch();
-    k_mirror_count<<<cfg_blocks, 256, 0, st>>>(P, d_skip, d_rownnz, d_mk, d_err);
-    TRYC(cudaGetLastError());
-    int herr = 0;
-    TRYC(cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ElemArgs<W> E = elem_args<W>(c, T);
+    E.row_nnz = d_rownnz;
+    E.segments = T.t.counter;
+    TRYC(cudaMemsetAsync(T.t.counter, 0, sizeof(unsigned long long), st));
+    // 3. count the kept elements of each row
+    if (vals) TRY((elems_launch<W, 0, true>(c, P, E)));
+    else TRY((elems_launch<W, 0, false>(c, P, E)));
+    TRYC(cudaEventRecord(ev[3], st));
+    t_d = tnow();
+    unsigned long long segs = 0;
+    TRYC(cudaMemcpyAsync(&segs, T.t.counter, sizeof(segs), cudaMemcpyDeviceToHost, st));
+    // 4. row offsets
     TRY(psoci_alloc(c, &c->d_rowptr, N + 1));
     TRY(psoci_scan_i64(c, d_rownnz, c->d_rowptr, N, &nnz));
-    if (herr) TRY(psoci_fail(c, PSOCI_ERR_CUDA, "H build: neighbour lists are not symmetric"));
+    c->nseg = nseg = (int64_t)segs;
     TRYC(cudaEventRecord(ev[4], st));
-    slab_used = nlower;
-    c->slab_hint = nlower;
     if (nnz < N) TRY(psoci_fail(c, PSOCI_ERR_CUDA, "H build: rows without their diagonal element"));
     TRY(psoci_alloc(c, &c->d_col, nnz));
     TRY(psoci_alloc(c, &c->d_val, nnz));
     if (mode == PSOCI_HMODE_CSR_BOTH) TRY(psoci_alloc(c, &c->d_val32, nnz));
-    TRY(psoci_alloc(c, &c->d_diag, N));
-    P.rowptr = c->d_rowptr; P.col = c->d_col; P.val = c->d_val; P.val32 = c->d_val32; P.diag = c->d_diag;
+    P.rowptr = c->d_rowptr; P.col = c->d_col; P.val = c->d_val; P.val32 = c->d_val32;
     t_e = tnow();
-    // 5. ordered assembly
-    psoci_note_launch();
-    k_assemble<<<cfg_blocks, ASM_THREADS, 0, st>>>(P, d_mk);
-    TRYC(cudaGetLastError());
+    // 5. write them
+    if (vals) TRY((elems_launch<W, 1, true>(c, P, E)));
+    else TRY((elems_launch<W, 1, false>(c, P, E)));
     TRYC(cudaEventRecord(ev[5], st));
     TRYC(cudaStreamSynchronize(st));
   } else {
@@ -2510,7 +2385,6 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
     k_hbuild<W, 0><<<hb_blocks, WARPS_PER_CTA * 32, smem, st>>>(P);
     TRYC(cudaGetLastError());
     TRYC(cudaEventRecord(ev[3], st));
-    ++evaluations;
     t_d = tnow();
     // 4. offsets
     TRY(psoci_alloc(c, &d_rownnz, N + 1));
@@ -2537,19 +2411,18 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
   if (c->verbose) {
     auto d = [](auto a, auto b) { return std::chrono::duration<double>(b - a).count(); };
     fprintf(stderr,
-            "psoci: H build phases (%s kernel%s, %s screen): screen %.4f s, segments %.4f s, evaluate %.4f s, "
-            "offsets %.4f s, fill/copy %.4f s\n",
-            fast ? "fast" : "generic", split ? ", masks launched apart" : "", nsplit ? "all-pairs" : "lookup",
-            d(t_a, t_b), d(t_b, t_c), d(t_c, t_d),
-            d(t_d, t_e), d(t_e, t_f));
+            "psoci: H build phases (%s%s, %s screen): screen %.4f s, tables %.4f s, evaluate %.4f s, "
+            "offsets %.4f s, fill %.4f s\n",
+            fast ? "coupling tables" : "generic kernels", vals ? ", pair integrals listed" : "",
+            nsplit ? "all-pairs" : "lookup", d(t_a, t_b), d(t_b, t_c), d(t_c, t_d), d(t_d, t_e), d(t_e, t_f));
   }
   {
     psoci_build_info &b = c->binfo;
     b = psoci_build_info{};
     b.candidates = ncand; b.pairs = npairs; b.segments = nseg; b.nnz = nnz; b.nnz_lower = direct ? 0 : (nnz + N) / 2;
-    b.slab_slots = slab_used; b.evaluations = evaluations; b.fast = fast ? 1 : 0;
+    b.evaluations = direct ? 0 : 1; b.fast = (fast && !direct) ? 1 : 0;
     b.lookup_screen = c->join_ok ? 1 : 0;
-    b.eval_launches = fast ? (split ? 2 : 1) : 0;
+    b.eval_launches = (fast && !direct) ? (vals ? 2 : 1) : 0;
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, ev[0], ev[1]) == cudaSuccess) b.screen_ms = ms;
     if (cudaEventElapsedTime(&ms, ev[2], ev[3]) == cudaSuccess) b.evaluate_ms = ms;
@@ -2590,20 +2463,21 @@ psoci_status run_direct_sigma(psoci_ctx *c, int k, const double *dX, int ldx, do
   P.nbroff = c->dir_nbroff; P.nbr = c->dir_nbr;
   P.nseg = c->nseg; P.seg_cfg = c->dir_segcfg; P.seg_k0 = c->dir_segk0; P.seg_n = c->dir_segn;
   const int64_t N = c->nsef_total;
-  PSOCI_CUDA(c, cudaMemset2DAsync(dY, sizeof(double) * ldy, 0, sizeof(double) * k, N, st));
-  if (P.nseg == 0) return PSOCI_OK;
-  // configurations of at most 32 determinants: the connectivity-marking kernel, evaluating
-  // only the elements that can be non-zero; otherwise the generic one
-  const bool fast = c->max_ndet <= FAST_MAXDET;
-  const size_t smem = fast ? sizeof(FastSmem<W>) * WARPS_PER_CTA : sizeof(WarpSmem) * WARPS_PER_CTA;
+  psoci_status s;
+  const bool fast = c->dir_tabs != nullptr;
+  const size_t smem = sizeof(WarpSmem) * WARPS_PER_CTA;
+  ElemArgs<W> E = {};
   if (fast) {
-    PSOCI_CUDA(c, cudaFuncSetAttribute(k_hbuild_fast<W, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PSOCI_CUDA(c, cudaFuncSetAttribute(k_hbuild_fast<W, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  } else
+    E = elem_args<W>(c, dir_set<W>(static_cast<DirTabs *>(c->dir_tabs)));
+  } else {
+    PSOCI_CUDA(c, cudaMemset2DAsync(dY, sizeof(double) * ldy, 0, sizeof(double) * k, N, st));
+    if (P.nseg == 0) return PSOCI_OK;
     PSOCI_CUDA(c, cudaFuncSetAttribute(k_hbuild<W, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  }
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((P.nseg + WARPS_PER_CTA - 1) / WARPS_PER_CTA, 152 * 16));
-  // MIXED (connectivity-marking kernel only): FP32 element x FP32 input products
-  const bool mixed = fast && prec == PSOCI_PREC_MIXED && x32;
+  // MIXED (spaces of at most 32 determinants a configuration): FP32 element x FP32 input
+  // products; beyond them direct mode is FP64 whatever the precision asked for
+  const bool mixed = fast && c->max_ndet <= 32 && prec == PSOCI_PREC_MIXED && x32;
   for (int q0 = 0; q0 < k; q0 += 8) {
     P.dx = dX + q0; P.dy = dY + q0; P.ldx = ldx; P.ldy = ldy; P.kvec = std::min(8, k - q0);
     P.dx32 = nullptr;
@@ -2611,15 +2485,14 @@ psoci_status run_direct_sigma(psoci_ctx *c, int k, const double *dX, int ldx, do
       psoci_note_launch();
       k_direct_x32<<<(unsigned)std::min<int64_t>((N + 255) / 256, 152 * 16), 256, 0, st>>>(N, P.kvec, P.dx, ldx, x32);
       P.dx32 = x32;
-    }
-    psoci_note_launch();
-    if (fast && mixed)
-      k_hbuild_fast<W, 2><<<blocks, WARPS_PER_CTA * 32, smem, st>>>(P);
-    else if (fast)
-      k_hbuild_fast<W, 1><<<blocks, WARPS_PER_CTA * 32, smem, st>>>(P);
-    else
+      if ((s = elems_launch<W, 3, false>(c, P, E))) return s;
+    } else if (fast) {
+      if ((s = elems_launch<W, 2, false>(c, P, E))) return s;
+    } else {
+      psoci_note_launch();
       k_hbuild<W, 2><<<blocks, WARPS_PER_CTA * 32, smem, st>>>(P);
-    PSOCI_CUDA(c, cudaGetLastError());
+      PSOCI_CUDA(c, cudaGetLastError());
+    }
   }
   return PSOCI_OK;
 }
@@ -2839,6 +2712,13 @@ void psoci_h_release(psoci_ctx *c) {
   psoci_free(c->dir_segcfg);
   psoci_free(c->dir_segk0);
   psoci_free(c->dir_segn);
+  if (c->dir_tabs) {
+    DirTabs *d = static_cast<DirTabs *>(c->dir_tabs);
+    d->s1.free();
+    d->s2.free();
+    delete d;
+    c->dir_tabs = nullptr;
+  }
   c->direct = false;
   psoci_free(c->d_rowptr);
   psoci_free(c->d_col);

@@ -31,7 +31,7 @@ struct DevBuf {
 struct psoci_ctx {
   int device = 0;
   int verbose = 0;
-  int eval_launches = 0;  // 0: automatic; 1: the element evaluation in one launch
+  int eval_launches = 0;  // 0: automatic; 1: pair integrals evaluated in the element launches
   cudaStream_t stream = nullptr;
   std::string err;
   // released device blocks kept for reuse (size -> pointer), see psoci_alloc
@@ -100,7 +100,8 @@ struct psoci_ctx {
   int32_t *dir_nbr = nullptr;     // [npairs]
   int32_t *dir_segcfg = nullptr, *dir_segn = nullptr;
   int64_t *dir_segk0 = nullptr;
-  int64_t slab_hint = 0;  // value-slab slots the last build of this space used
+  void *dir_tabs = nullptr;       // coupling tables of the elements (hbuild.cu, DirTabs), or null
+  int64_t tab_words_hint = 0;     // words of coupling tables the last build used
   int64_t join_hint = 0;  // join-slab slots the last build of this space used
 
   // 1-particle density: configuration groups sharing a hole key (density.cu)

@@ -1,0 +1,89 @@
+"""H from coupling tables at the edges of what the tables hold: 7 to 10 open shells (rows of
+up to 256 SEFs, row offsets instead of 4-bit row counts), 11 open shells (the generic
+kernels), doubly emptied and filled orbitals, two-word strings, both electron parities — the
+stored matrix, and the direct product with no stored elements, against the oracle.
+
+Elements are the reference's sums in its order, so they agree to rounding (a few ulps of
+values up to about 50: 1e-12); products add at most a row of them."""
+import numpy as np
+import pytest
+
+from helpers import check_h_against_oracle, gpu_context, small_problem
+
+pytestmark = pytest.mark.gpu
+
+
+def neighbourhood(nbf, nelec, nopen, ksym, most, seed, shift=0):
+    """A configuration with `nopen` open shells and its first `most` neighbours within two
+    excitations (lexicographic order of the excitations), orbitals moved up by `shift`."""
+    from psoci_gb300.inputs import Problem, config_jsym, make_integrals, make_irreps, select_block
+
+    rng = np.random.default_rng(seed)
+    n = nbf + shift
+    irr = make_irreps(n, rng)
+    h, so, eri = make_integrals(n, irr, n, rng)
+    ref = np.zeros(n, np.uint8)
+    ndbl = (nelec - nopen) // 2
+    ref[shift:shift + ndbl] = 2
+    ref[shift + ndbl:shift + ndbl + nopen] = 1
+    occs = {tuple(ref)}
+    singles = []
+    for i in range(n):
+        for a in range(n):
+            o = ref.astype(int)
+            o[i] -= 1
+            o[a] += 1
+            if i != a and o[i] >= 0 and o[a] <= 2:
+                singles.append(tuple(o))
+    rng.shuffle(singles)
+    doubles = []
+    for s in singles[:40]:
+        for i, a in rng.integers(0, n, (6, 2)):
+            o = np.array(s)
+            o[i] -= 1
+            o[a] += 1
+            if i != a and o[i] >= 0 and o[a] <= 2:
+                doubles.append(tuple(int(x) for x in o))
+    for o in singles[:most // 2] + doubles:
+        if len(occs) >= most:
+            break
+        if sum(x == 1 for x in o) <= 11:
+            occs.add(tuple(int(x) for x in o))
+    occ = np.array(sorted(occs, reverse=True), np.uint8)
+    js = config_jsym(occ, irr)
+    occ, js = select_block(occ, js, ksym)
+    return Problem(nbf=n, nelec=nelec, ksym=ksym, mx_open=int((occ == 1).sum(1).max()), jsym=np.ascontiguousarray(js),
+                   occ=np.ascontiguousarray(occ), h=h, so=so, eri=eri, irreps=irr)
+
+
+CASES = {
+    "open7": lambda: neighbourhood(9, 9, 7, 1, 60, 1),
+    "open8": lambda: neighbourhood(10, 8, 8, 2, 40, 2),
+    "open9": lambda: neighbourhood(11, 9, 9, 1, 16, 3),
+    "open10": lambda: neighbourhood(11, 10, 10, 1, 10, 4),
+    "open10_two_words": lambda: neighbourhood(11, 10, 8, 3, 24, 5, shift=58),
+    "open11": lambda: neighbourhood(12, 11, 11, 2, 4, 6),
+    "pairs": lambda: neighbourhood(8, 8, 0, 1, 120, 7),
+    "one_electron": lambda: neighbourhood(6, 1, 1, 1, 6, 8),
+    "two_electrons": lambda: small_problem("fci_4e6o", 2),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_tables_match_oracle(oracle_mod, name):
+    p = CASES[name]()
+    O = oracle_mod.Oracle(p)
+    c = gpu_context(p)
+    F = check_h_against_oracle(c, O, p, tol=1e-12)
+    listed = c.get_hamiltonian()
+    assert c.build_stats()["fast"] == (1 if p.mx_open <= 10 else 0)
+    c.set_eval_launches(1)  # the pairs' integrals evaluated in the element launches
+    c.build_hamiltonian(mixed=True)
+    for a, b in zip(listed, c.get_hamiltonian()):
+        assert np.array_equal(a, b)
+    X = np.random.default_rng(9).standard_normal((c.nsef, 9))
+    Y = F @ X
+    c.build_hamiltonian(direct=True)
+    scale = np.abs(F).sum(axis=1).max() * np.abs(X).max()
+    assert np.abs(c.sigma(X) - Y).max() <= 1e-14 * scale
+    c.close()
