@@ -485,3 +485,96 @@ __device__ __noinline__ double tab_sum_value(uint32_t ent, uint32_t info, double
   if (c1 != TAB_NOTERM) t = t + tab_single_term(c1, v0, X);
   return tab_scale(t, info);
 }
+
+// ------------------------------------------------------------------------------------
+// adjoint
+// ------------------------------------------------------------------------------------
+// The derivative of a block's elements with respect to one of the pair's integrals is a list of
+// (row, column, sign): the program of a table is these lists end to end — doubles v0, v1;
+// spin-orbit v0; singles v0, X[0], X[1], ... (to the last that occurs) — with the lists' ends
+// (uint16, two a word) before it.  hdr[2 slot + 1].x: first word, .y: lists.  An entry: bits 0-7
+// column, 8-15 row, 31 sign.
+constexpr int TAB_LISTS = 1 + TAB_MAXOPEN;
+
+// signed count of integral `a` in an entry (0, +-1, +-2); singles: two terms a list may hold it twice
+__device__ __forceinline__ int tab_weight(uint32_t ent, bool single, int a) {
+  if (!single) {
+    constexpr int c0[12] = {1, 0, 1, 2, 0, 2, 1, 1, 2, 0, 1, -1}, c1[12] = {0, 1, -1, 0, 2, -2, 1, -1, -1, 1, 0, 2};
+    const int f = (int)(ent >> 8) & 15;
+    int w = 0;
+#pragma unroll
+    for (int u = 0; u < 12; ++u)
+      if (f == u) w = a == 0 ? c0[u] : c1[u];
+    return (ent >> 31) ? -w : w;
+  }
+  int w = 0;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const uint32_t c = u ? ent >> 20 : (ent >> 8) & 0xfffu;
+    if (u && c == TAB_NOTERM) continue;
+    int x = 0;
+    if (c & 0x400u) x = (a > 0 && (c & 0x3ffu) == (uint32_t)(a - 1)) ? 1 : 0;
+    else x = a == 0 ? 1 : ((c >> (a - 1)) & 1u) ? -1 : 0;
+    w += (c & 0x800u) ? -x : x;
+  }
+  return w;
+}
+
+// Programs of all occupied slots, from their entries; one warp a slot, lanes over the entries.
+__global__ void __launch_bounds__(128) k_tab_program(const uint64_t *__restrict__ keys, int64_t slots, uint4 *hdr,
+                                                     uint32_t *pool, unsigned long long *counter, int64_t cap) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t s0 = warp * 32; s0 < slots; s0 += nwarps * 32) {
+    unsigned todo = __ballot_sync(0xffffffffu, s0 + lane < slots && keys[s0 + lane] != 0ull);
+    while (todo) {
+      const int64_t s = s0 + __ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint4 h = hdr[2 * s];
+      const int nent = (int)(h.y & TAB_ENTRIES);
+      // entries that did not fit the pool were not written: the host, which sees the count, repeats
+      if ((int64_t)h.x + nent + (nent + 3) / 4 > cap) {
+        if (lane == 0) hdr[2 * s + 1] = make_uint4(0u, 0u, 0u, 0u);
+        continue;
+      }
+      const bool single = ((h.y >> TAB_KIND) & 7u) == 2u;
+      const uint8_t *rows = reinterpret_cast<const uint8_t *>(pool + h.x + nent);
+      const int most = single ? TAB_LISTS : 2;
+      uint32_t words = 0u, off = 0u;
+      int lists = 0;
+      bool fits = false;
+      for (int pass = 0; pass < 2; ++pass) {
+        int n = 0;
+        for (int a = 0; a < most; ++a) {
+          for (int e0 = 0; e0 < nent; e0 += 32) {
+            const int e = e0 + lane;
+            const uint32_t ent = e < nent ? pool[h.x + e] : 0u;
+            const int w = e < nent ? tab_weight(ent, single, a) : 0;
+            const unsigned b1 = __ballot_sync(0xffffffffu, w != 0), b2 = __ballot_sync(0xffffffffu, w == 2 || w == -2);
+            if (pass == 1 && fits && w != 0) {
+              const unsigned lt = (1u << lane) - 1u;
+              const uint32_t r = single ? rows[e] : (ent >> 12) & 0xffu;
+              const uint32_t x = (ent & 0xffu) | (r << 8) | (w < 0 ? 0x80000000u : 0u);
+              uint32_t *to = pool + off + (TAB_LISTS + 1) / 2 + n + __popc(b1 & lt) + __popc(b2 & lt);
+              to[0] = x;
+              if (w == 2 || w == -2) to[1] = x;
+            }
+            n += __popc(b1) + __popc(b2);
+            if (b1) lists = a + 1;
+          }
+          if (pass == 1 && fits && lane == 0) reinterpret_cast<uint16_t *>(pool + off)[a] = (uint16_t)n;
+        }
+        if (pass == 0) {
+          words = (uint32_t)(n + (TAB_LISTS + 1) / 2);
+          unsigned long long o = 0;
+          if (lane == 0) o = atomicAdd(counter, (unsigned long long)words);
+          o = __shfl_sync(0xffffffffu, o, 0);
+          fits = (int64_t)(o + words) <= cap;
+          off = (uint32_t)o;
+        }
+      }
+      if (lane == 0) hdr[2 * s + 1] = make_uint4(off, (uint32_t)lists, 0u, 0u);
+    }
+  }
+}

@@ -1278,8 +1278,9 @@ __device__ __forceinline__ bool pair_values(const Params &P, const CfgRec<W> &A,
 }
 
 // Slot of every pair (ordered; one warp a configuration, lanes over its list), and with VALS
-// its integrals.  drop: pairs whose integrals make the block zero get TAB_NONE.
-template <int W, bool VALS>
+// its integrals, pairs whose integrals make the block zero getting TAB_NONE.  LOWER: the pairs
+// J < I alone (the list's first; the slots of the others are not written).
+template <int W, bool VALS, bool LOWER>
 __global__ void __launch_bounds__(256) k_pair_slots(Params P, const CfgRec<W> *__restrict__ cfg,
                                                     const int64_t *__restrict__ nbroff, const int32_t *__restrict__ nbr,
                                                     uint64_t *keys, uint32_t mask, int *err, uint32_t *__restrict__ slot,
@@ -1292,6 +1293,7 @@ __global__ void __launch_bounds__(256) k_pair_slots(Params P, const CfgRec<W> *_
     const int64_t e = nbroff[I + 1];
     for (int64_t q = nbroff[I] + lane; q < e; q += 32) {
       const int J = nbr[q];
+      if (LOWER && J >= (int)I) break;
       uint32_t sl = TAB_NONE;
       double v0 = 0.0, v1 = 0.0;
       if (J == (int)I) {
@@ -2086,9 +2088,10 @@ int max_open_of(const psoci_ctx *c) {
 // Slots (and with vals the integrals) of the npairs pairs of the lists and the tables they
 // need.  ok = false: the patterns do not fit the tables and nothing is left allocated; the
 // generic kernels take the space.
+// grad: the lower pairs alone, with the tables' programs.
 template <int W>
 psoci_status tab_prepare(psoci_ctx *c, const Params &P, const int64_t *nbroff, const int32_t *nbr, int64_t npairs,
-                         bool vals, TabSet<W> &S, bool &ok) {
+                         bool vals, bool grad, TabSet<W> &S, bool &ok) {
   cudaStream_t st = c->stream;
   const int n = c->nconf;
   psoci_status s = PSOCI_OK;
@@ -2118,16 +2121,16 @@ psoci_status tab_prepare(psoci_ctx *c, const Params &P, const int64_t *nbroff, c
     if (e == cudaSuccess) e = cudaMemsetAsync(S.t.counter, 0, 2 * sizeof(unsigned long long), st);
     if (e != cudaSuccess) break;
     psoci_note_launch();
-    if (vals)
-      k_pair_slots<W, true><<<wblocks, 256, 0, st>>>(P, S.cfg, nbroff, nbr, S.t.keys, (uint32_t)(slots - 1), S.t.err,
-                                                     S.slot, S.vals);
-    else
-      k_pair_slots<W, false><<<wblocks, 256, 0, st>>>(P, S.cfg, nbroff, nbr, S.t.keys, (uint32_t)(slots - 1), S.t.err,
-                                                      S.slot, nullptr);
+    auto k = grad ? k_pair_slots<W, false, true> : vals ? k_pair_slots<W, true, false> : k_pair_slots<W, false, false>;
+    k<<<wblocks, 256, 0, st>>>(P, S.cfg, nbroff, nbr, S.t.keys, (uint32_t)(slots - 1), S.t.err, S.slot, S.vals);
     const TabBuildArgs B = {S.t.keys, slots, c->d_tmpl, c->d_tmpl_off, c->nelec, c->ksym & 1,
                             S.t.hdr, S.t.pool, S.t.counter, cap, S.t.err};
     psoci_note_launch();
     k_tab_build<<<(unsigned)((slots / 32 + TABB_WARPS - 1) / TABB_WARPS), TABB_WARPS * 32, 0, st>>>(B);
+    if (grad) {
+      psoci_note_launch();
+      k_tab_program<<<(unsigned)((slots / 32 + 3) / 4), 128, 0, st>>>(S.t.keys, slots, S.t.hdr, S.t.pool, S.t.counter, cap);
+    }
     if ((e = cudaGetLastError()) != cudaSuccess) break;
     unsigned long long back[2] = {0, 0};  // words used; error bits
     e = cudaMemcpyAsync(back, S.t.counter, sizeof(back), cudaMemcpyDeviceToHost, st);
@@ -2277,7 +2280,7 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
     TRYC(cudaMemGetInfo(&freeb, &totb));
     vals = !direct && c->eval_launches != 1 && (double)npairs * 16.0 <= 0.25 * ((double)freeb + (double)c->pool_bytes);
     TRYC(cudaEventRecord(ev[2], st));
-    TRY(tab_prepare<W>(c, P, d_nbroff, d_nbr, npairs, vals, T, fast));
+    TRY(tab_prepare<W>(c, P, d_nbroff, d_nbr, npairs, vals, false, T, fast));
   }
   auto t_c = tnow();
 
@@ -3183,8 +3186,8 @@ struct AdjRec {
   int32_t info;  // tag | (sgn < 0) << 4 | term << 8
 };
 
-// One warp per row configuration I (grid-stride); its lower neighbours J <= I in chunks of
-// 32 set up by the lanes.  Per pair: (1) lanes over the determinant pairs (x, y) test them for
+// One warp per row configuration I (grid-stride); its lower neighbours J <= I (diag_only: I
+// itself) in chunks of 32 set up by the lanes.  Per pair: (1) lanes over the determinant pairs (x, y) test them for
 // coupling and classify the coupled ones (det_adj), collecting the records in shared memory;
 // (2) lanes = (slot, root) take the records, slots over the records and roots over the lanes
 // of a slot, and add s * cd_I[x] * cd_J[y] to register accumulators of the pair's terms (v0,
@@ -3196,7 +3199,7 @@ template <int W, typename CT, typename ACC>
 __global__ void __launch_bounds__(ADJ_WARPS * 32) k_energy_grad(Params P, const int64_t *__restrict__ nbroff,
                                                                 const int32_t *__restrict__ nbr,
                                                                 const CT *__restrict__ CD, int k, double *G1,
-                                                                int64_t n1, double *G2, int64_t n2) {
+                                                                int64_t n1, double *G2, int64_t n2, bool diag_only) {
   __shared__ AdjSmem<W> sm[ADJ_WARPS];
   __shared__ AdjRec recs[ADJ_WARPS][ADJ_CONN];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -3211,10 +3214,10 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32) k_energy_grad(Params P, const 
   for (int e = lane; e < ADJ_NT * ADJ_MAXR; e += 32) (&S.acc[0][0])[e] = 0.0;
   __syncwarp();
   for (int64_t I = warp; I < P.nconf; I += nwarps) {
-    const int64_t b0 = nbroff[I], b1 = nbroff[I + 1];
+    const int64_t b0 = diag_only ? 0 : nbroff[I], b1 = diag_only ? 1 : nbroff[I + 1];
     for (int64_t c0 = b0; c0 < b1; c0 += 32) {
       const int64_t q = c0 + lane;
-      const int J = (q < b1) ? nbr[q] : INT_MAX;
+      const int J = (q < b1) ? (diag_only ? (int)I : nbr[q]) : INT_MAX;
       const bool lower = J <= (int)I;
       if (lower) adj_pair_setup<W>(P, (int)I, J, S.pi[lane]);
       const unsigned lm = __ballot_sync(0xffffffffu, lower);
@@ -3338,6 +3341,160 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32) k_energy_grad(Params P, const 
   }
 }
 
+// ------------------------------------------------------------------------------------
+// The same from coupling tables (at most TAB_MAXOPEN open shells), for the pairs J < I; the
+// diagonal blocks stay with k_energy_grad.
+// ------------------------------------------------------------------------------------
+// vectors (k per pass, root-major with stride ldv) side by side, KP a SEF (zero padded)
+template <typename CT, int KP>
+__global__ void k_grad_rows(int64_t n, const double *__restrict__ V, int64_t ldv, int k, CT *__restrict__ C) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+#pragma unroll
+    for (int q = 0; q < KP; ++q) C[i * KP + q] = q < k ? (CT)V[(int64_t)q * ldv + i] : (CT)0;
+  }
+}
+
+// G[q * n + i] += T[i * KP + q]
+template <int KP>
+__global__ void k_grad_out(int64_t n, int k, const double *__restrict__ T, double *__restrict__ G) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+#pragma unroll
+    for (int q = 0; q < KP; ++q)
+      if (q < k) G[(int64_t)q * n + i] += T[i * KP + q];
+}
+
+__device__ __forceinline__ double with_sign(double v, uint32_t x) { return flip_sign(v, x & 0x80000000u); }
+__device__ __forceinline__ float with_sign(float v, uint32_t x) {
+  return __int_as_float(__float_as_int(v) ^ (int)(x & 0x80000000u));
+}
+
+constexpr int GT_WARPS = 4;
+struct GradPair {
+  double f;          // sign, 2 (the pair's two places in H) and the pattern's constants
+  uint32_t prog;     // its program: first word
+  int lists, kind;
+  int ie, je, ex1, jy1;
+  uint32_t sefJ;
+  int B;
+};
+
+// One warp per configuration, 32 lower pairs set up at a time, KP lanes (a root each) to a pair:
+// the lists of its table's program give one sum of products c_I[row] c_J[column] an integral,
+// which goes to that integral's place in the gradient.  The sums are FP64 (CT double) or FP32
+// (float) within a pair; the places take FP64 atomics, the KP roots of one side by side (T1, T2:
+// KP a table entry).  Bound by the FP64 pipe, one FMA an entry of a list (16 clocks a warp
+// instruction an SM): mrcisd_6e8o_v16, 8 roots, 3.2 ms (determinant pair by determinant pair the
+// lower and diagonal blocks took 54.7 ms, of which the diagonal's 2.4 ms remain).
+template <int W, typename CT, int KP>
+__global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgRec<W> *__restrict__ cfg,
+                                                            const int64_t *__restrict__ nbroff,
+                                                            const int32_t *__restrict__ nbr,
+                                                            const uint32_t *__restrict__ slot,
+                                                            const uint4 *__restrict__ hdr,
+                                                            const uint32_t *__restrict__ pool,
+                                                            const CT *__restrict__ C, double *T1, double *T2) {
+  __shared__ GradPair pairs[GT_WARPS][PSOCI_SEG];
+  GradPair *gp = pairs[threadIdx.x >> 5];
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, q = lane % KP, grp = lane / KP;
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t I = warp; I < P.nconf; I += nwarps) {
+    const CfgRec<W> a = cfg[I];
+    const CT *cI = C + (int64_t)a.sef * KP + q;
+    const int64_t b1 = nbroff[I + 1];
+    for (int64_t k0 = nbroff[I]; k0 < b1; k0 += 32) {
+      const int J = (k0 + lane < b1) ? nbr[k0 + lane] : INT_MAX;
+      const bool low = J < (int)I;
+      const int np = __popc(__ballot_sync(FULL, low));  // they come first
+      if (np == 0) break;
+      if (low) {
+        const CfgRec<W> b = cfg[J];
+        const PairShape s = pair_shape<W>(a, b);
+        GradPair g;
+        g.kind = s.kind;
+        g.ie = s.ex0; g.je = s.jy0; g.ex1 = s.ex1; g.jy1 = s.jy1;
+        g.sefJ = b.sef;
+        g.B = J;
+        g.lists = 0;
+        const uint32_t sl = slot[k0 + lane];
+        if (sl != TAB_NONE) {
+          const uint4 h0 = __ldg(hdr + 2 * (size_t)(sl & ~TAB_SIGN)), h1 = __ldg(hdr + 2 * (size_t)(sl & ~TAB_SIGN) + 1);
+          g.prog = h1.x;
+          g.lists = (int)h1.y;
+          g.f = tab_scale(s.sign ? -2.0 : 2.0, h0.y);
+        }
+        gp[lane] = g;
+      }
+      __syncwarp();
+      for (int u = grp; u < np; u += 32 / KP) {
+        const GradPair &g = gp[u];
+        const CT *cJ = C + (int64_t)g.sefJ * KP + q;
+        const uint16_t *ends = reinterpret_cast<const uint16_t *>(pool + g.prog);
+        const uint32_t *pw = pool + g.prog + (TAB_LISTS + 1) / 2;
+        int e = 0;
+        for (int l = 0; l < g.lists; ++l) {
+          const int end = (int)__ldg(ends + l);
+          if (e == end) continue;
+          CT sum = 0;
+          for (; e + 2 <= end; e += 2) {
+            const uint32_t x0 = __ldg(pw + e), x1 = __ldg(pw + e + 1);
+            const CT i0 = __ldg(cI + (int)((x0 >> 8) & 0xffu) * KP), i1 = __ldg(cI + (int)((x1 >> 8) & 0xffu) * KP);
+            const CT j0 = __ldg(cJ + (int)(x0 & 0xffu) * KP), j1 = __ldg(cJ + (int)(x1 & 0xffu) * KP);
+            sum = fma(with_sign(i0, x0), j0, sum);
+            sum = fma(with_sign(i1, x1), j1, sum);
+          }
+          if (e < end) {
+            const uint32_t x0 = __ldg(pw + e);
+            sum = fma(with_sign(__ldg(cI + (int)((x0 >> 8) & 0xffu) * KP), x0), __ldg(cJ + (int)(x0 & 0xffu) * KP), sum);
+            ++e;
+          }
+          const double w = g.f * (double)sum;
+          if (g.kind == K_DOUBLE) {
+            atomicAdd(T2 + (l == 0 ? canon4(g.ie, g.je, g.ex1, g.jy1) : canon4(g.ie, g.jy1, g.ex1, g.je)) * KP + q, w);
+          } else if (g.kind == K_SO) {
+            // v = +-SO(ie, je) / 2, negated when je > ie (PsociHamiltonian.C:223-237)
+            atomicAdd(T1 + tri64(g.ie, g.je) * KP + q, (g.je > g.ie ? -0.5 : 0.5) * w);
+          } else if (l > 0) {  // X[l - 1]
+            int t = l - 1, o = 0;
+#pragma unroll
+            for (int x = 0; x < W; ++x) {
+              uint64_t m = a.e1[x] & ~a.e2[x];
+              const int n = __popcll(m);
+              if (t >= 0 && t < n) {
+                for (; t > 0; --t) m &= m - 1;
+                o = 64 * x + __ffsll((long long)m) - 1;
+                t = -1;
+              } else {
+                t -= n;
+              }
+            }
+            atomicAdd(T2 + canon4(g.ie, o, o, g.je) * KP + q, w);
+          } else {
+            // v0 = h(ie, je) - (ie je|ie ie) + sum over A's occupied p of occ (ie je|p p) less
+            // (ie p|p je) where p is doubly occupied in both (PsociHamiltonian.C:239-258)
+            atomicAdd(T1 + tri64(g.ie, g.je) * KP + q, w);
+            atomicAdd(T2 + canon4(g.ie, g.je, g.ie, g.ie) * KP + q, -w);
+#pragma unroll
+            for (int x = 0; x < W; ++x) {
+              uint64_t m = a.e1[x];
+              const uint64_t both = a.e2[x] & __ldg(&cfg[g.B].e2[x]);
+              while (m) {
+                const int bit = __ffsll((long long)m) - 1, o = 64 * x + bit;
+                m &= m - 1;
+                atomicAdd(T2 + canon4(g.ie, g.je, o, o) * KP + q, ((a.e2[x] >> bit) & 1ull) ? 2.0 * w : w);
+                if ((both >> bit) & 1ull) atomicAdd(T2 + canon4(g.ie, o, o, g.je) * KP + q, -w);
+              }
+            }
+          }
+        }
+      }
+      __syncwarp();
+      if (np < 32) break;
+    }
+  }
+}
+
 __global__ void k_fill(double *p, int64_t n, double v) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
 }
@@ -3350,6 +3507,47 @@ __global__ void k_mask_zero(const double *__restrict__ tab, int64_t n, int k, do
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     if (tab[i] == 0.0)
       for (int r = 0; r < k; ++r) G[(int64_t)r * n + i] = 0.0;
+}
+
+void grad_tabs_release(psoci_ctx *c) {
+  if (c->grad_tabs) {
+    DirTabs *d = static_cast<DirTabs *>(c->grad_tabs);
+    d->s1.free();
+    d->s2.free();
+    delete d;
+    c->grad_tabs = nullptr;
+  }
+  c->grad_generic = false;
+}
+
+// the pairs J < I of one pass of kk <= KP roots, added to G1 [kk][n1] and G2 [kk][n2]
+template <int W, int KP>
+cudaError_t grad_pass(psoci_ctx *c, const Params &P, const TabSet<W> &S, int kk, const double *V, int64_t ldv,
+                      psoci_prec prec, double *CS, double *T1, double *G1, double *G2) {
+  cudaStream_t st = c->stream;
+  const int64_t N = c->nsef_total, n1 = c->n1, n2 = c->n2;
+  double *T2 = T1 + n1 * KP;
+  cudaError_t e = cudaMemsetAsync(T1, 0, sizeof(double) * (n1 + n2) * KP, st);
+  if (e != cudaSuccess) return e;
+  const unsigned rb = (unsigned)std::min<int64_t>((N + 255) / 256, 152 * 16);
+  const unsigned gb = (unsigned)std::min<int64_t>((c->nconf + GT_WARPS - 1) / GT_WARPS, 1 << 20);
+  psoci_note_launch();
+  psoci_note_launch();
+  if (prec == PSOCI_PREC_MIXED) {
+    float *C = reinterpret_cast<float *>(CS);
+    k_grad_rows<float, KP><<<rb, 256, 0, st>>>(N, V, ldv, kk, C);
+    k_grad_tab<W, float, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, S.cfg, c->grad_nbroff, c->grad_nbr, S.slot, S.t.hdr,
+                                                           S.t.pool, C, T1, T2);
+  } else {
+    k_grad_rows<double, KP><<<rb, 256, 0, st>>>(N, V, ldv, kk, CS);
+    k_grad_tab<W, double, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, S.cfg, c->grad_nbroff, c->grad_nbr, S.slot, S.t.hdr,
+                                                            S.t.pool, CS, T1, T2);
+  }
+  psoci_note_launch();
+  psoci_note_launch();
+  k_grad_out<KP><<<(unsigned)std::min<int64_t>((n1 + 255) / 256, 152 * 8), 256, 0, st>>>(n1, kk, T1, G1);
+  k_grad_out<KP><<<(unsigned)std::min<int64_t>((n2 + 255) / 256, 152 * 8), 256, 0, st>>>(n2, kk, T2, G2);
+  return cudaGetLastError();
 }
 
 template <int W>
@@ -3370,6 +3568,7 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
   if (!c->grad_nbroff || c->grad_mode != mode) {
     psoci_free(c->grad_nbroff);
     psoci_free(c->grad_nbr);
+    grad_tabs_release(c);
     double *t1 = nullptr, *t2 = nullptr;
     if ((s = psoci_alloc(c, &t1, n1)) || (s = psoci_alloc(c, &t2, n2))) {
       psoci_free(t1);
@@ -3392,34 +3591,63 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
     c->grad_mode = mode;
     c->grad_npairs = npairs;
   }
+  // pairs J < I from coupling tables, kept with the lists; the generic kernel for spaces or
+  // patterns that the tables do not hold
+  if (!c->grad_tabs && !c->grad_generic) {
+    DirTabs *d = new DirTabs();
+    bool ok = tab_usable(c, false);
+    if (ok && (s = tab_prepare<W>(c, P, c->grad_nbroff, c->grad_nbr, c->grad_npairs, false, true, dir_set<W>(d), ok))) {
+      delete d;
+      return s;
+    }
+    if (ok) c->grad_tabs = d;
+    else delete d;
+    c->grad_generic = !ok;
+  }
+  const bool tabs = c->grad_tabs != nullptr;
   double *CD = nullptr;  // determinant-basis vectors (FP64, or FP32 for the FP32-bulk variant)
-  if ((s = psoci_alloc(c, &CD, (size_t)c->ndet_total * std::min(k, ADJ_MAXR)))) return s;
+  double *CS = nullptr, *T1 = nullptr;  // SEF-basis vectors and gradients, the roots of a pass side by side
+  auto done = [&](psoci_status r) {
+    psoci_free(CD); psoci_free(CS); psoci_free(T1);
+    return r;
+  };
+  const int kmax = std::min(k, ADJ_MAXR), kpmax = kmax <= 2 ? kmax : kmax <= 4 ? 4 : 8;
+  const int64_t N = c->nsef_total;
+  if ((s = psoci_alloc(c, &CD, (size_t)c->ndet_total * kmax))) return done(s);
+  if (tabs && ((s = psoci_alloc(c, &CS, (size_t)N * kpmax)) || (s = psoci_alloc(c, &T1, (size_t)(n1 + n2) * kpmax))))
+    return done(s);
   float *CD32 = reinterpret_cast<float *>(CD);
-  PSOCI_CUDA(c, cudaMemsetAsync(dG1, 0, sizeof(double) * n1 * k, st));
-  PSOCI_CUDA(c, cudaMemsetAsync(dG2, 0, sizeof(double) * n2 * k, st));
+  cudaError_t e = cudaMemsetAsync(dG1, 0, sizeof(double) * n1 * k, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(dG2, 0, sizeof(double) * n2 * k, st);
+  if (e != cudaSuccess) return done(psoci_cuda_fail(c, e, "energy_gradient"));
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n + ADJ_WARPS - 1) / ADJ_WARPS, 152 * 16));
   for (int r0 = 0; r0 < k; r0 += ADJ_MAXR) {
     const int kk = std::min(ADJ_MAXR, k - r0);
     const unsigned sb = (unsigned)(((int64_t)n * 32 + 255) / 256);
+    const double *V = dV + (int64_t)r0 * ldv;
     psoci_note_launch();
     if (prec == PSOCI_PREC_MIXED)
-      k_sef_to_det<float><<<sb, 256, 0, st>>>(n, c->nelec, c->ksym, c->d_sefoff, c->d_detoff, c->d_jsym, c->d_nopen,
-                                              dV + (int64_t)r0 * ldv, ldv, kk, CD32);
+      k_sef_to_det<float><<<sb, 256, 0, st>>>(n, c->nelec, c->ksym, c->d_sefoff, c->d_detoff, c->d_jsym, c->d_nopen, V,
+                                              ldv, kk, CD32);
     else
-      k_sef_to_det<double><<<sb, 256, 0, st>>>(n, c->nelec, c->ksym, c->d_sefoff, c->d_detoff, c->d_jsym, c->d_nopen,
-                                               dV + (int64_t)r0 * ldv, ldv, kk, CD);
+      k_sef_to_det<double><<<sb, 256, 0, st>>>(n, c->nelec, c->ksym, c->d_sefoff, c->d_detoff, c->d_jsym, c->d_nopen, V,
+                                               ldv, kk, CD);
     psoci_note_launch();
     if (prec == PSOCI_PREC_MIXED)
       k_energy_grad<W, float, float><<<blocks, ADJ_WARPS * 32, 0, st>>>(P, c->grad_nbroff, c->grad_nbr, CD32, kk,
-                                                                        dG1 + r0 * n1, n1, dG2 + r0 * n2, n2);
+                                                                        dG1 + r0 * n1, n1, dG2 + r0 * n2, n2, tabs);
     else
       k_energy_grad<W, double, double><<<blocks, ADJ_WARPS * 32, 0, st>>>(P, c->grad_nbroff, c->grad_nbr, CD, kk,
-                                                                          dG1 + r0 * n1, n1, dG2 + r0 * n2, n2);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-      psoci_free(CD);
-      return psoci_cuda_fail(c, e, "energy_gradient");
+                                                                          dG1 + r0 * n1, n1, dG2 + r0 * n2, n2, tabs);
+    e = cudaGetLastError();
+    if (e == cudaSuccess && tabs) {
+      const TabSet<W> &S = dir_set<W>(static_cast<DirTabs *>(c->grad_tabs));
+      e = kk <= 1 ? grad_pass<W, 1>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
+          : kk <= 2 ? grad_pass<W, 2>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
+          : kk <= 4 ? grad_pass<W, 4>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
+                    : grad_pass<W, 8>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2);
     }
+    if (e != cudaSuccess) return done(psoci_cuda_fail(c, e, "energy_gradient"));
   }
   if (mode == 1) {
     psoci_note_launch();
@@ -3427,10 +3655,9 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
     psoci_note_launch();
     k_mask_zero<<<152 * 8, 256, 0, st>>>(c->d_eri, n2, k, dG2);
   }
-  cudaError_t e = cudaStreamSynchronize(st);
-  psoci_free(CD);
-  if (e != cudaSuccess) return psoci_cuda_fail(c, e, "energy_gradient");
-  return PSOCI_OK;
+  e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return done(psoci_cuda_fail(c, e, "energy_gradient"));
+  return done(PSOCI_OK);
 }
 
 }  // namespace
@@ -3438,6 +3665,7 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
 void psoci_grad_release(psoci_ctx *c) {
   psoci_free(c->grad_nbroff);
   psoci_free(c->grad_nbr);
+  grad_tabs_release(c);
   c->grad_mode = -1;
   c->grad_npairs = 0;
 }

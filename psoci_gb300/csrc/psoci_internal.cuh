@@ -127,6 +127,8 @@ struct psoci_ctx {
   int32_t *grad_nbr = nullptr;
   int grad_mode = -1;
   int64_t grad_npairs = 0;
+  void *grad_tabs = nullptr;   // their coupling tables (hbuild.cu, DirTabs), or null
+  bool grad_generic = false;   // the tables do not hold them
 
   // step-level Davidson basis (psoci_basis_*, davidson.cu)
   struct psoci_dav_basis *basis = nullptr;

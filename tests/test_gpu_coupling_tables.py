@@ -8,7 +8,7 @@ values up to about 50: 1e-12); products add at most a row of them."""
 import numpy as np
 import pytest
 
-from helpers import check_h_against_oracle, gpu_context, small_problem
+from helpers import check_h_against_oracle, gpu_context, lower_to_full, small_problem
 
 pytestmark = pytest.mark.gpu
 
@@ -86,4 +86,38 @@ def test_tables_match_oracle(oracle_mod, name):
     c.build_hamiltonian(direct=True)
     scale = np.abs(F).sum(axis=1).max() * np.abs(X).max()
     assert np.abs(c.sigma(X) - Y).max() <= 1e-14 * scale
+    c.close()
+
+
+@pytest.mark.parametrize("name", ["open8", "open10", "open10_two_words", "open11", "pairs", "one_electron"])
+@pytest.mark.parametrize("k", [1, 3, 9])
+def test_gradient_contracts_to_the_energy(oracle_mod, name, k):
+    """c^T H c is linear in the integrals, so the gradient contracted with them is the energy of
+    each vector, with H from the oracle: 1, 3 and 9 vectors (a pass of eight and one of one); 11
+    open shells go by the generic kernel.  Elements under the 1e-8 that H keeps are in the
+    gradient and not in H: at most 1e-8 times |c|_1^2 <= 1e-8 N between the two."""
+    p = CASES[name]()
+    O = oracle_mod.Oracle(p)
+    rp, ci, va = O.build_lower(4)
+    v = np.random.default_rng(k).standard_normal((k, O.num_sefs()))
+    v /= np.linalg.norm(v, axis=1)[:, None]
+    F = lower_to_full(rp, ci, va, O.num_sefs())
+    E = np.einsum("kn,kn->k", v, (F @ v.T).T)
+    c = gpu_context(p)
+    g1, g2 = c.energy_gradient(v)
+    assert np.abs(g1 @ p.one_packed() + g2 @ p.eri - E).max() <= 1e-8 * O.num_sefs()
+    c.close()
+
+
+@pytest.mark.parametrize("k", [1, 9])
+def test_gradient_matches_oracle(oracle_mod, k):
+    """Doubly emptied and filled orbitals, entry by entry against the oracle's unit tables."""
+    p = neighbourhood(5, 4, 0, 1, 12, 7)
+    O = oracle_mod.Oracle(p)
+    v = np.random.default_rng(k).standard_normal((k, O.num_sefs()))
+    v /= np.linalg.norm(v, axis=1)[:, None]
+    r1, r2 = O.energy_gradient(v)
+    c = gpu_context(p)
+    g1, g2 = c.energy_gradient(v)
+    assert np.abs(g1 - r1).max() <= 1e-12 and np.abs(g2 - r2).max() <= 1e-12
     c.close()
