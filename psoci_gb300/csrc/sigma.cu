@@ -86,6 +86,13 @@ __device__ __forceinline__ void store_reduced_f64(double (&acc)[K], int lane, do
   if ((lane & 3) == 0 && q < K) yr[q] = tot;
 }
 
+// FP64: one warp per row.  Bound by the FP64 pipe (an FMA warp instruction every 16 clocks an SM,
+// K of them for 32 elements).  An element's row of X is read whole before its FMAs: with each
+// FMA behind its own load the pipe waited for the loads, and 8 vectors took 8.39 ms at
+// mrcisd_6e8o_v24 (3.5 ms of FMAs); now 4.04 ms, and 98 -> 78 us at 18,777 rows.  Two elements a
+// lane are in flight for 4 and 8 vectors (4.14 -> 4.04 ms); for the other widths one was faster
+// (5 vectors 2.72 against 2.80 ms, 1 vector 0.84 against 0.88 ms).  Rows packed for 256-bit loads
+// took 4.16 ms, and the packing its own time.
 template <int K>
 __global__ void __launch_bounds__(SIG_THREADS) k_spmm_f64(int64_t nrows, const int64_t *__restrict__ rowptr,
                                                           const int32_t *__restrict__ col,
@@ -95,26 +102,47 @@ __global__ void __launch_bounds__(SIG_THREADS) k_spmm_f64(int64_t nrows, const i
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  constexpr int UNR = K % 4 == 0 ? 2 : 1;
   for (int64_t r = warp; r < nrows; r += nwarps) {
     double acc[K];
 #pragma unroll
     for (int q = 0; q < K; ++q) acc[q] = 0.0;
     const int64_t e = rowptr[r + 1];
-    for (int64_t t = rowptr[r] + lane; t < e; t += 32) {
+    int64_t t = rowptr[r] + lane;
+    for (; t + 32 * (UNR - 1) < e; t += 32 * UNR) {
+      double v[UNR], xx[UNR][K];
+      int c[UNR];
+#pragma unroll
+      for (int u = 0; u < UNR; ++u) {
+        c[u] = ldg_stream(col + t + 32 * u);
+        v[u] = ldg_stream(val + t + 32 * u);
+      }
+#pragma unroll
+      for (int u = 0; u < UNR; ++u) {
+        const double *xr = x + (int64_t)c[u] * ldx;
+        if (K % 2 == 0 && vec2) {
+#pragma unroll
+          for (int q = 0; q < K; q += 2) {
+            const double2 w = __ldg(reinterpret_cast<const double2 *>(xr + q));
+            xx[u][q] = w.x;
+            xx[u][(q + 1) % K] = w.y;
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < K; ++q) xx[u][q] = __ldg(xr + q);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < UNR; ++u)
+#pragma unroll
+        for (int q = 0; q < K; ++q) acc[q] = fma(v[u], xx[u][q], acc[q]);
+    }
+    if (UNR > 1 && t < e) {
       const int c = ldg_stream(col + t);
       const double v = ldg_stream(val + t);
       const double *xr = x + (int64_t)c * ldx;
-      if (K % 2 == 0 && vec2) {
 #pragma unroll
-        for (int q = 0; q < K; q += 2) {
-          const double2 xx = __ldg(reinterpret_cast<const double2 *>(xr + q));
-          acc[q] = fma(v, xx.x, acc[q]);
-          acc[q + 1] = fma(v, xx.y, acc[q + 1]);
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < K; ++q) acc[q] = fma(v, __ldg(xr + q), acc[q]);
-      }
+      for (int q = 0; q < K; ++q) acc[q] = fma(v, __ldg(xr + q), acc[q]);
     }
     store_reduced_f64<K>(acc, lane, y + r * ldy);
   }
