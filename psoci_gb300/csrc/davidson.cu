@@ -17,7 +17,7 @@
 // (psoci_subspace_eigen, symeig.cpp), as the reference's dsygv is.
 //
 // Initial guess: the lowest eigenvectors of H on the 3072 lowest diagonal elements, found
-// by this same solver run on that dense block (a one-CTA Jacobi for blocks of at most 96).
+// by this same solver run on that block (a one-CTA Jacobi for blocks of at most 96).
 //
 // Vectors are N x ld row-major: the k entries of one SEF row are contiguous, which is
 // what the sigma kernel gathers.  All subspace arithmetic is FP64 or float-float.
@@ -90,6 +90,15 @@ __device__ __forceinline__ void ts_fma8(float (&h)[8], float (&l)[8], ts_elt<LOW
   }
 }
 
+// Blocks of k_tn: 256 rows each, at most four blocks an SM; where that leaves SMs without a block,
+// 32 rows or more each.  With 256 rows a basis of 2,044 rows ran on 8 SMs, 16.5 us a product
+// (9.9 us now).  More blocks than this make the sum over them the longer part: 608 instead of 350
+// for 89,404 rows took k_reduce_partials from 6.6 to 8.2 us.
+int ts_blocks(int64_t n) {
+  const int64_t b = std::max((n + 255) / 256, std::min<int64_t>((n + 31) / 32, 152));
+  return (int)std::min<int64_t>(std::max<int64_t>(1, b), 152 * 4);
+}
+
 // partial[blk][i*k + j] = sum over the block's rows r of A[r, a0+i] * B[r, b0+j]
 // (m <= MAX_SUB, k <= TN_MAXK).  Thread: output group g = (i, jb), the 8 outputs
 // j in [8jb, 8jb+8) of row i of C, over the rows sub, sub+S, ... of each tile; B's tile is
@@ -120,9 +129,9 @@ __global__ void __launch_bounds__(TS_THREADS) k_tn(int64_t n, const double *__re
   for (int64_t rt = r0; rt < r1; rt += TN_TILE) {
     const int rows = (int)min((int64_t)TN_TILE, r1 - rt);
 #pragma unroll 4
-    for (int e = tid; e < (TN_TILE << ksh); e += TS_THREADS) {
+    for (int e = tid; e < (rows << ksh); e += TS_THREADS) {
       const int rr = e >> ksh, j = e & (kp - 1);
-      Bs[e] = (rr < rows && j < k) ? ts_load<LOWP>(B[(rt + rr) * ldb + b0 + j]) : E{};
+      Bs[e] = j < k ? ts_load<LOWP>(B[(rt + rr) * ldb + b0 + j]) : E{};
     }
     __syncthreads();
     if (act) {
@@ -183,6 +192,7 @@ __global__ void k_reduce_partials(const double *__restrict__ partial, int nblk, 
   const int idx = blockIdx.x * 32 + lane;
   double s = 0.0;
   if (idx < nout)
+#pragma unroll 8
     for (int b = wid; b < nblk; b += 8) s += partial[(int64_t)b * nout + idx];
   red[wid][lane] = s;
   __syncthreads();
@@ -288,14 +298,6 @@ __global__ void k_residual(int64_t n, int nr, const double *__restrict__ X, cons
   }
 }
 
-__global__ void k_sum_cols(const double *partial, int nblk, int nr, double *out) {
-  int j = threadIdx.x;
-  if (j >= nr) return;
-  double s = 0.0;
-  for (int b = 0; b < nblk; ++b) s += partial[(int64_t)b * nr + j];
-  out[j] = s;
-}
-
 // T[r, c] = R[r, sel[c]] / (D[r] - theta[sel[c]]) where |D - theta| > dmin, else R.
 // The correction is a search direction (the basis is orthonormalised right after), so the
 // quotient is formed on the FP32 pipe: D - theta exactly enough in float-float (the
@@ -343,57 +345,52 @@ __global__ void k_precond(int64_t n, int nr, const double *__restrict__ R, const
 // Gram matrix S (b x b) -> upper-triangular inverse factor F (b x b'), columns of kept
 // vectors compacted, so that T * F has orthonormal columns.  Drops a column whose
 // Cholesky pivot falls below drop_tol^2 of its original norm (linear dependence).
+// One warp: lane c carries column c (each entry's sums in ascending row order, as a single thread
+// would form them; a single thread took 29 us for up to 8 columns, the warp 13 us).
 __global__ void k_cholqr_factor(const double *S, int b, const double *ref, int ldref, double drop_tol, double *F,
                                 int *nkept) {
-  __shared__ double Finv[16 * 16];
-  __shared__ int keep[16];
-  if (threadIdx.x != 0) return;
+  __shared__ double Rm[16][17], Fi[16][17];
+  const int c = threadIdx.x;  // blockDim.x == 32
+  if (c < 16)
+    for (int i = 0; i < 16; ++i) Rm[i][c] = Fi[i][c] = 0.0;
+  __syncwarp();
   // Cholesky S = R^T R with R upper; dropped columns get zero rows
-  double Rm[16][16];
-  for (int i = 0; i < b; ++i)
-    for (int j = 0; j < b; ++j) Rm[i][j] = 0.0;
-  int nk = 0;
+  unsigned keep = 0u;
   for (int j = 0; j < b; ++j) {
-    double s = S[j * b + j];
-    double orig = ref ? ref[j * ldref + j] : s;
-    for (int i = 0; i < j; ++i) s -= Rm[i][j] * Rm[i][j];
-    if (!(orig > 0.0) || s <= drop_tol * drop_tol * orig || !(s > 0.0)) {
-      keep[j] = 0;
-      continue;
-    }
-    keep[j] = 1;
-    ++nk;
-    double rjj = sqrt(s);
-    Rm[j][j] = rjj;
-    for (int c = j + 1; c < b; ++c) {
-      double t = S[j * b + c];
+    double t = 0.0;
+    if (c >= j && c < b) {
+      t = S[j * b + c];
       for (int i = 0; i < j; ++i) t -= Rm[i][j] * Rm[i][c];
-      Rm[j][c] = t / rjj;
     }
+    const double s = __shfl_sync(0xffffffffu, t, j);
+    const double orig = ref ? ref[j * ldref + j] : S[j * b + j];
+    if (!(orig > 0.0) || s <= drop_tol * drop_tol * orig || !(s > 0.0)) continue;
+    keep |= 1u << j;
+    const double rjj = sqrt(s);
+    if (c == j) Rm[j][j] = rjj;
+    else if (c > j && c < b) Rm[j][c] = t / rjj;
+    __syncwarp();
   }
   // invert the kept upper-triangular part: F = R^{-1} restricted to kept rows/cols
-  for (int i = 0; i < b * b; ++i) Finv[i] = 0.0;
-  for (int j = 0; j < b; ++j) {
-    if (!keep[j]) continue;
-    Finv[j * b + j] = 1.0 / Rm[j][j];
-    for (int i = j - 1; i >= 0; --i) {
-      if (!keep[i]) continue;
+  if (c < b && ((keep >> c) & 1u)) {
+    Fi[c][c] = 1.0 / Rm[c][c];
+    for (int i = c - 1; i >= 0; --i) {
+      if (!((keep >> i) & 1u)) continue;
       double t = 0.0;
-      for (int q = i + 1; q <= j; ++q)
-        if (keep[q]) t += Rm[i][q] * Finv[q * b + j];
-      Finv[i * b + j] = -t / Rm[i][i];
+      for (int q = i + 1; q <= c; ++q)
+        if ((keep >> q) & 1u) t += Rm[i][q] * Fi[q][c];
+      Fi[i][c] = -t / Rm[i][i];
     }
   }
+  __syncwarp();
   // compact kept columns
-  int c = 0;
-  for (int j = 0; j < b; ++j) {
-    if (!keep[j]) continue;
-    for (int i = 0; i < b; ++i) F[i * b + c] = Finv[i * b + j];
-    ++c;
+  const int nk = __popc(keep);
+  if (c < b) {
+    const bool k = (keep >> c) & 1u;
+    const int to = k ? __popc(keep & ((1u << c) - 1u)) : nk + __popc(~keep & ((1u << c) - 1u));
+    for (int i = 0; i < b; ++i) F[i * b + to] = k ? Fi[i][c] : 0.0;
   }
-  for (; c < b; ++c)
-    for (int i = 0; i < b; ++i) F[i * b + c] = 0.0;
-  *nkept = nk;
+  if (c == 0) *nkept = nk;
 }
 
 // G (ld x ld): mirror new columns [m0, m1) into rows and symmetrise the new diagonal block
@@ -526,18 +523,36 @@ __global__ void k_map_set(const int64_t *idx, int M, int32_t *map) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) map[idx[i]] = i;
 }
 
-// Hs[i*M + j] = H[idx[i], idx[j]] from the stored rows (one warp per row)
+// H[idx[i], idx[j]] from the stored rows (one warp per row): dense, Hs[i*M + j] (rp null), or in
+// CSR, cnt[i] elements a row (FILL false) placed from rp[i] on in the stored order (FILL true)
+template <bool FILL>
 __global__ void k_extract_block(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ col,
                                 const double *__restrict__ val, const int64_t *__restrict__ idx, int M,
-                                const int32_t *__restrict__ map, double *Hs) {
+                                const int32_t *__restrict__ map, double *Hs, int64_t *cnt, const int64_t *rp,
+                                int32_t *bcol, double *bval, double *diag) {
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (i >= M) return;
-  const int64_t row = idx[i];
-  for (int64_t t = rowptr[row] + lane; t < rowptr[row + 1]; t += 32) {
-    const int j = map[col[t]];
-    if (j >= 0) Hs[(int64_t)i * M + j] = val[t];
+  const int64_t row = idx[i], e = rowptr[row + 1];
+  int64_t n = FILL ? rp[i] : 0;
+  for (int64_t t0 = rowptr[row]; t0 < e; t0 += 32) {
+    const int64_t t = t0 + lane;
+    const int j = t < e ? map[col[t]] : -1;
+    if (Hs) {
+      if (j >= 0) Hs[(int64_t)i * M + j] = val[t];
+      continue;
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, j >= 0);
+    if (FILL && j >= 0) {
+      const int64_t at = n + __popc(b & ((1u << lane) - 1u));
+      const double v = val[t];
+      bcol[at] = j;
+      bval[at] = v;
+      if (j == i) diag[i] = v;
+    }
+    n += __popc(b);
   }
+  if (!FILL && !Hs && lane == 0) cnt[i] = n;
 }
 
 // V[idx[i], j] = Y[i, j]: the block's lowest eigenvectors as the first basis vectors
@@ -565,33 +580,11 @@ __global__ void k_copy_cols(int64_t n, const double *__restrict__ src, int lds, 
   }
 }
 
-// Y[i, j] = sum_l A[i*n + l] X[l*ldx + j], j < k (k <= 16): the dense guess block applied in
-// FP64.  One warp per row (lanes stride the row, coalesced), k sums reduced across lanes.
-__global__ void k_dense_mv(int n, const double *__restrict__ A, const double *__restrict__ X, int ldx,
-                           double *__restrict__ Y, int ldy, int k) {
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= n) return;
-  double acc[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) acc[j] = 0.0;
-  const double *a = A + (int64_t)i * n;
-  for (int l = lane; l < n; l += 32) {
-    const double h = a[l];
-    const double *x = X + (int64_t)l * ldx;
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (j < k) acc[j] = fma(h, x[j], acc[j]);
-  }
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    if (j >= k) break;
-    double v = acc[j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) Y[(int64_t)i * ldy + j] = v;
-  }
-}
+struct SubBlock {
+  const int64_t *rowptr;
+  const int32_t *col;
+  const double *val;
+};
 
 struct Work {
   psoci_ctx *c = nullptr;
@@ -603,9 +596,9 @@ struct Work {
   float *x32 = nullptr;
   int *sel = nullptr, *ibuf = nullptr;
   int64_t *idx = nullptr;
-  // the operator: the context's Hamiltonian, or (dense != nullptr) a dense N x N FP64 block
-  // of it, the initial guess's subproblem
-  const double *dense = nullptr;
+  // the operator: the context's Hamiltonian, or an N x N block of it in CSR, the initial
+  // guess's subproblem
+  const SubBlock *block = nullptr;
   int nblk = 0;
   int64_t rows_per_blk = 0;
   // FP32 subspace products allowed (the FP32-element phase of a mixed solve): used for the
@@ -680,10 +673,8 @@ psoci_status sigma_block(Work &w, const double *X, int ldx, double *Y, int ldy, 
   w.ev.push_back(e1);
   cudaEventRecord(e0, w.c->stream);
   psoci_status s = PSOCI_OK;
-  if (w.dense) {
-    psoci_note_launch();
-    k_dense_mv<<<(unsigned)((w.N + 7) / 8), 256, 0, w.c->stream>>>((int)w.N, w.dense, X, ldx, Y, ldy, k);
-    if (cudaGetLastError() != cudaSuccess) s = psoci_fail(w.c, PSOCI_ERR_CUDA, "davidson: guess block product");
+  if (w.block) {
+    s = psoci_csr_product(w.c, w.N, w.block->rowptr, w.block->col, w.block->val, k, X, ldx, Y, ldy);
   } else {
     s = psoci_sigma_launch(w.c, k, X, ldx, Y, ldy, prec, w.x32);
   }
@@ -861,10 +852,10 @@ psoci_status lowest_elements(psoci_ctx *c, const double *d, int64_t N, int M, st
 constexpr int GUESS_M = 3072;  // order of the initial guess's block of H (lowest diagonal elements)
 
 // The solver over an operator of order N with diagonal diag (device): the context's
-// Hamiltonian (dense == nullptr), or a dense block of it for the initial guess (inner: unit
+// Hamiltonian (block == nullptr), or a block of it for the initial guess (inner: unit
 // vectors as its own guess, no error text on non-convergence).  dX_out (device, N x nroots
 // row-major) receives the last Ritz vectors, converged or not.
-psoci_status davidson_run(psoci_ctx *c, int64_t N, const double *diag, const double *dense, const psoci_dav_opts *o,
+psoci_status davidson_run(psoci_ctx *c, int64_t N, const double *diag, const SubBlock *block, const psoci_dav_opts *o,
                           bool inner, double *evals, double *evecs, double *rnorms, psoci_dav_stats *stats,
                           double *dX_out) {
   const int nr = o->nroots;
@@ -878,7 +869,7 @@ psoci_status davidson_run(psoci_ctx *c, int64_t N, const double *diag, const dou
   if (maxsub < 2 * nr && N >= 2 * nr) return psoci_fail(c, PSOCI_ERR_INVALID_ARG, "davidson: subspace too small");
   if (o->prec != PSOCI_PREC_FP64 && o->prec != PSOCI_PREC_MIXED && o->prec != PSOCI_PREC_FF)
     return psoci_fail(c, PSOCI_ERR_INVALID_ARG, "davidson: unknown precision");
-  if (o->prec == PSOCI_PREC_MIXED && !dense && !c->d_val32 && !c->direct)
+  if (o->prec == PSOCI_PREC_MIXED && !block && !c->d_val32 && !c->direct)
     return psoci_fail(c, PSOCI_ERR_STATE, "davidson: MIXED needs PSOCI_HMODE_CSR_BOTH");
   const double rtol = o->rtol > 0 ? o->rtol : 1e-6;
   const double dmin = o->precond_min > 0 ? o->precond_min : 1e-3;
@@ -888,11 +879,11 @@ psoci_status davidson_run(psoci_ctx *c, int64_t N, const double *diag, const dou
   Work w;
   w.c = c;
   w.N = N;
-  w.dense = dense;
+  w.block = block;
   w.nr = nr;
   w.ld = (maxsub + 1) & ~1;
   const int ld = w.ld;
-  w.nblk = (int)std::min<int64_t>(std::max<int64_t>(1, (N + 255) / 256), 152 * 4);
+  w.nblk = ts_blocks(N);
   w.rows_per_blk = (N + w.nblk - 1) / w.nblk;
   psoci_status s;
   if ((s = psoci_alloc(c, &w.V, (size_t)N * ld)) || (s = psoci_alloc(c, &w.HV, (size_t)N * ld)) ||
@@ -940,17 +931,22 @@ psoci_status davidson_run(psoci_ctx *c, int64_t N, const double *diag, const dou
   } else if (!inner && !c->direct && c->d_val && M > nr) {
     // the block of H on the M lowest diagonal elements (a stored matrix), its lowest
     // eigenvectors scattered into V: a one-CTA Jacobi when it fits in shared memory, else
-    // this solver run on the dense block (FP64, residuals to 1e-4)
+    // this solver run on the block (FP64, residuals to 1e-4).  The block is as sparse as H, so it
+    // is kept in CSR: as a dense matrix its products of 8 vectors took 342 us at 3,072 rows
     int64_t *gidx = nullptr;
     int32_t *map = nullptr;
-    double *Hs = nullptr, *Ys = nullptr, *ths = nullptr, *dg = nullptr;
+    double *Hs = nullptr, *Ys = nullptr, *ths = nullptr, *dg = nullptr, *bval = nullptr;
+    int64_t *cnt = nullptr, *rp = nullptr;
+    int32_t *bcol = nullptr;
     int *jst = nullptr;
     auto release = [&]() {
       psoci_free(gidx); psoci_free(map); psoci_free(Hs); psoci_free(Ys); psoci_free(ths); psoci_free(jst);
-      psoci_free(dg);
+      psoci_free(dg); psoci_free(cnt); psoci_free(rp); psoci_free(bcol); psoci_free(bval);
     };
     const bool small = M <= MAX_SUB;
-    if ((s = psoci_alloc(c, &gidx, M)) || (s = psoci_alloc(c, &map, N)) || (s = psoci_alloc(c, &Hs, (size_t)M * M)) ||
+    if ((s = psoci_alloc(c, &gidx, M)) || (s = psoci_alloc(c, &map, N)) ||
+        (small ? (s = psoci_alloc(c, &Hs, (size_t)M * M))
+               : (s = psoci_alloc(c, &cnt, M)) || (s = psoci_alloc(c, &rp, M + 1))) ||
         (s = psoci_alloc(c, &Ys, small ? (size_t)M * M : (size_t)M * nr)) || (s = psoci_alloc(c, &ths, M)) ||
         (s = psoci_alloc(c, &jst, 1)) || (s = psoci_alloc(c, &dg, M))) {
       release();
@@ -958,12 +954,13 @@ psoci_status davidson_run(psoci_ctx *c, int64_t N, const double *diag, const dou
     }
     cudaError_t e = cudaMemcpyAsync(gidx, order.data(), sizeof(int64_t) * M, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(map, 0xff, sizeof(int32_t) * N, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(Hs, 0, sizeof(double) * M * M, st);
+    if (e == cudaSuccess && small) e = cudaMemsetAsync(Hs, 0, sizeof(double) * M * M, st);
     if (e == cudaSuccess) {
       psoci_note_launch();
       k_map_set<<<(M + 127) / 128, 128, 0, st>>>(gidx, M, map);
       psoci_note_launch();
-      k_extract_block<<<(M + 7) / 8, 256, 0, st>>>(c->d_rowptr, c->d_col, c->d_val, gidx, M, map, Hs);
+      k_extract_block<false><<<(M + 7) / 8, 256, 0, st>>>(c->d_rowptr, c->d_col, c->d_val, gidx, M, map, Hs, cnt,
+                                                          nullptr, nullptr, nullptr, nullptr);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess && small) {
@@ -973,17 +970,25 @@ psoci_status davidson_run(psoci_ctx *c, int64_t N, const double *diag, const dou
       k_scatter_guess<<<1, 256, 0, st>>>(Ys, M, gidx, M, nr, w.V, ld);
       e = cudaGetLastError();
     } else if (e == cudaSuccess) {
-      // diagonal of the block (stride M + 1), then the inner solve
-      e = cudaMemcpy2DAsync(dg, sizeof(double), Hs, sizeof(double) * (M + 1), sizeof(double), M,
-                            cudaMemcpyDeviceToDevice, st);
+      // the block and its diagonal, then the inner solve
+      int64_t bnnz = 0;
+      if ((s = psoci_scan_i64(c, cnt, rp, M, &bnnz)) || (s = psoci_alloc(c, &bcol, bnnz)) || (s = psoci_alloc(c, &bval, bnnz))) {
+        release();
+        return s;
+      }
+      psoci_note_launch();
+      k_extract_block<true><<<(M + 7) / 8, 256, 0, st>>>(c->d_rowptr, c->d_col, c->d_val, gidx, M, map, nullptr, nullptr,
+                                                         rp, bcol, bval, dg);
+      e = cudaGetLastError();
       if (e == cudaSuccess) {
+        const SubBlock sub = {rp, bcol, bval};
         psoci_dav_opts oi = *o;
         oi.rtol = 1e-4;
         oi.prec = PSOCI_PREC_FP64;
         oi.refine = 0;
         oi.block = 1;
         oi.max_iter = 100;
-        const psoci_status si = davidson_run(c, M, dg, Hs, &oi, true, nullptr, nullptr, nullptr, nullptr, Ys);
+        const psoci_status si = davidson_run(c, M, dg, &sub, &oi, true, nullptr, nullptr, nullptr, nullptr, Ys);
         if (si != PSOCI_OK && si != PSOCI_ERR_NOT_CONVERGED) {
           release();
           return si;
@@ -1035,7 +1040,7 @@ psoci_status davidson_run(psoci_ctx *c, int64_t N, const double *diag, const dou
     psoci_note_launch();
     k_residual<<<rb, 256, 0, st>>>(N, nr, w.X, w.HX, w.theta, w.R, w.partial);
     psoci_note_launch();
-    k_sum_cols<<<1, 32, 0, st>>>(w.partial, rb, nr, w.norms);
+    k_reduce_partials<<<1, 256, 0, st>>>(w.partial, rb, 1, nr, w.norms, nr, 0);
     PSOCI_CUDA(c, cudaGetLastError());
     PSOCI_CUDA(c, cudaMemcpyAsync(h_norm.data(), w.norms, sizeof(double) * nr, cudaMemcpyDeviceToHost, st));
     PSOCI_CUDA(c, cudaStreamSynchronize(st));
@@ -1276,7 +1281,7 @@ psoci_status psoci_basis_create(psoci_ctx *c, int nroots, int max_vectors) {
   w.nr = nroots;
   w.ld = (max_vectors + 1) & ~1;
   const int ld = w.ld;
-  w.nblk = (int)std::min<int64_t>(std::max<int64_t>(1, (N + 255) / 256), 152 * 4);
+  w.nblk = ts_blocks(N);
   w.rows_per_blk = (N + w.nblk - 1) / w.nblk;
   psoci_status s;
   if ((s = psoci_alloc(c, &w.V, (size_t)N * ld)) || (s = psoci_alloc(c, &w.HV, (size_t)N * ld)) ||
@@ -1463,7 +1468,7 @@ psoci_status basis_residual(psoci_ctx *c, int j, double *nrm2) {
   psoci_note_launch();
   k_residual_col<<<rb, 256, 0, c->stream>>>(b->N, nr, j, w.X, w.HX, w.theta + j, w.R, w.partial);
   psoci_note_launch();
-  k_sum_cols<<<1, 32, 0, c->stream>>>(w.partial, rb, 1, w.norms);
+  k_reduce_partials<<<1, 256, 0, c->stream>>>(w.partial, rb, 1, 1, w.norms, 1, 0);
   PSOCI_CUDA(c, cudaGetLastError());
   PSOCI_CUDA(c, cudaMemcpyAsync(nrm2, w.norms, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   PSOCI_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1723,7 +1728,7 @@ extern "C" psoci_status psoci_tsprod(psoci_ctx *c, int method, int64_t n, const 
     Work w;
     w.c = c;
     w.N = n;
-    w.nblk = (int)std::min<int64_t>(std::max<int64_t>(1, (n + 255) / 256), 152 * 4);
+    w.nblk = ts_blocks(n);
     w.rows_per_blk = (n + w.nblk - 1) / w.nblk;
     if ((s = psoci_alloc(c, &w.partial, (size_t)w.nblk * MAX_SUB * TN_MAXK))) return s;
     s = tn(w, dA, lda, 0, m, dB, ldb, 0, k, dC, k, 0);

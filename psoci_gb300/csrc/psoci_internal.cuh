@@ -212,6 +212,9 @@ psoci_status psoci_scan_i64(psoci_ctx *c, const int64_t *d_in, int64_t *d_out, i
 psoci_status psoci_sigma_launch(psoci_ctx *c, int k, const double *dX, int ldx, double *dY, int ldy,
                                 psoci_prec prec, float *dX32);
 
+psoci_status psoci_csr_product(psoci_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *col, const double *val,
+                               int k, const double *dX, int ldx, double *dY, int ldy);
+
 psoci_status psoci_sigma_autotune_run(psoci_ctx *c, int k, int *choice, float *times_ms);
 
 // determinant templates (dets.cu)

@@ -364,6 +364,16 @@ __global__ void k_to_f32(int64_t n, int k, const double *__restrict__ x, int ldx
   }
 }
 
+bool rows_vec2(const double *x, int ldx) { return ((uintptr_t)x % 16 == 0) && (ldx % 2 == 0); }
+
+template <int K>
+void launch_f64(psoci_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *col, const double *val, const double *dX,
+                int ldx, double *dY, int ldy) {
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n * 32 + SIG_THREADS - 1) / SIG_THREADS, 152 * 8 * 4));
+  psoci_note_launch();
+  k_spmm_f64<K><<<blocks, SIG_THREADS, 0, c->stream>>>(n, rowptr, col, val, dX, ldx, dY, ldy, rows_vec2(dX, ldx));
+}
+
 template <int K>
 void launch_k(psoci_ctx *c, int64_t n, const double *dX, int ldx, double *dY, int ldy, psoci_prec prec,
               const float *x32, int ld32) {
@@ -373,7 +383,7 @@ void launch_k(psoci_ctx *c, int64_t n, const double *dX, int ldx, double *dY, in
   psoci_note_launch();
   if (prec == PSOCI_PREC_FP64)
     k_spmm_f64<K><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val, dX, ldx, dY, ldy,
-                                                         ((uintptr_t)dX % 16 == 0) && (ldx % 2 == 0));
+                                                         rows_vec2(dX, ldx));
   else if (prec == PSOCI_PREC_FF)
     k_spmm_ff<K><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val,
                                                         reinterpret_cast<const float2 *>(x32), dY, ldy);
@@ -444,6 +454,27 @@ psoci_status psoci_sigma_launch(psoci_ctx *c, int k, const double *dX, int ldx, 
       case 6: launch_k<6>(c, n, xs, ldx, ys, ldy, prec, x32, 6); break;
       case 7: launch_k<7>(c, n, xs, ldx, ys, ldy, prec, x32, 7); break;
       default: launch_k<8>(c, n, xs, ldx, ys, ldy, prec, x32, 8); break;
+    }
+    PSOCI_CUDA(c, cudaGetLastError());
+  }
+  return PSOCI_OK;
+}
+
+// Y = A X for a square CSR matrix A of n rows, k vectors, FP64
+psoci_status psoci_csr_product(psoci_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *col, const double *val,
+                               int k, const double *dX, int ldx, double *dY, int ldy) {
+  for (int q0 = 0; q0 < k; q0 += 8) {
+    const double *x = dX + q0;
+    double *y = dY + q0;
+    switch (std::min(8, k - q0)) {
+      case 1: launch_f64<1>(c, n, rowptr, col, val, x, ldx, y, ldy); break;
+      case 2: launch_f64<2>(c, n, rowptr, col, val, x, ldx, y, ldy); break;
+      case 3: launch_f64<3>(c, n, rowptr, col, val, x, ldx, y, ldy); break;
+      case 4: launch_f64<4>(c, n, rowptr, col, val, x, ldx, y, ldy); break;
+      case 5: launch_f64<5>(c, n, rowptr, col, val, x, ldx, y, ldy); break;
+      case 6: launch_f64<6>(c, n, rowptr, col, val, x, ldx, y, ldy); break;
+      case 7: launch_f64<7>(c, n, rowptr, col, val, x, ldx, y, ldy); break;
+      default: launch_f64<8>(c, n, rowptr, col, val, x, ldx, y, ldy); break;
     }
     PSOCI_CUDA(c, cudaGetLastError());
   }
