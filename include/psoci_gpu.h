@@ -110,7 +110,9 @@ PSOCI_API psoci_status psoci_get_determinants(const psoci_ctx *ctx, uint64_t *al
  * PSOCI_HMODE_DIRECT stands in for the reference's direct products
  * (matrixVectorProductsSplitChunkMultipleJchunksLowLevelAccumulateDirectFetch,
  * PsociGAhamiltonian.C:7549-7826, built with DIRECTMATRIXPRODUCTS): only the screened
- * neighbour lists and the diagonal are kept (*nnz = 0); psoci_sigma / psoci_sigma_device /
+ * neighbour lists with their coupling tables, the diagonal blocks and, where they take at most a
+ * quarter of the device memory at hand, the pairs' integrals (16 bytes a pair) are kept (*nnz =
+ * 0); psoci_sigma / psoci_sigma_device /
  * psoci_davidson then evaluate every element again on each call, in FP64 whatever the
  * precision asked for, applying the same |x| >= 1e-8 rule.  psoci_get_hamiltonian,
  * psoci_save_hamiltonian and psoci_sigma_mixed_noalloc answer PSOCI_ERR_STATE. */

@@ -25,7 +25,11 @@
 constexpr int TAB_MAXOPEN = 10;        // open shells a configuration may have (256 SEFs)
 constexpr int TAB_MAXDET = 512;        // determinants of 10 open shells
 constexpr int TAB_SYMS = 12;           // orbitals of a pattern
-constexpr uint32_t TAB_SIGN = 0x80000000u;  // of a pair's slot: the stripped doubles' sign
+// a pair's slot: the table, the forms v0, v1, v0 - v1 that pass the threshold of storage (listed
+// pairs only) and the stripped doubles' sign
+constexpr uint32_t TAB_SLOT = 0x01ffffffu;
+constexpr int TAB_KEPT = 26;
+constexpr uint32_t TAB_SIGN = 0x80000000u;
 constexpr uint32_t TAB_DIAG = 0x7ffffffeu;  // slot of a configuration with itself
 constexpr uint32_t TAB_NONE = 0x7fffffffu;  // slot of a pair whose block is zero
 

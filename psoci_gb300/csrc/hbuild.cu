@@ -1213,9 +1213,9 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32) k_hbuild(Params P) {
 //   MODE 2  multiplies them with X (direct mode), MODE 3 with X in FP32.
 // Both triangles are evaluated: an element costs so little that reading its pair twice is cheaper
 // than mirroring it.  mrcisd_6e8o_v48 (2.18 million SEFs, 1.25e9 elements): pair slots, tables and
-// diagonal 10.7 ms, count 6.9 ms, fill 17.5 ms (12.5 GB of CSR: 1.9 ms at the copy rate), where
+// diagonal 8.7 ms, count 6.2 ms, fill 17.0 ms (20 GB of CSR: 3 ms at the copy rate), where
 // evaluating the lower triangle determinant by determinant, counting its mirror image and
-// assembling the rows took 98 + 7 + 27 ms; 31,650 SEFs with up to 8 open shells: 14.6 -> 2.1 ms.
+// assembling the rows took 98 + 7 + 27 ms; 31,650 SEFs with up to 8 open shells: 14.6 -> 2.0 ms.
 // ------------------------------------------------------------------------------------
 template <int W>
 __global__ void k_cfg_rec(Params P, CfgRec<W> *__restrict__ out) {
@@ -1232,6 +1232,24 @@ __global__ void k_cfg_rec(Params P, CfgRec<W> *__restrict__ out) {
     r.pad = 0u;
     out[i] = r;
   }
+}
+
+// Rounding to FP32 on the integer pipe (round to nearest even; values outside FP32's normal
+// range by the conversion instruction, which shares the narrow FP64 pipe).
+__device__ __forceinline__ float f32_of(double v) {
+  const uint32_t hi = (uint32_t)__double2hiint(v);
+  const uint64_t a = ((uint64_t)(hi & 0x7fffffffu) << 32) | (uint32_t)__double2loint(v);
+  const uint64_t r = (a + 0x0fffffffull + ((a >> 29) & 1ull)) >> 29;  // 11 exponent bits, 23 mantissa bits
+  const uint64_t f = r - (896ull << 23);
+  if (f - 0x00800000ull >= 0x7f000000ull) return (float)v;
+  return __uint_as_float((uint32_t)f | (hi & 0x80000000u));
+}
+// |v| >= PSOCI_MIN_VALUE (not NaN) by its bits, word by word: masking the sign of the 64-bit
+// pattern compiles to an FP64 absolute value
+__device__ __forceinline__ bool kept_value(double v) {
+  const uint64_t a = ((uint64_t)((uint32_t)__double2hiint(v) & 0x7fffffffu) << 32) | (uint32_t)__double2loint(v);
+  constexpr uint64_t lo = 0x3e45798ee2308c3aull, inf = 0x7ff0000000000000ull;  // the bits of 1e-8
+  return a - lo <= inf - lo;
 }
 
 __device__ __forceinline__ bool is_zero(double v) { return ((uint64_t)__double_as_longlong(v) << 1) == 0ull; }
@@ -1279,21 +1297,60 @@ __device__ __forceinline__ bool pair_values(const Params &P, const CfgRec<W> &A,
 
 // Slot of every pair (ordered; one warp a configuration, lanes over its list), and with VALS
 // its integrals, pairs whose integrals make the block zero getting TAB_NONE.  LOWER: the pairs
-// J < I alone (the list's first; the slots of the others are not written).
+// J < I alone (the list's first; the slots of the others are not written).  The sum over occupied
+// orbitals of a single's integral is the longest part and one pair in twenty has it, so a
+// configuration's singles are set aside and summed by full warps (evaluated where they came up:
+// 7.4 ms at mrcisd_6e8o_v48, now 6.5 ms, of it 0.6 ms for the kept-form bits that the count reads; bound by integer issue).
 template <int W, bool VALS, bool LOWER>
 __global__ void __launch_bounds__(256) k_pair_slots(Params P, const CfgRec<W> *__restrict__ cfg,
                                                     const int64_t *__restrict__ nbroff, const int32_t *__restrict__ nbr,
                                                     uint64_t *keys, uint32_t mask, int *err, uint32_t *__restrict__ slot,
                                                     double2 *__restrict__ vals) {
-  const int lane = threadIdx.x & 31;
+  __shared__ int64_t s_q[8][64];   // singles set aside: place in the lists ...
+  __shared__ uint32_t s_m[8][64];  // ... ie | je << 8 | J > I << 16 | sign
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t I = warp; I < P.nconf; I += nwarps) {
     const CfgRec<W> a = cfg[I];
     const int64_t e = nbroff[I + 1];
-    for (int64_t q = nbroff[I] + lane; q < e; q += 32) {
-      const int J = nbr[q];
-      if (LOWER && J >= (int)I) break;
+    int ns = 0;  // singles set aside
+    auto sum_singles = [&](int n) {
+      __syncwarp();
+      if (lane < n) {
+        const int64_t q = s_q[wib][lane];
+        const uint32_t m = s_m[wib][lane];
+        const CfgRec<W> b = cfg[nbr[q]];
+        const bool up = (m >> 16) & 1u;
+        CfgRec<W> A, B;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          A.e1[w] = up ? b.e1[w] : a.e1[w]; A.e2[w] = up ? b.e2[w] : a.e2[w];
+          B.e2[w] = up ? a.e2[w] : b.e2[w];
+        }
+        const PairShape s{K_SINGLE, (int)(m & 0xffu), -1, (int)((m >> 8) & 0xffu), -1, m & TAB_SIGN};
+        double v0, v1;
+        if (!pair_values<W>(P, A, B, s, v0, v1)) slot[q] = TAB_NONE;
+        vals[q] = make_double2(v0, v1);
+      }
+      __syncwarp();
+      if (lane < ns - n) {  // the rest moves up (at most 32)
+        const int64_t q = s_q[wib][lane + n];
+        const uint32_t m = s_m[wib][lane + n];
+        s_q[wib][lane] = q;
+        s_m[wib][lane] = m;
+      }
+      ns -= n;
+      __syncwarp();
+    };
+    for (int64_t q0 = nbroff[I]; q0 < e; q0 += 32) {
+      const int64_t q = q0 + lane;
+      const int J = q < e ? nbr[q] : INT_MAX;
+      const bool in = LOWER ? J < (int)I : q < e;
+      if (LOWER && __ballot_sync(0xffffffffu, in) == 0u) break;
+      bool single = false;
+      uint32_t meta = 0u;
+      if (in) {
       uint32_t sl = TAB_NONE;
       double v0 = 0.0, v1 = 0.0;
       if (J == (int)I) {
@@ -1311,28 +1368,53 @@ __global__ void __launch_bounds__(256) k_pair_slots(Params P, const CfgRec<W> *_
         B.flags = up ? a.flags : b.flags; B.jsym = up ? a.jsym : b.jsym;
         const PairShape s = pair_shape<W>(A, B);
         bool any = s.kind != K_NONE;
-        if (VALS && any) any = pair_values<W>(P, A, B, s, v0, v1);
+        single = VALS && s.kind == K_SINGLE;
+        meta = (uint32_t)s.ex0 | ((uint32_t)s.jy0 << 8) | ((uint32_t)up << 16) | s.sign;
+        if (VALS && any && !single) any = pair_values<W>(P, A, B, s, v0, v1);
         if (any) {
           sl = tab_insert(keys, mask, pair_key<W>(A, B, s.kind, up), err);
           if (sl != TAB_NONE) sl |= s.sign;
+          if (VALS && !single && sl != TAB_NONE) {
+            const uint32_t oa = A.flags & 15u, ob = B.flags & 15u;
+            const uint32_t fc = (P.nelec & 1) ? 0u : ((oa ? 2u : 0u) | (ob ? 1u : 0u)) << TAB_FACTORS;
+            sl |= (kept_value(tab_scale(v0, fc)) ? 1u : 0u) << TAB_KEPT;
+            if (s.kind == K_DOUBLE)
+              sl |= ((kept_value(tab_scale(v1, fc)) ? 2u : 0u) | (kept_value(tab_scale(v0 - v1, fc)) ? 4u : 0u)) << TAB_KEPT;
+          }
         }
       }
       slot[q] = sl;
-      if (VALS) vals[q] = make_double2(v0, v1);
+      if (VALS && !single) vals[q] = make_double2(v0, v1);
+      }
+      if (VALS) {
+        const unsigned sb = __ballot_sync(0xffffffffu, single);
+        if (sb) {
+          if (single) {
+            const int at = ns + __popc(sb & ((1u << lane) - 1u));
+            s_q[wib][at] = q;
+            s_m[wib][at] = meta;
+          }
+          ns += __popc(sb);
+          if (ns >= 32) sum_singles(32);
+        }
+      }
     }
+    if (VALS && ns > 0) sum_singles(ns);
   }
 }
 
 // Diagonal blocks: D[(sef r) * ldd + t], the lower half as the reference computes it and its
 // mirror image, and the diagonal.  One warp a configuration: the diagonal's integral sums with
 // their loads spread over the lanes and added in the reference's order, then lanes over the
-// elements.
+// elements that can differ from zero (all of them evaluated: 3.2 ms at mrcisd_6e8o_v48, now
+// 2.1 ms).
 constexpr int DG_WARPS = 4;
 template <int W>
 __global__ void __launch_bounds__(DG_WARPS * 32) k_diag_blocks(Params P, int ldd, double *__restrict__ D,
                                                                double *__restrict__ diag) {
   __shared__ PairInfo spi[DG_WARPS];
   __shared__ double sK[DG_WARPS][MAXK];
+  __shared__ uint16_t list[DG_WARPS][64];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1409,34 +1491,55 @@ __global__ void __launch_bounds__(DG_WARPS * 32) k_diag_blocks(Params P, int ldd
       for (int w = 0; w < W; ++w) pi.SA[w] = so[w];
     }
     __syncwarp();
-    for (int e = lane; e < nsef * nsef; e += 32) {
-      const int r = e / nsef, t = e - r * nsef;
-      if (t > r) continue;
-      const double x = sef_elem<W>(P, pi, Kd, r, t);
-      D[(row0 + r) * ldd + t] = x;
-      if (t != r) D[(row0 + t) * ldd + r] = x;
-      else diag[row0 + r] = x;
+    // elements whose determinants couple (at most one alpha and one beta move apart, equal alpha
+    // counts), gathered 32 at a time; the others are zero
+    const bool open2 = !(P.nelec & 1) && nop != 0;
+    const int64_t d0 = P.detoff[I];
+    int n = 0;
+    auto eval = [&](int m) {
+      __syncwarp();
+      if (lane < m) {
+        const int r = list[wib][lane] >> 8, t = list[wib][lane] & 255;
+        const double x = sef_elem<W>(P, pi, Kd, r, t);
+        D[(row0 + r) * ldd + t] = x;
+        if (t != r) D[(row0 + t) * ldd + r] = x;
+        else diag[row0 + r] = x;
+      }
+      __syncwarp();
+      if (lane < n - m) list[wib][lane] = list[wib][lane + m];
+      n -= m;
+      __syncwarp();
+    };
+    const int lg = __ffs(nsef) - 1;  // a power of two
+    for (int e0 = 0; e0 < nsef << lg; e0 += 32) {
+      const int e = e0 + lane, r = e >> lg, t = e & (nsef - 1);
+      bool couple = false;
+      if (e < nsef << lg && t <= r) {
+        for (int x = 0; x <= (int)open2; ++x) {  // the first column determinant: the second pairs are its flips
+          int na = 0, nb = 0, ca = 0;
+          const int64_t ia = d0 + (open2 ? 2 * r + x : r), ib = d0 + (open2 ? 2 * t : t);
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            const uint64_t aa = P.alpha[ia * W + w], ab = P.alpha[ib * W + w];
+            na += __popcll(ab & ~aa);
+            ca += __popcll(aa & ~ab);
+            nb += __popcll(P.beta[ib * W + w] & ~P.beta[ia * W + w]);
+          }
+          couple |= na == ca && na <= 1 && nb <= 1;
+        }
+        if (!couple) {
+          D[(row0 + r) * ldd + t] = 0.0;
+          D[(row0 + t) * ldd + r] = 0.0;
+        }
+      }
+      const unsigned cb = __ballot_sync(0xffffffffu, couple);
+      if (couple) list[wib][n + __popc(cb & ((1u << lane) - 1u))] = (uint16_t)((r << 8) | t);
+      n += __popc(cb);
+      if (n >= 32) eval(32);
     }
+    if (n > 0) eval(n);
     __syncwarp();
   }
-}
-
-// Rounding to FP32 on the integer pipe (round to nearest even; values outside FP32's normal
-// range by the conversion instruction, which shares the narrow FP64 pipe).
-__device__ __forceinline__ float f32_of(double v) {
-  const uint32_t hi = (uint32_t)__double2hiint(v);
-  const uint64_t a = ((uint64_t)(hi & 0x7fffffffu) << 32) | (uint32_t)__double2loint(v);
-  const uint64_t r = (a + 0x0fffffffull + ((a >> 29) & 1ull)) >> 29;  // 11 exponent bits, 23 mantissa bits
-  const uint64_t f = r - (896ull << 23);
-  if (f - 0x00800000ull >= 0x7f000000ull) return (float)v;
-  return __uint_as_float((uint32_t)f | (hi & 0x80000000u));
-}
-// |v| >= PSOCI_MIN_VALUE (not NaN) by its bits, word by word: masking the sign of the 64-bit
-// pattern compiles to an FP64 absolute value
-__device__ __forceinline__ bool kept_value(double v) {
-  const uint64_t a = ((uint64_t)((uint32_t)__double2hiint(v) & 0x7fffffffu) << 32) | (uint32_t)__double2loint(v);
-  constexpr uint64_t lo = 0x3e45798ee2308c3aull, inf = 0x7ff0000000000000ull;  // the bits of 1e-8
-  return a - lo <= inf - lo;
 }
 
 // Per warp, followed by X (ms doubles a pair) and, MODE 0 and 1, an int32 a row (count, write
@@ -1556,14 +1659,18 @@ __global__ void __launch_bounds__(EL_WARPS * 32) k_elems(Params P, ElemArgs<W> E
         pr.x = EL_DIAG;
         pr.y = (uint32_t)row0;
       } else if (sl != TAB_NONE) {
-        const uint4 h = __ldg(E.hdr + 2 * (size_t)(sl & ~TAB_SIGN));
+        const uint4 h = __ldg(E.hdr + 2 * (size_t)(sl & TAB_SLOT));
         single = ((h.y >> TAB_KIND) & 7u) == K_SINGLE;
+        two = !single && (h.y >> (TAB_FORMS + 3)) != 0u;
+        const bool counted = MODE == 0 && !single && !two && !(h.y & TAB_NOCOUNTS);  // by the table's rows alone
 #pragma unroll
         for (int w = 0; w < W; ++w) sa[w] = a.e1[w] & ~a.e2[w];
         if (VALS) {
-          const double2 v = __ldg(E.vals + k0 + lane);
-          v0 = v.x;
-          v1 = v.y;
+          if (!counted) {
+            const double2 v = __ldg(E.vals + k0 + lane);
+            v0 = v.x;
+            v1 = v.y;
+          }
           if (MODE != 0) pr.y = __ldg(&E.cfg[J].sef);
           if (single && J > (int)I) {
 #pragma unroll
@@ -1593,19 +1700,20 @@ __global__ void __launch_bounds__(EL_WARPS * 32) k_elems(Params P, ElemArgs<W> E
         if (single) {
           pr.x |= EL_SUMS;
         } else {
-          const uint32_t forms = (h.y >> TAB_FORMS) & 0xfffu;
-          f0 = tab_scale(v0, h.y);
-          if (forms & ~1u) {  // more than v0 in use
-            f1 = tab_scale(v1, h.y);
-            f2 = tab_scale(v0 - v1, h.y);
+          uint32_t keep = (sl >> TAB_KEPT) & 7u;
+          if (!VALS || !counted) {
+            f0 = tab_scale(v0, h.y);
+            if ((h.y >> TAB_FORMS) & 0xffeu) {  // more than v0 in use
+              f1 = tab_scale(v1, h.y);
+              f2 = tab_scale(v0 - v1, h.y);
+            }
+            if (!VALS) keep = (kept_value(f0) ? 1u : 0u) | (kept_value(f1) ? 2u : 0u) | (kept_value(f2) ? 4u : 0u);
           }
-          const uint32_t keep = (kept_value(f0) ? 1u : 0u) | (kept_value(f1) ? 2u : 0u) | (kept_value(f2) ? 4u : 0u);
           pr.x |= keep << EL_KEPT;
-          two = (forms >> 3) != 0u;
           if (two) pr.x |= EL_SUMS;
-          if (MODE == 0 && !two && !(h.y & TAB_NOCOUNTS)) {
+          if (counted) {
             c = 0;
-            const uint4 h2 = __ldg(E.hdr + 2 * (size_t)(sl & ~TAB_SIGN) + 1);
+            const uint4 h2 = __ldg(E.hdr + 2 * (size_t)(sl & TAB_SLOT) + 1);
             const uint64_t m = 0x000f000f000f000full;
             const uint64_t n1 = (uint64_t)h2.x | ((uint64_t)h2.y << 32), n2 = (uint64_t)h2.z | ((uint64_t)h2.w << 32);
             const uint64_t nib = ((keep & 1u) ? rows - n1 - n2 : 0ull) + ((keep & 2u) ? n1 : 0ull) + ((keep & 4u) ? n2 : 0ull);
@@ -1687,20 +1795,35 @@ __global__ void __launch_bounds__(EL_WARPS * 32) k_elems(Params P, ElemArgs<W> E
       if (cg > 0) ws.run[__popc(nzg & lt)] = make_uint2(ent0 - (uint32_t)st, (uint32_t)me);
       ent0 += (uint32_t)cg;
       __syncwarp();
+      // an element's run (by the runs that start at or below it), pair and entry, fetched a pass ahead
       int started = 0;
+      uint2 run_n = make_uint2(0u, 0u);
+      uint4 q_n = make_uint4(0u, 0u, 0u, 0u);
+      uint32_t ent_n = 0u;
+      auto fetch = [&](int e0) {
+        const unsigned bw = __reduce_or_sync(FULL, (cg > 0 && (unsigned)(st - e0) < 32u) ? 1u << ((st - e0) & 31) : 0u);
+        if (e0 + lane < T) {
+          run_n = ws.run[started + __popc(bw & le) - 1];
+          q_n = ws.pair[run_n.y];
+          if (!(q_n.x & EL_DIAG)) ent_n = __ldg(E.pool + (run_n.x + (uint32_t)(e0 + lane)));
+        }
+        started += __popc(bw);
+      };
+      if (MODE != 0 && T > 0) fetch(0);
       for (int e0 = 0; e0 < T; e0 += 32) {
         const int e = e0 + lane;
-        // runs starting in this pass, and with them this element's run
-        const unsigned bw = __reduce_or_sync(FULL, (cg > 0 && (unsigned)(st - e0) < 32u) ? 1u << ((st - e0) & 31) : 0u);
+        if (MODE == 0) fetch(e0);  // few passes: not worth the registers
+        const uint2 run = run_n;
+        const uint4 q = q_n;
+        const uint32_t ent = ent_n;
+        if (MODE != 0 && e0 + 32 < T) fetch(e0 + 32);
         bool keep = false;
         double v = 0.0;
         float v32 = 0.f;
         int r = 0;
         uint32_t col = 0u;
         if (e < T) {
-          const uint2 run = ws.run[started + __popc(bw & le) - 1];
           const int p = (int)run.y;
-          const uint4 q = ws.pair[p];
           const uint32_t at = run.x + (uint32_t)e;
           if (q.x & EL_DIAG) {
             const int b = (int)at, t = b & (nsefI - 1);
@@ -1710,7 +1833,6 @@ __global__ void __launch_bounds__(EL_WARPS * 32) k_elems(Params P, ElemArgs<W> E
             keep = t == r || kept_value(v);
             col = q.y + (uint32_t)t;
           } else {
-            const uint32_t ent = __ldg(E.pool + at);
             const int f = (int)(ent >> 8) & 15;
             col = q.y + (ent & 0xffu);
             r = (int)(ent >> 12) & 0xff;
@@ -1727,7 +1849,6 @@ __global__ void __launch_bounds__(EL_WARPS * 32) k_elems(Params P, ElemArgs<W> E
             }
           }
         }
-        started += __popc(bw);
         if (MODE < 2) {
           unsigned same = __ballot_sync(FULL, keep);  // the kept elements of this one's row
 #pragma unroll
@@ -2278,7 +2399,7 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
     // memory there is, evaluated in each element launch otherwise
     size_t freeb = 0, totb = 0;
     TRYC(cudaMemGetInfo(&freeb, &totb));
-    vals = !direct && c->eval_launches != 1 && (double)npairs * 16.0 <= 0.25 * ((double)freeb + (double)c->pool_bytes);
+    vals = c->eval_launches != 1 && (double)npairs * 16.0 <= 0.25 * ((double)freeb + (double)c->pool_bytes);
     TRYC(cudaEventRecord(ev[2], st));
     TRY(tab_prepare<W>(c, P, d_nbroff, d_nbr, npairs, vals, false, T, fast));
   }
@@ -2488,9 +2609,9 @@ psoci_status run_direct_sigma(psoci_ctx *c, int k, const double *dX, int ldx, do
       psoci_note_launch();
       k_direct_x32<<<(unsigned)std::min<int64_t>((N + 255) / 256, 152 * 16), 256, 0, st>>>(N, P.kvec, P.dx, ldx, x32);
       P.dx32 = x32;
-      if ((s = elems_launch<W, 3, false>(c, P, E))) return s;
+      if ((s = E.vals ? elems_launch<W, 3, true>(c, P, E) : elems_launch<W, 3, false>(c, P, E))) return s;
     } else if (fast) {
-      if ((s = elems_launch<W, 2, false>(c, P, E))) return s;
+      if ((s = E.vals ? elems_launch<W, 2, true>(c, P, E) : elems_launch<W, 2, false>(c, P, E))) return s;
     } else {
       psoci_note_launch();
       k_hbuild<W, 2><<<blocks, WARPS_PER_CTA * 32, smem, st>>>(P);
@@ -3419,7 +3540,7 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgR
         g.lists = 0;
         const uint32_t sl = slot[k0 + lane];
         if (sl != TAB_NONE) {
-          const uint4 h0 = __ldg(hdr + 2 * (size_t)(sl & ~TAB_SIGN)), h1 = __ldg(hdr + 2 * (size_t)(sl & ~TAB_SIGN) + 1);
+          const uint4 h0 = __ldg(hdr + 2 * (size_t)(sl & TAB_SLOT)), h1 = __ldg(hdr + 2 * (size_t)(sl & TAB_SLOT) + 1);
           g.prog = h1.x;
           g.lists = (int)h1.y;
           g.f = tab_scale(s.sign ? -2.0 : 2.0, h0.y);
