@@ -2206,18 +2206,16 @@ int max_open_of(const psoci_ctx *c) {
   return no;
 }
 
-// Slots (and with vals the integrals) of the npairs pairs of the lists and the tables they
-// need.  ok = false: the patterns do not fit the tables and nothing is left allocated; the
-// generic kernels take the space.
-// grad: the lower pairs alone, with the tables' programs.
-template <int W>
-psoci_status tab_prepare(psoci_ctx *c, const Params &P, const int64_t *nbroff, const int32_t *nbr, int64_t npairs,
-                         bool vals, bool grad, TabSet<W> &S, bool &ok) {
+// Tables of the pairs whose slots `slots_of(S)` writes (a launch on the stream): S.slot and with
+// vals S.vals for npairs pairs.  grad: with the tables' programs.  ok = false: the patterns do not
+// fit the tables and nothing is left allocated; the generic kernels take the space.
+template <int W, class F>
+psoci_status tab_prepare(psoci_ctx *c, const Params &P, int64_t npairs, bool vals, bool grad, TabSet<W> &S, bool &ok,
+                         F &&slots_of) {
   cudaStream_t st = c->stream;
   const int n = c->nconf;
   psoci_status s = PSOCI_OK;
   ok = false;
-  const int wblocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n * 32 + 255) / 256, 1 << 20));
   if ((s = psoci_alloc(c, &S.cfg, n)) || (s = psoci_alloc(c, &S.slot, npairs)) ||
       (vals && (s = psoci_alloc(c, &S.vals, npairs))) || (s = psoci_alloc(c, &S.t.counter, 2))) {
     S.free();
@@ -2242,8 +2240,7 @@ psoci_status tab_prepare(psoci_ctx *c, const Params &P, const int64_t *nbroff, c
     if (e == cudaSuccess) e = cudaMemsetAsync(S.t.counter, 0, 2 * sizeof(unsigned long long), st);
     if (e != cudaSuccess) break;
     psoci_note_launch();
-    auto k = grad ? k_pair_slots<W, false, true> : vals ? k_pair_slots<W, true, false> : k_pair_slots<W, false, false>;
-    k<<<wblocks, 256, 0, st>>>(P, S.cfg, nbroff, nbr, S.t.keys, (uint32_t)(slots - 1), S.t.err, S.slot, S.vals);
+    slots_of(S);
     const TabBuildArgs B = {S.t.keys, slots, c->d_tmpl, c->d_tmpl_off, c->nelec, c->ksym & 1,
                             S.t.hdr, S.t.pool, S.t.counter, cap, S.t.err};
     psoci_note_launch();
@@ -2274,6 +2271,17 @@ psoci_status tab_prepare(psoci_ctx *c, const Params &P, const int64_t *nbroff, c
   }
   if (!ok) S.free();
   return PSOCI_OK;
+}
+
+// The same for the pairs of neighbour lists (grad: the lower pairs alone).
+template <int W>
+psoci_status tab_prepare_lists(psoci_ctx *c, const Params &P, const int64_t *nbroff, const int32_t *nbr, int64_t npairs,
+                               bool vals, bool grad, TabSet<W> &S, bool &ok) {
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)c->nconf * 32 + 255) / 256, 1 << 20));
+  auto k = grad ? k_pair_slots<W, false, true> : vals ? k_pair_slots<W, true, false> : k_pair_slots<W, false, false>;
+  return tab_prepare<W>(c, P, npairs, vals, grad, S, ok, [&](TabSet<W> &T) {
+    k<<<blocks, 256, 0, c->stream>>>(P, T.cfg, nbroff, nbr, T.t.keys, (uint32_t)(T.t.slots - 1), T.t.err, T.slot, T.vals);
+  });
 }
 
 // The diagonal blocks and the diagonal of H.
@@ -2401,7 +2409,7 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
     TRYC(cudaMemGetInfo(&freeb, &totb));
     vals = c->eval_launches != 1 && (double)npairs * 16.0 <= 0.25 * ((double)freeb + (double)c->pool_bytes);
     TRYC(cudaEventRecord(ev[2], st));
-    TRY(tab_prepare<W>(c, P, d_nbroff, d_nbr, npairs, vals, false, T, fast));
+    TRY(tab_prepare_lists<W>(c, P, d_nbroff, d_nbr, npairs, vals, false, T, fast));
   }
   auto t_c = tnow();
 
@@ -3717,7 +3725,7 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
   if (!c->grad_tabs && !c->grad_generic) {
     DirTabs *d = new DirTabs();
     bool ok = tab_usable(c, false);
-    if (ok && (s = tab_prepare<W>(c, P, c->grad_nbroff, c->grad_nbr, c->grad_npairs, false, true, dir_set<W>(d), ok))) {
+    if (ok && (s = tab_prepare_lists<W>(c, P, c->grad_nbroff, c->grad_nbr, c->grad_npairs, false, true, dir_set<W>(d), ok))) {
       delete d;
       return s;
     }
@@ -3802,4 +3810,237 @@ psoci_status psoci_energy_grad_run(psoci_ctx *c, int k, const double *dV, int64_
     return psoci_fail(c, PSOCI_ERR_INVALID_ARG, "energy_gradient: precision must be FP64 or MIXED");
   return (c->words == 1) ? run_energy_grad<1>(c, k, dV, ldv, mode, prec, dG1, dG2)
                          : run_energy_grad<2>(c, k, dV, ldv, mode, prec, dG1, dG2);
+}
+
+// ------------------------------------------------------------------------------------
+// 1-particle density from coupling tables (density.cu finds the pairs and holds the plan).  An
+// element of a single-excitation block of equal symmetries contains v0 with the coefficient of
+// the reference's CIDEN block (PsociHamiltonian.C:572-705), so c_I^T S_IJ c_J is the first list of
+// the table's program.
+// ------------------------------------------------------------------------------------
+namespace {
+
+// Pair t of the groups: its slot and what the density kernel reads of it, {table and sign,
+// first SEF of I, first SEF of J, place in the packed triangle}.  One thread a chunk of pairs.
+constexpr int DEN_CHUNK = 4;
+template <int W>
+__global__ void __launch_bounds__(256) k_den_slots(Params P, const CfgRec<W> *__restrict__ cfg, int64_t ng, int64_t np,
+                                                   const int64_t *__restrict__ geoff, const int64_t *__restrict__ gpoff,
+                                                   const int32_t *__restrict__ gcfg, const uint8_t *__restrict__ gorb,
+                                                   uint64_t *keys, uint32_t mask, int *err, uint4 *__restrict__ recs) {
+  const int64_t nchunk = (np + DEN_CHUNK - 1) / DEN_CHUNK;
+  for (int64_t ch = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; ch < nchunk; ch += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t t0 = ch * DEN_CHUNK;
+    int64_t lo = 0, hi = ng - 1;  // group holding pair t0: last g with gpoff[g] <= t0
+    while (lo < hi) {
+      const int64_t mid = (lo + hi + 1) >> 1;
+      if (gpoff[mid] <= t0) lo = mid;
+      else hi = mid - 1;
+    }
+    int64_t g = lo, e0 = geoff[g];
+    int m = (int)(geoff[g + 1] - e0);
+    int64_t u = t0 - gpoff[g];
+    int a = 0;
+    while (u >= m - 1 - a) { u -= m - 1 - a; ++a; }
+    int b = a + 1 + (int)u;
+    const int64_t tend = min(t0 + DEN_CHUNK, np);
+    for (int64_t t = t0; t < tend; ++t) {
+      const int I = gcfg[e0 + a], J = gcfg[e0 + b], p = gorb[e0 + a], q = gorb[e0 + b];
+      const CfgRec<W> A = cfg[I], B = cfg[J];
+      uint32_t sl = TAB_NONE;
+      const PairShape s = pair_shape<W>(A, B);
+      // members of a group share a hash, not always the occupation: only p -> q singles count
+      if (s.kind == K_SINGLE && s.ex0 == p && s.jy0 == q) {
+        sl = tab_insert(keys, mask, pair_key<W>(A, B, s.kind, false), err);
+        if (sl != TAB_NONE) sl |= s.sign;
+      }
+      const int x = max(p, q), y = min(p, q);
+      recs[t] = make_uint4(sl, A.sef, B.sef, (uint32_t)(x * (x + 1) / 2 + y));
+      if (++b == m) {
+        if (++a == m - 1) {
+          if (++g >= ng) break;
+          e0 = geoff[g];
+          m = (int)(geoff[g + 1] - e0);
+          a = 0;
+        }
+        b = a + 1;
+      }
+    }
+  }
+}
+
+// Off-diagonal: KP lanes (a root each) to a pair, the signed products of its list added in FP64,
+// and to the packed triangle T [place][KP] by FP64 atomics.  mrcisd_6e8o_v24, 8 roots: the whole
+// density 339 us, where a warp took the determinants of a pair in float-float sums,
+// four roots a pass, for 1,560 us.
+template <int KP>
+__global__ void __launch_bounds__(256) k_den_pairs(int64_t np, const uint4 *__restrict__ recs,
+                                                   const uint4 *__restrict__ hdr, const uint32_t *__restrict__ pool,
+                                                   const double *__restrict__ C, double *T) {
+  const int q = threadIdx.x % KP;
+  const int64_t ngrp = (int64_t)gridDim.x * blockDim.x / KP;
+  for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / KP; u < np; u += ngrp) {
+    const uint4 r = __ldg(recs + u);
+    if (r.x == TAB_NONE) continue;
+    const uint4 h0 = __ldg(hdr + 2 * (size_t)(r.x & TAB_SLOT)), h1 = __ldg(hdr + 2 * (size_t)(r.x & TAB_SLOT) + 1);
+    const double *cI = C + (int64_t)r.y * KP + q, *cJ = C + (int64_t)r.z * KP + q;
+    const int end = h1.y ? (int)__ldg(reinterpret_cast<const uint16_t *>(pool + h1.x)) : 0;
+    const uint32_t *pw = pool + h1.x + (TAB_LISTS + 1) / 2;
+    double s0 = 0.0, s1 = 0.0;
+    int e = 0;
+#pragma unroll 2
+    for (; e + 2 <= end; e += 2) {
+      const uint32_t x0 = __ldg(pw + e), x1 = __ldg(pw + e + 1);
+      s0 = fma(with_sign(__ldg(cI + (int)((x0 >> 8) & 0xffu) * KP), x0), __ldg(cJ + (int)(x0 & 0xffu) * KP), s0);
+      s1 = fma(with_sign(__ldg(cI + (int)((x1 >> 8) & 0xffu) * KP), x1), __ldg(cJ + (int)(x1 & 0xffu) * KP), s1);
+    }
+    if (e < end) {
+      const uint32_t x0 = __ldg(pw + e);
+      s0 = fma(with_sign(__ldg(cI + (int)((x0 >> 8) & 0xffu) * KP), x0), __ldg(cJ + (int)(x0 & 0xffu) * KP), s0);
+    }
+    if (end) atomicAdd(T + (int64_t)r.w * KP + q, flip_sign(tab_scale(s0 + s1, h0.y), r.x & TAB_SIGN));
+  }
+}
+
+// Diagonal: T[p][p] += occ_p(I) |c_I|^2.  One warp a run of configurations; lane l holds orbitals
+// l, l + 32, ... for all KP roots, the norms are summed by lanes (SEF, root).
+template <int W, int KP>
+__global__ void __launch_bounds__(128) k_den_diag(Params P, const CfgRec<W> *__restrict__ cfg,
+                                                  const double *__restrict__ C, double *T) {
+  constexpr int NO = 2 * W;
+  const int lane = threadIdx.x & 31, q = lane % KP;
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const double r2 = sqrt(0.5), ssd = r2 * r2 + r2 * r2;  // (C C^T)_aa of an open-shell SEF, even electron count
+  double acc[NO][KP];
+#pragma unroll
+  for (int w = 0; w < NO; ++w)
+#pragma unroll
+    for (int u = 0; u < KP; ++u) acc[w][u] = 0.0;
+  for (int64_t I = warp; I < P.nconf; I += nwarps) {
+    const CfgRec<W> a = cfg[I];
+    const int nsef = (int)(a.flags >> 16) & 0x1ff;
+    double s = 0.0;
+    for (int x = lane / KP; x < nsef; x += 32 / KP) {
+      const double c = __ldg(C + ((int64_t)a.sef + x) * KP + q);
+      s = fma(c, c, s);
+    }
+#pragma unroll
+    for (int o = KP; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (!(P.nelec & 1) && (a.flags & 15u)) s *= ssd;
+    double n2[KP];
+#pragma unroll
+    for (int u = 0; u < KP; ++u) n2[u] = __shfl_sync(0xffffffffu, s, u);
+#pragma unroll
+    for (int w = 0; w < NO; ++w) {
+      const uint32_t o1 = (uint32_t)(a.e1[w / 2] >> (32 * (w & 1))), o2 = (uint32_t)(a.e2[w / 2] >> (32 * (w & 1)));
+      if (o1 == 0u) continue;
+      const int occ = (int)((o1 >> lane) & 1u) + (int)((o2 >> lane) & 1u);
+      const double f = occ == 0 ? 0.0 : occ == 1 ? 1.0 : 2.0;
+#pragma unroll
+      for (int u = 0; u < KP; ++u) acc[w][u] = fma(f, n2[u], acc[w][u]);
+    }
+  }
+#pragma unroll
+  for (int w = 0; w < NO; ++w) {
+    const int64_t p = 32 * w + lane;
+    if (p < P.nbf)
+#pragma unroll
+      for (int u = 0; u < KP; ++u)
+        if (acc[w][u] != 0.0) atomicAdd(T + (p * (p + 1) / 2 + p) * KP + u, acc[w][u]);
+  }
+}
+
+// D[q * n + i] = T[i * KP + q]
+template <int KP>
+__global__ void k_den_out(int n, int k, const double *__restrict__ T, double *__restrict__ D) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * k; e += gridDim.x * blockDim.x)
+    D[e] = T[(int64_t)(e % n) * KP + e / n];
+}
+
+Params den_params(const psoci_ctx *c) {
+  Params P = {};
+  P.nconf = c->nconf; P.nbf = c->nbf; P.nelec = c->nelec; P.ksym = c->ksym;
+  P.e1 = c->d_e1; P.e2 = c->d_e2; P.jsym = c->d_jsym; P.nopen = c->d_nopen;
+  P.sefoff = c->d_sefoff; P.detoff = c->d_detoff; P.phase = c->d_phase;
+  return P;
+}
+
+template <int W>
+psoci_status den_plan(psoci_ctx *c) {
+  const Params P = den_params(c);
+  DirTabs *d = new DirTabs();
+  bool ok = false;
+  const int64_t np = c->den_npairs;
+  psoci_status s = psoci_alloc(c, &c->den_recs, np);
+  if (s == PSOCI_OK)
+    s = tab_prepare<W>(c, P, np, false, true, dir_set<W>(d), ok, [&](TabSet<W> &T) {
+      k_den_slots<W><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((np + 1023) / 1024, 152 * 32)), 256, 0, c->stream>>>(
+          P, T.cfg, c->den_ng, np, c->den_geoff, c->den_gpoff, c->den_gcfg, c->den_gorb, T.t.keys,
+          (uint32_t)(T.t.slots - 1), T.t.err, c->den_recs);
+    });
+  if (s != PSOCI_OK || !ok) {
+    delete d;
+    psoci_free(c->den_recs);
+    return s;
+  }
+  c->den_tabs = d;
+  return PSOCI_OK;
+}
+
+template <int W, int KP>
+cudaError_t den_pass(psoci_ctx *c, int k, const double *V, int64_t ldv, double *D) {
+  cudaStream_t st = c->stream;
+  const TabSet<W> &S = dir_set<W>(static_cast<DirTabs *>(c->den_tabs));
+  const int64_t N = c->nsef_total, np = c->den_npairs;
+  const int ntri = c->nbf * (c->nbf + 1) / 2;
+  double *T = c->den_rows + N * KP;  // the packed triangles, the roots of an entry side by side
+  cudaError_t e = cudaMemsetAsync(T, 0, sizeof(double) * ntri * KP, st);
+  if (e != cudaSuccess) return e;
+  for (int q = 0; q < 4; ++q) psoci_note_launch();
+  k_grad_rows<double, KP><<<(unsigned)std::min<int64_t>((N + 255) / 256, 152 * 16), 256, 0, st>>>(N, V, ldv, k, c->den_rows);
+  k_den_diag<W, KP><<<(unsigned)std::min<int64_t>((c->nconf + 31) / 32, 152 * 4), 128, 0, st>>>(den_params(c), S.cfg,
+                                                                                            c->den_rows, T);
+  if (np > 0)
+    k_den_pairs<KP><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((np * KP + 255) / 256, 152 * 32)), 256, 0, st>>>(
+        np, c->den_recs, S.t.hdr, S.t.pool, c->den_rows, T);
+  k_den_out<KP><<<(ntri * k + 255) / 256, 256, 0, st>>>(ntri, k, T, D);
+  return cudaGetLastError();
+}
+
+template <int W>
+psoci_status den_run(psoci_ctx *c, int k, const double *V, int64_t ldv, double *D) {
+  const int ntri = c->nbf * (c->nbf + 1) / 2;
+  psoci_status s;
+  if (!c->den_rows && (s = psoci_alloc(c, &c->den_rows, (size_t)(c->nsef_total + ntri) * 8))) return s;
+  for (int r0 = 0; r0 < k; r0 += 8) {
+    const int kk = std::min(8, k - r0);
+    const double *v = V + (int64_t)r0 * ldv;
+    double *d = D + (int64_t)r0 * ntri;
+    const cudaError_t e = kk <= 1 ? den_pass<W, 1>(c, kk, v, ldv, d) : kk <= 2 ? den_pass<W, 2>(c, kk, v, ldv, d)
+                        : kk <= 4 ? den_pass<W, 4>(c, kk, v, ldv, d) : den_pass<W, 8>(c, kk, v, ldv, d);
+    if (e != cudaSuccess) return psoci_cuda_fail(c, e, "density1");
+  }
+  return PSOCI_OK;
+}
+
+}  // namespace
+
+psoci_status psoci_density_plan(psoci_ctx *c) {
+  if (c->max_ndet > TAB_MAXDET) return PSOCI_OK;
+  return c->words == 1 ? den_plan<1>(c) : den_plan<2>(c);
+}
+psoci_status psoci_density_tab_run(psoci_ctx *c, int k, const double *dV, int64_t ldv, double *dD) {
+  return c->words == 1 ? den_run<1>(c, k, dV, ldv, dD) : den_run<2>(c, k, dV, ldv, dD);
+}
+void psoci_density_tabs_release(psoci_ctx *c) {
+  if (c->den_tabs) {
+    DirTabs *d = static_cast<DirTabs *>(c->den_tabs);
+    d->s1.free();
+    d->s2.free();
+    delete d;
+    c->den_tabs = nullptr;
+  }
+  psoci_free(c->den_recs);
+  psoci_free(c->den_rows);
 }

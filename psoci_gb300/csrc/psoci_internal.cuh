@@ -111,11 +111,9 @@ struct psoci_ctx {
   int64_t *den_gpoff = nullptr;  // [ng+1] first candidate pair of each group
   int32_t *den_gcfg = nullptr;   // members: configuration
   uint8_t *den_gorb = nullptr;   // members: orbital the key removed
-  int4 *den_gmem = nullptr;      // members packed with their configuration's offsets
-  uint8_t *den_gflag = nullptr;  // [ng] 1: members' exact keys differ (hash collision)
-  uint64_t *den_gopen = nullptr; // members: open shells of the configuration [words]
-  float2 *den_vs = nullptr;      // float-float copy of the roots of one pass
-  size_t den_vs_cap = 0;
+  void *den_tabs = nullptr;      // their coupling tables (hbuild.cu, DirTabs), or null: generic kernel
+  uint4 *den_recs = nullptr;     // [npairs] what the table kernel reads of a pair
+  double *den_rows = nullptr;    // the roots of a pass (at most 8) side by side, and the triangles being summed
 
   // mixed-sigma variant in use (sigma.cu; psoci_autotune_sigma picks it, a build resets it)
   int sigma_variant = PSOCI_SIGMA_DEFAULT;
@@ -229,6 +227,11 @@ void psoci_join_release(psoci_ctx *c);
 void psoci_h_release(psoci_ctx *c);
 void psoci_dets_release(psoci_ctx *c);
 void psoci_density_release(psoci_ctx *c);
+// density from coupling tables (hbuild.cu): tables and pair records of the groups (den_tabs stays
+// null where the tables do not hold the space), the density, their release
+psoci_status psoci_density_plan(psoci_ctx *c);
+psoci_status psoci_density_tab_run(psoci_ctx *c, int k, const double *dV, int64_t ldv, double *dD);
+void psoci_density_tabs_release(psoci_ctx *c);
 void psoci_basis_release(psoci_ctx *c);
 void psoci_grad_release(psoci_ctx *c);
 // energy gradient with respect to the integral tables (hbuild.cu): device vectors k x ldv

@@ -121,3 +121,17 @@ def test_gradient_matches_oracle(oracle_mod, k):
     g1, g2 = c.energy_gradient(v)
     assert np.abs(g1 - r1).max() <= 1e-12 and np.abs(g2 - r2).max() <= 1e-12
     c.close()
+
+
+@pytest.mark.parametrize("name", ["open8", "open10_two_words", "open11", "pairs", "one_electron"])
+@pytest.mark.parametrize("k", [1, 2, 3, 9])
+def test_density_matches_oracle(oracle_mod, name, k):
+    """1-particle densities, passes of 1, 2, 4 and 8 roots; unit vectors, sums of at most N^2
+    products of their entries."""
+    p = CASES[name]()
+    O = oracle_mod.Oracle(p)
+    v = np.random.default_rng(k).standard_normal((k, O.num_sefs()))
+    v /= np.linalg.norm(v, axis=1)[:, None]
+    c = gpu_context(p)
+    assert np.abs(c.density1(v) - O.density1(v)).max() <= 1e-12
+    c.close()
