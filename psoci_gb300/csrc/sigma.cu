@@ -22,6 +22,10 @@
 namespace {
 
 constexpr int SIG_THREADS = 256;
+// threads of a block of the mixed kernel: narrow blocks of vectors run 9-15% faster with 512 (k = 1:
+// 155 -> 138 us at 60.0 M elements, 753 -> 640 at 267 M), wide ones are slower (k = 8: 111 -> 129 at
+// 25.7 M)
+__host__ __device__ constexpr int mix_threads(int k) { return k <= 4 ? 512 : 256; }
 // stored elements per lane whose gathers are in flight together; 4 was fastest for 8
 // vectors (8.96 ms at the benchmark block, 9.13 with 6, 9.67 with 8)
 constexpr int SIG_UNROLL = 4;
@@ -187,7 +191,7 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float prod) {
 // per row; 16: two rows per warp, for short rows) and UNR stored elements per lane whose
 // gathers are in flight together.
 template <int K, int LPR, int UNR>
-__global__ void __launch_bounds__(SIG_THREADS) k_spmm_mixed(int64_t nrows, const int64_t *__restrict__ rowptr,
+__global__ void __launch_bounds__(mix_threads(K)) k_spmm_mixed(int64_t nrows, const int64_t *__restrict__ rowptr,
                                                             const int32_t *__restrict__ col,
                                                             const float *__restrict__ val,
                                                             const float *__restrict__ x, double *__restrict__ y,
@@ -289,13 +293,24 @@ __device__ __forceinline__ void store_reduced_ff(ff2 (&v)[8], int lane, double *
   if ((lane & 3) == 0 && qq < K) yr[qq] = (double)cc.h + (double)cc.l;
 }
 
-// FF: FP64 elements split as they stream, inputs pre-split into float pairs (x2, K per row)
-template <int K>
+// pairs in a row of the FF inputs for k vectors: a gathered row is one load up to 4 vectors, two
+// from 5 on, and never crosses a 32-byte sector more than its size asks for.  Rows of exactly k
+// pairs took k 8-byte loads, which bound the kernel: 592 us at k = 4 and 573 at k = 5 against 532
+// with the full rows of k = 8 (60.0 M elements); padded they take 273, 424 and (two elements a lane
+// in flight) 459.  One and two vectors keep rows of 8 and 16 bytes: a wider row would only move more.
+__host__ __device__ constexpr int ff_row(int k) { return k <= 2 ? k : (k <= 4 ? 4 : 8); }
+
+// FF: FP64 elements split as they stream, inputs pre-split into float pairs (x2: ff_row(K) a row).
+// Bound by the gathered rows from L2 (64 bytes an element at k > 4: 9 TB/s at k = 8) and by the
+// ~20 FP32 operations a product.  Two elements a lane in flight (UNR) for k >= 2; one vector loses by
+// it (232 us against 208).
+template <int K, int UNR>
 __global__ void __launch_bounds__(SIG_THREADS) k_spmm_ff(int64_t nrows, const int64_t *__restrict__ rowptr,
                                                          const int32_t *__restrict__ col,
                                                          const double *__restrict__ val,
                                                          const float2 *__restrict__ x2, double *__restrict__ y,
                                                          int ldy) {
+  constexpr int XS = ff_row(K);
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -304,29 +319,43 @@ __global__ void __launch_bounds__(SIG_THREADS) k_spmm_ff(int64_t nrows, const in
 #pragma unroll
     for (int q = 0; q < K; ++q) { sh[q] = 0.f; sl[q] = 0.f; }
     const int64_t e = rowptr[r + 1];
-    for (int64_t t = rowptr[r] + lane; t < e; t += 32) {
-      const int c = ldg_stream(col + t);
-      const float2 v = split_f64(ldg_stream(val + t));
-      const float2 *xr = x2 + (int64_t)c * K;
-      float2 xv[K];
-      if (K == 8) {
-        // 8 pairs = 64 contiguous, 64-byte-aligned bytes: two 256-bit loads
-        float f[16];
-        asm("ld.global.cg.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-            : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7])
-            : "l"(xr));
-        asm("ld.global.cg.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-            : "=f"(f[8]), "=f"(f[9]), "=f"(f[10]), "=f"(f[11]), "=f"(f[12]), "=f"(f[13]), "=f"(f[14]), "=f"(f[15])
-            : "l"(xr + 4));
+    int64_t t = rowptr[r] + lane;
+    auto add = [&](int m) {  // m elements from t on, 32 apart
+      double v[UNR];
+      float f[UNR][2 * XS];
 #pragma unroll
-        for (int q = 0; q < K; ++q) xv[q] = make_float2(f[2 * q], f[2 * q + 1]);
-      } else {
+      for (int u = 0; u < UNR; ++u)
+        if (u < m) {
+          const int c = ldg_stream(col + t + 32 * u);
+          v[u] = ldg_stream(val + t + 32 * u);
+          const float *xr = reinterpret_cast<const float *>(x2 + (int64_t)c * XS);
 #pragma unroll
-        for (int q = 0; q < K; ++q) xv[q] = __ldg(xr + q);
-      }
+          for (int h = 0; h < (XS >= 4 ? XS / 4 : 0); ++h) {
+            float g[8];
+            ldg_row8(g, xr + 8 * h);
 #pragma unroll
-      for (int q = 0; q < K; ++q) ff_fma(sh[q], sl[q], v, xv[q]);
-    }
+            for (int q = 0; q < 8; ++q) f[u][8 * h + q] = g[q];
+          }
+          if constexpr (XS == 2) {
+            const float4 g = __ldcg(reinterpret_cast<const float4 *>(xr));
+            f[u][0] = g.x; f[u][1] = g.y; f[u][2] = g.z; f[u][3] = g.w;
+          }
+          if constexpr (XS == 1) {
+            const float2 g = __ldcg(reinterpret_cast<const float2 *>(xr));
+            f[u][0] = g.x; f[u][1] = g.y;
+          }
+        }
+#pragma unroll
+      for (int u = 0; u < UNR; ++u)
+        if (u < m) {
+          const float2 w = split_f64(v[u]);
+#pragma unroll
+          for (int q = 0; q < K; ++q) ff_fma(sh[q], sl[q], w, make_float2(f[u][2 * q], f[u][2 * q + 1]));
+        }
+    };
+    for (; t + 32 * (UNR - 1) < e; t += 32 * UNR) add(UNR);
+    if (UNR > 1)
+      for (; t < e; t += 32) add(1);
     ff2 vv[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -342,10 +371,14 @@ __global__ void __launch_bounds__(SIG_THREADS) k_spmm_ff(int64_t nrows, const in
   }
 }
 
-// X (FP64, leading dim ldx) -> X2 (float pairs, leading dim k); one thread per row
+// X (FP64, leading dim ldx, k <= 8 columns) -> X2 (float pairs, ff_row(k) a row, zero padded);
+// one thread a pair
 __global__ void k_split_x(int64_t n, int k, const double *__restrict__ x, int ldx, float2 *__restrict__ x2) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-    for (int q = 0; q < k; ++q) x2[r * k + q] = split_f64(x[r * ldx + q]);
+  const int sh = 31 - __clz(ff_row(k));
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n << sh; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = e >> sh;
+    const int q = (int)(e - (r << sh));
+    x2[e] = q < k ? split_f64(x[r * ldx + q]) : make_float2(0.f, 0.f);
   }
 }
 
@@ -364,12 +397,17 @@ __global__ void k_to_f32(int64_t n, int k, const double *__restrict__ x, int ldx
   }
 }
 
+// blocks of a kernel with a warp a row
+int sig_blocks(int64_t n, int threads) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>((n * 32 + threads - 1) / threads, 152 * 8 * 4));
+}
+
 bool rows_vec2(const double *x, int ldx) { return ((uintptr_t)x % 16 == 0) && (ldx % 2 == 0); }
 
 template <int K>
 void launch_f64(psoci_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *col, const double *val, const double *dX,
                 int ldx, double *dY, int ldy) {
-  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n * 32 + SIG_THREADS - 1) / SIG_THREADS, 152 * 8 * 4));
+  const int blocks = sig_blocks(n, SIG_THREADS);
   psoci_note_launch();
   k_spmm_f64<K><<<blocks, SIG_THREADS, 0, c->stream>>>(n, rowptr, col, val, dX, ldx, dY, ldy, rows_vec2(dX, ldx));
 }
@@ -377,37 +415,37 @@ void launch_f64(psoci_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *c
 template <int K>
 void launch_k(psoci_ctx *c, int64_t n, const double *dX, int ldx, double *dY, int ldy, psoci_prec prec,
               const float *x32, int ld32) {
-  int64_t warps = n;
-  int blocks = (int)std::min<int64_t>((warps * 32 + SIG_THREADS - 1) / SIG_THREADS, 152 * 8 * 4);
-  if (blocks < 1) blocks = 1;
+  int blocks = sig_blocks(n, SIG_THREADS);
   psoci_note_launch();
   if (prec == PSOCI_PREC_FP64)
     k_spmm_f64<K><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val, dX, ldx, dY, ldy,
                                                          rows_vec2(dX, ldx));
   else if (prec == PSOCI_PREC_FF)
-    k_spmm_ff<K><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val,
+    k_spmm_ff<K, K == 1 ? 1 : 2><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val,
                                                         reinterpret_cast<const float2 *>(x32), dY, ldy);
   else {
+    constexpr int T = mix_threads(K);
+    blocks = sig_blocks(n, T);
     // the variant chosen by psoci_autotune_sigma for this Hamiltonian (PSOCI_SIGMA_DEFAULT
     // until it runs)
     switch (c->sigma_variant) {
       case 1:
-        k_spmm_mixed<K, 32, 2><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
+        k_spmm_mixed<K, 32, 2><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
         break;
       case 2:
-        k_spmm_mixed<K, 16, 4><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
+        k_spmm_mixed<K, 16, 4><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
         break;
       case 3:
-        k_spmm_mixed<K, 16, 2><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
+        k_spmm_mixed<K, 16, 2><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
         break;
       case 4:
-        k_spmm_mixed<K, 8, 4><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
+        k_spmm_mixed<K, 8, 4><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
         break;
       case 5:
-        k_spmm_mixed<K, 16, 6><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
+        k_spmm_mixed<K, 16, 6><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
         break;
       default:
-        k_spmm_mixed<K, 32, SIG_UNROLL><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32,
+        k_spmm_mixed<K, 32, SIG_UNROLL><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32,
                                                                               dY, ldy);
     }
   }
@@ -440,7 +478,7 @@ psoci_status psoci_sigma_launch(psoci_ctx *c, int k, const double *dX, int ldx, 
       x32 = dX32;
     } else if (prec == PSOCI_PREC_FF) {
       if (!dX32) return psoci_fail(c, PSOCI_ERR_INVALID_ARG, "sigma: FF without staging");
-      int blocks = (int)std::min<int64_t>((n + 255) / 256, 152 * 16);
+      int blocks = (int)std::min<int64_t>((n * ff_row(kk) + 255) / 256, 152 * 16);
       psoci_note_launch();
       k_split_x<<<std::max(blocks, 1), 256, 0, c->stream>>>(n, kk, xs, ldx, reinterpret_cast<float2 *>(dX32));
       x32 = dX32;
