@@ -3315,8 +3315,8 @@ struct AdjRec {
   int32_t info;  // tag | (sgn < 0) << 4 | term << 8
 };
 
-// One warp per row configuration I (grid-stride); its lower neighbours J <= I (diag_only: I
-// itself) in chunks of 32 set up by the lanes.  Per pair: (1) lanes over the determinant pairs (x, y) test them for
+// One warp per row configuration I (grid-stride); its lower neighbours J <= I in chunks of 32
+// set up by the lanes.  Per pair: (1) lanes over the determinant pairs (x, y) test them for
 // coupling and classify the coupled ones (det_adj), collecting the records in shared memory;
 // (2) lanes = (slot, root) take the records, slots over the records and roots over the lanes
 // of a slot, and add s * cd_I[x] * cd_J[y] to register accumulators of the pair's terms (v0,
@@ -3328,7 +3328,7 @@ template <int W, typename CT, typename ACC>
 __global__ void __launch_bounds__(ADJ_WARPS * 32) k_energy_grad(Params P, const int64_t *__restrict__ nbroff,
                                                                 const int32_t *__restrict__ nbr,
                                                                 const CT *__restrict__ CD, int k, double *G1,
-                                                                int64_t n1, double *G2, int64_t n2, bool diag_only) {
+                                                                int64_t n1, double *G2, int64_t n2) {
   __shared__ AdjSmem<W> sm[ADJ_WARPS];
   __shared__ AdjRec recs[ADJ_WARPS][ADJ_CONN];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -3343,10 +3343,10 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32) k_energy_grad(Params P, const 
   for (int e = lane; e < ADJ_NT * ADJ_MAXR; e += 32) (&S.acc[0][0])[e] = 0.0;
   __syncwarp();
   for (int64_t I = warp; I < P.nconf; I += nwarps) {
-    const int64_t b0 = diag_only ? 0 : nbroff[I], b1 = diag_only ? 1 : nbroff[I + 1];
+    const int64_t b0 = nbroff[I], b1 = nbroff[I + 1];
     for (int64_t c0 = b0; c0 < b1; c0 += 32) {
       const int64_t q = c0 + lane;
-      const int J = (q < b1) ? (diag_only ? (int)I : nbr[q]) : INT_MAX;
+      const int J = (q < b1) ? nbr[q] : INT_MAX;
       const bool lower = J <= (int)I;
       if (lower) adj_pair_setup<W>(P, (int)I, J, S.pi[lane]);
       const unsigned lm = __ballot_sync(0xffffffffu, lower);
@@ -3471,8 +3471,8 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32) k_energy_grad(Params P, const 
 }
 
 // ------------------------------------------------------------------------------------
-// The same from coupling tables (at most TAB_MAXOPEN open shells), for the pairs J < I; the
-// diagonal blocks stay with k_energy_grad.
+// The same from coupling tables (at most TAB_MAXOPEN open shells), pairs J < I and diagonal
+// blocks apart.
 // ------------------------------------------------------------------------------------
 // vectors (k per pass, root-major with stride ldv) side by side, KP a SEF (zero padded)
 template <typename CT, int KP>
@@ -3513,7 +3513,7 @@ struct GradPair {
 // (float) within a pair; the places take FP64 atomics, the KP roots of one side by side (T1, T2:
 // KP a table entry).  Bound by the FP64 pipe, one FMA an entry of a list (16 clocks a warp
 // instruction an SM): mrcisd_6e8o_v16, 8 roots, 3.2 ms (determinant pair by determinant pair the
-// lower and diagonal blocks took 54.7 ms, of which the diagonal's 2.4 ms remain).
+// lower blocks took 52 ms).
 template <int W, typename CT, int KP>
 __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgRec<W> *__restrict__ cfg,
                                                             const int64_t *__restrict__ nbroff,
@@ -3624,6 +3624,111 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgR
   }
 }
 
+// Diagonal blocks.  The determinants of a configuration are spin patterns of its open shells, and two
+// of them couple only by exchanging the spins of two shells a > b, with the sign of their phases and
+// of the a - b - 1 shells between.  So with c' the coefficients times their phases the integral
+// (ab|ba) gets, over the patterns x of equal spins in a and b and the pairs x, y that differ by the
+// exchange (PsociHamiltonian.C:306-388),
+//   -sum c'x^2 + sum 2 s c'x c'y = -sum over all of c'x^2 + sum over the pairs of (c'x + s c'y)^2 ,
+// 2^(n-2) squares instead of a test of every determinant with every other.  One warp a configuration,
+// KP lanes (a root each) to a shell pair or an integral.  Of 2.4 ms at mrcisd_6e8o_v16, 8 roots,
+// 0.14 ms remain.
+template <int W, typename CT, int KP>
+__global__ void __launch_bounds__(GT_WARPS * 32) k_grad_diag(Params P, const CT *__restrict__ C, double *T1, double *T2) {
+  // of a spin pattern: SEF in the block, bit 15 the sign of c'; NO_DET without a determinant
+  __shared__ uint16_t maps[GT_WARPS][1 << TAB_MAXOPEN];
+  constexpr unsigned FULL = 0xffffffffu, NO_DET = 0x7fffu;
+  uint16_t *map = maps[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31, q = lane % KP, grp = lane / KP, ngrp = 32 / KP;
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t I = warp; I < P.nconf; I += nwarps) {
+    uint64_t o1[W], o2[W], so[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      o1[w] = P.e1[I * W + w];
+      o2[w] = P.e2[I * W + w];
+      so[w] = o1[w] & ~o2[w];
+    }
+    auto nth = [](const uint64_t(&x)[W], int p) {  // the p-th lowest set bit of x
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        uint64_t u = x[w];
+        const int c = __popcll(u);
+        if (p < c) {
+          for (; p > 0; --p) u &= u - 1;
+          return 64 * w + __ffsll((long long)u) - 1;
+        }
+        p -= c;
+      }
+      return 0;
+    };
+    const int nop = popc_w<W>(so), nocc = popc_w<W>(o1);
+    const int64_t s0 = P.sefoff[I], d0 = P.detoff[I];
+    const int nsef = (int)(P.sefoff[I + 1] - s0), ndet = (int)(P.detoff[I + 1] - d0);
+    const bool open2 = !(P.nelec & 1) && nop != 0;
+    const bool flip = open2 && P.jsym[I] % 2 != P.ksym % 2;  // second determinants with the other sign
+    const CT *c = C + s0 * KP + q;
+    for (int m = lane; m < 1 << nop; m += 32) map[m] = NO_DET;
+    __syncwarp();
+    if (nop > 1)
+      for (int d = lane; d < ndet; d += 32) {
+        int m = 0, b = 0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const uint64_t al = P.alpha[(d0 + d) * W + w];
+          for (uint64_t u = so[w]; u; u &= u - 1, ++b) m |= (int)((al >> (__ffsll((long long)u) - 1)) & 1ull) << b;
+        }
+        const int neg = (P.phase[d0 + d] & 1) ^ (int)(flip && (d & 1));
+        map[m] = (uint16_t)((open2 ? d >> 1 : d) | (neg << 15));
+      }
+    __syncwarp();
+    CT n0 = 0;
+    for (int s = grp; s < nsef; s += ngrp) {
+      const CT v = __ldg(c + s * KP);
+      n0 = fma(v, v, n0);
+    }
+    double a0 = (double)n0;
+#pragma unroll
+    for (int o = KP; o < 32; o <<= 1) a0 += __shfl_xor_sync(FULL, a0, o);
+    // exchange integrals of the open-shell pairs
+    for (int mm = grp; mm < nop * (nop - 1) / 2; mm += ngrp) {
+      int a = 1, b = mm;
+      while (b >= a) { b -= a; ++a; }
+      const uint32_t between = (uint32_t)(a - b - 1) << 31;
+      CT sum = 0;
+      for (int i = 0; i < 1 << (nop - 2); ++i) {
+        // bits a and b put into i: a set, b clear
+        int m = (i & ((1 << b) - 1)) | ((i >> b) << (b + 1));
+        m = (m & ((1 << a) - 1)) | ((m >> a) << (a + 1)) | (1 << a);
+        const uint32_t x = map[m], y = map[m ^ (1 << a) ^ (1 << b)];
+        if (x == NO_DET && y == NO_DET) continue;
+        const CT cx = x == NO_DET ? (CT)0 : __ldg(c + (int)(x & 0x7fffu) * KP);
+        const CT cy = y == NO_DET ? (CT)0 : __ldg(c + (int)(y & 0x7fffu) * KP);
+        const CT v = cx + with_sign(cy, ((x ^ y) << 16) ^ between);
+        sum = fma(v, v, sum);
+      }
+      const int oa = nth(so, a), ob = nth(so, b);
+      atomicAdd(T2 + canon4(oa, ob, ob, oa) * KP + q, (open2 ? 0.5 : 1.0) * (double)sum - a0);
+    }
+    // orbital energies and the other pairs of occupied orbitals j < i; j = i: the orbital itself
+    for (int e = grp; e < nocc * (nocc + 1) / 2; e += ngrp) {
+      int i = 0, j = e;
+      while (j > i) { j -= i + 1; ++i; }
+      const int ib = nth(o1, i), occi = 1 + (int)bit_w<W>(o2, ib);
+      if (j == i) {
+        atomicAdd(T1 + tri64(ib, ib) * KP + q, occi * a0);
+        if (occi == 2) atomicAdd(T2 + canon4(ib, ib, ib, ib) * KP + q, a0);
+        continue;
+      }
+      const int jb = nth(o1, j), ninj = occi * (1 + (int)bit_w<W>(o2, jb));
+      atomicAdd(T2 + canon4(ib, ib, jb, jb) * KP + q, ninj * a0);
+      if (ninj > 1) atomicAdd(T2 + canon4(ib, jb, ib, jb) * KP + q, ninj == 2 ? -a0 : -2.0 * a0);
+    }
+    __syncwarp();
+  }
+}
+
 __global__ void k_fill(double *p, int64_t n, double v) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
 }
@@ -3649,7 +3754,7 @@ void grad_tabs_release(psoci_ctx *c) {
   c->grad_generic = false;
 }
 
-// the pairs J < I of one pass of kk <= KP roots, added to G1 [kk][n1] and G2 [kk][n2]
+// one pass of kk <= KP roots, added to G1 [kk][n1] and G2 [kk][n2]
 template <int W, int KP>
 cudaError_t grad_pass(psoci_ctx *c, const Params &P, const TabSet<W> &S, int kk, const double *V, int64_t ldv,
                       psoci_prec prec, double *CS, double *T1, double *G1, double *G2) {
@@ -3662,15 +3767,18 @@ cudaError_t grad_pass(psoci_ctx *c, const Params &P, const TabSet<W> &S, int kk,
   const unsigned gb = (unsigned)std::min<int64_t>((c->nconf + GT_WARPS - 1) / GT_WARPS, 1 << 20);
   psoci_note_launch();
   psoci_note_launch();
+  psoci_note_launch();
   if (prec == PSOCI_PREC_MIXED) {
     float *C = reinterpret_cast<float *>(CS);
     k_grad_rows<float, KP><<<rb, 256, 0, st>>>(N, V, ldv, kk, C);
     k_grad_tab<W, float, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, S.cfg, c->grad_nbroff, c->grad_nbr, S.slot, S.t.hdr,
                                                            S.t.pool, C, T1, T2);
+    k_grad_diag<W, float, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, C, T1, T2);
   } else {
     k_grad_rows<double, KP><<<rb, 256, 0, st>>>(N, V, ldv, kk, CS);
     k_grad_tab<W, double, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, S.cfg, c->grad_nbroff, c->grad_nbr, S.slot, S.t.hdr,
                                                             S.t.pool, CS, T1, T2);
+    k_grad_diag<W, double, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, CS, T1, T2);
   }
   psoci_note_launch();
   psoci_note_launch();
@@ -3720,8 +3828,8 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
     c->grad_mode = mode;
     c->grad_npairs = npairs;
   }
-  // pairs J < I from coupling tables, kept with the lists; the generic kernel for spaces or
-  // patterns that the tables do not hold
+  // coupling tables, kept with the lists; the generic kernel for spaces or patterns that they do
+  // not hold
   if (!c->grad_tabs && !c->grad_generic) {
     DirTabs *d = new DirTabs();
     bool ok = tab_usable(c, false);
@@ -3742,7 +3850,7 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
   };
   const int kmax = std::min(k, ADJ_MAXR), kpmax = kmax <= 2 ? kmax : kmax <= 4 ? 4 : 8;
   const int64_t N = c->nsef_total;
-  if ((s = psoci_alloc(c, &CD, (size_t)c->ndet_total * kmax))) return done(s);
+  if (!tabs && (s = psoci_alloc(c, &CD, (size_t)c->ndet_total * kmax))) return done(s);
   if (tabs && ((s = psoci_alloc(c, &CS, (size_t)N * kpmax)) || (s = psoci_alloc(c, &T1, (size_t)(n1 + n2) * kpmax))))
     return done(s);
   float *CD32 = reinterpret_cast<float *>(CD);
@@ -3754,27 +3862,28 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
     const int kk = std::min(ADJ_MAXR, k - r0);
     const unsigned sb = (unsigned)(((int64_t)n * 32 + 255) / 256);
     const double *V = dV + (int64_t)r0 * ldv;
-    psoci_note_launch();
-    if (prec == PSOCI_PREC_MIXED)
-      k_sef_to_det<float><<<sb, 256, 0, st>>>(n, c->nelec, c->ksym, c->d_sefoff, c->d_detoff, c->d_jsym, c->d_nopen, V,
-                                              ldv, kk, CD32);
-    else
-      k_sef_to_det<double><<<sb, 256, 0, st>>>(n, c->nelec, c->ksym, c->d_sefoff, c->d_detoff, c->d_jsym, c->d_nopen, V,
-                                               ldv, kk, CD);
-    psoci_note_launch();
-    if (prec == PSOCI_PREC_MIXED)
-      k_energy_grad<W, float, float><<<blocks, ADJ_WARPS * 32, 0, st>>>(P, c->grad_nbroff, c->grad_nbr, CD32, kk,
-                                                                        dG1 + r0 * n1, n1, dG2 + r0 * n2, n2, tabs);
-    else
-      k_energy_grad<W, double, double><<<blocks, ADJ_WARPS * 32, 0, st>>>(P, c->grad_nbroff, c->grad_nbr, CD, kk,
-                                                                          dG1 + r0 * n1, n1, dG2 + r0 * n2, n2, tabs);
-    e = cudaGetLastError();
-    if (e == cudaSuccess && tabs) {
+    if (tabs) {
       const TabSet<W> &S = dir_set<W>(static_cast<DirTabs *>(c->grad_tabs));
       e = kk <= 1 ? grad_pass<W, 1>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
           : kk <= 2 ? grad_pass<W, 2>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
           : kk <= 4 ? grad_pass<W, 4>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
                     : grad_pass<W, 8>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2);
+    } else {
+      psoci_note_launch();
+      if (prec == PSOCI_PREC_MIXED)
+        k_sef_to_det<float><<<sb, 256, 0, st>>>(n, c->nelec, c->ksym, c->d_sefoff, c->d_detoff, c->d_jsym, c->d_nopen, V,
+                                                ldv, kk, CD32);
+      else
+        k_sef_to_det<double><<<sb, 256, 0, st>>>(n, c->nelec, c->ksym, c->d_sefoff, c->d_detoff, c->d_jsym, c->d_nopen, V,
+                                                 ldv, kk, CD);
+      psoci_note_launch();
+      if (prec == PSOCI_PREC_MIXED)
+        k_energy_grad<W, float, float><<<blocks, ADJ_WARPS * 32, 0, st>>>(P, c->grad_nbroff, c->grad_nbr, CD32, kk,
+                                                                          dG1 + r0 * n1, n1, dG2 + r0 * n2, n2);
+      else
+        k_energy_grad<W, double, double><<<blocks, ADJ_WARPS * 32, 0, st>>>(P, c->grad_nbroff, c->grad_nbr, CD, kk,
+                                                                            dG1 + r0 * n1, n1, dG2 + r0 * n2, n2);
+      e = cudaGetLastError();
     }
     if (e != cudaSuccess) return done(psoci_cuda_fail(c, e, "energy_gradient"));
   }

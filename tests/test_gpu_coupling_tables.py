@@ -135,3 +135,49 @@ def test_density_matches_oracle(oracle_mod, name, k):
     c = gpu_context(p)
     assert np.abs(c.density1(v) - O.density1(v)).max() <= 1e-12
     c.close()
+
+
+@pytest.mark.parametrize("nbf,nelec,nopen", [(3, 4, 0), (4, 5, 1), (4, 6, 2), (5, 5, 3), (66, 6, 4), (6, 6, 6), (9, 9, 7)])
+@pytest.mark.parametrize("ksym", [1, 2])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_gradient_of_one_configuration(oracle_mod, nbf, nelec, nopen, ksym, prec):
+    """A diagonal block alone, in either symmetry block (the second determinants' sign), by the
+    closed form of its derivatives: E = sum occ h_ii + (ii|ii) of doubly occupied + pairs, the
+    exchange of two open shells from the oracle's element with that integral alone.  Unit vectors;
+    FP32 sums of at most 2^6 squares and products err by less than 2^6 2^-24 times their norm."""
+    p = neighbourhood(8 if nbf == 66 else nbf, nelec, nopen, 1, 1, 3, shift=58 if nbf == 66 else 0)
+    p.ksym = ksym
+    O = oracle_mod.Oracle(p)
+    N = O.num_sefs()
+    v = np.random.default_rng(nopen).standard_normal((3, N))
+    v /= np.linalg.norm(v, axis=1)[:, None]
+    c = gpu_context(p)
+    g1, g2 = c.energy_gradient(v, prec=prec)
+    c.close()
+    occ = p.occ[0].astype(int)
+    tri = lambda a, b: max(a, b) * (max(a, b) + 1) // 2 + min(a, b)
+    r1, r2 = np.zeros_like(g1), np.zeros_like(g2)
+    orb = np.flatnonzero(occ)
+    for i in orb:
+        r1[:, tri(i, i)] += occ[i]
+        if occ[i] == 2:
+            r2[:, tri(tri(i, i), tri(i, i))] += 1.0
+        for j in orb[orb < i]:
+            r2[:, tri(tri(i, i), tri(j, j))] += occ[i] * occ[j]
+            if occ[i] * occ[j] > 1:
+                r2[:, tri(tri(i, j), tri(i, j))] -= occ[i] * occ[j] / 2
+            else:
+                q = oracle_mod.Oracle(_only(p, tri(tri(i, j), tri(i, j))))
+                F = lower_to_full(*q.build_lower(1), N)
+                r2[:, tri(tri(i, j), tri(i, j))] += np.einsum("kn,kn->k", v, (F @ v.T).T)
+    tol = 2.0 ** -18 if prec else 1e-13
+    assert np.abs(g1 - r1).max() <= tol * 2 and np.abs(g2 - r2).max() <= tol * 4
+
+
+def _only(p, at):
+    """p with one two-electron integral, 1, and nothing else."""
+    import dataclasses
+
+    eri = np.zeros_like(p.eri)
+    eri[at] = 1.0
+    return dataclasses.replace(p, h=np.zeros_like(p.h), so=np.zeros_like(p.so), eri=eri)
