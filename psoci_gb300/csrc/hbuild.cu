@@ -3512,8 +3512,9 @@ struct GradPair {
 // which goes to that integral's place in the gradient.  The sums are FP64 (CT double) or FP32
 // (float) within a pair; the places take FP64 atomics, the KP roots of one side by side (T1, T2:
 // KP a table entry).  Bound by the FP64 pipe, one FMA an entry of a list (16 clocks a warp
-// instruction an SM): mrcisd_6e8o_v16, 8 roots, 3.2 ms (determinant pair by determinant pair the
-// lower blocks took 52 ms).
+// instruction an SM, whatever its active lanes): mrcisd_6e8o_v16, 8 roots, 2.5 ms (3.2 with the
+// pairs in their lists' order, 19 of 32 lanes active; determinant pair by determinant pair the lower
+// blocks took 52 ms).
 template <int W, typename CT, int KP>
 __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgRec<W> *__restrict__ cfg,
                                                             const int64_t *__restrict__ nbroff,
@@ -3537,24 +3538,33 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgR
       const bool low = J < (int)I;
       const int np = __popc(__ballot_sync(FULL, low));  // they come first
       if (np == 0) break;
+      uint32_t key = 0xffffffe0u | lane;
+      GradPair g;
       if (low) {
         const CfgRec<W> b = cfg[J];
         const PairShape s = pair_shape<W>(a, b);
-        GradPair g;
         g.kind = s.kind;
         g.ie = s.ex0; g.je = s.jy0; g.ex1 = s.ex1; g.jy1 = s.jy1;
         g.sefJ = b.sef;
         g.B = J;
         g.lists = 0;
+        g.prog = 0;
+        uint32_t len = 0;
         const uint32_t sl = slot[k0 + lane];
         if (sl != TAB_NONE) {
           const uint4 h0 = __ldg(hdr + 2 * (size_t)(sl & TAB_SLOT)), h1 = __ldg(hdr + 2 * (size_t)(sl & TAB_SLOT) + 1);
           g.prog = h1.x;
           g.lists = (int)h1.y;
           g.f = tab_scale(s.sign ? -2.0 : 2.0, h0.y);
+          if (g.lists > 0) len = __ldg(reinterpret_cast<const uint16_t *>(pool + g.prog) + g.lists - 1);
         }
-        gp[lane] = g;
+        key = ((uint32_t)(s.kind & 3) << 30) | (min(len, 1023u) << 20) | ((g.prog & 0x7fffu) << 5) | lane;
       }
+      // pairs of one kind and similar programs go together: a warp's groups take as long as the longest
+      int rank = 0;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) rank += __shfl_sync(FULL, key, j) < key;
+      if (low) gp[rank] = g;
       __syncwarp();
       for (int u = grp; u < np; u += 32 / KP) {
         const GradPair &g = gp[u];
@@ -3583,7 +3593,7 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgR
             atomicAdd(T2 + (l == 0 ? canon4(g.ie, g.je, g.ex1, g.jy1) : canon4(g.ie, g.jy1, g.ex1, g.je)) * KP + q, w);
           } else if (g.kind == K_SO) {
             // v = +-SO(ie, je) / 2, negated when je > ie (PsociHamiltonian.C:223-237)
-            atomicAdd(T1 + tri64(g.ie, g.je) * KP + q, (g.je > g.ie ? -0.5 : 0.5) * w);
+            atomicAdd(T1 + tri64(g.ie, g.je) * KP + q, flip_sign(0.5 * w, g.je > g.ie ? 0x80000000u : 0u));
           } else if (l > 0) {  // X[l - 1]
             int t = l - 1, o = 0;
 #pragma unroll
@@ -3603,7 +3613,8 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgR
             // v0 = h(ie, je) - (ie je|ie ie) + sum over A's occupied p of occ (ie je|p p) less
             // (ie p|p je) where p is doubly occupied in both (PsociHamiltonian.C:239-258)
             atomicAdd(T1 + tri64(g.ie, g.je) * KP + q, w);
-            atomicAdd(T2 + canon4(g.ie, g.je, g.ie, g.ie) * KP + q, -w);
+            const double w2 = w + w, nw = flip_sign(w, 0x80000000u);
+            atomicAdd(T2 + canon4(g.ie, g.je, g.ie, g.ie) * KP + q, nw);
 #pragma unroll
             for (int x = 0; x < W; ++x) {
               uint64_t m = a.e1[x];
@@ -3611,8 +3622,8 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgR
               while (m) {
                 const int bit = __ffsll((long long)m) - 1, o = 64 * x + bit;
                 m &= m - 1;
-                atomicAdd(T2 + canon4(g.ie, g.je, o, o) * KP + q, ((a.e2[x] >> bit) & 1ull) ? 2.0 * w : w);
-                if ((both >> bit) & 1ull) atomicAdd(T2 + canon4(g.ie, o, o, g.je) * KP + q, -w);
+                atomicAdd(T2 + canon4(g.ie, g.je, o, o) * KP + q, ((a.e2[x] >> bit) & 1ull) ? w2 : w);
+                if ((both >> bit) & 1ull) atomicAdd(T2 + canon4(g.ie, o, o, g.je) * KP + q, nw);
               }
             }
           }
