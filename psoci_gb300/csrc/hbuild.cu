@@ -393,7 +393,7 @@ struct JoinTabs {
   const int64_t *goff;    // per hi pattern g: its list of hi patterns h to visit ...
   const uint32_t *glist;  // ... h | d_hi(g, h) << 28, ascending h
   const uint32_t *dkept;  // double_block_kept of (ex0 <= ex1) -> (jy0 <= jy1), bit tri(ex)*NT + tri(jy)
-  int64_t nt;             // NT = nbf(nbf+1)/2
+  int64_t nt;             // NT = nbf(nbf+1)/2; at most 128 orbitals, so NT^2 bits have 32-bit places
 };
 
 // The pruning decision of every double excitation, as bits: word q holds the pairs
@@ -488,15 +488,22 @@ struct JoinSlab {
   int64_t cap;
   int64_t *start;  // [nconf] slab position of each configuration's list
 };
-constexpr int JOIN_CHUNK = 4096;
+constexpr int JOIN_CHUNK = 4096, JOIN_ALONE = -1;
 
+// One warp a configuration, lanes over its lookups in (hi pattern, lo pattern) order.  Bound by
+// instruction issue (67% of the slots) and the lookups' latency: 1.04 G lookups of mrcisd_6e8o_v48,
+// of which 181 M pairs stay, 9.9 -> 7.7 ms with a lookup's run found by ballot instead of a binary
+// search, the orbitals of two electrons taken as the lowest and the highest set bit (9.9 -> 8.7), and
+// the table T by hi pattern, so that a list's ascending lo patterns share its sectors (8.7 -> 7.7).
 template <int W, int MODE>
 __global__ void __launch_bounds__(256) k_join(Params P, JoinTabs J, int64_t *cnt, int64_t *ncand, const int64_t *off,
                                               JoinSlab S) {
-  __shared__ int s_pre[8][33], s_q0[8][32], s_lp[8][32], s_h[8][32];
-  __shared__ uint32_t s_hx[8][32];  // per hi pattern: its part of the excitation from i (see below)
-  __shared__ int s_hn[8][32];
+  // per hi pattern with lo patterns to visit: x, the first of them in J.ln less the first lookup (l_i
+  // itself when the hi patterns are disjoint); y, the pattern; z, w, its part of the excitation from
+  // i: orbitals, electrons (JOIN_ALONE when the hi patterns are disjoint)
+  __shared__ uint4 s_run[8][32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u, le = lt | (1u << lane);
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const uint32_t lomask = (1u << J.s) - 1u;
@@ -509,7 +516,7 @@ __global__ void __launch_bounds__(256) k_join(Params P, JoinTabs J, int64_t *cnt
     // orbitals come first in each list
     uint64_t g1[W], g2[W];
     hi_bits<W>(J.hdec[gi], J.s, g1, g2);
-    const uint32_t keyi = J.lokey[li], e1i = keyi & lomask, e2i = keyi >> J.s;
+    const uint32_t keyi = J.lokey[li];
     int64_t nk = 0, nc = 0;
     int64_t base = (MODE == 1) ? off[i] : 0;
     unsigned long long lstart = cursor;  // MODE 2: where this configuration's list begins
@@ -520,7 +527,8 @@ __global__ void __launch_bounds__(256) k_join(Params P, JoinTabs J, int64_t *cnt
       // hi patterns are disjoint: those blocks passed the integral test when the list was
       // built)
       int h = 0;
-      int len = 0, q0 = 0, lp0 = li;
+      int len = 0, q0 = li, hn = JOIN_ALONE;
+      uint32_t hx = 0u;
       if (h0 + lane < gl1) {
         const uint32_t ent = J.glist[h0 + lane];
         h = (int)(ent & 0x0fffffffu);
@@ -528,7 +536,7 @@ __global__ void __launch_bounds__(256) k_join(Params P, JoinTabs J, int64_t *cnt
         const int tau = 4 - d;
         const int code = J.hdec[h];
         const int k = ne_i - hi_electrons(code) + 2;  // lo electrons of l' minus l_i's, + 2
-        if (tau <= 0) { len = (k == 2); q0 = -1; }
+        if (tau <= 0) len = (k == 2);
         else {
           const int64_t at = (int64_t)(tau - 1) * (5 * (int64_t)J.L + 1) + 5 * (int64_t)li + k;
           q0 = J.lnoff[at];
@@ -538,9 +546,9 @@ __global__ void __launch_bounds__(256) k_join(Params P, JoinTabs J, int64_t *cnt
           uint64_t b1[W], b2[W];
           hi_bits<W>(code, J.s, b1, b2);
           int x0, x1, y0, y1;
-          s_hn[wib][lane] = excitation_r<W>(g1, g2, b1, b2, x0, x1, y0, y1);
-          s_hx[wib][lane] = (uint32_t)(x0 & 0xff) | ((uint32_t)(x1 & 0xff) << 8) | ((uint32_t)(y0 & 0xff) << 16) |
-                            ((uint32_t)(y1 & 0xff) << 24);
+          hn = excitation_r<W>(g1, g2, b1, b2, x0, x1, y0, y1);
+          hx = (uint32_t)(x0 & 0xff) | ((uint32_t)(x1 & 0xff) << 8) | ((uint32_t)(y0 & 0xff) << 16) |
+               ((uint32_t)(y1 & 0xff) << 24);
         }
       }
       int incl = len;
@@ -550,54 +558,50 @@ __global__ void __launch_bounds__(256) k_join(Params P, JoinTabs J, int64_t *cnt
         if (lane >= o) incl += v;
       }
       const int tot = __shfl_sync(0xffffffffu, incl, 31);
-      s_pre[wib][lane] = incl - len;
-      s_q0[wib][lane] = q0;
-      s_lp[wib][lane] = lp0;
-      s_h[wib][lane] = h;
+      const int st = incl - len;
+      const unsigned runs = __ballot_sync(0xffffffffu, len > 0);
+      if (len > 0)
+        s_run[wib][__popc(runs & lt)] = make_uint4((uint32_t)(hn == JOIN_ALONE ? q0 : q0 - st), (uint32_t)h, hx, (uint32_t)hn);
       __syncwarp();
-      // the chunk's lookups, spread evenly over the lanes in (h, l') order
+      // the chunk's lookups, spread evenly over the lanes in (h, l') order; a lookup's run is the
+      // last that starts at or before it
+      int started = 0;
       for (int e0 = 0; e0 < tot; e0 += 32) {
-        const int e = e0 + lane;
+        const unsigned bw =
+            __reduce_or_sync(0xffffffffu, (len > 0 && (unsigned)(st - e0) < 32u) ? 1u << ((st - e0) & 31) : 0u);
         bool found = false, keep = false;
         int j = -1;
-        if (e < tot) {
-          int o = 0;
-#pragma unroll
-          for (int st = 16; st > 0; st >>= 1)
-            if (s_pre[wib][o + st] <= e) o += st;
-          const int qo = s_q0[wib][o], ho = s_h[wib][o];
-          const int lp = (qo < 0) ? s_lp[wib][o] : J.ln[qo + (e - s_pre[wib][o])];
-          j = J.T[(int64_t)lp * J.G + ho];
-          if (j >= 0) {
-            found = true;
-            keep = true;
-            if (j != (int)i && qo >= 0) {
-              // lo part from the keys (bit q: orbital q occupied; bit s + q: doubly)
-              const uint32_t key = J.lokey[lp], e1j = key & lomask, e2j = key >> J.s;
-              const uint32_t i1 = e1i & ~e1j, i2 = e2i & ~e2j, j1 = e1j & ~e1i, j2 = e2j & ~e2i;
-              const int lni = __popc(i1) + __popc(i2), lnj = __popc(j1) + __popc(j2);
-              const int ni = lni + s_hn[wib][o];
-              const uint32_t hx = s_hx[wib][o];
-              const int hx0 = (int)(hx & 0xffu), hx1 = (int)((hx >> 8) & 0xffu);
-              const int hy0 = (int)((hx >> 16) & 0xffu), hy1 = (int)(hx >> 24);
-              // first two orbitals of each list: lo ones (a doubly emptied / filled orbital
-              // twice), then hi ones
-              const int la0 = __ffs(i1 | i2) - 1, lb0 = __ffs(j1 | j2) - 1;
-              const int la1 = (lni < 2) ? -1 : ((i1 & i2) >> la0) & 1u ? la0 : __ffs((i1 | i2) & ~(1u << la0)) - 1;
-              const int lb1 = (lnj < 2) ? -1 : ((j1 & j2) >> lb0) & 1u ? lb0 : __ffs((j1 | j2) & ~(1u << lb0)) - 1;
-              const int ex0 = (lni >= 1) ? la0 : hx0, jy0 = (lnj >= 1) ? lb0 : hy0;
-              const int ex1 = (lni >= 2) ? la1 : (lni == 1) ? hx0 : hx1;
-              const int jy1 = (lnj >= 2) ? lb1 : (lnj == 1) ? hy0 : hy1;
+        if (e0 + lane < tot) {
+          const uint4 u = s_run[wib][started + __popc(bw & le) - 1];
+          const bool alone = (int)u.w == JOIN_ALONE;
+          const int lp = alone ? (int)u.x : __ldg(J.ln + (int)u.x + (e0 + lane));
+          j = __ldg(J.T + ((int64_t)u.y * J.L + lp));
+          found = keep = j >= 0;
+          if (found && j != (int)i && !alone) {
+            // lo part from the keys (bit q: orbital q occupied; bit s + q: doubly)
+            const uint32_t keyj = __ldg(J.lokey + lp), di = keyi & ~keyj, dj = keyj & ~keyi;
+            const int lni = __popc(di), ni = lni + (int)u.w;
+            if (ni <= 2) {
+              // first two orbitals of each list: lo ones (of two electrons the lowest and the highest
+              // orbital, the same if they share one), then hi ones
+              const uint32_t ui = (di | (di >> J.s)) & lomask, uj = (dj | (dj >> J.s)) & lomask;
+              const int lnj = __popc(dj);
+              const int ex0 = lni >= 1 ? __ffs(ui) - 1 : (int)(u.z & 0xffu);
+              const int jy0 = lnj >= 1 ? __ffs(uj) - 1 : (int)((u.z >> 16) & 0xffu);
               // the tests below are symmetric in the two configurations' roles
               if (ni == 2) {
-                const int64_t e = ((int64_t)ex1 * (ex1 + 1) / 2 + ex0) * J.nt + (int64_t)jy1 * (jy1 + 1) / 2 + jy0;
-                keep = (__ldg(J.dkept + (e >> 5)) >> (e & 31)) & 1u;
+                const int ex1 = lni >= 2 ? 31 - __clz(ui) : (int)((lni == 1 ? u.z : u.z >> 8) & 0xffu);
+                const int jy1 = lnj >= 2 ? 31 - __clz(uj) : (int)((lnj == 1 ? u.z >> 16 : u.z >> 24) & 0xffu);
+                const uint32_t at = (uint32_t)(ex1 * (ex1 + 1) / 2 + ex0) * (uint32_t)J.nt +
+                                    (uint32_t)(jy1 * (jy1 + 1) / 2 + jy0);
+                keep = (__ldg(J.dkept + (at >> 5)) >> (at & 31u)) & 1u;
               } else if (ni == 1 && __ldg(P.jsym + j) != js_i) {
                 keep = __ldg(P.one + tri64(ex0, jy0)) != 0.0;
               }
             }
           }
         }
+        started += __popc(bw);
         const unsigned kb = __ballot_sync(0xffffffffu, keep);
         if (MODE == 0) {
           nc += __popc(__ballot_sync(0xffffffffu, found));
@@ -2656,10 +2660,10 @@ void psoci_join_release(psoci_ctx *c) {
 // is used.  Not qualifying is not an error.
 namespace {
 // the configuration of each (lo pattern, hi pattern) cell; the pairs are unique
-__global__ void k_fill_T(int n, const int32_t *__restrict__ gid, const int32_t *__restrict__ lid, int64_t G,
+__global__ void k_fill_T(int n, const int32_t *__restrict__ gid, const int32_t *__restrict__ lid, int64_t L,
                          int32_t *__restrict__ T) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    T[(int64_t)lid[i] * G + gid[i]] = i;
+    T[(int64_t)gid[i] * L + lid[i]] = i;
 }
 }  // namespace
 
@@ -2820,10 +2824,10 @@ psoci_status psoci_join_prepare(psoci_ctx *c) {
   cudaStream_t q = c->stream;
   PSOCI_CUDA(c, cudaMemcpyAsync(c->d_jgid, gid.data(), 4 * gid.size(), cudaMemcpyHostToDevice, q));
   PSOCI_CUDA(c, cudaMemcpyAsync(c->d_jlid, lid.data(), 4 * lid.size(), cudaMemcpyHostToDevice, q));
-  // T[lo pattern][hi pattern] = configuration (or -1), filled on the device
+  // T[hi pattern][lo pattern] = configuration (or -1), filled on the device
   PSOCI_CUDA(c, cudaMemsetAsync(c->d_jT, 0xff, sizeof(int32_t) * (size_t)(G * L), q));
   psoci_note_launch();
-  k_fill_T<<<(n + 255) / 256, 256, 0, q>>>(n, c->d_jgid, c->d_jlid, G, c->d_jT);
+  k_fill_T<<<(n + 255) / 256, 256, 0, q>>>(n, c->d_jgid, c->d_jlid, L, c->d_jT);
   PSOCI_CUDA(c, cudaGetLastError());
   PSOCI_CUDA(c, cudaMemcpyAsync(c->d_jlnoff, lnoff.data(), 4 * lnoff.size(), cudaMemcpyHostToDevice, q));
   PSOCI_CUDA(c, cudaMemcpyAsync(c->d_jln, ln.data(), 4 * std::max<size_t>(ln.size(), 1), cudaMemcpyHostToDevice, q));
