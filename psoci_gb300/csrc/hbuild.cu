@@ -2665,6 +2665,52 @@ __global__ void k_fill_T(int n, const int32_t *__restrict__ gid, const int32_t *
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     T[(int64_t)gid[i] * L + lid[i]] = i;
 }
+
+// lo patterns within tau = 1..4 of each lo pattern (itself included), ascending inside each of five
+// groups: the lo electron count minus l's, -2..2 (a hi pattern holds 0-2 electrons, so a partner lo
+// pattern differs by at most 2; the others never make a configuration and are left out).  Lists
+// tau-major, then by pattern, then by group.  One warp a pattern, lanes over the others; MODE 0
+// counts to out[((tau - 1) * L + l) * 5 + k], MODE 1 writes the lists.  (On the host's cores the L^2
+// distances took 2 of the 4.6 ms of psoci_set_configs at mrcis_6e8o_v40.)
+constexpr int LN_GRP = 5, LN_TAU = 4;
+template <int MODE>
+__global__ void __launch_bounds__(256) k_lo_lists(int L, const uint32_t *__restrict__ key, const int32_t *__restrict__ off,
+                                                  int32_t *__restrict__ out) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), nwarps = (int)((gridDim.x * blockDim.x) >> 5);
+  for (int l = warp; l < L; l += nwarps) {
+    const uint32_t kl = key[l];
+    const int nel = __popc(kl);
+    // lane LN_GRP (tau - 1) + k: this list's entries, or its next place
+    const int t = lane / LN_GRP, g = lane - LN_GRP * t;
+    const int64_t own = t < LN_TAU ? (int64_t)t * LN_GRP * L + (int64_t)LN_GRP * l + g : 0;
+    int n = (MODE == 1 && t < LN_TAU) ? off[own + t] : 0;
+    for (int m0 = 0; m0 < L; m0 += 32) {
+      const int m = m0 + lane;
+      int d = LN_TAU + 1, k = 0;
+      if (m < L) {
+        const uint32_t km = key[m];
+        k = __popc(km) - nel + 2;
+        d = (k < 0 || k >= LN_GRP) ? LN_TAU + 1 : max(__popc(kl ^ km), 1);
+      }
+      if (!__any_sync(FULL, d <= LN_TAU)) continue;
+#pragma unroll
+      for (int tt = 0; tt < LN_TAU; ++tt)
+#pragma unroll
+        for (int kk = 0; kk < LN_GRP; ++kk) {
+          const bool in = d <= tt + 1 && k == kk;
+          const unsigned b = __ballot_sync(FULL, in);
+          if (MODE == 1) {
+            const int at = __shfl_sync(FULL, n, LN_GRP * tt + kk);
+            if (in) out[at + __popc(b & ((1u << lane) - 1u))] = m;
+          }
+          if (lane == LN_GRP * tt + kk) n += __popc(b);
+        }
+    }
+    if (MODE == 0 && t < LN_TAU) out[own] = n;
+  }
+}
 }  // namespace
 
 psoci_status psoci_join_prepare(psoci_ctx *c) {
@@ -2769,59 +2815,44 @@ psoci_status psoci_join_prepare(psoci_ctx *c) {
   for (int b = 0; b < nh; ++b)
     for (int a = 0; a <= b; ++a)
       hdec[1 + nh + (size_t)b * (b + 1) / 2 + a] = (a == b) ? (3 | (a << 8)) : (2 | (a << 8) | (b << 20));
-  // lo patterns within tau = 1..4 of each lo pattern (itself included), ascending inside
-  // each of five groups: the lo electron count minus l's, -2..2 (a hi pattern holds 0-2
-  // electrons, so a partner lo pattern differs by at most 2; the others never make a
-  // configuration and are left out).  Lists tau-major, then by pattern, then by group; one
-  // distance per pair, counted then written in parallel.
-  constexpr int NGRP = 5;
-  std::vector<int32_t> lnoff(4 * (NGRP * L + 1)), ln, lcnt((size_t)4 * NGRP * L, 0);
-  psoci_parallel_ranges(L, [&](int64_t lo, int64_t hi, int) {
-    for (int64_t l = lo; l < hi; ++l) {
-      const int nel = __builtin_popcount(lokey[l]);
-      for (int64_t m = 0; m < L; ++m) {
-        const int k = __builtin_popcount(lokey[m]) - nel + 2;
-        if (k < 0 || k >= NGRP) continue;
-        const int d = __builtin_popcount(lokey[l] ^ lokey[m]);
-        for (int tau = std::max(d, 1); tau <= 4; ++tau) ++lcnt[((size_t)(tau - 1) * L + l) * NGRP + k];
-      }
-    }
-  }, 64);
-  {
-    int64_t run = 0;
-    for (int tau = 1; tau <= 4; ++tau) {
-      for (int64_t g = 0; g < NGRP * L; ++g) {
-        lnoff[(tau - 1) * (NGRP * L + 1) + g] = (int32_t)run;
-        run += lcnt[(size_t)(tau - 1) * NGRP * L + g];
-      }
-      lnoff[(tau - 1) * (NGRP * L + 1) + NGRP * L] = (int32_t)run;
-    }
-    if (run > INT32_MAX) return PSOCI_OK;
-    ln.resize((size_t)run);
-  }
-  psoci_parallel_ranges(L, [&](int64_t lo, int64_t hi, int) {
-    for (int64_t l = lo; l < hi; ++l) {
-      const int nel = __builtin_popcount(lokey[l]);
-      int32_t pos[4][NGRP];
-      for (int tau = 1; tau <= 4; ++tau)
-        for (int k = 0; k < NGRP; ++k) pos[tau - 1][k] = lnoff[(tau - 1) * (NGRP * L + 1) + NGRP * l + k];
-      for (int64_t m = 0; m < L; ++m) {
-        const int k = __builtin_popcount(lokey[m]) - nel + 2;
-        if (k < 0 || k >= NGRP) continue;
-        const int d = __builtin_popcount(lokey[l] ^ lokey[m]);
-        for (int tau = std::max(d, 1); tau <= 4; ++tau) ln[pos[tau - 1][k]++] = (int32_t)m;
-      }
-    }
-  }, 64);
+  // lists of lo patterns (k_lo_lists): counted, their places summed here, then written
+  std::vector<int32_t> lnoff((size_t)LN_TAU * (LN_GRP * L + 1)), lcnt((size_t)LN_TAU * LN_GRP * L);
+  cudaStream_t q = c->stream;
   psoci_status st;
+  int32_t *d_cnt = nullptr;
+  const int lblocks = (int)std::min<int64_t>((L + 7) / 8, 152 * 8);
+  auto fail = [&](psoci_status r) {
+    psoci_free(d_cnt);
+    psoci_join_release(c);
+    return r;
+  };
+  if ((st = psoci_alloc(c, &c->d_jlokey, lokey.size())) || (st = psoci_alloc(c, &d_cnt, lcnt.size()))) return fail(st);
+  cudaError_t e = cudaMemcpyAsync(c->d_jlokey, lokey.data(), 4 * lokey.size(), cudaMemcpyHostToDevice, q);
+  if (e == cudaSuccess) {
+    psoci_note_launch();
+    k_lo_lists<0><<<lblocks, 256, 0, q>>>((int)L, c->d_jlokey, nullptr, d_cnt);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(lcnt.data(), d_cnt, 4 * lcnt.size(), cudaMemcpyDeviceToHost, q);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(q);
+  if (e != cudaSuccess) return fail(psoci_cuda_fail(c, e, "lookup screen"));
+  psoci_free(d_cnt);
+  int64_t nln = 0;
+  for (int tau = 1; tau <= LN_TAU; ++tau) {
+    for (int64_t g = 0; g < LN_GRP * L; ++g) {
+      lnoff[(tau - 1) * (LN_GRP * L + 1) + g] = (int32_t)nln;
+      nln += lcnt[(size_t)(tau - 1) * LN_GRP * L + g];
+    }
+    lnoff[(tau - 1) * (LN_GRP * L + 1) + LN_GRP * L] = (int32_t)nln;
+    if (nln > INT32_MAX) {
+      psoci_join_release(c);
+      return PSOCI_OK;
+    }
+  }
   if ((st = psoci_alloc(c, &c->d_jgid, n)) || (st = psoci_alloc(c, &c->d_jlid, n)) ||
       (st = psoci_alloc(c, &c->d_jT, (size_t)(G * L))) || (st = psoci_alloc(c, &c->d_jlnoff, lnoff.size())) ||
-      (st = psoci_alloc(c, &c->d_jln, ln.size())) || (st = psoci_alloc(c, &c->d_jhdec, hdec.size())) ||
-      (st = psoci_alloc(c, &c->d_jlokey, lokey.size()))) {
-    psoci_join_release(c);
-    return st;
-  }
-  cudaStream_t q = c->stream;
+      (st = psoci_alloc(c, &c->d_jln, (size_t)nln)) || (st = psoci_alloc(c, &c->d_jhdec, hdec.size())))
+    return fail(st);
   PSOCI_CUDA(c, cudaMemcpyAsync(c->d_jgid, gid.data(), 4 * gid.size(), cudaMemcpyHostToDevice, q));
   PSOCI_CUDA(c, cudaMemcpyAsync(c->d_jlid, lid.data(), 4 * lid.size(), cudaMemcpyHostToDevice, q));
   // T[hi pattern][lo pattern] = configuration (or -1), filled on the device
@@ -2830,9 +2861,10 @@ psoci_status psoci_join_prepare(psoci_ctx *c) {
   k_fill_T<<<(n + 255) / 256, 256, 0, q>>>(n, c->d_jgid, c->d_jlid, L, c->d_jT);
   PSOCI_CUDA(c, cudaGetLastError());
   PSOCI_CUDA(c, cudaMemcpyAsync(c->d_jlnoff, lnoff.data(), 4 * lnoff.size(), cudaMemcpyHostToDevice, q));
-  PSOCI_CUDA(c, cudaMemcpyAsync(c->d_jln, ln.data(), 4 * std::max<size_t>(ln.size(), 1), cudaMemcpyHostToDevice, q));
+  psoci_note_launch();
+  k_lo_lists<1><<<lblocks, 256, 0, q>>>((int)L, c->d_jlokey, c->d_jlnoff, c->d_jln);
+  PSOCI_CUDA(c, cudaGetLastError());
   PSOCI_CUDA(c, cudaMemcpyAsync(c->d_jhdec, hdec.data(), 4 * hdec.size(), cudaMemcpyHostToDevice, q));
-  PSOCI_CUDA(c, cudaMemcpyAsync(c->d_jlokey, lokey.data(), 4 * lokey.size(), cudaMemcpyHostToDevice, q));
   PSOCI_CUDA(c, cudaStreamSynchronize(q));
   c->join_s = s; c->join_nh = nh; c->join_G = (int)G; c->join_L = (int)L;
   c->join_ok = true;
