@@ -29,8 +29,12 @@
 #include <type_traits>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "ffmath.cuh"
 #include "psoci_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -347,10 +351,13 @@ __global__ void k_precond(int64_t n, int nr, const double *__restrict__ R, const
 // Cholesky pivot falls below drop_tol^2 of its original norm (linear dependence).
 // One warp: lane c carries column c (each entry's sums in ascending row order, as a single thread
 // would form them; a single thread took 29 us for up to 8 columns, the warp 13 us).
-__global__ void k_cholqr_factor(const double *S, int b, const double *ref, int ldref, double drop_tol, double *F,
-                                int *nkept) {
-  __shared__ double Rm[16][17], Fi[16][17];
-  const int c = threadIdx.x;  // blockDim.x == 32
+struct CholSmem {
+  double Rm[16][17], Fi[16][17];
+};
+__device__ int cholqr_factor(CholSmem &sm, const double *S, int b, const double *ref, int ldref, double drop_tol,
+                             double *F) {
+  auto &Rm = sm.Rm, &Fi = sm.Fi;
+  const int c = threadIdx.x & 31;
   if (c < 16)
     for (int i = 0; i < 16; ++i) Rm[i][c] = Fi[i][c] = 0.0;
   __syncwarp();
@@ -390,7 +397,211 @@ __global__ void k_cholqr_factor(const double *S, int b, const double *ref, int l
     const int to = k ? __popc(keep & ((1u << c) - 1u)) : nk + __popc(~keep & ((1u << c) - 1u));
     for (int i = 0; i < b; ++i) F[i * b + to] = k ? Fi[i][c] : 0.0;
   }
-  if (c == 0) *nkept = nk;
+  return nk;
+}
+
+__global__ void k_cholqr_factor(const double *S, int b, const double *ref, int ldref, double drop_tol, double *F,
+                                int *nkept) {
+  __shared__ CholSmem sm;
+  const int nk = cholqr_factor(sm, S, b, ref, ldref, drop_tol, F);  // blockDim.x == 32
+  if (threadIdx.x == 0) *nkept = nk;
+}
+
+// ------------------------------------------------------------------------------------
+// The whole orthonormalisation of a new block against a small basis (at most OC_ROWS rows) in
+// one kernel, a cluster of OC_CTAS CTAs that hold the new block's rows in shared memory: two
+// projections and two Cholesky-QR passes, the steps of orthonormalize().  As separate kernels
+// they were 16 launches, 110 us of kernel time at 2,044 rows and 4 roots, and two waits for the
+// host; this is one of 44 us.  The sums of the CTAs meet in distributed shared memory, added by
+// every CTA in the same order, so all take the same decisions; float-float sums over a share of
+// the rows, combined in FP64, as in k_tn and k_nn.  Bound by the latency of the small steps (the
+// factors take 12 us) and, towards 4,096 rows, by the float-float arithmetic of 16 SMs.
+//   With a CTA's conversions to FP64 after every row or two, its rows of V read from global memory
+// in each step, and 128 shares added one by one it took 105 us.
+// ------------------------------------------------------------------------------------
+constexpr int OC_CTAS = 16, OC_THREADS = 512, OC_MAXR = 256, OC_ROWS = OC_CTAS * OC_MAXR;
+constexpr int OC_SUMS = (MAX_SUB + 16) * 16;
+
+struct __align__(16) OcSmem {
+  double sums[2][OC_SUMS];      // this CTA's sums, two phases in turn (peers read them)
+  float2 Cf[MAX_SUB * 16];      // coefficients, split, zero-padded to kq columns
+  double red[OC_THREADS * 4];
+  double S[256], ref[256], F[256];
+  CholSmem chol;
+  int nk;
+};
+// followed by the CTA's rows of T, split (kq float pairs a row) and in FP64 (b a row), and, where
+// they fit, its rows of V, split (an odd number of pairs a row: no bank conflicts down a column)
+constexpr size_t OC_SMEM_MAX = 227 * 1024;
+int oc_per(int64_t n) { return (int)((n + OC_CTAS - 1) / OC_CTAS); }
+size_t oc_smem(int64_t n, int m, int b, bool &staged) {
+  const size_t per = oc_per(n), base = sizeof(OcSmem) + per * 8 * (size_t)(((b + 3) & ~3) + b);
+  const size_t all = base + per * 8 * (size_t)(m | 1);
+  staged = m > 0 && all <= OC_SMEM_MAX;
+  return staged ? all : base;
+}
+
+// four consecutive float pairs
+__device__ __forceinline__ void oc_load4(const float2 *p, float2 (&v)[4]) {
+  const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
+  v[0] = make_float2(a.x, a.y); v[1] = make_float2(a.z, a.w);
+  v[2] = make_float2(b.x, b.y); v[3] = make_float2(b.z, b.w);
+}
+
+// out[i * k + j] = sum over this CTA's rows of a(r, i) * T[r, j], i < m.  A thread takes four columns
+// of an i over every S-th row, eight rows or more (a share's combination in FP64 costs as much as
+// several rows).
+template <typename LOAD>
+__device__ void oc_tn(OcSmem &s, const float2 *Tf, int kq, int rows, int per, int m, int k, LOAD a, double *out) {
+  const int tid = threadIdx.x, ng = (k + 3) >> 2;
+  const int G = m * ng, S = max(1, min(OC_THREADS / G, per >> 3));  // G <= (MAX_SUB + 16) * 4
+  const int g = tid % G, sub = tid / G, i = g % m, jb = g / m;
+  if (sub < S) {
+    float h[4] = {0.f, 0.f, 0.f, 0.f}, l[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int r = sub; r < rows; r += S) {
+      float2 b[4];
+      const float2 v = a(r, i);
+      oc_load4(Tf + r * kq + 4 * jb, b);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ff_fma(h[j], l[j], v, b[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      ff_renorm(h[j], l[j]);
+      s.red[(sub * G + g) * 4 + j] = (double)h[j] + (double)l[j];
+    }
+  }
+  __syncthreads();
+  for (int o = tid; o < G * 4; o += OC_THREADS) {
+    const int g2 = o >> 2, jj = (g2 / m) * 4 + (o & 3);
+    if (jj >= k) continue;
+    double v = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < S; ++q) v += s.red[q * G * 4 + o];
+    out[(g2 % m) * k + jj] = v;
+  }
+  __syncthreads();
+}
+
+// sum of an entry of the CTAs' sums, in their order
+__device__ __forceinline__ double oc_total(cg::cluster_group &cl, double *sums, int o) {
+  double v[OC_CTAS], t = 0.0;
+#pragma unroll
+  for (int q = 0; q < OC_CTAS; ++q) v[q] = *cl.map_shared_rank(sums + o, q);
+#pragma unroll
+  for (int q = 0; q < OC_CTAS; ++q) t += v[q];
+  return t;
+}
+
+// out(r, j, sum over i < m of a(r, i) * Cf[i, j]) for this CTA's rows; a thread takes a row and four
+// columns
+template <typename LOAD, typename STORE>
+__device__ void oc_nn(OcSmem &s, int kq, int rows, int m, int k, LOAD a, STORE out) {
+  for (int e = threadIdx.x; e < rows * ((k + 3) >> 2); e += OC_THREADS) {
+    const int j0 = 4 * (e / rows), r = e % rows;
+    float h[4] = {0.f, 0.f, 0.f, 0.f}, l[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int i = 0; i < m; ++i) {
+      float2 y[4];
+      const float2 v = a(r, i);
+      oc_load4(s.Cf + i * kq + j0, y);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ff_fma(h[j], l[j], v, y[j]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (j0 + q < k) out(r, j0 + q, (double)h[q] + (double)l[q]);
+  }
+  __syncthreads();
+}
+
+// T[:, 0:b] against V[:, 0:m] and within itself; the kept columns to V[:, m:m+nk]
+template <bool STAGED>
+__global__ void __launch_bounds__(OC_THREADS) k_ortho_cluster(int64_t n, double *V, int ld, int m,
+                                                              const double *__restrict__ Tin, int ldt, int b,
+                                                              double drop_tol, int *nkept) {
+  extern __shared__ __align__(16) unsigned char oc_raw[];
+  OcSmem &s = *reinterpret_cast<OcSmem *>(oc_raw);
+  cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x, rank = (int)cl.block_rank();
+  const int per = (int)((n + OC_CTAS - 1) / OC_CTAS);
+  const int64_t r0 = min(n, (int64_t)rank * per);
+  const int rows = (int)(min(n, r0 + per) - r0);
+  const int kq = (b + 3) & ~3, vs = m | 1;
+  float2 *Tf = reinterpret_cast<float2 *>(&s + 1);
+  double *T = reinterpret_cast<double *>(Tf + per * kq);
+  float2 *Vs = reinterpret_cast<float2 *>(T + per * b);
+  const double *Vr = V + r0 * ld;
+  auto v_at = [&](int r, int i) { return STAGED ? Vs[r * vs + i] : split_f64(__ldg(Vr + (int64_t)r * ld + i)); };
+  auto t_at = [&](int r, int i) { return Tf[r * kq + i]; };
+  auto split_rows = [&](int k) {
+    for (int e = tid; e < rows * kq; e += OC_THREADS) {
+      const int r = e / kq, j = e - r * kq;
+      Tf[e] = j < k ? split_f64(T[r * b + j]) : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+  };
+  // the CTAs' sums of a phase are complete; the buffer of the phase before is free for the next
+  int ph = 0;
+  auto meet = [&]() -> double * {
+    cl.sync();
+    double *p = s.sums[ph];
+    ph ^= 1;
+    return p;
+  };
+  for (int e = tid; e < rows * b; e += OC_THREADS) T[e] = Tin[(r0 + e / b) * ldt + e % b];
+  if (STAGED)
+    for (int e = tid; e < rows * m; e += OC_THREADS) {
+      const int r = e / m, i = e - r * m;
+      Vs[r * vs + i] = split_f64(__ldg(Vr + (int64_t)r * ld + i));
+    }
+  __syncthreads();
+  split_rows(b);
+  // two projections; the squared norms before them with the first
+  for (int pass = 0; pass < (m > 0 ? 2 : 1); ++pass) {
+    oc_tn(s, Tf, kq, rows, per, pass == 0 ? m + b : m, b,
+          [&](int r, int i) { return i < m ? v_at(r, i) : t_at(r, i - m); }, s.sums[ph]);
+    double *sums = meet();
+    if (pass == 0)
+      for (int o = tid; o < b; o += OC_THREADS) s.ref[o * b + o] = oc_total(cl, sums, (m + o) * b + o);
+    if (m > 0) {
+      for (int e = tid; e < m * kq; e += OC_THREADS) {
+        const int i = e / kq, j = e - i * kq;
+        s.Cf[e] = j < b ? split_f64(oc_total(cl, sums, i * b + j)) : make_float2(0.f, 0.f);
+      }
+      __syncthreads();
+      oc_nn(s, kq, rows, m, b, v_at, [&](int r, int j, double x) { T[r * b + j] -= x; });
+      split_rows(b);
+    }
+  }
+  int nk = b;
+  for (int pass = 0; pass < 2 && nk > 0; ++pass) {
+    oc_tn(s, Tf, kq, rows, per, nk, nk, t_at, s.sums[ph]);
+    double *sums = meet();
+    for (int o = tid; o < nk * nk; o += OC_THREADS) s.S[o] = oc_total(cl, sums, o);
+    __syncthreads();
+    if (tid < 32) {
+      const int q = cholqr_factor(s.chol, s.S, nk, pass == 0 ? s.ref : nullptr, b, drop_tol, s.F);
+      if (tid == 0) s.nk = q;
+    }
+    __syncthreads();
+    const int nk2 = s.nk;
+    for (int e = tid; e < nk * kq; e += OC_THREADS) {
+      const int i = e / kq, j = e - i * kq;
+      s.Cf[e] = j < nk2 ? split_f64(s.F[i * nk + j]) : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    if (pass == 0) {
+      oc_nn(s, kq, rows, nk, nk2, t_at, [&](int r, int j, double x) { T[r * b + j] = x; });
+      split_rows(nk2);
+    } else {
+      oc_nn(s, kq, rows, nk, nk2, t_at, [&](int r, int j, double x) { V[(r0 + r) * ld + m + j] = x; });
+    }
+    nk = nk2;
+  }
+  if (rank == 0 && tid == 0) *nkept = nk;
+  cl.sync();  // no CTA ends while a peer reads its sums
 }
 
 // G (ld x ld): mirror new columns [m0, m1) into rows and symmetrise the new diagonal block
@@ -606,6 +817,7 @@ struct Work {
   // phase resolves; Ritz vectors, their images and collapses keep float-float sums, since
   // the residuals are formed from them
   bool lowp = false;
+  int cluster = -1;  // whether k_ortho_cluster runs here: not asked yet, no, yes
   std::vector<cudaEvent_t> ev;
   ~Work() {
     psoci_free(V); psoci_free(HV); psoci_free(G); psoci_free(Y); psoci_free(theta); psoci_free(X); psoci_free(HX);
@@ -682,12 +894,56 @@ psoci_status sigma_block(Work &w, const double *X, int ldx, double *Y, int ldy, 
   return s;
 }
 
+// k_ortho_cluster launched; false where the device has no room for its cluster
+bool ortho_cluster(Work &w, int m, int b, cudaError_t &e) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = OC_CTAS;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(OC_CTAS);
+  cfg.blockDim = dim3(OC_THREADS);
+  cfg.stream = w.c->stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (w.cluster < 0) {
+    w.cluster = 1;
+    cfg.dynamicSmemBytes = OC_SMEM_MAX;
+    for (auto k : {k_ortho_cluster<false>, k_ortho_cluster<true>}) {
+      int n = 0;
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OC_SMEM_MAX) != cudaSuccess ||
+          cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        w.cluster = 0;
+      }
+    }
+  }
+  if (!w.cluster) return false;
+  bool staged = false;
+  cfg.dynamicSmemBytes = oc_smem(w.N, m, b, staged);
+  psoci_note_launch();
+  e = cudaLaunchKernelEx(&cfg, staged ? k_ortho_cluster<true> : k_ortho_cluster<false>, w.N, w.V, w.ld, m,
+                         (const double *)w.T, w.nr, b, 1e-10, w.ibuf);
+  return true;
+}
+
 // orthonormalise T[:, 0:b] against V[:, 0:m] and within itself; kept columns land in
 // V[:, m:m+b'].  Returns b' through *bk.
 psoci_status orthonormalize(Work &w, int m, int b, int *bk) {
   psoci_ctx *c = w.c;
   psoci_status s;
   const int ld = w.ld, tld = w.nr;
+  // small bases: one kernel
+  cudaError_t e = cudaSuccess;
+  if (w.N <= OC_ROWS && m <= MAX_SUB && b >= 1 && b <= TN_MAXK && ortho_cluster(w, m, b, e)) {
+    int nk = 0;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&nk, w.ibuf, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e != cudaSuccess) return psoci_cuda_fail(c, e, "davidson: orthonormalisation");
+    *bk = nk;
+    return PSOCI_OK;
+  }
   // squared norms before the projection: a column that loses all but 1e-10 of its norm
   // against V (or the block's earlier columns) carries no new direction and is dropped
   double *ref = w.small + (size_t)ld * ld / 2;

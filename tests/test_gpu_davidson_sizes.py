@@ -43,3 +43,26 @@ def test_roots_by_guess_block(kw, ksym, mixed):
     r = c.davidson(3, rtol=1e-8, mixed=mixed)
     assert np.abs(r.evals - w[:3]).max() <= 1e-10
     c.close()
+
+
+@pytest.mark.parametrize("kw,nroots", [(dict(nbf=4, nelec=2), 1), (dict(nbf=5, nelec=3), 16), (dict(nbf=6, nelec=4), 9),
+                                       (dict(nbf=7, nelec=5), 16), (dict(nbf=8, nelec=5), 8), (dict(nbf=9, nelec=5), 3)])
+@pytest.mark.parametrize("max_subspace", [0, 48])
+def test_orthonormal_vectors(kw, nroots, max_subspace):
+    """Bases on both sides of 4,096 rows (one cluster's kernel below), 1 to 16 new vectors, with
+    collapses (48 vectors): vectors orthonormal to the float-float sums (2^-45 of at most 1, well
+    under 1e-12) and residuals as asked for."""
+    import scipy.sparse as sp
+
+    from psoci_gb300.inputs import make_problem
+
+    c = gpu_context(make_problem("fci", seed=5, **kw))
+    c.build_hamiltonian(mixed=False)
+    rp, ci, va = c.get_hamiltonian()
+    H = sp.csr_matrix((va, ci, rp), shape=(c.nsef, c.nsef))
+    nroots = min(nroots, c.nsef)
+    r = c.davidson(nroots, rtol=1e-8, mixed=False, max_subspace=max_subspace, want_vectors=True)
+    v = r.evecs.reshape(nroots, c.nsef)
+    assert np.abs(v @ v.T - np.eye(nroots)).max() <= 1e-12
+    assert np.linalg.norm(H @ v.T - v.T * r.evals, axis=0).max() <= 2e-8
+    c.close()
