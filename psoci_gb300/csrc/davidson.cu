@@ -66,42 +66,43 @@ __device__ __forceinline__ ts_elt<LOWP> ts_load(double x) {
   else return split_f64(x);
 }
 
-// 8 consecutive elements from 16-byte aligned shared memory
-template <bool LOWP>
-__device__ __forceinline__ void ts_load8(const ts_elt<LOWP> *p, ts_elt<LOWP> (&v)[8]) {
-  const float4 *q = reinterpret_cast<const float4 *>(p);
-  if constexpr (LOWP) {
-    const float4 u = q[0], w = q[1];
-    v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
-    v[4] = w.x; v[5] = w.y; v[6] = w.z; v[7] = w.w;
+// N (2, 4 or 8) consecutive elements from shared memory aligned to 2 of them
+template <bool LOWP, int N>
+__device__ __forceinline__ void ts_loadn(const ts_elt<LOWP> *p, ts_elt<LOWP> (&v)[N]) {
+  if constexpr (LOWP && N == 2) {
+    const float2 u = *reinterpret_cast<const float2 *>(p);
+    v[0] = u.x; v[1] = u.y;
+  } else if constexpr (LOWP) {
+#pragma unroll
+    for (int t = 0; t < N / 4; ++t) {
+      const float4 u = reinterpret_cast<const float4 *>(p)[t];
+      v[4 * t] = u.x; v[4 * t + 1] = u.y; v[4 * t + 2] = u.z; v[4 * t + 3] = u.w;
+    }
   } else {
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const float4 u = q[t];
+    for (int t = 0; t < N / 2; ++t) {
+      const float4 u = reinterpret_cast<const float4 *>(p)[t];
       v[2 * t] = make_float2(u.x, u.y);
       v[2 * t + 1] = make_float2(u.z, u.w);
     }
   }
 }
 
-// acc[j] += a * b[j] for the 8 outputs of a thread (float-float, or FP32 when LOWP)
-template <bool LOWP>
-__device__ __forceinline__ void ts_fma8(float (&h)[8], float (&l)[8], ts_elt<LOWP> a, const ts_elt<LOWP> (&b)[8]) {
+// acc[j] += a * b[j] for the N outputs of a thread (float-float, or FP32 when LOWP)
+template <bool LOWP, int N>
+__device__ __forceinline__ void ts_fman(float (&h)[N], float (&l)[N], ts_elt<LOWP> a, const ts_elt<LOWP> (&b)[N]) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int j = 0; j < N; ++j) {
     if constexpr (LOWP) h[j] = __fmaf_rn(a, b[j], h[j]);
     else ff_fma(h[j], l[j], a, b[j]);
   }
 }
 
-// Blocks of k_tn: 256 rows each, at most four blocks an SM; where that leaves SMs without a block,
-// 32 rows or more each.  With 256 rows a basis of 2,044 rows ran on 8 SMs, 16.5 us a product
-// (9.9 us now).  More blocks than this make the sum over them the longer part: 608 instead of 350
-// for 89,404 rows took k_reduce_partials from 6.6 to 8.2 us.
-int ts_blocks(int64_t n) {
-  const int64_t b = std::max((n + 255) / 256, std::min<int64_t>((n + 31) / 32, 152));
-  return (int)std::min<int64_t>(std::max<int64_t>(1, b), 152 * 4);
-}
+// Blocks of k_tn: 256 rows each, at most four blocks an SM.  The grouping of the sums fixes their
+// rounding, and with it the signs of Ritz vectors (the host's eigen-solve takes them from products
+// that vanish but for rounding, where the basis holds eigenvectors of the whole matrix): it does not
+// change with the launch shape below.
+int ts_blocks(int64_t n) { return (int)std::min<int64_t>(std::max<int64_t>(1, (n + 255) / 256), 152 * 4); }
 
 // partial[blk][i*k + j] = sum over the block's rows r of A[r, a0+i] * B[r, b0+j]
 // (m <= MAX_SUB, k <= TN_MAXK).  Thread: output group g = (i, jb), the 8 outputs
@@ -109,7 +110,9 @@ int ts_blocks(int64_t n) {
 // split into shared memory once, A is read from global memory (lanes of a warp take
 // consecutive i of one row).  The S shares of a group are added in FP64 at the end, in a
 // fixed order.
-template <bool LOWP>
+// NJ outputs a thread, gridDim.y = 8 / NJ CTAs for the 8 of a group: with all 8 a basis of 2,044 rows
+// ran on 8 SMs, 16.5 us a product of 32 and 4 columns (13.3 us with NJ = 2 on 32 SMs).
+template <bool LOWP, int NJ>
 __global__ void __launch_bounds__(TS_THREADS) k_tn(int64_t n, const double *__restrict__ A, int lda, int a0, int m,
                                                    const double *__restrict__ B, int ldb, int b0, int k,
                                                    double *__restrict__ partial, int64_t rows_per_blk) {
@@ -124,9 +127,10 @@ __global__ void __launch_bounds__(TS_THREADS) k_tn(int64_t n, const double *__re
   const int g = tid % G, sub = tid / G;
   const int i = g % m, jb = g / m;
   const bool act = sub < S;
-  float h[8], l[8], t[8];
+  const int j0 = 8 * jb + NJ * blockIdx.y;     // this thread's first output
+  float h[NJ], l[NJ], t[NJ];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) { h[j] = 0.f; l[j] = 0.f; }
+  for (int j = 0; j < NJ; ++j) { h[j] = 0.f; l[j] = 0.f; }
   const int64_t r0 = (int64_t)blockIdx.x * rows_per_blk;
   const int64_t r1 = min(n, r0 + rows_per_blk);
   const double *ai = A + a0 + i;
@@ -140,7 +144,7 @@ __global__ void __launch_bounds__(TS_THREADS) k_tn(int64_t n, const double *__re
     __syncthreads();
     if (act) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) t[j] = 0.f;
+      for (int j = 0; j < NJ; ++j) t[j] = 0.f;
       const double *ar = ai + rt * lda;
       int rr = sub;
       for (; rr + 3 * S < rows; rr += 4 * S) {  // four rows in flight
@@ -149,38 +153,39 @@ __global__ void __launch_bounds__(TS_THREADS) k_tn(int64_t n, const double *__re
         for (int u = 0; u < 4; ++u) av[u] = __ldg(ar + (int64_t)(rr + u * S) * lda);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          E b[8];
-          ts_load8<LOWP>(Bs + ((rr + u * S) << ksh) + 8 * jb, b);
-          if constexpr (LOWP) ts_fma8<true>(t, l, ts_load<true>(av[u]), b);
-          else ts_fma8<false>(h, l, ts_load<false>(av[u]), b);
+          E b[NJ];
+          ts_loadn<LOWP, NJ>(Bs + ((rr + u * S) << ksh) + j0, b);
+          if constexpr (LOWP) ts_fman<true, NJ>(t, l, ts_load<true>(av[u]), b);
+          else ts_fman<false, NJ>(h, l, ts_load<false>(av[u]), b);
         }
       }
       for (; rr < rows; rr += S) {
-        E b[8];
-        ts_load8<LOWP>(Bs + (rr << ksh) + 8 * jb, b);
-        if constexpr (LOWP) ts_fma8<true>(t, l, ts_load<true>(__ldg(ar + (int64_t)rr * lda)), b);
-        else ts_fma8<false>(h, l, ts_load<false>(__ldg(ar + (int64_t)rr * lda)), b);
+        E b[NJ];
+        ts_loadn<LOWP, NJ>(Bs + (rr << ksh) + j0, b);
+        if constexpr (LOWP) ts_fman<true, NJ>(t, l, ts_load<true>(__ldg(ar + (int64_t)rr * lda)), b);
+        else ts_fman<false, NJ>(h, l, ts_load<false>(__ldg(ar + (int64_t)rr * lda)), b);
       }
       if constexpr (LOWP)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ff_fma(h[j], l[j], make_float2(t[j], 0.f), make_float2(1.f, 0.f));
+        for (int j = 0; j < NJ; ++j) ff_fma(h[j], l[j], make_float2(t[j], 0.f), make_float2(1.f, 0.f));
 #pragma unroll
-      for (int j = 0; j < 8; ++j) ff_renorm(h[j], l[j]);
+      for (int j = 0; j < NJ; ++j) ff_renorm(h[j], l[j]);
     }
     __syncthreads();
   }
   // combine the S shares of each output in FP64 (the tile is no longer needed)
-  double *red = sm;  // [S][G][8]
+  double *red = sm;  // [S][G][NJ]
   if (act)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) red[(sub * G + g) * 8 + j] = (double)h[j] + (double)l[j];
+    for (int j = 0; j < NJ; ++j) red[(sub * G + g) * NJ + j] = (double)h[j] + (double)l[j];
   __syncthreads();
   const int nout = m * k;
-  for (int o = tid; o < G * 8; o += TS_THREADS) {
-    const int g2 = o >> 3, jj = (g2 / m) * 8 + (o & 7);
+  for (int o = tid; o < G * NJ; o += TS_THREADS) {
+    const int g2 = o / NJ, jj = (g2 / m) * 8 + NJ * blockIdx.y + (o % NJ);
     if (jj >= k) continue;
     double s = 0.0;
-    for (int q = 0; q < S; ++q) s += red[(q * G + g2) * 8 + (o & 7)];
+#pragma unroll 4
+    for (int q = 0; q < S; ++q) s += red[q * G * NJ + o];
     partial[(int64_t)blockIdx.x * nout + (g2 % m) * k + jj] = s;
   }
 }
@@ -244,17 +249,17 @@ __global__ void __launch_bounds__(NN_THREADS) k_nn(int64_t n, const double *__re
     for (; i + 1 < m; i += 2) {
       const double2 v = __ldg(reinterpret_cast<const double2 *>(ar + i));
       E y[8];
-      ts_load8<LOWP>(yj + i * kp, y);
-      ts_fma8<LOWP>(h, l, ts_load<LOWP>(v.x), y);
-      ts_load8<LOWP>(yj + (i + 1) * kp, y);
-      ts_fma8<LOWP>(h, l, ts_load<LOWP>(v.y), y);
+      ts_loadn<LOWP, 8>(yj + i * kp, y);
+      ts_fman<LOWP, 8>(h, l, ts_load<LOWP>(v.x), y);
+      ts_loadn<LOWP, 8>(yj + (i + 1) * kp, y);
+      ts_fman<LOWP, 8>(h, l, ts_load<LOWP>(v.y), y);
     }
   }
 #pragma unroll 4
   for (; i < m; ++i) {
     E y[8];
-    ts_load8<LOWP>(yj + i * kp, y);
-    ts_fma8<LOWP>(h, l, ts_load<LOWP>(__ldg(ar + i)), y);
+    ts_loadn<LOWP, 8>(yj + i * kp, y);
+    ts_fman<LOWP, 8>(h, l, ts_load<LOWP>(__ldg(ar + i)), y);
   }
   double *o = Out + r * ldo + o0 + 8 * jb;
 #pragma unroll
@@ -265,40 +270,89 @@ __global__ void __launch_bounds__(NN_THREADS) k_nn(int64_t n, const double *__re
   }
 }
 
-// R[r, j] = HX[r, j] - theta[j] * X[r, j]; partial squared norms per block.  A thread takes
-// whole rows (the nr values of a row are contiguous), so each row is read once.
-__global__ void k_residual(int64_t n, int nr, const double *__restrict__ X, const double *__restrict__ HX,
-                           const double *__restrict__ theta, double *__restrict__ R, double *__restrict__ partial) {
-  __shared__ double red[16][8];  // [root][warp], blockDim.x == 256
-  double th[16], s[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    th[j] = (j < nr) ? theta[j] : 0.0;
-    s[j] = 0.0;
-  }
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      if (j >= nr) break;
-      const double v = HX[r * nr + j] - th[j] * X[r * nr + j];
-      R[r * nr + j] = v;
-      s[j] = fma(v, v, s[j]);
-    }
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    if (j >= nr) break;
-    double v = s[j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[j][wid] = v;
+// Ritz vectors and residuals: X[r, j] = sum_i V[r, i] Y[i*ldy + j], R[r, j] = sum_i HV[r, i] Y[i*ldy + j]
+// - theta[j] * X[r, j], partial squared norms of R per block.  Float-float sums as in k_nn, a thread a
+// row and NJ outputs of both products; the images are not stored.  Bound by the float-float
+// arithmetic (13 FP32 instructions a product).  Two k_nn and a pass over their results took 54 us for
+// 89,404 rows and 8 roots, 38 us now (averages over the solve of mrcis_6e8o_v40); for 2,044 rows and
+// 4 roots 23 us, 9.8 now with two outputs a thread, so that the rows fill more SMs.
+template <int NJ>
+__global__ void __launch_bounds__(NN_THREADS) k_ritz(int64_t n, const double *__restrict__ V,
+                                                     const double *__restrict__ HV, int ld, int m,
+                                                     const double *__restrict__ Y, int ldy, int k,
+                                                     const double *__restrict__ theta, double *__restrict__ X,
+                                                     double *__restrict__ R, double *__restrict__ partial, int jbp) {
+  extern __shared__ double sm[];
+  __shared__ double red[NN_THREADS / 32][NJ];
+  const int kp = (k + 7) & ~7;
+  float2 *Ys = reinterpret_cast<float2 *>(sm);  // [m][kp]
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int e = tid; e < m * kp; e += NN_THREADS) {
+    const int i = e / kp, j = e - i * kp;
+    Ys[e] = (j < k) ? split_f64(Y[i * ldy + j]) : make_float2(0.f, 0.f);
   }
   __syncthreads();
-  if ((int)threadIdx.x < nr) {
+  const int TR = NN_THREADS / jbp;  // a multiple of 32: a warp has one group
+  const int rr = tid % TR, jb = tid / TR;
+  const float2 *yj = Ys + NJ * jb;
+  double s[NJ];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) s[j] = 0.0;
+  if (NJ * jb < k)
+    for (int64_t r = (int64_t)blockIdx.x * TR + rr; r < n; r += (int64_t)gridDim.x * TR) {
+      const double *ar = V + r * ld, *hr = HV + r * ld;
+      float xh[NJ], xl[NJ], hh[NJ], hl[NJ];
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) { xh[j] = xl[j] = hh[j] = hl[j] = 0.f; }
+      int i = 0;
+#pragma unroll 2
+      for (; i + 1 < m; i += 2) {  // rows start at even elements: ld is even
+        const double2 a = __ldg(reinterpret_cast<const double2 *>(ar + i));
+        const double2 h = __ldg(reinterpret_cast<const double2 *>(hr + i));
+        float2 y[NJ];
+        ts_loadn<false, NJ>(yj + i * kp, y);
+        ts_fman<false, NJ>(xh, xl, split_f64(a.x), y);
+        ts_fman<false, NJ>(hh, hl, split_f64(h.x), y);
+        ts_loadn<false, NJ>(yj + (i + 1) * kp, y);
+        ts_fman<false, NJ>(xh, xl, split_f64(a.y), y);
+        ts_fman<false, NJ>(hh, hl, split_f64(h.y), y);
+      }
+      if (i < m) {
+        float2 y[NJ];
+        ts_loadn<false, NJ>(yj + i * kp, y);
+        ts_fman<false, NJ>(xh, xl, split_f64(__ldg(ar + i)), y);
+        ts_fman<false, NJ>(hh, hl, split_f64(__ldg(hr + i)), y);
+      }
+      const int64_t o = r * k + NJ * jb;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        if (NJ * jb + j >= k) break;
+        const double x = (double)xh[j] + (double)xl[j], hx = (double)hh[j] + (double)hl[j];
+        const double v = hx - theta[NJ * jb + j] * x;
+        X[o + j] = x;
+        R[o + j] = v;
+        s[j] = fma(v, v, s[j]);
+      }
+    }
+  // the warp's sums: halving exchanges leave each lane one of the NJ, butterflies finish it
+#pragma unroll
+  for (int h = NJ / 2, o = 16; h > 0; h >>= 1, o >>= 1)
+#pragma unroll
+    for (int j = 0; j < h; ++j) {
+      const bool hi = lane & o;
+      const double keep = hi ? s[j + h] : s[j], give = hi ? s[j] : s[j + h];
+      s[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  double v = s[0];
+#pragma unroll
+  for (int o = 16 / NJ; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane % (32 / NJ) == 0) red[tid >> 5][lane / (32 / NJ)] = v;  // the lane's high bits are the output
+  __syncthreads();
+  if (tid < k) {
+    const int wpg = TR / 32, w0 = (tid / NJ) * wpg;
     double t = 0.0;
-    for (int w = 0; w < 8; ++w) t += red[threadIdx.x][w];
-    partial[(int64_t)blockIdx.x * nr + threadIdx.x] = t;
+    for (int w = 0; w < wpg; ++w) t += red[w0 + w][tid % NJ];
+    partial[(int64_t)blockIdx.x * k + tid] = t;
   }
 }
 
@@ -412,12 +466,11 @@ __global__ void k_cholqr_factor(const double *S, int b, const double *ref, int l
 // one kernel, a cluster of OC_CTAS CTAs that hold the new block's rows in shared memory: two
 // projections and two Cholesky-QR passes, the steps of orthonormalize().  As separate kernels
 // they were 16 launches, 110 us of kernel time at 2,044 rows and 4 roots, and two waits for the
-// host; this is one of 44 us.  The sums of the CTAs meet in distributed shared memory, added by
-// every CTA in the same order, so all take the same decisions; float-float sums over a share of
-// the rows, combined in FP64, as in k_tn and k_nn.  Bound by the latency of the small steps (the
-// factors take 12 us) and, towards 4,096 rows, by the float-float arithmetic of 16 SMs.
-//   With a CTA's conversions to FP64 after every row or two, its rows of V read from global memory
-// in each step, and 128 shares added one by one it took 105 us.
+// host; this is one of 69 us.  A CTA takes a block of k_tn and sums its shares as k_tn does, and the
+// CTAs' sums meet in distributed shared memory in the order of k_reduce_partials: the same vectors
+// to the bit, and the same decisions in every CTA.  Bound by the latency of the small steps (the
+// factors take 12 us).  Shares of 128 rows on all 16 CTAs took 44 us, but other roundings, and with
+// them one solve in ten other signs of its vectors.
 // ------------------------------------------------------------------------------------
 constexpr int OC_CTAS = 16, OC_THREADS = 512, OC_MAXR = 256, OC_ROWS = OC_CTAS * OC_MAXR;
 constexpr int OC_SUMS = (MAX_SUB + 16) * 16;
@@ -433,64 +486,80 @@ struct __align__(16) OcSmem {
 // followed by the CTA's rows of T, split (kq float pairs a row) and in FP64 (b a row), and, where
 // they fit, its rows of V, split (an odd number of pairs a row: no bank conflicts down a column)
 constexpr size_t OC_SMEM_MAX = 227 * 1024;
-int oc_per(int64_t n) { return (int)((n + OC_CTAS - 1) / OC_CTAS); }
-size_t oc_smem(int64_t n, int m, int b, bool &staged) {
-  const size_t per = oc_per(n), base = sizeof(OcSmem) + per * 8 * (size_t)(((b + 3) & ~3) + b);
+size_t oc_smem(size_t per, int m, int b, bool &staged) {
+  const size_t base = sizeof(OcSmem) + per * 8 * (size_t)(((b + 3) & ~3) + b);
   const size_t all = base + per * 8 * (size_t)(m | 1);
   staged = m > 0 && all <= OC_SMEM_MAX;
   return staged ? all : base;
 }
 
-// four consecutive float pairs
-__device__ __forceinline__ void oc_load4(const float2 *p, float2 (&v)[4]) {
-  const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
-  v[0] = make_float2(a.x, a.y); v[1] = make_float2(a.z, a.w);
-  v[2] = make_float2(b.x, b.y); v[3] = make_float2(b.z, b.w);
-}
-
-// out[i * k + j] = sum over this CTA's rows of a(r, i) * T[r, j], i < m.  A thread takes four columns
-// of an i over every S-th row, eight rows or more (a share's combination in FP64 costs as much as
-// several rows).
-template <typename LOAD>
-__device__ void oc_tn(OcSmem &s, const float2 *Tf, int kq, int rows, int per, int m, int k, LOAD a, double *out) {
-  const int tid = threadIdx.x, ng = (k + 3) >> 2;
-  const int G = m * ng, S = max(1, min(OC_THREADS / G, per >> 3));  // G <= (MAX_SUB + 16) * 4
-  const int g = tid % G, sub = tid / G, i = g % m, jb = g / m;
-  if (sub < S) {
-    float h[4] = {0.f, 0.f, 0.f, 0.f}, l[4] = {0.f, 0.f, 0.f, 0.f};
+// out[i * k + j] = sum over this CTA's rows of a(r, i) * T[r, j], i < m: the shares of a block of k_tn,
+// NJ outputs of a share a thread, and their sum in FP64
+template <int NJ, typename LOAD>
+__device__ void oc_tn(OcSmem &s, const float2 *Tf, int kq, int rows, int m, int k, LOAD a, double *out) {
+  const int S = max(1, TS_THREADS / (m * ((k + 7) >> 3))), nj = (k + NJ - 1) / NJ;
+  for (int e = threadIdx.x; e < S * m * nj; e += OC_THREADS) {
+    const int g = e / m, i = e - g * m, sub = g / nj, j0 = NJ * (g - sub * nj);
+    float h[NJ], l[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) { h[j] = 0.f; l[j] = 0.f; }
 #pragma unroll 4
     for (int r = sub; r < rows; r += S) {
-      float2 b[4];
+      float2 b[NJ];
       const float2 v = a(r, i);
-      oc_load4(Tf + r * kq + 4 * jb, b);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) ff_fma(h[j], l[j], v, b[j]);
+      ts_loadn<false, NJ>(Tf + r * kq + j0, b);
+      ts_fman<false, NJ>(h, l, v, b);
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < NJ; ++j) {
       ff_renorm(h[j], l[j]);
-      s.red[(sub * G + g) * 4 + j] = (double)h[j] + (double)l[j];
+      s.red[(sub * m + i) * kq + j0 + j] = (double)h[j] + (double)l[j];
     }
   }
   __syncthreads();
-  for (int o = tid; o < G * 4; o += OC_THREADS) {
-    const int g2 = o >> 2, jj = (g2 / m) * 4 + (o & 3);
-    if (jj >= k) continue;
+  for (int o = threadIdx.x; o < m * k; o += OC_THREADS) {
+    const int i = o / k, j = o - i * k;
     double v = 0.0;
 #pragma unroll 4
-    for (int q = 0; q < S; ++q) v += s.red[q * G * 4 + o];
-    out[(g2 % m) * k + jj] = v;
+    for (int q = 0; q < S; ++q) v += s.red[(q * m + i) * kq + j];
+    out[o] = v;
+  }
+  __syncthreads();
+}
+template <typename LOAD>
+__device__ __forceinline__ void oc_tn(OcSmem &s, const float2 *Tf, int kq, int rows, int m, int k, LOAD a, double *out) {
+  // four outputs a thread where that still gives each thread an item
+  if (max(1, TS_THREADS / (m * ((k + 7) >> 3))) * m * (kq >> 2) >= OC_THREADS) oc_tn<4>(s, Tf, kq, rows, m, k, a, out);
+  else oc_tn<2>(s, Tf, kq, rows, m, k, a, out);
+}
+// its diagonal for a = T: out[j] = sum T[r, j]^2
+__device__ void oc_norms(OcSmem &s, const float2 *Tf, int kq, int rows, int k, double *out) {
+  const int S = max(1, TS_THREADS / (k * ((k + 7) >> 3)));
+  for (int e = threadIdx.x; e < S * k; e += OC_THREADS) {
+    const int sub = e / k, j = e - sub * k;
+    float h = 0.f, l = 0.f;
+#pragma unroll 4
+    for (int r = sub; r < rows; r += S) ff_fma(h, l, Tf[r * kq + j], Tf[r * kq + j]);
+    ff_renorm(h, l);
+    s.red[e] = (double)h + (double)l;
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < k) {
+    double v = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < S; ++q) v += s.red[q * k + threadIdx.x];
+    out[threadIdx.x] = v;
   }
   __syncthreads();
 }
 
-// sum of an entry of the CTAs' sums, in their order
+// sum of an entry of the CTAs' sums, in the order of k_reduce_partials
 __device__ __forceinline__ double oc_total(cg::cluster_group &cl, double *sums, int o) {
   double v[OC_CTAS], t = 0.0;
 #pragma unroll
   for (int q = 0; q < OC_CTAS; ++q) v[q] = *cl.map_shared_rank(sums + o, q);
 #pragma unroll
-  for (int q = 0; q < OC_CTAS; ++q) t += v[q];
+  for (int q = 0; q < 8; ++q) t += v[q] + v[q + 8];
   return t;
 }
 
@@ -505,9 +574,8 @@ __device__ void oc_nn(OcSmem &s, int kq, int rows, int m, int k, LOAD a, STORE o
     for (int i = 0; i < m; ++i) {
       float2 y[4];
       const float2 v = a(r, i);
-      oc_load4(s.Cf + i * kq + j0, y);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) ff_fma(h[j], l[j], v, y[j]);
+      ts_loadn<false, 4>(s.Cf + i * kq + j0, y);
+      ts_fman<false, 4>(h, l, v, y);
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q)
@@ -520,12 +588,11 @@ __device__ void oc_nn(OcSmem &s, int kq, int rows, int m, int k, LOAD a, STORE o
 template <bool STAGED>
 __global__ void __launch_bounds__(OC_THREADS) k_ortho_cluster(int64_t n, double *V, int ld, int m,
                                                               const double *__restrict__ Tin, int ldt, int b,
-                                                              double drop_tol, int *nkept) {
+                                                              double drop_tol, int per, int *nkept) {
   extern __shared__ __align__(16) unsigned char oc_raw[];
   OcSmem &s = *reinterpret_cast<OcSmem *>(oc_raw);
   cg::cluster_group cl = cg::this_cluster();
   const int tid = threadIdx.x, rank = (int)cl.block_rank();
-  const int per = (int)((n + OC_CTAS - 1) / OC_CTAS);
   const int64_t r0 = min(n, (int64_t)rank * per);
   const int rows = (int)(min(n, r0 + per) - r0);
   const int kq = (b + 3) & ~3, vs = m | 1;
@@ -560,11 +627,10 @@ __global__ void __launch_bounds__(OC_THREADS) k_ortho_cluster(int64_t n, double 
   split_rows(b);
   // two projections; the squared norms before them with the first
   for (int pass = 0; pass < (m > 0 ? 2 : 1); ++pass) {
-    oc_tn(s, Tf, kq, rows, per, pass == 0 ? m + b : m, b,
-          [&](int r, int i) { return i < m ? v_at(r, i) : t_at(r, i - m); }, s.sums[ph]);
+    if (m > 0) oc_tn(s, Tf, kq, rows, m, b, v_at, s.sums[ph]);
+    if (pass == 0) oc_norms(s, Tf, kq, rows, b, s.sums[ph] + m * b);
     double *sums = meet();
-    if (pass == 0)
-      for (int o = tid; o < b; o += OC_THREADS) s.ref[o * b + o] = oc_total(cl, sums, (m + o) * b + o);
+    if (pass == 0 && tid < b) s.ref[tid * b + tid] = oc_total(cl, sums, m * b + tid);
     if (m > 0) {
       for (int e = tid; e < m * kq; e += OC_THREADS) {
         const int i = e / kq, j = e - i * kq;
@@ -577,7 +643,7 @@ __global__ void __launch_bounds__(OC_THREADS) k_ortho_cluster(int64_t n, double 
   }
   int nk = b;
   for (int pass = 0; pass < 2 && nk > 0; ++pass) {
-    oc_tn(s, Tf, kq, rows, per, nk, nk, t_at, s.sums[ph]);
+    oc_tn(s, Tf, kq, rows, nk, nk, t_at, s.sums[ph]);
     double *sums = meet();
     for (int o = tid; o < nk * nk; o += OC_THREADS) s.S[o] = oc_total(cl, sums, o);
     __syncthreads();
@@ -735,35 +801,65 @@ __global__ void k_map_set(const int64_t *idx, int M, int32_t *map) {
 }
 
 // H[idx[i], idx[j]] from the stored rows (one warp per row): dense, Hs[i*M + j] (rp null), or in
-// CSR, cnt[i] elements a row (FILL false) placed from rp[i] on in the stored order (FILL true)
+// CSR with the columns of a row dealt to the 32 lanes of its product, lane j % 32 taking its columns
+// in ascending order: a lane's sum is that of the dense row read 32 at a time, to the bit.  Rows are
+// padded with zeros to the longest lane: cnt[i] places a row (FILL false), from rp[i] on (FILL true).
+constexpr int EB_WARPS = 8;
 template <bool FILL>
-__global__ void k_extract_block(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ col,
-                                const double *__restrict__ val, const int64_t *__restrict__ idx, int M,
-                                const int32_t *__restrict__ map, double *Hs, int64_t *cnt, const int64_t *rp,
-                                int32_t *bcol, double *bval, double *diag) {
+__global__ void __launch_bounds__(EB_WARPS * 32) k_extract_block(const int64_t *__restrict__ rowptr,
+                                                                 const int32_t *__restrict__ col,
+                                                                 const double *__restrict__ val,
+                                                                 const int64_t *__restrict__ idx, int M,
+                                                                 const int32_t *__restrict__ map, double *Hs, int64_t *cnt,
+                                                                 const int64_t *rp, int32_t *bcol, double *bval,
+                                                                 double *diag) {
+  __shared__ int s_n[EB_WARPS][32];
   const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int i = blockIdx.x * EB_WARPS + (threadIdx.x >> 5);
   if (i >= M) return;
-  const int64_t row = idx[i], e = rowptr[row + 1];
-  int64_t n = FILL ? rp[i] : 0;
-  for (int64_t t0 = rowptr[row]; t0 < e; t0 += 32) {
-    const int64_t t = t0 + lane;
-    const int j = t < e ? map[col[t]] : -1;
+  int *n = s_n[threadIdx.x >> 5];
+  n[lane] = 0;
+  __syncwarp();
+  const int64_t row = idx[i], e = rowptr[row + 1], p0 = FILL ? rp[i] : 0;
+  for (int64_t t = rowptr[row] + lane; t < e; t += 32) {
+    const int j = map[col[t]];
+    if (j < 0) continue;
     if (Hs) {
-      if (j >= 0) Hs[(int64_t)i * M + j] = val[t];
+      Hs[(int64_t)i * M + j] = val[t];
       continue;
     }
-    const unsigned b = __ballot_sync(0xffffffffu, j >= 0);
-    if (FILL && j >= 0) {
-      const int64_t at = n + __popc(b & ((1u << lane) - 1u));
+    const int64_t at = p0 + 32 * atomicAdd(n + (j & 31), 1) + (j & 31);
+    if (FILL) {
       const double v = val[t];
       bcol[at] = j;
       bval[at] = v;
       if (j == i) diag[i] = v;
     }
-    n += __popc(b);
   }
-  if (!FILL && !Hs && lane == 0) cnt[i] = n;
+  if (Hs) return;
+  __syncwarp();
+  const int mine = n[lane], most = (int)__reduce_max_sync(0xffffffffu, (unsigned)mine);
+  if (!FILL) {
+    if (lane == 0) cnt[i] = 32 * (int64_t)most;
+    return;
+  }
+  int32_t *c = bcol + p0 + lane;
+  double *v = bval + p0 + lane;
+  for (int a = 1; a < mine; ++a) {  // few a lane: by insertion
+    const int ca = c[32 * a];
+    const double va = v[32 * a];
+    int b = a;
+    for (; b > 0 && c[32 * (b - 1)] > ca; --b) {
+      c[32 * b] = c[32 * (b - 1)];
+      v[32 * b] = v[32 * (b - 1)];
+    }
+    c[32 * b] = ca;
+    v[32 * b] = va;
+  }
+  for (int a = mine; a < most; ++a) {
+    c[32 * a] = i;
+    v[32 * a] = 0.0;
+  }
 }
 
 // V[idx[i], j] = Y[i, j]: the block's lowest eigenvectors as the first basis vectors
@@ -838,10 +934,10 @@ psoci_status tn(Work &w, const double *A, int lda, int a0, int m, const double *
   const size_t smem = std::max<size_t>((size_t)TN_TILE * kp * (lowp ? sizeof(float) : sizeof(float2)),
                                        sizeof(double) * TS_THREADS * 8);
   psoci_note_launch();
-  if (lowp)
-    k_tn<true><<<w.nblk, TS_THREADS, smem, c->stream>>>(w.N, A, lda, a0, m, B, ldb, b0, k, w.partial, w.rows_per_blk);
-  else
-    k_tn<false><<<w.nblk, TS_THREADS, smem, c->stream>>>(w.N, A, lda, a0, m, B, ldb, b0, k, w.partial, w.rows_per_blk);
+  const bool few = w.nblk <= 76;  // half the SMs
+  auto *kern = few ? (lowp ? k_tn<true, 2> : k_tn<false, 2>) : (lowp ? k_tn<true, 8> : k_tn<false, 8>);
+  kern<<<dim3(w.nblk, few ? 4 : 1), TS_THREADS, smem, c->stream>>>(w.N, A, lda, a0, m, B, ldb, b0, k, w.partial,
+                                                                   w.rows_per_blk);
   psoci_note_launch();
   k_reduce_partials<<<(m * k + 31) / 32, 256, 0, c->stream>>>(w.partial, w.nblk, m, k, C, ldc, c0);
   PSOCI_CUDA(c, cudaGetLastError());
@@ -921,10 +1017,10 @@ bool ortho_cluster(Work &w, int m, int b, cudaError_t &e) {
   }
   if (!w.cluster) return false;
   bool staged = false;
-  cfg.dynamicSmemBytes = oc_smem(w.N, m, b, staged);
+  cfg.dynamicSmemBytes = oc_smem((size_t)w.rows_per_blk, m, b, staged);
   psoci_note_launch();
   e = cudaLaunchKernelEx(&cfg, staged ? k_ortho_cluster<true> : k_ortho_cluster<false>, w.N, w.V, w.ld, m,
-                         (const double *)w.T, w.nr, b, 1e-10, w.ibuf);
+                         (const double *)w.T, w.nr, b, 1e-10, (int)w.rows_per_blk, w.ibuf);
   return true;
 }
 
@@ -936,7 +1032,7 @@ psoci_status orthonormalize(Work &w, int m, int b, int *bk) {
   const int ld = w.ld, tld = w.nr;
   // small bases: one kernel
   cudaError_t e = cudaSuccess;
-  if (w.N <= OC_ROWS && m <= MAX_SUB && b >= 1 && b <= TN_MAXK && ortho_cluster(w, m, b, e)) {
+  if (w.N <= OC_ROWS && !w.lowp && m <= MAX_SUB && b >= 1 && b <= TN_MAXK && ortho_cluster(w, m, b, e)) {
     int nk = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&nk, w.ibuf, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -1145,7 +1241,7 @@ psoci_status davidson_run(psoci_ctx *c, int64_t N, const double *diag, const Sub
   if ((s = psoci_alloc(c, &w.V, (size_t)N * ld)) || (s = psoci_alloc(c, &w.HV, (size_t)N * ld)) ||
       (s = psoci_alloc(c, &w.G, (size_t)ld * ld)) || (s = psoci_alloc(c, &w.Y, (size_t)ld * ld)) ||
       (s = psoci_alloc(c, &w.theta, ld)) || (s = psoci_alloc(c, &w.X, (size_t)N * nr)) ||
-      (s = psoci_alloc(c, &w.HX, (size_t)N * nr)) || (s = psoci_alloc(c, &w.R, (size_t)N * nr)) ||
+      (s = psoci_alloc(c, &w.R, (size_t)N * nr)) ||
       (s = psoci_alloc(c, &w.T, (size_t)N * nr)) || (s = psoci_alloc(c, &w.tmp, (size_t)N * std::max(nr, 2 * nr))) ||
       (s = psoci_alloc(c, &w.partial, (size_t)w.nblk * MAX_SUB * TN_MAXK)) ||
       (s = psoci_alloc(c, &w.small, (size_t)ld * ld)) || (s = psoci_alloc(c, &w.F, 16 * 16)) ||
@@ -1289,12 +1385,14 @@ psoci_status davidson_run(psoci_ctx *c, int64_t N, const double *diag, const Sub
     PSOCI_CUDA(c, cudaMemcpy2DAsync(w.Y, sizeof(double) * ld, h_y.data(), sizeof(double) * ld, sizeof(double) * m, m,
                                     cudaMemcpyHostToDevice, st));
     PSOCI_CUDA(c, cudaMemcpyAsync(w.theta, h_theta.data(), sizeof(double) * m, cudaMemcpyHostToDevice, st));
-    // Ritz vectors, their images and residuals
-    if ((s = nn(w, w.V, ld, 0, m, w.Y, ld, 0, nr, 1.0, 0.0, w.X, nr, 0))) return s;
-    if ((s = nn(w, w.HV, ld, 0, m, w.Y, ld, 0, nr, 1.0, 0.0, w.HX, nr, 0))) return s;
-    int rb = (int)std::min<int64_t>((N + 255) / 256, 152 * 4);
+    // Ritz vectors and residuals
+    const int nj = N > 76 * 256 ? 8 : nr <= 8 ? 2 : 4;
+    const int jbp = (nr + nj - 1) / nj <= 1 ? 1 : (nr + nj - 1) / nj <= 2 ? 2 : 4;
+    const int rb = (int)std::min<int64_t>((N * jbp + NN_THREADS - 1) / NN_THREADS, 152 * 8);
+    auto *ritz = nj == 8 ? k_ritz<8> : nj == 4 ? k_ritz<4> : k_ritz<2>;
     psoci_note_launch();
-    k_residual<<<rb, 256, 0, st>>>(N, nr, w.X, w.HX, w.theta, w.R, w.partial);
+    ritz<<<rb, NN_THREADS, sizeof(float2) * (size_t)m * ((nr + 7) & ~7), st>>>(N, w.V, w.HV, ld, m, w.Y, ld, nr, w.theta,
+                                                                              w.X, w.R, w.partial, jbp);
     psoci_note_launch();
     k_reduce_partials<<<1, 256, 0, st>>>(w.partial, rb, 1, nr, w.norms, nr, 0);
     PSOCI_CUDA(c, cudaGetLastError());
