@@ -330,17 +330,21 @@ __device__ __forceinline__ bool double_block_kept(double v0, double v1) { return
 // Screen, stage 2: drop candidates whose block stores nothing, judged from its integral
 // prefactors alone — double excitations as above and spin-orbit singles with SO_ij = 0
 // (PsociHamiltonian.C:227); both tests are symmetric in (i, j).  One warp per row configuration, candidates in order, ballot
-// compaction; MODE 0 counts, MODE 1 writes.
+// compaction; MODE 0 tests and counts, and marks a dropped candidate by its complement, MODE 1 writes
+// (with the tests again it took 98 us for the 4.3 M candidates of 6 electrons in 12 orbitals, 20 now).
 template <int W, int MODE>
-__global__ void k_prune(Params P, const int64_t *candoff, const int32_t *cand, int64_t *cnt) {
+__global__ void k_prune(Params P, const int64_t *candoff, int32_t *cand, int64_t *cnt) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t i = warp; i < P.nconf; i += nwarps) {
     uint64_t a1[W], a2[W];
+    int js_i = 0;
+    if (MODE == 0) {
 #pragma unroll
-    for (int w = 0; w < W; ++w) { a1[w] = P.e1[i * W + w]; a2[w] = P.e2[i * W + w]; }
-    const int js_i = P.jsym[i];
+      for (int w = 0; w < W; ++w) { a1[w] = P.e1[i * W + w]; a2[w] = P.e2[i * W + w]; }
+      js_i = P.jsym[i];
+    }
     const int64_t c0 = candoff[i], c1 = candoff[i + 1];
     int64_t n = 0;
     const int64_t out = (MODE == 1) ? P.nbroff[i] : 0;
@@ -350,8 +354,8 @@ __global__ void k_prune(Params P, const int64_t *candoff, const int32_t *cand, i
       int32_t j = 0;
       if (t < c1) {
         j = cand[t];
-        keep = true;
-        if (j != i) {
+        keep = j >= 0;
+        if (MODE == 0 && j != i) {
           uint64_t b1[W], b2[W];
 #pragma unroll
           for (int w = 0; w < W; ++w) { b1[w] = __ldg(P.e1 + (int64_t)j * W + w); b2[w] = __ldg(P.e2 + (int64_t)j * W + w); }
@@ -363,6 +367,7 @@ __global__ void k_prune(Params P, const int64_t *candoff, const int32_t *cand, i
           } else if (ni == 1 && __ldg(P.jsym + j) != js_i) {
             keep = __ldg(P.one + tri64(ex[0], jy[0])) != 0.0;
           }
+          if (!keep) cand[t] = ~j;
         }
       }
       const unsigned b = __ballot_sync(0xffffffffu, keep);
