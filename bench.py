@@ -33,15 +33,7 @@ sys.path.insert(0, ROOT)
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from ncu captures of
 # a smaller case of the same space, scaled to the full launch by the units processed; the
 # captures and the scaling are summarised under profiles/.
-EVAL = "k_hbuild_masks+k_hbuild_fast"  # the element evaluation: masks launch, then elements
-TRAFFIC = {(EVAL, "mrcisd_6e8o_v64"): 3.62e10, ("k_spmm_mixed", "mrcisd_6e8o_v64"): 1.91e10}
-# Warp instructions the element evaluation issues (smsp__inst_executed.sum, a one-pass ncu
-# capture of its two launches at the benchmark block, summed; profiles/).  The evaluation is
-# bound by instruction issue, so its roofline is issued instructions per second against the
-# SMs' issue peak: 152 SMs x 4 schedulers x 1 warp instruction per clock at the sampled SM
-# clock, over the library's CUDA-event time of the two launches.
-INST_PER_LAUNCH = {(EVAL, "mrcisd_6e8o_v64"): 24055006943 + 105044569354}
-SM_COUNT, ISSUE_PER_SM_CLK = 152, 4
+TRAFFIC = {("k_elems", "mrcisd_6e8o_v64"): 5.54e10, ("k_spmm_mixed", "mrcisd_6e8o_v64"): 1.91e10}
 
 NROOTS = 8
 RTOL = 1e-5          # residual norm; |dE| ~ r^2/gap, well inside 1e-7 Eh (checked below)
@@ -264,34 +256,32 @@ def run_ours(args):
     del V, Dd
 
     hbm, peak_kind = peaks()
-    clocks_now = clk.summary()
-    sm_hz = (clocks_now["sm_mhz"] or 2070.0) * 1e6
-    # dominant kernel: the element evaluation of the H build (k_hbuild_masks, then
-    # k_hbuild_fast), timed by the library's CUDA events on its stream in every timed mixed step.  Algorithmic bytes: the
-    # reference's stored lower triangle (values 8 + columns 4 per element, row pointers 8
-    # per row) written, plus the per-configuration tables (occupancies 2 x 8, offsets 8)
-    # and the integral tables read once.
+    # the largest launch of the H build: k_elems writing the stored elements, timed by the library's
+    # CUDA events on its stream in every timed mixed step (assemble_ms).  Algorithmic bytes: both
+    # triangles in FP64 and FP32 with their columns (8 + 4 + 4 per element), the neighbour lists (4 a
+    # pair), row pointers and per-configuration tables read once.
     bs = bstats[-1]
-    eval_s = float(np.mean([b["evaluate_ms"] for b in bstats])) * 1e-3
-    b_eval = bs["nnz_lower"] * (8 + 4) + (N + 1) * 8 + p.nconf * (2 * 8 + 8) + one.nbytes + p.eri.nbytes
-    ach_e = b_eval / eval_s / 1e9
-    inst = INST_PER_LAUNCH.get((EVAL, args.workload))
-    issue_peak = SM_COUNT * ISSUE_PER_SM_CLK * sm_hz
-    roofline_issue = {"kernel": "k_hbuild_masks + k_hbuild_fast<2,0,2> (H build element evaluation, lower "
-                      "blocks: masks launch, then elements)", "bound": "issue",
-                      "achieved": round(inst / eval_s / 1e9, 1) if inst else None, "peak": round(issue_peak / 1e9, 1),
-                      "unit": "G warp-instructions/s", "frac": round(inst / eval_s / issue_peak, 4) if inst else None,
-                      "traffic": TRAFFIC.get((EVAL, args.workload)), "peak_kind": "152 SMs x 4 issue/clk x "
-                      "sampled SM clock", "instructions_per_launch": inst, "launch_s": round(eval_s, 6),
-                      "instructions_per_lower_element": round(inst / bs["nnz_lower"], 1) if inst else None,
-                      "elements_per_s": round(bs["nnz_lower"] / eval_s, 1),
-                      "note": "issued warp instructions (ncu, one pass, both launches) over their CUDA-event time"}
+    fill_s = float(np.mean([b["assemble_ms"] for b in bstats])) * 1e-3
+    b_fill = nnz * (8 + 4 + 4) + bs["pairs"] * 4 + (N + 1) * 8 + p.nconf * (2 * 8 + 8) + one.nbytes + p.eri.nbytes
+    ach_e = b_fill / fill_s / 1e9
     # sigma: values + column indices + row pointers + x gathered once per row of the block +
     # y written (mixed: FP32 x staged from FP64, conversion kernel included)
     b_mixed = nnz * (4 + 4) + (N + 1) * 8 + N * k * (8 + 4 + 4 + 8)
     b_fp64 = nnz * (8 + 4) + (N + 1) * 8 + N * k * (8 + 8)
     ach_m = b_mixed / sig["mixed"] / 1e9
     ach_d = b_fp64 / sig["fp64"] / 1e9
+
+    # the dominant kernel of the step: 12 of its launches in a mixed solve
+    roofline_sigma = {"kernel": "k_spmm_mixed<8> (sigma, 8 vectors, timed alone)", "bound": "hbm",
+                      "achieved": round(ach_m, 1), "peak": hbm, "unit": "GB/s", "frac": round(ach_m / hbm, 4),
+                      "traffic": TRAFFIC.get(("k_spmm_mixed", args.workload)), "peak_kind": peak_kind,
+                      "bytes_per_launch": int(b_mixed), "launch_s": sig["mixed"],
+                      "l2_gather_bytes_per_launch": int(nnz * 32),
+                      "l2_gather_gbs": round(nnz * 32 / sig["mixed"] / 1e9, 1),
+                      "note": "bound by L2 gathers, not HBM: one 32-byte input row (8 FP32 vectors) per "
+                              "stored element, about one element per column of a configuration-pair block, so "
+                              "rows are rarely reused; ncu lts__throughput 79% of peak at mrcisd_6e8o_v24 "
+                              "(profiles/)"}
 
     # e2e: the user-facing call with host buffers, timed around the whole C-ABI sequence
     e2e_times = []
@@ -358,22 +348,14 @@ def run_ours(args):
                                "iterations": rr.iterations, "sigma_vectors": rr.sigma_calls,
                                "refine_iters": rr.refine_iters, "sigma_s": round(rr.sigma_seconds, 6)},
             "evals": [float(x) for x in r_mixed.evals],
-            "roofline": roofline_issue,
-            "roofline_hbm_element": {"kernel": "k_hbuild_masks + k_hbuild_fast", "bound": "hbm", "achieved": round(ach_e, 2),
-                                     "peak": hbm, "unit": "GB/s", "frac": round(ach_e / hbm, 5),
-                                     "traffic": TRAFFIC.get((EVAL, args.workload)), "peak_kind": peak_kind,
-                                     "bytes_per_launch": int(b_eval), "launch_s": round(eval_s, 6),
-                                     "note": "the element kernel's algorithmic bytes against HBM: not its bound"},
-            "roofline_sigma": {"kernel": "k_spmm_mixed<8> (sigma, 8 vectors, timed alone)", "bound": "hbm",
-                               "achieved": round(ach_m, 1), "peak": hbm, "unit": "GB/s", "frac": round(ach_m / hbm, 4),
-                               "traffic": TRAFFIC.get(("k_spmm_mixed", args.workload)), "peak_kind": peak_kind,
-                               "bytes_per_launch": int(b_mixed), "launch_s": sig["mixed"],
-                               "l2_gather_bytes_per_launch": int(nnz * 32),
-                               "l2_gather_gbs": round(nnz * 32 / sig["mixed"] / 1e9, 1),
-                               "note": "bound by L2 gathers, not HBM: one 32-byte input row (8 FP32 vectors) per "
-                                       "stored element, about one element per column of a configuration-pair block, so "
-                                       "rows are rarely reused; ncu lts__throughput 79% of peak at mrcisd_6e8o_v24 "
-                                       "(profiles/)"},
+            "roofline": roofline_sigma,
+            "roofline_elements": {"kernel": "k_elems<1,1,1,1> (H build: stored elements from coupling tables)",
+                                  "bound": "hbm", "achieved": round(ach_e, 1), "peak": hbm, "unit": "GB/s",
+                                  "frac": round(ach_e / hbm, 4), "traffic": TRAFFIC.get(("k_elems", args.workload)),
+                                  "peak_kind": peak_kind, "bytes_per_launch": int(b_fill), "launch_s": round(fill_s, 6),
+                                  "elements_per_s": round(nnz / fill_s, 1),
+                                  "note": "the elements' bytes against HBM; the kernel waits on table and pair "
+                                          "look-ups (profiles/)"},
             "roofline_fp64_sigma": {"achieved": round(ach_d, 1), "frac": round(ach_d / hbm, 4),
                                     "bytes_per_launch": int(b_fp64), "launch_s": sig["fp64"]},
             "h_build_ms": {k: round(bs[k], 3) for k in ("screen_ms", "evaluate_ms", "rows_ms", "assemble_ms",
