@@ -22,10 +22,6 @@
 namespace {
 
 constexpr int SIG_THREADS = 256;
-// threads of a block of the mixed kernel: narrow blocks of vectors run 9-15% faster with 512 (k = 1:
-// 155 -> 138 us at 60.0 M elements, 753 -> 640 at 267 M), wide ones are slower (k = 8: 111 -> 129 at
-// 25.7 M)
-__host__ __device__ constexpr int mix_threads(int k) { return k <= 4 ? 512 : 256; }
 // stored elements per lane whose gathers are in flight together; 4 was fastest for 8
 // vectors (8.96 ms at the benchmark block, 9.13 with 6, 9.67 with 8)
 constexpr int SIG_UNROLL = 4;
@@ -191,7 +187,7 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float prod) {
 // per row; 16: two rows per warp, for short rows) and UNR stored elements per lane whose
 // gathers are in flight together.
 template <int K, int LPR, int UNR>
-__global__ void __launch_bounds__(mix_threads(K)) k_spmm_mixed(int64_t nrows, const int64_t *__restrict__ rowptr,
+__global__ void __launch_bounds__(SIG_THREADS) k_spmm_mixed(int64_t nrows, const int64_t *__restrict__ rowptr,
                                                             const int32_t *__restrict__ col,
                                                             const float *__restrict__ val,
                                                             const float *__restrict__ x, double *__restrict__ y,
@@ -337,11 +333,11 @@ __global__ void __launch_bounds__(SIG_THREADS) k_spmm_ff(int64_t nrows, const in
             for (int q = 0; q < 8; ++q) f[u][8 * h + q] = g[q];
           }
           if constexpr (XS == 2) {
-            const float4 g = __ldcg(reinterpret_cast<const float4 *>(xr));
+            const float4 g = __ldg(reinterpret_cast<const float4 *>(xr));
             f[u][0] = g.x; f[u][1] = g.y; f[u][2] = g.z; f[u][3] = g.w;
           }
           if constexpr (XS == 1) {
-            const float2 g = __ldcg(reinterpret_cast<const float2 *>(xr));
+            const float2 g = __ldg(reinterpret_cast<const float2 *>(xr));
             f[u][0] = g.x; f[u][1] = g.y;
           }
         }
@@ -415,7 +411,7 @@ void launch_f64(psoci_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *c
 template <int K>
 void launch_k(psoci_ctx *c, int64_t n, const double *dX, int ldx, double *dY, int ldy, psoci_prec prec,
               const float *x32, int ld32) {
-  int blocks = sig_blocks(n, SIG_THREADS);
+  const int blocks = sig_blocks(n, SIG_THREADS);
   psoci_note_launch();
   if (prec == PSOCI_PREC_FP64)
     k_spmm_f64<K><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val, dX, ldx, dY, ldy,
@@ -424,28 +420,26 @@ void launch_k(psoci_ctx *c, int64_t n, const double *dX, int ldx, double *dY, in
     k_spmm_ff<K, K == 1 ? 1 : 2><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val,
                                                         reinterpret_cast<const float2 *>(x32), dY, ldy);
   else {
-    constexpr int T = mix_threads(K);
-    blocks = sig_blocks(n, T);
     // the variant chosen by psoci_autotune_sigma for this Hamiltonian (PSOCI_SIGMA_DEFAULT
     // until it runs)
     switch (c->sigma_variant) {
       case 1:
-        k_spmm_mixed<K, 32, 2><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
+        k_spmm_mixed<K, 32, 2><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
         break;
       case 2:
-        k_spmm_mixed<K, 16, 4><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
+        k_spmm_mixed<K, 16, 4><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
         break;
       case 3:
-        k_spmm_mixed<K, 16, 2><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
+        k_spmm_mixed<K, 16, 2><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
         break;
       case 4:
-        k_spmm_mixed<K, 8, 4><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
+        k_spmm_mixed<K, 8, 4><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
         break;
       case 5:
-        k_spmm_mixed<K, 16, 6><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
+        k_spmm_mixed<K, 16, 6><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32, dY, ldy);
         break;
       default:
-        k_spmm_mixed<K, 32, SIG_UNROLL><<<blocks, T, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32,
+        k_spmm_mixed<K, 32, SIG_UNROLL><<<blocks, SIG_THREADS, 0, c->stream>>>(n, c->d_rowptr, c->d_col, c->d_val32, x32,
                                                                               dY, ldy);
     }
   }
