@@ -1044,20 +1044,33 @@ __device__ __forceinline__ double det_elem(const double *eri, const PairInfo &pi
   return (ncount & 1) ? -v : v;
 }
 
-// SEF element (a, b) of the reference block (A, B): ciout / transformCDCt.  The determinant elements are
+// Where sef_elem finds the determinants of A: the global tables, or a copy of A's own
+// determinants in shared memory (rows indexed from A's first determinant).
+struct RowDets {
+  const uint64_t *al, *be;
+  const uint8_t *ph, *na;
+};
+
+// SEF element (a, b) of the reference block (A, B): ciout / transformCDCt.  conn bit
+// (x << 1 | y) says whether determinant x of SEF a and determinant y of SEF b can couple;
+// a determinant element that cannot is exactly zero and is not evaluated (adding the zero
+// it would return leaves every partial sum unchanged).  The determinant elements are
 // added in the reference's order: t = d00 + mB d01, u = d10 + mB d11, r (r t) + mA r (r u).
 template <int W>
-__device__ double sef_elem(const Params &PP, const PairInfo &pi, const double *Kd, int a, int b) {
+__device__ double sef_elem(const Params &PP, const PairInfo &pi, const double *Kd, int a, int b,
+                           unsigned conn = 0xFu, const RowDets *rowA = nullptr) {
   if (pi.kind == K_NONE) return 0.0;
   const bool odd = PP.nelec & 1;
   const bool oa = !odd && pi.nopenA != 0, ob = !odd && pi.nopenB != 0;
   const int64_t a0 = odd ? a : (oa ? 2 * a : 0), b0 = pi.detB + (odd ? b : (ob ? 2 * b : 0));
-  const unsigned conn = (ob ? 0xFu : 0x5u) & (oa ? 0xFu : 0x3u);  // determinant pairs there are: bit x << 1 | y
+  if (!ob) conn &= 0x5u;
+  if (!oa) conn &= 0x3u;
   DetBits<W> A[2] = {}, B[2] = {};
 #pragma unroll
   for (int x = 0; x < 2; ++x) {
     if (x == 1 && !oa) break;
-    load_det<W>(A[x], PP.alpha, PP.beta, PP.phase, PP.nalpha, pi.detA + a0 + x);
+    if (rowA) load_det<W>(A[x], rowA->al, rowA->be, rowA->ph, rowA->na, a0 + x);
+    else load_det<W>(A[x], PP.alpha, PP.beta, PP.phase, PP.nalpha, pi.detA + a0 + x);
   }
 #pragma unroll
   for (int y = 0; y < 2; ++y) {
@@ -1219,7 +1232,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32) k_hbuild(Params P) {
 // k_elems then walks each configuration's list, 32 pairs at a time, and
 //   MODE 0  counts the kept elements of its rows,
 //   MODE 1  writes them, columns ascending, at the rows' places,
-//   MODE 2  multiplies them with X (direct mode), MODE 3 with X in FP32.
+//   MODE 2  multiplies them with X (direct mode).
 // Both triangles are evaluated: an element costs so little that reading its pair twice is cheaper
 // than mirroring it.  mrcisd_6e8o_v48 (2.18 million SEFs, 1.25e9 elements): pair slots, tables and
 // diagonal 8.7 ms, count 6.2 ms, fill 17.0 ms (20 GB of CSR: 3 ms at the copy rate), where
@@ -1552,7 +1565,7 @@ __global__ void __launch_bounds__(DG_WARPS * 32) k_diag_blocks(Params P, int ldd
 }
 
 // Per warp, followed by X (ms doubles a pair) and, MODE 0 and 1, an int32 a row (count, write
-// position from the configuration's first), MODE 2 and 3 four times eight doubles a row (its
+// position from the configuration's first), MODE 2 four times eight doubles a row (its
 // products).  The pairs that have elements, in order.
 struct ElemWarp {
   uint2 run[PSOCI_SEG];        // runs of elements: first entry less first element, pair
@@ -1892,22 +1905,12 @@ __global__ void __launch_bounds__(EL_WARPS * 32) k_elems(Params P, ElemArgs<W> E
               const uint32_t cc = __shfl_sync(FULL, col, l);
               const bool ok = cc != 0xffffffffu && q < P.kvec;
               if (!ok) vv[u] = 0.0;
-              if (MODE == 2) xx[u] = ok ? __ldg(P.dx + (int64_t)cc * P.ldx + q) : 0.0;
-              else xx[u] = __hiloint2double(0, __float_as_int(ok ? __ldg(P.dx32 + (int64_t)cc * 8 + q) : 0.f));
+              xx[u] = ok ? __ldg(P.dx + (int64_t)cc * P.ldx + q) : 0.0;
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-              if (MODE == 2) {
-                double *y = ya + rr[u] * 8;
-                *y = fma(vv[u], xx[u], *y);
-              } else {
-                // FP32 product, Kahan sum: the rounding error of each addition is carried in .y
-                float2 *y = reinterpret_cast<float2 *>(ya + rr[u] * 8);
-                const float2 sc = *y;
-                const float pr32 = __fmul_rn(f32_of(vv[u]), __int_as_float(__double2loint(xx[u])));
-                const float yv = __fsub_rn(pr32, sc.y), tt = __fadd_rn(sc.x, yv);
-                *y = make_float2(tt, __fsub_rn(__fsub_rn(tt, sc.x), yv));
-              }
+              double *y = ya + rr[u] * 8;
+              *y = fma(vv[u], xx[u], *y);
             }
           }
         }
@@ -1921,14 +1924,11 @@ __global__ void __launch_bounds__(EL_WARPS * 32) k_elems(Params P, ElemArgs<W> E
       for (int r = lane; r < nsefI; r += 32) E.row_nnz[row0 + r] = pos[r];
       if (lane == 0) atomicAdd(E.segments, (unsigned long long)((b1 - b0 + 31) / 32));
     }
-    if (MODE >= 2)
+    if (MODE == 2)
       for (int r = lane; r < nsefI * 8; r += 32) {
         double y[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          y[u] = yacc[u * nsefI * 8 + r];
-          if (MODE == 3) y[u] = (double)__int_as_float(__double2loint(y[u])) - (double)__int_as_float(__double2hiint(y[u]));
-        }
+        for (int u = 0; u < 4; ++u) y[u] = yacc[u * nsefI * 8 + r];
         if ((r & 7) < P.kvec) P.dy[(row0 + (r >> 3)) * P.ldy + (r & 7)] = (y[0] + y[1]) + (y[2] + y[3]);
       }
     __syncwarp();
@@ -2422,9 +2422,11 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
   }
   auto t_c = tnow();
 
-  // 2. segments of the generic kernels (<= 32 neighbours of a configuration, one warp each)
+  // 2. segments of the generic kernels and of direct mode's FP32 products (<= 32 neighbours of a
+  // configuration, one warp each)
   int64_t nseg = 0, nslots = 0;
-  if (!fast) {
+  const bool segs = !fast || (direct && c->max_ndet <= 32);
+  if (segs) {
     TRY(psoci_alloc(c, &d_nseg, n + 1));
     TRY(psoci_alloc(c, &d_nrow, n + 1));
     TRY(psoci_alloc(c, &d_segoff, n + 1));
@@ -2438,7 +2440,7 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
     TRY(psoci_alloc(c, &d_segk0, nseg));
     TRY(psoci_alloc(c, &d_segn, nseg));
     TRY(psoci_alloc(c, &d_segrow, nseg));
-    TRY(psoci_alloc(c, &d_segcnt, nslots));
+    if (!fast) TRY(psoci_alloc(c, &d_segcnt, nslots));
     psoci_note_launch();
     k_seg_init<<<(n + 255) / 256, 256, 0, st>>>(n, d_nbroff, c->d_sefoff, d_segoff, d_rowslot, d_segcfg, d_segk0,
                                                 d_segn, d_segrow);
@@ -2459,7 +2461,7 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
     P.diag = c->d_diag;
     if (fast) {
       TRY(tab_diagonal<W>(c, P, T, c->d_diag));
-      c->nseg = nseg = (npairs + PSOCI_SEG - 1) / PSOCI_SEG;
+      if (!segs) c->nseg = nseg = (npairs + PSOCI_SEG - 1) / PSOCI_SEG;
     } else {
       const size_t smem = sizeof(WarpSmem) * WARPS_PER_CTA;
       TRYC(cudaFuncSetAttribute(k_hbuild<W, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2479,11 +2481,10 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
       dir_set<W>(d) = T;
       T = TabSet<W>();
       c->dir_tabs = d;
-    } else {
-      c->dir_segcfg = d_segcfg; d_segcfg = nullptr;
-      c->dir_segk0 = d_segk0; d_segk0 = nullptr;
-      c->dir_segn = d_segn; d_segn = nullptr;
     }
+    c->dir_segcfg = d_segcfg; d_segcfg = nullptr;
+    c->dir_segk0 = d_segk0; d_segk0 = nullptr;
+    c->dir_segn = d_segn; d_segn = nullptr;
     c->direct = true;
   } else if (fast) {
     TRY(psoci_alloc(c, &c->d_diag, N));
@@ -2579,6 +2580,254 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
 #undef TRYC
 }
 
+// ------------------------------------------------------------------------------------
+// Direct mode with FP32 elements and inputs (configurations of at most 32 determinants, <= 6 open
+// shells with an even electron count, <= 5 with an odd one; at most 16 SEFs).  The compensated FP32
+// sums of a lane round by the order of its products, so they keep the order of the determinants:
+// a lane owns a neighbour and marks, per row SEF r of I, the column SEFs t whose determinants are
+// within two spin-orbital substitutions with the same spin projection (one, any spin, for spin-orbit
+// pairs); a row's marked elements, by pair kind, neighbour and column, go to the lanes in turn.
+// Elements from the coupling tables in the order of k_elems took a tenth of the time (46 against 118 us
+// and 85 against 442 us at two small spaces) but agreed with these sums to 3e-8 only.  FP64 products
+// (k_elems MODE 2) are the faster choice in direct mode, and what its solves use.
+// ------------------------------------------------------------------------------------
+constexpr int FAST_MAXDET = 32;
+constexpr int FAST_MAXSEF = 16;
+constexpr int FAST_MAXOPEN = 6;  // 2^(6-1) = 32 determinants
+constexpr int FAST_MAXK = 1 + FAST_MAXOPEN * (FAST_MAXOPEN - 1) / 2;  // diagonal list, <= 6 open shells
+
+__device__ __forceinline__ bool tbit(const uint64_t *x, int p) { return (x[p >> 6] >> (p & 63)) & 1ull; }
+
+template <int W>
+struct FastSmem {
+  PairInfo pi[PSOCI_SEG];
+  double K[FAST_MAXK];
+  uint64_t ra[FAST_MAXDET * W], rb[FAST_MAXDET * W];
+  uint8_t rna[FAST_MAXDET], rph[FAST_MAXDET];
+  // of a row: connectivity of the marked elements of each slot (the marked columns are its four
+  // 16-bit quarters or-ed) and their exclusive prefix
+  uint64_t cm[PSOCI_SEG];
+  int16_t pre[PSOCI_SEG];
+  int8_t perm[PSOCI_SEG];  // evaluation order: slot -> neighbour lane, grouped by pair kind
+};
+
+template <int W>
+__global__ void __launch_bounds__(WARPS_PER_CTA * 32) k_direct_mixed(Params P) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  FastSmem<W> *ws = reinterpret_cast<FastSmem<W> *>(smem_raw) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const bool odd = P.nelec & 1;
+  for (int64_t s = warp; s < P.nseg; s += nwarps) {
+    const int I = P.seg_cfg[s];
+    const int64_t k0 = P.seg_k0[s];
+    const int n = P.seg_n[s];
+    const int nsefI = (int)(P.sefoff[I + 1] - P.sefoff[I]);
+    const int64_t d0I = P.detoff[I];
+    const int ndI = (int)(P.detoff[I + 1] - d0I);
+    const int nopI = P.nopen[I];
+    if (lane < n) pair_setup<W>(P, I, P.nbr[k0 + lane], ws->pi[lane], ws->K);
+    for (int d = lane; d < ndI; d += 32) {
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        ws->ra[d * W + w] = P.alpha[(d0I + d) * W + w];
+        ws->rb[d * W + w] = P.beta[(d0I + d) * W + w];
+      }
+      ws->rna[d] = P.nalpha[d0I + d];
+      ws->rph[d] = P.phase[d0I + d];
+    }
+    __syncwarp();
+    // phase 1: connectivity masks C[r] for this lane's neighbour, bit-parallel over the
+    // row determinants.  With m_a the alpha pattern of row det a on I's open shells, a column
+    // det b (alpha ab, beta bb) differs from a in
+    //   c(a) = F + #{p in x : p not in m_a} + #{p in y : p in m_a}
+    // spin-orbitals of b, where x, y are b's alpha / beta patterns on I's open shells and F
+    // counts b's electrons in orbitals empty in I.  Non-spin-orbit pairs need c(a) <= 2 and
+    // equal alpha counts, spin-orbit pairs c(a) <= 1 (the tests det_elem starts with).  The sets
+    // {a : p in m_a} and {a : |m_a| = k} are warp ballots; c(a) is kept as a saturating
+    // bit-sliced counter over all row dets at once.
+    uint32_t Ap[FAST_MAXOPEN], Nk[FAST_MAXOPEN + 1];
+    int sI[FAST_MAXOPEN];
+    uint64_t occI[W];
+    {
+      uint64_t SI[W];
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        occI[w] = P.e1[(int64_t)I * W + w];
+        SI[w] = occI[w] & ~P.e2[(int64_t)I * W + w];
+      }
+      // open shells of I, ascending (fixed-size loops keep these arrays in registers)
+#pragma unroll
+      for (int p = 0; p < FAST_MAXOPEN; ++p) {
+        sI[p] = lowest_bit<W>(SI);
+        bool done = false;
+#pragma unroll
+        for (int w = 0; w < W; ++w)
+          if (!done && SI[w]) { SI[w] &= SI[w] - 1; done = true; }
+      }
+      uint32_t ma = 0u;
+      if (lane < ndI)
+#pragma unroll
+        for (int p = 0; p < FAST_MAXOPEN; ++p)
+          if (p < nopI) ma |= (uint32_t)tbit(&ws->ra[lane * W], sI[p]) << p;
+#pragma unroll
+      for (int p = 0; p < FAST_MAXOPEN; ++p) Ap[p] = __ballot_sync(0xffffffffu, (lane < ndI) && ((ma >> p) & 1u));
+#pragma unroll
+      for (int k = 0; k <= FAST_MAXOPEN; ++k) Nk[k] = __ballot_sync(0xffffffffu, (lane < ndI) && __popc(ma) == k);
+    }
+    const int ndblI = P.nelec - nopI;  // electrons in I's doubly occupied orbitals
+    // C[r]: for row SEF r and column SEF t, bit t + 16 (x << 1 | y) says that determinant x
+    // of SEF r and determinant y of SEF t can couple; the SEF element is marked when any can.
+    uint64_t C[FAST_MAXSEF];
+    for (int r = 0; r < FAST_MAXSEF; ++r) C[r] = 0ull;
+    if (lane < n) {
+      const PairInfo &pi = ws->pi[lane];
+      if (pi.kind != K_NONE) {
+        const bool so = (pi.kind == K_SO);
+        const int64_t d0J = pi.swap ? pi.detA : pi.detB;
+        const int nopJ = pi.swap ? pi.nopenA : pi.nopenB;
+        const int ndJ = 1 << (nopJ > 1 ? nopJ - 1 : 0);
+        const int thr = so ? 1 : 2;
+        const uint32_t rows_valid = (ndI >= 32) ? 0xffffffffu : ((1u << ndI) - 1u);
+        for (int b = 0; b < ndJ; ++b) {
+          uint64_t ja[W], jb[W];
+#pragma unroll
+          for (int w = 0; w < W; ++w) { ja[w] = __ldg(P.alpha + (d0J + b) * W + w); jb[w] = __ldg(P.beta + (d0J + b) * W + w); }
+          int F = 0;
+#pragma unroll
+          for (int w = 0; w < W; ++w) F += __popcll(ja[w] & ~occI[w]) + __popcll(jb[w] & ~occI[w]);
+          if (F > thr) continue;
+          uint32_t ok = 0u;
+          {
+            // saturating counter over the row dets: S0 (c'=0), S1, S2, S3 (>= 3)
+            uint32_t S0 = 0xffffffffu, S1 = 0u, S2 = 0u;
+#pragma unroll
+            for (int p = 0; p < FAST_MAXOPEN; ++p) {
+              if (p >= nopI) break;
+              const bool xa = bit_w<W>(ja, sI[p]), yb = bit_w<W>(jb, sI[p]);
+              if (xa) {  // mismatch where row det has beta on p
+                const uint32_t T = ~Ap[p];
+                S2 = (S2 & ~T) | (S1 & T);
+                S1 = (S1 & ~T) | (S0 & T);
+                S0 &= ~T;
+              }
+              if (yb) {  // mismatch where row det has alpha on p
+                const uint32_t T = Ap[p];
+                S2 = (S2 & ~T) | (S1 & T);
+                S1 = (S1 & ~T) | (S0 & T);
+                S0 &= ~T;
+              }
+            }
+            ok = (thr - F >= 2) ? (S0 | S1 | S2) : (thr - F == 1) ? (S0 | S1) : S0;
+          }
+          int na = 0;
+#pragma unroll
+          for (int w = 0; w < W; ++w) na += __popcll(ja[w]);
+          const int need = na - (ndblI / 2);  // alpha open shells a row det needs for equal counts
+          ok &= rows_valid;
+          if (!so) {
+            uint32_t nk = 0u;
+#pragma unroll
+            for (int k = 0; k <= FAST_MAXOPEN; ++k)
+              if (k == need) nk = Nk[k];
+            ok &= (need >= 0 && need <= nopI) ? nk : 0u;
+          }
+          const int t = odd ? b : (nopJ ? (b >> 1) : 0);
+          const int y = (!odd && nopJ) ? (b & 1) : 0;
+          while (ok) {
+            const int a = __ffs(ok) - 1;
+            ok &= ok - 1;
+            const int x = (!odd && nopI) ? (a & 1) : 0;
+            C[odd ? a : (nopI ? (a >> 1) : 0)] |= 1ull << (t + 16 * ((x << 1) | y));
+          }
+        }
+      }
+    }
+    const RowDets rowA = {ws->ra, ws->rb, ws->rph, ws->rna};  // I's determinants (A = I)
+    // evaluation order of the neighbours: grouped by pair kind (doubles, singles, spin-orbit,
+    // diagonal), ascending within a kind, so that neighbouring lanes mostly run the same
+    // branch of the element code.  With the marked elements' numbers it fixes the order of the sums.
+    {
+      const int kd = (lane < n) ? ws->pi[lane].kind : -1;
+      const int key = (kd == K_DOUBLE) ? 0 : (kd == K_SINGLE) ? 1 : (kd == K_SO) ? 2 : (kd == K_DIAG) ? 3
+                                                                                         : (kd == K_NONE) ? 4 : 5;
+      int rank = 0, base = 0;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const unsigned m = __ballot_sync(0xffffffffu, key == k);
+        if (key == k) rank = base + __popc(m & ((1u << lane) - 1u));
+        base += __popc(m);
+      }
+      ws->perm[rank] = (int8_t)lane;
+      __syncwarp();
+    }
+    const int src = ws->perm[lane];  // the neighbour lane at evaluation slot `lane`
+    for (int r = 0; r < nsefI; ++r) {
+      // marked columns of each slot and their exclusive prefix
+      const uint64_t cr = __shfl_sync(0xffffffffu, (lane < n) ? C[r] : 0ull, src);
+      const int cm = __popc((uint32_t)((cr | (cr >> 16) | (cr >> 32) | (cr >> 48)) & 0xffffull));
+      int inclm = cm;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inclm, o);
+        if (lane >= o) inclm += v;
+      }
+      ws->pre[lane] = (int16_t)(inclm - cm);
+      ws->cm[lane] = cr;
+      const int T = __shfl_sync(0xffffffffu, inclm, 31);
+      double acc[8];
+      float accs[8], accc[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) { accs[q] = 0.f; accc[q] = 0.f; }
+      __syncwarp();
+      for (int e = lane; e < T; e += 32) {
+        int o = 0;  // the slot owning element e: last slot whose prefix is <= e
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+          if (ws->pre[o + step] <= e) o += step;
+        const uint64_t cw = ws->cm[o];
+        uint32_t m = (uint32_t)((cw | (cw >> 16) | (cw >> 32) | (cw >> 48)) & 0xffffull);
+        for (int q = e - ws->pre[o]; q > 0; --q) m &= m - 1;
+        const int t = __ffs(m) - 1;
+        const PairInfo &pi = ws->pi[ws->perm[o]];
+        // reference roles: the lower half of a diagonal block, block (J, I) for J > I
+        const bool diag_blk = (pi.kind == K_DIAG);
+        const bool flip = diag_blk ? (t > r) : (pi.swap != 0);
+        const uint64_t co = cw >> t;
+        unsigned conn = (unsigned)((co & 1ull) | ((co >> 15) & 2ull) | ((co >> 30) & 4ull) | ((co >> 45) & 8ull));
+        // a diagonal block is symmetric: the transposed element swaps the determinant roles
+        if (flip) conn = (conn & 9u) | ((conn & 2u) << 1) | ((conn & 4u) >> 1);
+        // A's determinants come from shared memory when A = I (a pair J > I has A = J, read from the
+        // tables)
+        const double v = sef_elem<W>(P, pi, ws->K, flip ? t : r, flip ? r : t, conn, pi.swap ? nullptr : &rowA);
+        if (fabs(v) >= PSOCI_MIN_VALUE || (diag_blk && t == r)) {
+          const float vf = (float)v;
+          const float4 *xr = reinterpret_cast<const float4 *>(P.dx32 + (pi.colbase + t) * 8);
+          const float4 xa = __ldg(xr), xb = __ldg(xr + 1);
+          const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            // Kahan: the rounding error of each addition is carried in accc and fed back
+            const float yv = __fsub_rn(__fmul_rn(vf, xv[q]), accc[q]);
+            const float tt = __fadd_rn(accs[q], yv);
+            accc[q] = __fsub_rn(__fsub_rn(tt, accs[q]), yv);
+            accs[q] = tt;
+          }
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[q] = (double)accs[q] - (double)accc[q];
+      const double tot = reduce_scatter8_f64(acc, lane);
+      const int q = lane >> 2;
+      if ((lane & 3) == 0 && q < P.kvec && tot != 0.0) atomicAdd(P.dy + (P.sefoff[I] + r) * P.ldy + q, tot);
+      __syncwarp();
+    }
+    __syncwarp();
+  }
+}
+
 // X (FP64, leading dim ldx, k <= 8 columns) -> X32 (FP32, row stride 8, zero padded)
 __global__ void k_direct_x32(int64_t n, int k, const double *__restrict__ x, int ldx, float *__restrict__ x32) {
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
@@ -2618,7 +2867,12 @@ psoci_status run_direct_sigma(psoci_ctx *c, int k, const double *dX, int ldx, do
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((P.nseg + WARPS_PER_CTA - 1) / WARPS_PER_CTA, 152 * 16));
   // MIXED (spaces of at most 32 determinants a configuration): FP32 element x FP32 input
   // products; beyond them direct mode is FP64 whatever the precision asked for
-  const bool mixed = fast && c->max_ndet <= 32 && prec == PSOCI_PREC_MIXED && x32;
+  const bool mixed = c->max_ndet <= FAST_MAXDET && prec == PSOCI_PREC_MIXED && x32 && P.nseg > 0;
+  const size_t fsmem = sizeof(FastSmem<W>) * WARPS_PER_CTA;
+  if (mixed) {
+    PSOCI_CUDA(c, cudaFuncSetAttribute(k_direct_mixed<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
+    if (fast) PSOCI_CUDA(c, cudaMemset2DAsync(dY, sizeof(double) * ldy, 0, sizeof(double) * k, N, st));
+  }
   for (int q0 = 0; q0 < k; q0 += 8) {
     P.dx = dX + q0; P.dy = dY + q0; P.ldx = ldx; P.ldy = ldy; P.kvec = std::min(8, k - q0);
     P.dx32 = nullptr;
@@ -2626,7 +2880,9 @@ psoci_status run_direct_sigma(psoci_ctx *c, int k, const double *dX, int ldx, do
       psoci_note_launch();
       k_direct_x32<<<(unsigned)std::min<int64_t>((N + 255) / 256, 152 * 16), 256, 0, st>>>(N, P.kvec, P.dx, ldx, x32);
       P.dx32 = x32;
-      if ((s = E.vals ? elems_launch<W, 3, true>(c, P, E) : elems_launch<W, 3, false>(c, P, E))) return s;
+      psoci_note_launch();
+      k_direct_mixed<W><<<blocks, WARPS_PER_CTA * 32, fsmem, st>>>(P);
+      PSOCI_CUDA(c, cudaGetLastError());
     } else if (fast) {
       if ((s = E.vals ? elems_launch<W, 2, true>(c, P, E) : elems_launch<W, 2, false>(c, P, E))) return s;
     } else {
@@ -3516,11 +3772,11 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32) k_energy_grad(Params P, const 
 // blocks apart.
 // ------------------------------------------------------------------------------------
 // vectors (k per pass, root-major with stride ldv) side by side, KP a SEF (zero padded)
-template <typename CT, int KP>
-__global__ void k_grad_rows(int64_t n, const double *__restrict__ V, int64_t ldv, int k, CT *__restrict__ C) {
+template <int KP>
+__global__ void k_grad_rows(int64_t n, const double *__restrict__ V, int64_t ldv, int k, double *__restrict__ C) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
 #pragma unroll
-    for (int q = 0; q < KP; ++q) C[i * KP + q] = q < k ? (CT)V[(int64_t)q * ldv + i] : (CT)0;
+    for (int q = 0; q < KP; ++q) C[i * KP + q] = q < k ? V[(int64_t)q * ldv + i] : 0.0;
   }
 }
 
@@ -3534,9 +3790,6 @@ __global__ void k_grad_out(int64_t n, int k, const double *__restrict__ T, doubl
 }
 
 __device__ __forceinline__ double with_sign(double v, uint32_t x) { return flip_sign(v, x & 0x80000000u); }
-__device__ __forceinline__ float with_sign(float v, uint32_t x) {
-  return __int_as_float(__float_as_int(v) ^ (int)(x & 0x80000000u));
-}
 
 constexpr int GT_WARPS = 4;
 struct GradPair {
@@ -3550,20 +3803,20 @@ struct GradPair {
 
 // One warp per configuration, 32 lower pairs set up at a time, KP lanes (a root each) to a pair:
 // the lists of its table's program give one sum of products c_I[row] c_J[column] an integral,
-// which goes to that integral's place in the gradient.  The sums are FP64 (CT double) or FP32
-// (float) within a pair; the places take FP64 atomics, the KP roots of one side by side (T1, T2:
+// which goes to that integral's place in the gradient.  The sums are FP64
+// and the places take FP64 atomics, the KP roots of one side by side (T1, T2:
 // KP a table entry).  Bound by the FP64 pipe, one FMA an entry of a list (16 clocks a warp
 // instruction an SM, whatever its active lanes): mrcisd_6e8o_v16, 8 roots, 2.5 ms (3.2 with the
 // pairs in their lists' order, 19 of 32 lanes active; determinant pair by determinant pair the lower
 // blocks took 52 ms).
-template <int W, typename CT, int KP>
+template <int W, int KP>
 __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgRec<W> *__restrict__ cfg,
                                                             const int64_t *__restrict__ nbroff,
                                                             const int32_t *__restrict__ nbr,
                                                             const uint32_t *__restrict__ slot,
                                                             const uint4 *__restrict__ hdr,
                                                             const uint32_t *__restrict__ pool,
-                                                            const CT *__restrict__ C, double *T1, double *T2) {
+                                                            const double *__restrict__ C, double *T1, double *T2) {
   __shared__ GradPair pairs[GT_WARPS][PSOCI_SEG];
   GradPair *gp = pairs[threadIdx.x >> 5];
   constexpr unsigned FULL = 0xffffffffu;
@@ -3572,7 +3825,7 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgR
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t I = warp; I < P.nconf; I += nwarps) {
     const CfgRec<W> a = cfg[I];
-    const CT *cI = C + (int64_t)a.sef * KP + q;
+    const double *cI = C + (int64_t)a.sef * KP + q;
     const int64_t b1 = nbroff[I + 1];
     for (int64_t k0 = nbroff[I]; k0 < b1; k0 += 32) {
       const int J = (k0 + lane < b1) ? nbr[k0 + lane] : INT_MAX;
@@ -3609,18 +3862,18 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgR
       __syncwarp();
       for (int u = grp; u < np; u += 32 / KP) {
         const GradPair &g = gp[u];
-        const CT *cJ = C + (int64_t)g.sefJ * KP + q;
+        const double *cJ = C + (int64_t)g.sefJ * KP + q;
         const uint16_t *ends = reinterpret_cast<const uint16_t *>(pool + g.prog);
         const uint32_t *pw = pool + g.prog + (TAB_LISTS + 1) / 2;
         int e = 0;
         for (int l = 0; l < g.lists; ++l) {
           const int end = (int)__ldg(ends + l);
           if (e == end) continue;
-          CT sum = 0;
+          double sum = 0;
           for (; e + 2 <= end; e += 2) {
             const uint32_t x0 = __ldg(pw + e), x1 = __ldg(pw + e + 1);
-            const CT i0 = __ldg(cI + (int)((x0 >> 8) & 0xffu) * KP), i1 = __ldg(cI + (int)((x1 >> 8) & 0xffu) * KP);
-            const CT j0 = __ldg(cJ + (int)(x0 & 0xffu) * KP), j1 = __ldg(cJ + (int)(x1 & 0xffu) * KP);
+            const double i0 = __ldg(cI + (int)((x0 >> 8) & 0xffu) * KP), i1 = __ldg(cI + (int)((x1 >> 8) & 0xffu) * KP);
+            const double j0 = __ldg(cJ + (int)(x0 & 0xffu) * KP), j1 = __ldg(cJ + (int)(x1 & 0xffu) * KP);
             sum = fma(with_sign(i0, x0), j0, sum);
             sum = fma(with_sign(i1, x1), j1, sum);
           }
@@ -3629,7 +3882,7 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgR
             sum = fma(with_sign(__ldg(cI + (int)((x0 >> 8) & 0xffu) * KP), x0), __ldg(cJ + (int)(x0 & 0xffu) * KP), sum);
             ++e;
           }
-          const double w = g.f * (double)sum;
+          const double w = g.f * sum;
           if (g.kind == K_DOUBLE) {
             atomicAdd(T2 + (l == 0 ? canon4(g.ie, g.je, g.ex1, g.jy1) : canon4(g.ie, g.jy1, g.ex1, g.je)) * KP + q, w);
           } else if (g.kind == K_SO) {
@@ -3685,8 +3938,8 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_tab(Params P, const CfgR
 // 2^(n-2) squares instead of a test of every determinant with every other.  One warp a configuration,
 // KP lanes (a root each) to a shell pair or an integral.  Of 2.4 ms at mrcisd_6e8o_v16, 8 roots,
 // 0.14 ms remain.
-template <int W, typename CT, int KP>
-__global__ void __launch_bounds__(GT_WARPS * 32) k_grad_diag(Params P, const CT *__restrict__ C, double *T1, double *T2) {
+template <int W, int KP>
+__global__ void __launch_bounds__(GT_WARPS * 32) k_grad_diag(Params P, const double *__restrict__ C, double *T1, double *T2) {
   // of a spin pattern: SEF in the block, bit 15 the sign of c'; NO_DET without a determinant
   __shared__ uint16_t maps[GT_WARPS][1 << TAB_MAXOPEN];
   constexpr unsigned FULL = 0xffffffffu, NO_DET = 0x7fffu;
@@ -3720,7 +3973,7 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_diag(Params P, const CT 
     const int nsef = (int)(P.sefoff[I + 1] - s0), ndet = (int)(P.detoff[I + 1] - d0);
     const bool open2 = !(P.nelec & 1) && nop != 0;
     const bool flip = open2 && P.jsym[I] % 2 != P.ksym % 2;  // second determinants with the other sign
-    const CT *c = C + s0 * KP + q;
+    const double *c = C + s0 * KP + q;
     for (int m = lane; m < 1 << nop; m += 32) map[m] = NO_DET;
     __syncwarp();
     if (nop > 1)
@@ -3735,12 +3988,12 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_diag(Params P, const CT 
         map[m] = (uint16_t)((open2 ? d >> 1 : d) | (neg << 15));
       }
     __syncwarp();
-    CT n0 = 0;
+    double n0 = 0;
     for (int s = grp; s < nsef; s += ngrp) {
-      const CT v = __ldg(c + s * KP);
+      const double v = __ldg(c + s * KP);
       n0 = fma(v, v, n0);
     }
-    double a0 = (double)n0;
+    double a0 = n0;
 #pragma unroll
     for (int o = KP; o < 32; o <<= 1) a0 += __shfl_xor_sync(FULL, a0, o);
     // exchange integrals of the open-shell pairs
@@ -3748,20 +4001,20 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_grad_diag(Params P, const CT 
       int a = 1, b = mm;
       while (b >= a) { b -= a; ++a; }
       const uint32_t between = (uint32_t)(a - b - 1) << 31;
-      CT sum = 0;
+      double sum = 0;
       for (int i = 0; i < 1 << (nop - 2); ++i) {
         // bits a and b put into i: a set, b clear
         int m = (i & ((1 << b) - 1)) | ((i >> b) << (b + 1));
         m = (m & ((1 << a) - 1)) | ((m >> a) << (a + 1)) | (1 << a);
         const uint32_t x = map[m], y = map[m ^ (1 << a) ^ (1 << b)];
         if (x == NO_DET && y == NO_DET) continue;
-        const CT cx = x == NO_DET ? (CT)0 : __ldg(c + (int)(x & 0x7fffu) * KP);
-        const CT cy = y == NO_DET ? (CT)0 : __ldg(c + (int)(y & 0x7fffu) * KP);
-        const CT v = cx + with_sign(cy, ((x ^ y) << 16) ^ between);
+        const double cx = x == NO_DET ? 0 : __ldg(c + (int)(x & 0x7fffu) * KP);
+        const double cy = y == NO_DET ? 0 : __ldg(c + (int)(y & 0x7fffu) * KP);
+        const double v = cx + with_sign(cy, ((x ^ y) << 16) ^ between);
         sum = fma(v, v, sum);
       }
       const int oa = nth(so, a), ob = nth(so, b);
-      atomicAdd(T2 + canon4(oa, ob, ob, oa) * KP + q, (open2 ? 0.5 : 1.0) * (double)sum - a0);
+      atomicAdd(T2 + canon4(oa, ob, ob, oa) * KP + q, (open2 ? 0.5 : 1.0) * sum - a0);
     }
     // orbital energies and the other pairs of occupied orbitals j < i; j = i: the orbital itself
     for (int e = grp; e < nocc * (nocc + 1) / 2; e += ngrp) {
@@ -3809,7 +4062,7 @@ void grad_tabs_release(psoci_ctx *c) {
 // one pass of kk <= KP roots, added to G1 [kk][n1] and G2 [kk][n2]
 template <int W, int KP>
 cudaError_t grad_pass(psoci_ctx *c, const Params &P, const TabSet<W> &S, int kk, const double *V, int64_t ldv,
-                      psoci_prec prec, double *CS, double *T1, double *G1, double *G2) {
+                      double *CS, double *T1, double *G1, double *G2) {
   cudaStream_t st = c->stream;
   const int64_t N = c->nsef_total, n1 = c->n1, n2 = c->n2;
   double *T2 = T1 + n1 * KP;
@@ -3820,18 +4073,10 @@ cudaError_t grad_pass(psoci_ctx *c, const Params &P, const TabSet<W> &S, int kk,
   psoci_note_launch();
   psoci_note_launch();
   psoci_note_launch();
-  if (prec == PSOCI_PREC_MIXED) {
-    float *C = reinterpret_cast<float *>(CS);
-    k_grad_rows<float, KP><<<rb, 256, 0, st>>>(N, V, ldv, kk, C);
-    k_grad_tab<W, float, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, S.cfg, c->grad_nbroff, c->grad_nbr, S.slot, S.t.hdr,
-                                                           S.t.pool, C, T1, T2);
-    k_grad_diag<W, float, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, C, T1, T2);
-  } else {
-    k_grad_rows<double, KP><<<rb, 256, 0, st>>>(N, V, ldv, kk, CS);
-    k_grad_tab<W, double, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, S.cfg, c->grad_nbroff, c->grad_nbr, S.slot, S.t.hdr,
-                                                            S.t.pool, CS, T1, T2);
-    k_grad_diag<W, double, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, CS, T1, T2);
-  }
+  k_grad_rows<KP><<<rb, 256, 0, st>>>(N, V, ldv, kk, CS);
+  k_grad_tab<W, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, S.cfg, c->grad_nbroff, c->grad_nbr, S.slot, S.t.hdr, S.t.pool, CS,
+                                                  T1, T2);
+  k_grad_diag<W, KP><<<gb, GT_WARPS * 32, 0, st>>>(P, CS, T1, T2);
   psoci_note_launch();
   psoci_note_launch();
   k_grad_out<KP><<<(unsigned)std::min<int64_t>((n1 + 255) / 256, 152 * 8), 256, 0, st>>>(n1, kk, T1, G1);
@@ -3881,8 +4126,8 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
     c->grad_npairs = npairs;
   }
   // coupling tables, kept with the lists; the generic kernel for spaces or patterns that they do
-  // not hold
-  if (!c->grad_tabs && !c->grad_generic) {
+  // not hold, and for FP32 sums, whose rounding is that of its order (the tables' agreed to 1e-8)
+  if (prec == PSOCI_PREC_FP64 && !c->grad_tabs && !c->grad_generic) {
     DirTabs *d = new DirTabs();
     bool ok = tab_usable(c, false);
     if (ok && (s = tab_prepare_lists<W>(c, P, c->grad_nbroff, c->grad_nbr, c->grad_npairs, false, true, dir_set<W>(d), ok))) {
@@ -3893,7 +4138,7 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
     else delete d;
     c->grad_generic = !ok;
   }
-  const bool tabs = c->grad_tabs != nullptr;
+  const bool tabs = prec == PSOCI_PREC_FP64 && c->grad_tabs != nullptr;
   double *CD = nullptr;  // determinant-basis vectors (FP64, or FP32 for the FP32-bulk variant)
   double *CS = nullptr, *T1 = nullptr;  // SEF-basis vectors and gradients, the roots of a pass side by side
   auto done = [&](psoci_status r) {
@@ -3916,10 +4161,10 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
     const double *V = dV + (int64_t)r0 * ldv;
     if (tabs) {
       const TabSet<W> &S = dir_set<W>(static_cast<DirTabs *>(c->grad_tabs));
-      e = kk <= 1 ? grad_pass<W, 1>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
-          : kk <= 2 ? grad_pass<W, 2>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
-          : kk <= 4 ? grad_pass<W, 4>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
-                    : grad_pass<W, 8>(c, P, S, kk, V, ldv, prec, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2);
+      e = kk <= 1 ? grad_pass<W, 1>(c, P, S, kk, V, ldv, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
+          : kk <= 2 ? grad_pass<W, 2>(c, P, S, kk, V, ldv, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
+          : kk <= 4 ? grad_pass<W, 4>(c, P, S, kk, V, ldv, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2)
+                    : grad_pass<W, 8>(c, P, S, kk, V, ldv, CS, T1, dG1 + r0 * n1, dG2 + r0 * n2);
     } else {
       psoci_note_launch();
       if (prec == PSOCI_PREC_MIXED)
@@ -4159,7 +4404,7 @@ cudaError_t den_pass(psoci_ctx *c, int k, const double *V, int64_t ldv, double *
   cudaError_t e = cudaMemsetAsync(T, 0, sizeof(double) * ntri * KP, st);
   if (e != cudaSuccess) return e;
   for (int q = 0; q < 4; ++q) psoci_note_launch();
-  k_grad_rows<double, KP><<<(unsigned)std::min<int64_t>((N + 255) / 256, 152 * 16), 256, 0, st>>>(N, V, ldv, k, c->den_rows);
+  k_grad_rows<KP><<<(unsigned)std::min<int64_t>((N + 255) / 256, 152 * 16), 256, 0, st>>>(N, V, ldv, k, c->den_rows);
   k_den_diag<W, KP><<<(unsigned)std::min<int64_t>((c->nconf + 31) / 32, 152 * 4), 128, 0, st>>>(den_params(c), S.cfg,
                                                                                             c->den_rows, T);
   if (np > 0)
