@@ -2587,9 +2587,9 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
 // a lane owns a neighbour and marks, per row SEF r of I, the column SEFs t whose determinants are
 // within two spin-orbital substitutions with the same spin projection (one, any spin, for spin-orbit
 // pairs); a row's marked elements, by pair kind, neighbour and column, go to the lanes in turn.
-// Elements from the coupling tables in the order of k_elems took a tenth of the time (46 against 118 us
-// and 85 against 442 us at two small spaces) but agreed with these sums to 3e-8 only.  FP64 products
-// (k_elems MODE 2) are the faster choice in direct mode, and what its solves use.
+// Elements from the coupling tables, in the order of k_elems, took 46 us for 118 and 85 for 442 at two
+// small spaces, but agreed with these sums to 3e-8 only.  FP64 products (k_elems MODE 2) are the
+// faster choice in direct mode, and what its solves use.
 // ------------------------------------------------------------------------------------
 constexpr int FAST_MAXDET = 32;
 constexpr int FAST_MAXSEF = 16;
