@@ -4276,9 +4276,9 @@ __global__ void __launch_bounds__(256) k_den_slots(Params P, const CfgRec<W> *__
 }
 
 // Off-diagonal: KP lanes (a root each) to a pair, the signed products of its list added in FP64,
-// and to the packed triangle T [place][KP] by FP64 atomics.  mrcisd_6e8o_v24, 8 roots: the whole
-// density 339 us, where a warp took the determinants of a pair in float-float sums,
-// four roots a pass, for 1,560 us.
+// and to the packed triangle T [place][KP] by FP64 atomics.  Bound by the latency of record, table
+// header, list and vectors (FP64 pipe 40%).  mrcisd_6e8o_v24, 8 roots: the whole density 240 us,
+// where a warp took the determinants of a pair in float-float sums, four roots a pass, for 1,440 us.
 template <int KP>
 __global__ void __launch_bounds__(256) k_den_pairs(int64_t np, const uint4 *__restrict__ recs,
                                                    const uint4 *__restrict__ hdr, const uint32_t *__restrict__ pool,
