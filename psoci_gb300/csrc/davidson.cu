@@ -474,11 +474,14 @@ __global__ void k_cholqr_factor(const double *S, int b, const double *ref, int l
 // ------------------------------------------------------------------------------------
 constexpr int OC_CTAS = 16, OC_THREADS = 512, OC_MAXR = 256, OC_ROWS = OC_CTAS * OC_MAXR;
 constexpr int OC_SUMS = (MAX_SUB + 16) * 16;
+// shares of a block of k_tn: at most TS_THREADS / ceil(k / 8) rows (share, output) of k values padded
+// to a multiple of 4
+constexpr int OC_RED = TS_THREADS * 8;
 
 struct __align__(16) OcSmem {
   double sums[2][OC_SUMS];      // this CTA's sums, two phases in turn (peers read them)
   float2 Cf[MAX_SUB * 16];      // coefficients, split, zero-padded to kq columns
-  double red[OC_THREADS * 4];
+  double red[OC_RED];
   double S[256], ref[256], F[256];
   CholSmem chol;
   int nk;
@@ -498,6 +501,7 @@ size_t oc_smem(size_t per, int m, int b, bool &staged) {
 template <int NJ, typename LOAD>
 __device__ void oc_tn(OcSmem &s, const float2 *Tf, int kq, int rows, int m, int k, LOAD a, double *out) {
   const int S = max(1, TS_THREADS / (m * ((k + 7) >> 3))), nj = (k + NJ - 1) / NJ;
+  const int ks = (k + 3) & ~3;  // of the sums: T's rows (kq) may be wider, where columns were dropped
   for (int e = threadIdx.x; e < S * m * nj; e += OC_THREADS) {
     const int g = e / m, i = e - g * m, sub = g / nj, j0 = NJ * (g - sub * nj);
     float h[NJ], l[NJ];
@@ -513,7 +517,7 @@ __device__ void oc_tn(OcSmem &s, const float2 *Tf, int kq, int rows, int m, int 
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
       ff_renorm(h[j], l[j]);
-      s.red[(sub * m + i) * kq + j0 + j] = (double)h[j] + (double)l[j];
+      s.red[(sub * m + i) * ks + j0 + j] = (double)h[j] + (double)l[j];
     }
   }
   __syncthreads();
@@ -521,7 +525,7 @@ __device__ void oc_tn(OcSmem &s, const float2 *Tf, int kq, int rows, int m, int 
     const int i = o / k, j = o - i * k;
     double v = 0.0;
 #pragma unroll 4
-    for (int q = 0; q < S; ++q) v += s.red[(q * m + i) * kq + j];
+    for (int q = 0; q < S; ++q) v += s.red[(q * m + i) * ks + j];
     out[o] = v;
   }
   __syncthreads();
@@ -529,7 +533,7 @@ __device__ void oc_tn(OcSmem &s, const float2 *Tf, int kq, int rows, int m, int 
 template <typename LOAD>
 __device__ __forceinline__ void oc_tn(OcSmem &s, const float2 *Tf, int kq, int rows, int m, int k, LOAD a, double *out) {
   // four outputs a thread where that still gives each thread an item
-  if (max(1, TS_THREADS / (m * ((k + 7) >> 3))) * m * (kq >> 2) >= OC_THREADS) oc_tn<4>(s, Tf, kq, rows, m, k, a, out);
+  if (max(1, TS_THREADS / (m * ((k + 7) >> 3))) * m * ((k + 3) >> 2) >= OC_THREADS) oc_tn<4>(s, Tf, kq, rows, m, k, a, out);
   else oc_tn<2>(s, Tf, kq, rows, m, k, a, out);
 }
 // its diagonal for a = T: out[j] = sum T[r, j]^2
