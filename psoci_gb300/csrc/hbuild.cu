@@ -1685,6 +1685,7 @@ __global__ void __launch_bounds__(EL_WARPS * 32) k_elems(Params P, ElemArgs<W> E
         single = ((h.y >> TAB_KIND) & 7u) == K_SINGLE;
         two = !single && (h.y >> (TAB_FORMS + 3)) != 0u;
         const bool counted = MODE == 0 && !single && !two && !(h.y & TAB_NOCOUNTS);  // by the table's rows alone
+        bool any = true;
 #pragma unroll
         for (int w = 0; w < W; ++w) sa[w] = a.e1[w] & ~a.e2[w];
         if (VALS) {
@@ -1711,12 +1712,12 @@ __global__ void __launch_bounds__(EL_WARPS * 32) k_elems(Params P, ElemArgs<W> E
           A.flags = up ? b.flags : a.flags; A.jsym = up ? b.jsym : a.jsym;
           B.flags = up ? a.flags : b.flags; B.jsym = up ? a.jsym : b.jsym;
           const PairShape s = pair_shape<W>(A, B);
-          pair_values<W>(P, A, B, s, v0, v1);
+          any = pair_values<W>(P, A, B, s, v0, v1);  // not: skipped whole, as in the list
           pr.y = b.sef;
         }
-        c = (int)(h.y & TAB_ENTRIES);
+        c = any ? (int)(h.y & TAB_ENTRIES) : 0;
         ent0 = h.x;
-        rows = (uint64_t)h.z | ((uint64_t)h.w << 32);
+        rows = any ? (uint64_t)h.z | ((uint64_t)h.w << 32) : 0ull;
         pr.z = 3u * h.x + 4u * (uint32_t)c;  // row indices: a byte each, after the entries
         pr.x = h.y & ((3u << TAB_FACTORS) | (7u << TAB_KIND));
         if (single) {
