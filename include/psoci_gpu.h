@@ -146,6 +146,13 @@ PSOCI_API psoci_status psoci_build_stats(const psoci_ctx *ctx, psoci_build_info 
  * the same bit for bit either way.  No counterpart in the reference (a GPU scheduling choice). */
 PSOCI_API psoci_status psoci_set_eval_launches(psoci_ctx *ctx, int launches);
 
+/* Device memory that the context may take, its cache of released blocks included, in bytes (0, the
+ * default: no limit).  What does not need the memory to run (lists of pair integrals, coupling
+ * tables) is left out within it; calls that need more answer PSOCI_ERR_NOMEM.  *held (may be
+ * NULL): the bytes in use now.  The reference's counterpart is the fixed memory of its Global
+ * Arrays processes. */
+PSOCI_API psoci_status psoci_set_memory_limit(psoci_ctx *ctx, int64_t bytes, int64_t *held);
+
 /* Replaces PsociHamiltonian::generateSOCIblocks (PsociHamiltonian.C:401-558) for a batch of
  * configuration pairs: block q is the reference's nsef_A x nsef_B sefsef matrix for
  * (A[q], B[q]) in the reference's roles, row-major, stored consecutively in out (host) in

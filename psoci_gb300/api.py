@@ -98,6 +98,7 @@ SIGNATURES = {
                                     ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]),
     "psoci_autotune_sigma": (ctypes.c_int, [_P, ctypes.c_int, _IP, ctypes.POINTER(ctypes.c_float)]),
     "psoci_set_eval_launches": (ctypes.c_int, [_P, ctypes.c_int]),
+    "psoci_set_memory_limit": (ctypes.c_int, [_P, ctypes.c_int64, ctypes.POINTER(ctypes.c_int64)]),
     "psoci_davidson_batch": (ctypes.c_int, [ctypes.POINTER(_P), ctypes.c_int, ctypes.POINTER(DavOpts),
                                             ctypes.POINTER(_DP), ctypes.POINTER(_DP), ctypes.POINTER(_DP),
                                             ctypes.POINTER(DavStats), _IP]),
@@ -356,6 +357,12 @@ class Context:
         """1: the H build's pair integrals evaluated in the element launches; 0: automatic (listed
         by a launch of their own when the list fits)."""
         self._check(self.lib.psoci_set_eval_launches(self.ctx, launches), "set_eval_launches")
+
+    def set_memory_limit(self, nbytes: int) -> int:
+        """Device memory that this context may take (0: no limit); returns the bytes in use."""
+        held = ctypes.c_int64()
+        self._check(self.lib.psoci_set_memory_limit(self.ctx, nbytes, ctypes.byref(held)), "set_memory_limit")
+        return held.value
 
     def set_sigma_variant(self, v: int):
         """Install mixed-sigma variant v (0..5) without timing."""

@@ -507,7 +507,7 @@ extern "C" psoci_status psoci_density1_device(psoci_ctx *c, int k, const double 
   PSOCI_CUDA(c, cudaSetDevice(c->device));
   psoci_status s;
   if ((s = density_groups(c))) return s;
-  if (c->den_tabs) return psoci_density_tab_run(c, k, dV, ldv, dD);
+  if (c->den_tabs && (s = psoci_density_tab_run(c, k, dV, ldv, dD)) != PSOCI_ERR_NOMEM) return s;
   cudaStream_t st = c->stream;
   const int ntri = c->nbf * (c->nbf + 1) / 2;
   PSOCI_CUDA(c, cudaMemsetAsync(dD, 0, sizeof(double) * (size_t)k * ntri, st));

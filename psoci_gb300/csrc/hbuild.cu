@@ -2098,8 +2098,8 @@ psoci_status screen_pairs(psoci_ctx *c, const Params &P0, const double *prune_on
     JoinSlab S = {};
     bool single = false;
     {
-      size_t freeb = 0, totb = 0;
-      TRYC(cudaMemGetInfo(&freeb, &totb));
+      size_t freeb = 0;
+      TRYC(psoci_mem_free(c, &freeb));
       const int64_t tails = (int64_t)jblocks * 8 * 2 * JOIN_CHUNK;
       int64_t cap = std::max<int64_t>(c->join_hint + c->join_hint / 8, 1024 * (int64_t)n) + tails;
       cap = std::min<int64_t>(cap, (int64_t)(freeb * 0.4) / 4);
@@ -2202,11 +2202,11 @@ struct TabSet {
 
 // Whether a space goes by coupling tables: every configuration within TAB_MAXOPEN open shells
 // and room for the diagonal blocks (N rows of the largest configuration's SEFs).
-bool tab_usable(const psoci_ctx *c, bool want_diag) {
+bool tab_usable(psoci_ctx *c, bool want_diag) {
   if (c->max_ndet > TAB_MAXDET) return false;
   if (!want_diag) return true;
-  size_t freeb = 0, totb = 0;
-  if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess) return false;
+  size_t freeb = 0;
+  if (psoci_mem_free(c, &freeb) != cudaSuccess) return false;
   return (double)c->nsef_total * c->max_nsef * 8.0 <= 0.25 * ((double)freeb + (double)c->pool_bytes);
 }
 
@@ -2216,17 +2216,17 @@ int max_open_of(const psoci_ctx *c) {
   return no;
 }
 
-// Tables of the pairs whose slots `slots_of(S)` writes (a launch on the stream): S.slot and with
-// vals S.vals for npairs pairs.  grad: with the tables' programs.  ok = false: the patterns do not
-// fit the tables and nothing is left allocated; the generic kernels take the space.
+// Tables of the pairs whose slots `slots_of(S)` writes (a launch on the stream): with own S.slot and
+// with vals S.vals for npairs pairs.  grad: with the tables' programs.  ok = false: the patterns do
+// not fit the tables and nothing is left allocated; the generic kernels take the space.
 template <int W, class F>
-psoci_status tab_prepare(psoci_ctx *c, const Params &P, int64_t npairs, bool vals, bool grad, TabSet<W> &S, bool &ok,
-                         F &&slots_of) {
+psoci_status tab_prepare(psoci_ctx *c, const Params &P, int64_t npairs, bool own, bool vals, bool grad, TabSet<W> &S,
+                         bool &ok, F &&slots_of) {
   cudaStream_t st = c->stream;
   const int n = c->nconf;
   psoci_status s = PSOCI_OK;
   ok = false;
-  if ((s = psoci_alloc(c, &S.cfg, n)) || (s = psoci_alloc(c, &S.slot, npairs)) ||
+  if ((s = psoci_alloc(c, &S.cfg, n)) || (own && (s = psoci_alloc(c, &S.slot, npairs))) ||
       (vals && (s = psoci_alloc(c, &S.vals, npairs))) || (s = psoci_alloc(c, &S.t.counter, 2))) {
     S.free();
     return s;
@@ -2289,7 +2289,7 @@ psoci_status tab_prepare_lists(psoci_ctx *c, const Params &P, const int64_t *nbr
                                bool vals, bool grad, TabSet<W> &S, bool &ok) {
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)c->nconf * 32 + 255) / 256, 1 << 20));
   auto k = grad ? k_pair_slots<W, false, true> : vals ? k_pair_slots<W, true, false> : k_pair_slots<W, false, false>;
-  return tab_prepare<W>(c, P, npairs, vals, grad, S, ok, [&](TabSet<W> &T) {
+  return tab_prepare<W>(c, P, npairs, true, vals, grad, S, ok, [&](TabSet<W> &T) {
     k<<<blocks, 256, 0, c->stream>>>(P, T.cfg, nbroff, nbr, T.t.keys, (uint32_t)(T.t.slots - 1), T.t.err, T.slot, T.vals);
   });
 }
@@ -2415,8 +2415,8 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
   if (fast) {
     // the pairs' integrals in a list (16 bytes a pair) when it takes at most a quarter of the
     // memory there is, evaluated in each element launch otherwise
-    size_t freeb = 0, totb = 0;
-    TRYC(cudaMemGetInfo(&freeb, &totb));
+    size_t freeb = 0;
+    TRYC(psoci_mem_free(c, &freeb));
     vals = c->eval_launches != 1 && (double)npairs * 16.0 <= 0.25 * ((double)freeb + (double)c->pool_bytes);
     TRYC(cudaEventRecord(ev[2], st));
     TRY(tab_prepare_lists<W>(c, P, d_nbroff, d_nbr, npairs, vals, false, T, fast));
@@ -4373,15 +4373,20 @@ Params den_params(const psoci_ctx *c) {
   return P;
 }
 
+// den_tabs and den_recs, where the records take at most a quarter of the memory at hand and the
+// tables hold the patterns and have room; the generic kernels need neither.
 template <int W>
 psoci_status den_plan(psoci_ctx *c) {
   const Params P = den_params(c);
+  const int64_t np = c->den_npairs;
+  size_t freeb = 0;
+  PSOCI_CUDA(c, psoci_mem_free(c, &freeb));
+  if ((double)np * sizeof(uint4) > 0.25 * ((double)freeb + (double)c->pool_bytes)) return PSOCI_OK;
   DirTabs *d = new DirTabs();
   bool ok = false;
-  const int64_t np = c->den_npairs;
   psoci_status s = psoci_alloc(c, &c->den_recs, np);
   if (s == PSOCI_OK)
-    s = tab_prepare<W>(c, P, np, false, true, dir_set<W>(d), ok, [&](TabSet<W> &T) {
+    s = tab_prepare<W>(c, P, np, false, false, true, dir_set<W>(d), ok, [&](TabSet<W> &T) {
       k_den_slots<W><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((np + 1023) / 1024, 152 * 32)), 256, 0, c->stream>>>(
           P, T.cfg, c->den_ng, np, c->den_geoff, c->den_gpoff, c->den_gcfg, c->den_gorb, T.t.keys,
           (uint32_t)(T.t.slots - 1), T.t.err, c->den_recs);
@@ -4389,7 +4394,9 @@ psoci_status den_plan(psoci_ctx *c) {
   if (s != PSOCI_OK || !ok) {
     delete d;
     psoci_free(c->den_recs);
-    return s;
+    if (s != PSOCI_ERR_NOMEM) return s;
+    c->err.clear();
+    return PSOCI_OK;
   }
   c->den_tabs = d;
   return PSOCI_OK;
@@ -4419,7 +4426,16 @@ template <int W>
 psoci_status den_run(psoci_ctx *c, int k, const double *V, int64_t ldv, double *D) {
   const int ntri = c->nbf * (c->nbf + 1) / 2;
   psoci_status s;
-  if (!c->den_rows && (s = psoci_alloc(c, &c->den_rows, (size_t)(c->nsef_total + ntri) * 8))) return s;
+  // for eight roots, so that later calls only launch, unless they take more than 1% of the memory
+  int width = k <= 2 ? k : k <= 4 ? 4 : 8;
+  if (c->den_width < width) {
+    size_t freeb = 0;
+    PSOCI_CUDA(c, psoci_mem_free(c, &freeb));
+    if ((c->nsef_total + ntri) * 64.0 <= 0.01 * ((double)freeb + (double)c->pool_bytes)) width = 8;
+    c->den_width = 0;
+    if ((s = psoci_alloc(c, &c->den_rows, (size_t)(c->nsef_total + ntri) * width))) return s;
+    c->den_width = width;
+  }
   for (int r0 = 0; r0 < k; r0 += 8) {
     const int kk = std::min(8, k - r0);
     const double *v = V + (int64_t)r0 * ldv;
@@ -4450,4 +4466,5 @@ void psoci_density_tabs_release(psoci_ctx *c) {
   }
   psoci_free(c->den_recs);
   psoci_free(c->den_rows);
+  c->den_width = 0;
 }

@@ -37,6 +37,7 @@ struct psoci_ctx {
   // released device blocks kept for reuse (size -> pointer), see psoci_alloc
   std::multimap<size_t, void *> pool;
   size_t pool_bytes = 0, pool_cap = 0;
+  size_t held = 0, mem_limit = 0;  // bytes in use; most that they and the pool may take (0: no limit)
 
   // integrals
   int nbf = 0;
@@ -114,6 +115,7 @@ struct psoci_ctx {
   void *den_tabs = nullptr;      // their coupling tables (hbuild.cu, DirTabs), or null: generic kernel
   uint4 *den_recs = nullptr;     // [npairs] what the table kernel reads of a pair
   double *den_rows = nullptr;    // the roots of a pass (at most 8) side by side, and the triangles being summed
+  int den_width = 0;             // roots that it has room for
 
   // mixed-sigma variant in use (sigma.cu; psoci_autotune_sigma picks it, a build resets it)
   int sigma_variant = PSOCI_SIGMA_DEFAULT;
@@ -181,6 +183,8 @@ void *psoci_device_alloc(psoci_ctx *c, size_t bytes, cudaError_t *err);
 void psoci_device_free(void *p);
 void psoci_pool_flush(psoci_ctx *c);
 void psoci_pool_forget(psoci_ctx *c);
+// cudaMemGetInfo's free bytes, within the context's limit (psoci_set_memory_limit)
+cudaError_t psoci_mem_free(psoci_ctx *c, size_t *bytes);
 
 template <typename T>
 psoci_status psoci_alloc(psoci_ctx *c, T **p, size_t count) {
@@ -228,7 +232,8 @@ void psoci_h_release(psoci_ctx *c);
 void psoci_dets_release(psoci_ctx *c);
 void psoci_density_release(psoci_ctx *c);
 // density from coupling tables (hbuild.cu): tables and pair records of the groups (den_tabs stays
-// null where the tables do not hold the space), the density, their release
+// null where the tables do not hold the space or there is no room for them), the density
+// (PSOCI_ERR_NOMEM: nothing done, no room for the vectors' rows), their release
 psoci_status psoci_density_plan(psoci_ctx *c);
 psoci_status psoci_density_tab_run(psoci_ctx *c, int k, const double *dV, int64_t ldv, double *dD);
 void psoci_density_tabs_release(psoci_ctx *c);

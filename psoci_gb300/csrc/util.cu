@@ -40,6 +40,14 @@ void flush_device_locked(int dev) {
     }
   g_pooled[dev] = 0;
 }
+
+// one context's released blocks (g_mu held)
+void flush_pool_locked(psoci_ctx *c) {
+  for (auto &kv : c->pool) cudaFree(kv.second);
+  c->pool.clear();
+  g_pooled[c->device] -= c->pool_bytes;
+  c->pool_bytes = 0;
+}
 }  // namespace
 
 void psoci_pool_register(psoci_ctx *c) {
@@ -54,7 +62,8 @@ void *psoci_device_alloc(psoci_ctx *c, size_t bytes, cudaError_t *err) {
     *err = cudaMalloc(&p, bytes);
     return (*err == cudaSuccess) ? p : nullptr;
   }
-  bool reused = false;
+  bool reused = false, over = false;
+  size_t held = 0;
   {
     std::lock_guard<std::mutex> g(g_mu);
     auto it = c->pool.lower_bound(bytes);
@@ -65,7 +74,11 @@ void *psoci_device_alloc(psoci_ctx *c, size_t bytes, cudaError_t *err) {
       c->pool_bytes -= sz;
       g_pooled[c->device] -= sz;
       g_blocks[p] = {c, sz};
+      c->held += held = sz;
       reused = true;
+    } else if (c->mem_limit && c->held + c->pool_bytes + bytes > c->mem_limit) {
+      flush_pool_locked(c);
+      over = c->held + bytes > c->mem_limit;
     }
   }
   if (reused) {
@@ -76,6 +89,7 @@ void *psoci_device_alloc(psoci_ctx *c, size_t bytes, cudaError_t *err) {
       {
         std::lock_guard<std::mutex> g(g_mu);
         g_blocks.erase(p);
+        c->held -= held;
       }
       cudaFree(p);
       *err = e;
@@ -84,8 +98,8 @@ void *psoci_device_alloc(psoci_ctx *c, size_t bytes, cudaError_t *err) {
     *err = cudaSuccess;
     return p;
   }
-  cudaError_t e = cudaMalloc(&p, bytes);
-  if (e == cudaErrorMemoryAllocation) {
+  cudaError_t e = over ? cudaErrorMemoryAllocation : cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation && !over) {
     cudaGetLastError();
     bool had = false;
     {
@@ -101,6 +115,7 @@ void *psoci_device_alloc(psoci_ctx *c, size_t bytes, cudaError_t *err) {
   }
   std::lock_guard<std::mutex> g(g_mu);
   g_blocks[p] = {c, bytes};
+  c->held += bytes;
   *err = cudaSuccess;
   return p;
 }
@@ -114,6 +129,7 @@ void psoci_device_free(void *p) {
       psoci_ctx *c = it->second.first;
       const size_t sz = it->second.second;
       g_blocks.erase(it);
+      if (c) c->held -= sz;
       // the cap holds for all contexts of the device together
       if (c && g_pooled[c->device] + sz <= c->pool_cap) {
         c->pool.insert({sz, p});
@@ -128,10 +144,27 @@ void psoci_device_free(void *p) {
 
 void psoci_pool_flush(psoci_ctx *c) {
   std::lock_guard<std::mutex> g(g_mu);
-  for (auto &kv : c->pool) cudaFree(kv.second);
-  c->pool.clear();
-  g_pooled[c->device] -= c->pool_bytes;
-  c->pool_bytes = 0;
+  flush_pool_locked(c);
+}
+
+cudaError_t psoci_mem_free(psoci_ctx *c, size_t *bytes) {
+  size_t total = 0;
+  const cudaError_t e = cudaMemGetInfo(bytes, &total);
+  std::lock_guard<std::mutex> g(g_mu);
+  if (e == cudaSuccess && c->mem_limit) {
+    const size_t used = c->held + c->pool_bytes;
+    *bytes = std::min(*bytes, used < c->mem_limit ? c->mem_limit - used : 0);
+  }
+  return e;
+}
+
+extern "C" psoci_status psoci_set_memory_limit(psoci_ctx *c, int64_t bytes, int64_t *held) {
+  if (!c) return PSOCI_ERR_INVALID_ARG;
+  if (bytes < 0) return psoci_fail(c, PSOCI_ERR_INVALID_ARG, "set_memory_limit: negative limit");
+  std::lock_guard<std::mutex> g(g_mu);
+  c->mem_limit = (size_t)bytes;
+  if (held) *held = (int64_t)c->held;
+  return PSOCI_OK;
 }
 
 // blocks of a context that is going away and were never released; the context leaves the
