@@ -4127,19 +4127,20 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
     c->grad_npairs = npairs;
   }
   // coupling tables, kept with the lists; the generic kernel for spaces or patterns that they do
-  // not hold, and for FP32 sums, whose rounding is that of its order (the tables' agreed to 1e-8)
+  // not hold, where there is no room for them, and for FP32 sums, whose rounding is that of its order
+  // (the tables' agreed to 1e-8)
   if (prec == PSOCI_PREC_FP64 && !c->grad_tabs && !c->grad_generic) {
     DirTabs *d = new DirTabs();
     bool ok = tab_usable(c, false);
-    if (ok && (s = tab_prepare_lists<W>(c, P, c->grad_nbroff, c->grad_nbr, c->grad_npairs, false, true, dir_set<W>(d), ok))) {
-      delete d;
-      return s;
-    }
-    if (ok) c->grad_tabs = d;
+    s = PSOCI_OK;
+    if (ok) s = tab_prepare_lists<W>(c, P, c->grad_nbroff, c->grad_nbr, c->grad_npairs, false, true, dir_set<W>(d), ok);
+    if (s == PSOCI_OK && ok) c->grad_tabs = d;
     else delete d;
-    c->grad_generic = !ok;
+    if (s != PSOCI_OK && s != PSOCI_ERR_NOMEM) return s;
+    if (s != PSOCI_OK) c->err.clear();
+    c->grad_generic = !c->grad_tabs;
   }
-  const bool tabs = prec == PSOCI_PREC_FP64 && c->grad_tabs != nullptr;
+  bool tabs = prec == PSOCI_PREC_FP64 && c->grad_tabs != nullptr;
   double *CD = nullptr;  // determinant-basis vectors (FP64, or FP32 for the FP32-bulk variant)
   double *CS = nullptr, *T1 = nullptr;  // SEF-basis vectors and gradients, the roots of a pass side by side
   auto done = [&](psoci_status r) {
@@ -4148,9 +4149,15 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
   };
   const int kmax = std::min(k, ADJ_MAXR), kpmax = kmax <= 2 ? kmax : kmax <= 4 ? 4 : 8;
   const int64_t N = c->nsef_total;
+  if (tabs && ((s = psoci_alloc(c, &CS, (size_t)N * kpmax)) || (s = psoci_alloc(c, &T1, (size_t)(n1 + n2) * kpmax)))) {
+    if (s != PSOCI_ERR_NOMEM) return done(s);
+    c->err.clear();
+    done(s);
+    grad_tabs_release(c);
+    c->grad_generic = true;
+    tabs = false;
+  }
   if (!tabs && (s = psoci_alloc(c, &CD, (size_t)c->ndet_total * kmax))) return done(s);
-  if (tabs && ((s = psoci_alloc(c, &CS, (size_t)N * kpmax)) || (s = psoci_alloc(c, &T1, (size_t)(n1 + n2) * kpmax))))
-    return done(s);
   float *CD32 = reinterpret_cast<float *>(CD);
   cudaError_t e = cudaMemsetAsync(dG1, 0, sizeof(double) * n1 * k, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(dG2, 0, sizeof(double) * n2 * k, st);

@@ -44,3 +44,35 @@ def test_density(oracle_mod, name, ksym, k):
     c = limited(p)
     assert np.abs(c.density1(v) - O.density1(v)).max() <= 1e-12
     c.close()
+
+
+@pytest.mark.parametrize("k", [1, 5])
+@pytest.mark.parametrize("room", [ROOM, 1 << 20])
+@pytest.mark.parametrize("nonzero", [False, True])
+def test_gradient(room, k, nonzero):
+    """Sums of at most N^2 products of unit vectors in either kernel."""
+    p = small_problem("fci_5e6o", 1)
+    c = gpu_context(p)
+    v = unit_vectors(k, c.nsef)
+    free = c.energy_gradient(v, nonzero_only=nonzero)
+    c.close()
+    c = limited(p, room)
+    for a, b in zip(free, c.energy_gradient(v, nonzero_only=nonzero)):
+        assert np.abs(a - b).max() <= 1e-12
+    c.close()
+
+
+def test_gradient_vectors_without_room():
+    """The lists, tables and eight vectors with their gradients (172 KB) have room, the vectors' rows
+    (128 KB) beside them do not."""
+    p = small_problem("fci_6e8o", 1)
+    c = gpu_context(p)
+    v = unit_vectors(8, c.nsef)
+    free = c.energy_gradient(v)
+    c.close()
+    c = gpu_context(p)
+    c.energy_gradient(v[:1])  # the plan, and a first pass
+    c.set_memory_limit(c.set_memory_limit(0) + (240 << 10))
+    for a, b in zip(free, c.energy_gradient(v)):
+        assert np.abs(a - b).max() <= 1e-12
+    c.close()
