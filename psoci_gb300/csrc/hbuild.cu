@@ -2347,8 +2347,15 @@ TabSet<W> &dir_set(DirTabs *d) {
   else return d->s2;
 }
 
+// Kernels of a build: by coupling tables with the pairs' integrals listed or evaluated in the element
+// launches, or the generic ones.  `form` comes in as the first that may be taken and leaves as the
+// one that was; each needs less memory than the one before.
+enum { FORM_LISTED, FORM_UNLISTED, FORM_GENERIC };
+
 template <int W>
-psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
+psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int &form, int64_t *nnz_out) {
+  const int first = form;
+  form = FORM_GENERIC;
   cudaStream_t st = c->stream;
   const int n = c->nconf;
   Params P = {};
@@ -2411,15 +2418,17 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz_out) {
   // for others, and for patterns the tables do not hold
   const bool direct = (mode == PSOCI_HMODE_DIRECT);
   const int64_t N = c->nsef_total;
-  bool fast = tab_usable(c, true), vals = false;
+  bool fast = first < FORM_GENERIC && tab_usable(c, true), vals = false;
   if (fast) {
     // the pairs' integrals in a list (16 bytes a pair) when it takes at most a quarter of the
     // memory there is, evaluated in each element launch otherwise
     size_t freeb = 0;
     TRYC(psoci_mem_free(c, &freeb));
-    vals = c->eval_launches != 1 && (double)npairs * 16.0 <= 0.25 * ((double)freeb + (double)c->pool_bytes);
+    vals = first == FORM_LISTED && (double)npairs * 16.0 <= 0.25 * ((double)freeb + (double)c->pool_bytes);
+    form = vals ? FORM_LISTED : FORM_UNLISTED;
     TRYC(cudaEventRecord(ev[2], st));
     TRY(tab_prepare_lists<W>(c, P, d_nbroff, d_nbr, npairs, vals, false, T, fast));
+    if (!fast) form = FORM_GENERIC;
   }
   auto t_c = tnow();
 
@@ -3175,10 +3184,17 @@ psoci_status psoci_h_build(psoci_ctx *c, psoci_hmode mode, int64_t *nnz) {
     return psoci_fail(c, PSOCI_ERR_INVALID_ARG, "integral and configuration orbital counts differ");
   psoci_h_release(c);
   auto t0 = std::chrono::steady_clock::now();
-  psoci_status s = (c->words == 1) ? run_build<1>(c, mode, nnz) : run_build<2>(c, mode, nnz);
-  if (s != PSOCI_OK) {
+  int form = c->eval_launches == 1 ? FORM_UNLISTED : FORM_LISTED;
+  psoci_status s;
+  for (bool again = false;; again = true) {
+    s = (c->words == 1) ? run_build<1>(c, mode, form, nnz) : run_build<2>(c, mode, form, nnz);
+    if (s == PSOCI_OK) {
+      if (again) c->err.clear();
+      break;
+    }
     psoci_h_release(c);
-    return s;
+    if (s != PSOCI_ERR_NOMEM || form == FORM_GENERIC) return s;
+    ++form;  // no room: the next form
   }
   c->build_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   c->have_h = true;

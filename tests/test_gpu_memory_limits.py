@@ -76,3 +76,36 @@ def test_gradient_vectors_without_room():
     for a, b in zip(free, c.energy_gradient(v)):
         assert np.abs(a - b).max() <= 1e-12
     c.close()
+
+
+@pytest.mark.parametrize("name,ksym", [("fci_5e6o", 1), ("fci_6e8o", 1)])
+def test_build_and_direct_product(name, ksym):
+    """From room for everything to none for the tables: the matrix without a limit to rounding (the
+    generic kernels form an element's sum in the reference's order, as the tables do), and the direct
+    product."""
+    p = small_problem(name, ksym)
+    c = gpu_context(p)
+    nnz = c.build_hamiltonian(mixed=True)
+    rp, ci, va = c.get_hamiltonian()
+    x = unit_vectors(3, c.nsef).T.copy()
+    y = c.sigma(x)
+    scale = np.abs(va).max() * np.diff(rp).max()
+    c.close()
+    stored = set()
+    for room in [64 << 20] + [(ROOM + 16 * nnz) + (q << 19) for q in range(16)]:
+        c = limited(p, room)
+        c.build_hamiltonian(mixed=True)
+        st = c.build_stats()
+        stored.add(st["eval_launches"])
+        assert st["fast"] == (st["eval_launches"] > 0)
+        for a, b in zip((rp, ci), c.get_hamiltonian()):
+            assert np.array_equal(a, b)
+        assert np.abs(c.get_hamiltonian()[2] - va).max() <= 1e-12
+        c.build_hamiltonian(direct=True)
+        assert np.abs(c.sigma(x) - y).max() <= 1e-14 * scale
+        c.close()
+    assert {0, 2} <= stored
+    c = limited(p, ROOM)
+    c.build_hamiltonian(direct=True)
+    assert np.abs(c.sigma(x) - y).max() <= 1e-14 * scale
+    c.close()
