@@ -60,7 +60,7 @@ typedef enum {
   PSOCI_HMODE_CSR_FP64 = 0,   /* stored FP64 CSR only                                   */
   PSOCI_HMODE_CSR_BOTH = 1,   /* stored FP64 CSR plus an FP32 copy of the elements      */
   PSOCI_HMODE_DIRECT = 2      /* nothing stored: neighbour lists and the diagonal only;  */
-                              /* every sigma evaluates the elements again (FP64)         */
+                              /* every sigma evaluates the elements again                */
 } psoci_hmode;
 
 /* Replaces GA::Initialize + the PsociGAhamiltonian constructor
@@ -110,11 +110,14 @@ PSOCI_API psoci_status psoci_get_determinants(const psoci_ctx *ctx, uint64_t *al
  * PSOCI_HMODE_DIRECT stands in for the reference's direct products
  * (matrixVectorProductsSplitChunkMultipleJchunksLowLevelAccumulateDirectFetch,
  * PsociGAhamiltonian.C:7549-7826, built with DIRECTMATRIXPRODUCTS): only the screened
- * neighbour lists with their coupling tables, the diagonal blocks and, where they take at most a
- * quarter of the device memory at hand, the pairs' integrals (16 bytes a pair) are kept (*nnz =
- * 0); psoci_sigma / psoci_sigma_device /
- * psoci_davidson then evaluate every element again on each call, in FP64 whatever the
- * precision asked for, applying the same |x| >= 1e-8 rule.  psoci_get_hamiltonian,
+ * neighbour lists (4 bytes a pair) with their coupling tables (4 bytes a pair, the diagonal blocks)
+ * and, where they take at most a quarter of the device memory at hand, the pairs' integrals (16
+ * bytes a pair; not with psoci_set_eval_launches(ctx, 1)) are kept (*nnz = 0), the integrals and
+ * the tables until this context needs their memory; psoci_sigma / psoci_sigma_device /
+ * psoci_davidson then evaluate every element again on each call, applying the same |x| >= 1e-8
+ * rule.  Products are FP64, but for PSOCI_PREC_MIXED of psoci_sigma / psoci_sigma_device where no
+ * configuration has more than 32 determinants: FP32 elements and inputs with compensated FP32
+ * sums, the slower choice (psoci_davidson takes FP64 ones).  psoci_get_hamiltonian,
  * psoci_save_hamiltonian and psoci_sigma_mixed_noalloc answer PSOCI_ERR_STATE. */
 PSOCI_API psoci_status psoci_build_hamiltonian(psoci_ctx *ctx, psoci_hmode mode, int64_t *nnz);
 /* Counters and phase times of the last psoci_build_hamiltonian.  Times are CUDA-event

@@ -988,8 +988,9 @@ psoci_status sigma_block(Work &w, const double *X, int ldx, double *Y, int ldy, 
   if (w.block) {
     s = psoci_csr_product(w.c, w.N, w.block->rowptr, w.block->col, w.block->val, k, X, ldx, Y, ldy);
   } else {
-    // direct mode: FP64 products are the faster ones (0.084 against 0.83 s for 8 vectors of 3.84 M SEFs)
-    const psoci_prec p = (w.c->direct && prec == PSOCI_PREC_MIXED) ? PSOCI_PREC_FP64 : prec;
+    // direct mode by coupling tables: FP64 products are the faster ones (0.084 against 0.83 s for 8
+    // vectors of 3.84 M SEFs)
+    const psoci_prec p = (w.c->direct && w.c->dir_tabs && prec == PSOCI_PREC_MIXED) ? PSOCI_PREC_FP64 : prec;
     s = psoci_sigma_launch(w.c, k, X, ldx, Y, ldy, p, w.x32);
   }
   cudaEventRecord(e1, w.c->stream);

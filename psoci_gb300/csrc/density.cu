@@ -505,6 +505,7 @@ extern "C" psoci_status psoci_density1_device(psoci_ctx *c, int k, const double 
   if (!c->have_dets) return psoci_fail(c, PSOCI_ERR_STATE, "density1: build the determinants first");
   if (ldv < c->nsef_total) return psoci_fail(c, PSOCI_ERR_INVALID_ARG, "density1: ldv < N");
   PSOCI_CUDA(c, cudaSetDevice(c->device));
+  const PsociKeep own(c, PSOCI_KEEP_DENSITY);
   psoci_status s;
   if ((s = density_groups(c))) return s;
   if (c->den_tabs && (s = psoci_density_tab_run(c, k, dV, ldv, dD)) != PSOCI_ERR_NOMEM) return s;

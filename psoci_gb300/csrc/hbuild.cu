@@ -2432,10 +2432,10 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int &form, int64_t *nnz_o
   }
   auto t_c = tnow();
 
-  // 2. segments of the generic kernels and of direct mode's FP32 products (<= 32 neighbours of a
-  // configuration, one warp each)
+  // 2. segments of the generic kernels, which direct mode may come to at any time (psoci_give_back),
+  // and of its FP32 products (<= 32 neighbours of a configuration, one warp each)
   int64_t nseg = 0, nslots = 0;
-  const bool segs = !fast || (direct && c->max_ndet <= 32);
+  const bool segs = !fast || direct;
   if (segs) {
     TRY(psoci_alloc(c, &d_nseg, n + 1));
     TRY(psoci_alloc(c, &d_nrow, n + 1));
@@ -2471,7 +2471,6 @@ psoci_status run_build(psoci_ctx *c, psoci_hmode mode, int &form, int64_t *nnz_o
     P.diag = c->d_diag;
     if (fast) {
       TRY(tab_diagonal<W>(c, P, T, c->d_diag));
-      if (!segs) c->nseg = nseg = (npairs + PSOCI_SEG - 1) / PSOCI_SEG;
     } else {
       const size_t smem = sizeof(WarpSmem) * WARPS_PER_CTA;
       TRYC(cudaFuncSetAttribute(k_hbuild<W, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -3142,6 +3141,34 @@ psoci_status psoci_join_prepare(psoci_ctx *c) {
   return PSOCI_OK;
 }
 
+static void dir_tabs_release(psoci_ctx *c) {
+  if (!c->dir_tabs) return;
+  DirTabs *d = static_cast<DirTabs *>(c->dir_tabs);
+  d->s1.free();
+  d->s2.free();
+  delete d;
+  c->dir_tabs = nullptr;
+}
+
+bool psoci_give_back(psoci_ctx *c) {
+  if (c->den_tabs && !(c->keep & PSOCI_KEEP_DENSITY)) {
+    psoci_density_release(c);
+  } else if (c->grad_nbroff && !(c->keep & PSOCI_KEEP_GRAD)) {
+    psoci_grad_release(c);
+  } else if (c->dir_tabs && !(c->keep & PSOCI_KEEP_DIRECT)) {
+    DirTabs *d = static_cast<DirTabs *>(c->dir_tabs);
+    if (d->s1.vals || d->s2.vals) {
+      psoci_free(d->s1.vals);
+      psoci_free(d->s2.vals);
+    } else {
+      dir_tabs_release(c);
+    }
+  } else {
+    return false;
+  }
+  return true;
+}
+
 void psoci_h_release(psoci_ctx *c) {
   psoci_grad_release(c);
   c->sigma_variant = PSOCI_SIGMA_DEFAULT;
@@ -3151,13 +3178,7 @@ void psoci_h_release(psoci_ctx *c) {
   psoci_free(c->dir_segcfg);
   psoci_free(c->dir_segk0);
   psoci_free(c->dir_segn);
-  if (c->dir_tabs) {
-    DirTabs *d = static_cast<DirTabs *>(c->dir_tabs);
-    d->s1.free();
-    d->s2.free();
-    delete d;
-    c->dir_tabs = nullptr;
-  }
+  dir_tabs_release(c);
   c->direct = false;
   psoci_free(c->d_rowptr);
   psoci_free(c->d_col);
@@ -4104,6 +4125,7 @@ cudaError_t grad_pass(psoci_ctx *c, const Params &P, const TabSet<W> &S, int kk,
 template <int W>
 psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv, int mode, psoci_prec prec,
                              double *dG1, double *dG2) {
+  const PsociKeep own(c, PSOCI_KEEP_GRAD);
   cudaStream_t st = c->stream;
   const int n = c->nconf;
   Params P = {};
@@ -4146,6 +4168,7 @@ psoci_status run_energy_grad(psoci_ctx *c, int k, const double *dV, int64_t ldv,
   // not hold, where there is no room for them, and for FP32 sums, whose rounding is that of its order
   // (the tables' agreed to 1e-8)
   if (prec == PSOCI_PREC_FP64 && !c->grad_tabs && !c->grad_generic) {
+    const PsociKeep plans(c, PSOCI_KEEP_ALL);
     DirTabs *d = new DirTabs();
     bool ok = tab_usable(c, false);
     s = PSOCI_OK;
@@ -4405,6 +4428,7 @@ psoci_status den_plan(psoci_ctx *c) {
   size_t freeb = 0;
   PSOCI_CUDA(c, psoci_mem_free(c, &freeb));
   if ((double)np * sizeof(uint4) > 0.25 * ((double)freeb + (double)c->pool_bytes)) return PSOCI_OK;
+  const PsociKeep plans(c, PSOCI_KEEP_ALL);
   DirTabs *d = new DirTabs();
   bool ok = false;
   psoci_status s = psoci_alloc(c, &c->den_recs, np);

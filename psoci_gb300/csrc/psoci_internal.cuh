@@ -38,6 +38,7 @@ struct psoci_ctx {
   std::multimap<size_t, void *> pool;
   size_t pool_bytes = 0, pool_cap = 0;
   size_t held = 0, mem_limit = 0;  // bytes in use; most that they and the pool may take (0: no limit)
+  unsigned keep = 0;               // PSOCI_KEEP_*: plans that psoci_give_back leaves alone
 
   // integrals
   int nbf = 0;
@@ -177,12 +178,24 @@ psoci_status psoci_cuda_fail(psoci_ctx *c, cudaError_t e, const char *where);
 // cudaMalloc (page mapping) for tens of GB each time.  Reuse waits for the context's stream
 // first, as cudaFree would have.  The caches of all contexts on one device hold at most
 // half its memory together; all of them are emptied when a cudaMalloc on that device fails
-// (and the allocation is retried), and a context's own on psoci_destroy.
+// (and the allocation is retried), and a context's own on psoci_destroy.  If that does not make
+// room, the context gives back what it keeps to be faster (psoci_give_back).
 void psoci_pool_register(psoci_ctx *c);
 void *psoci_device_alloc(psoci_ctx *c, size_t bytes, cudaError_t *err);
 void psoci_device_free(void *p);
 void psoci_pool_flush(psoci_ctx *c);
 void psoci_pool_forget(psoci_ctx *c);
+// One of the plans that the context keeps to be faster and can do without (hbuild.cu), the least
+// missed first: of the density, of the gradient, the pair integrals of direct mode, its coupling
+// tables.  False when nothing is left, or what is left is in use (PsociKeep).
+bool psoci_give_back(psoci_ctx *c);
+enum : unsigned { PSOCI_KEEP_DENSITY = 1, PSOCI_KEEP_GRAD = 2, PSOCI_KEEP_DIRECT = 4, PSOCI_KEEP_ALL = 7 };
+struct PsociKeep {
+  psoci_ctx *c;
+  unsigned before;
+  PsociKeep(psoci_ctx *ctx, unsigned what) : c(ctx), before(ctx->keep) { c->keep |= what; }
+  ~PsociKeep() { c->keep = before; }
+};
 // cudaMemGetInfo's free bytes, within the context's limit (psoci_set_memory_limit)
 cudaError_t psoci_mem_free(psoci_ctx *c, size_t *bytes);
 

@@ -55,8 +55,7 @@ void psoci_pool_register(psoci_ctx *c) {
   g_ctxs[c->device].push_back(c);
 }
 
-void *psoci_device_alloc(psoci_ctx *c, size_t bytes, cudaError_t *err) {
-  if (bytes == 0) bytes = 1;
+static void *alloc_once(psoci_ctx *c, size_t bytes, cudaError_t *err) {
   void *p = nullptr;
   if (!c) {
     *err = cudaMalloc(&p, bytes);
@@ -117,6 +116,16 @@ void *psoci_device_alloc(psoci_ctx *c, size_t bytes, cudaError_t *err) {
   g_blocks[p] = {c, bytes};
   c->held += bytes;
   *err = cudaSuccess;
+  return p;
+}
+
+void *psoci_device_alloc(psoci_ctx *c, size_t bytes, cudaError_t *err) {
+  if (bytes == 0) bytes = 1;
+  void *p = alloc_once(c, bytes, err);
+  while (!p && c && *err == cudaErrorMemoryAllocation && psoci_give_back(c)) {
+    cudaGetLastError();
+    p = alloc_once(c, bytes, err);
+  }
   return p;
 }
 

@@ -109,3 +109,35 @@ def test_build_and_direct_product(name, ksym):
     c.build_hamiltonian(direct=True)
     assert np.abs(c.sigma(x) - y).max() <= 1e-14 * scale
     c.close()
+
+
+@pytest.mark.parametrize("below", [-(1 << 18), 0, 3 << 20])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_direct_solve_takes_the_tables_memory(below, mixed):
+    """A direct build's pair integrals, then its tables, go when the solve's basis (2 MB) needs their
+    room: limits of 256 KB above to 3 MB below what the build holds."""
+    p = small_problem("fci_6e8o", 1)
+    c = gpu_context(p)
+    c.build_hamiltonian(direct=True)
+    full = c.davidson(4, rtol=1e-8, mixed=mixed)
+    c.close()
+    c = gpu_context(p)
+    c.build_hamiltonian(direct=True)
+    held = c.set_memory_limit(0)
+    c.set_memory_limit(held - below)
+    r = c.davidson(4, rtol=1e-8, mixed=mixed)
+    assert np.abs(r.evals - full.evals).max() <= 1e-10
+    assert c.set_memory_limit(0) < held - max(below, 0)
+    c.close()
+
+
+def test_build_takes_the_densitys_memory():
+    p = small_problem("fci_6e8o", 1)
+    c = gpu_context(p)
+    v = unit_vectors(2, c.nsef)
+    d = c.density1(v)
+    c.set_memory_limit(c.set_memory_limit(0) + (1 << 20))
+    c.build_hamiltonian(mixed=True)  # 3.4 MB of elements
+    c.set_memory_limit(0)
+    assert np.abs(c.density1(v) - d).max() <= 1e-14
+    c.close()
