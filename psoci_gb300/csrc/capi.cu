@@ -217,7 +217,7 @@ psoci_status psoci_set_configs(psoci_ctx *c, int nbf, int nelec, int ksym, int m
   psoci_parallel_ranges(nconf, [&](int64_t lo, int64_t hi, int) {
     memcpy(c->h_occ.data() + (size_t)lo * nbf, occ + (size_t)lo * nbf, (size_t)(hi - lo) * nbf);
   });
-  c->tab_words_hint = 0;
+  for (auto &h : c->tab_words_hint) h = 0;
   c->join_hint = 0;
   c->have_cfgs = true;
   return psoci_join_prepare(c);

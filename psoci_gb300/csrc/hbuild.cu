@@ -2222,6 +2222,7 @@ int max_open_of(const psoci_ctx *c) {
 template <int W, class F>
 psoci_status tab_prepare(psoci_ctx *c, const Params &P, int64_t npairs, bool own, bool vals, bool grad, TabSet<W> &S,
                          bool &ok, F &&slots_of) {
+  int64_t &hint = c->tab_words_hint[!grad ? 0 : own ? 1 : 2];
   cudaStream_t st = c->stream;
   const int n = c->nconf;
   psoci_status s = PSOCI_OK;
@@ -2235,22 +2236,27 @@ psoci_status tab_prepare(psoci_ctx *c, const Params &P, int64_t npairs, bool own
   cudaError_t e = cudaSuccess;
   psoci_note_launch();
   k_cfg_rec<W><<<(int)std::min<int64_t>((n + 255) / 256, 152 * 16), 256, 0, st>>>(P, S.cfg);
-  // 2^18 key slots hold every space measured (up to 6 * 10^4 patterns); a full table grows
-  int64_t slots = 1 << 14, cap = std::max<int64_t>(c->tab_words_hint + c->tab_words_hint / 8, 1 << 20);
+  // 2^18 key slots hold every space measured (up to 6 * 10^4 patterns); a full table grows, and a
+  // pool that was too small, whose keys and slots stay (the tables of 10 open shells go beyond 2^20
+  // words)
+  int64_t slots = 1 << 14, cap = std::max<int64_t>(hint + hint / 8, 1 << 20);
   while (slots < 4 * npairs && slots < (1 << 18)) slots <<= 1;
+  bool keyed = false;
   for (int attempt = 0; attempt < 6 && e == cudaSuccess; ++attempt) {
-    if ((s = psoci_alloc(c, &S.t.keys, slots)) || (s = psoci_alloc(c, &S.t.hdr, 2 * slots)) ||
+    if ((!keyed && ((s = psoci_alloc(c, &S.t.keys, slots)) || (s = psoci_alloc(c, &S.t.hdr, 2 * slots)))) ||
         (s = psoci_alloc(c, &S.t.pool, cap))) {
       S.free();
       return s;
     }
     S.t.slots = slots;
     S.t.cap = cap;
-    e = cudaMemsetAsync(S.t.keys, 0, sizeof(uint64_t) * slots, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(S.t.counter, 0, 2 * sizeof(unsigned long long), st);
+    e = cudaMemsetAsync(S.t.counter, 0, 2 * sizeof(unsigned long long), st);
+    if (e == cudaSuccess && !keyed) e = cudaMemsetAsync(S.t.keys, 0, sizeof(uint64_t) * slots, st);
     if (e != cudaSuccess) break;
-    psoci_note_launch();
-    slots_of(S);
+    if (!keyed) {
+      psoci_note_launch();
+      slots_of(S);
+    }
     const TabBuildArgs B = {S.t.keys, slots, c->d_tmpl, c->d_tmpl_off, c->nelec, c->ksym & 1,
                             S.t.hdr, S.t.pool, S.t.counter, cap, S.t.err};
     psoci_note_launch();
@@ -2265,8 +2271,9 @@ psoci_status tab_prepare(psoci_ctx *c, const Params &P, int64_t npairs, bool own
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) break;
     const int err = (int)(uint32_t)back[1];
-    c->tab_words_hint = (int64_t)back[0];
     if (err & 2) break;  // a pattern outside the tables' form
+    keyed = !(err & 1);
+    if (keyed) hint = (int64_t)back[0];
     if (!(err & 1) && (int64_t)back[0] <= cap) {
       ok = true;
       break;

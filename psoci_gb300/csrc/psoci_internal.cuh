@@ -103,7 +103,7 @@ struct psoci_ctx {
   int32_t *dir_segcfg = nullptr, *dir_segn = nullptr;
   int64_t *dir_segk0 = nullptr;
   void *dir_tabs = nullptr;       // coupling tables of the elements (hbuild.cu, DirTabs), or null
-  int64_t tab_words_hint = 0;     // words of coupling tables the last build used
+  int64_t tab_words_hint[3] = {};  // words of coupling tables the last build, gradient and density plan used
   int64_t join_hint = 0;  // join-slab slots the last build of this space used
 
   // 1-particle density: configuration groups sharing a hole key (density.cu)
