@@ -268,6 +268,7 @@ __device__ __forceinline__ uint32_t red_sum(uint32_t d0, uint32_t d1, bool m, ui
 }
 
 constexpr int TABB_WARPS = 4, TABB_LIST = 1024;
+constexpr int TABB_SLOTS = 8;  // key slots a warp looks through (up to one in eight is taken)
 struct TabBuildSmem {
   uint16_t aA[TAB_MAXDET], bA[TAB_MAXDET], aB[TAB_MAXDET], bB[TAB_MAXDET];
   uint32_t ent[TABB_LIST];  // the first entries and their rows
@@ -316,8 +317,8 @@ __global__ void __launch_bounds__(TABB_WARPS * 32) k_tab_build(TabBuildArgs T) {
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const bool odd = T.nelec & 1;
-  for (int64_t s0 = warp * 32; s0 < T.slots; s0 += nwarps * 32) {
-    const uint64_t mykey = (s0 + lane < T.slots) ? T.keys[s0 + lane] : 0ull;
+  for (int64_t s0 = warp * TABB_SLOTS; s0 < T.slots; s0 += nwarps * TABB_SLOTS) {
+    const uint64_t mykey = (lane < TABB_SLOTS && s0 + lane < T.slots) ? T.keys[s0 + lane] : 0ull;
     unsigned todo = __ballot_sync(0xffffffffu, mykey != 0ull);
     while (todo) {
       const int src = __ffs(todo) - 1;
@@ -541,14 +542,16 @@ __device__ __forceinline__ int tab_weight(uint32_t ent, bool single, int a) {
   return w;
 }
 
-// Programs of all occupied slots, from their entries; one warp a slot, lanes over the entries.
-__global__ void __launch_bounds__(128) k_tab_program(const uint64_t *__restrict__ keys, int64_t slots, uint4 *hdr,
-                                                     uint32_t *pool, unsigned long long *counter, int64_t cap) {
+// Programs of all occupied slots, from their entries (at most the first `want` lists); one warp a slot,
+// lanes over the entries.
+__global__ void __launch_bounds__(128) k_tab_program(const uint64_t *__restrict__ keys, int64_t slots, int want,
+                                                     uint4 *hdr, uint32_t *pool, unsigned long long *counter,
+                                                     int64_t cap) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t s0 = warp * 32; s0 < slots; s0 += nwarps * 32) {
-    unsigned todo = __ballot_sync(0xffffffffu, s0 + lane < slots && keys[s0 + lane] != 0ull);
+  for (int64_t s0 = warp * TABB_SLOTS; s0 < slots; s0 += nwarps * TABB_SLOTS) {
+    unsigned todo = __ballot_sync(0xffffffffu, lane < TABB_SLOTS && s0 + lane < slots && keys[s0 + lane] != 0ull);
     while (todo) {
       const int64_t s = s0 + __ffs(todo) - 1;
       todo &= todo - 1;
@@ -561,7 +564,7 @@ __global__ void __launch_bounds__(128) k_tab_program(const uint64_t *__restrict_
       }
       const bool single = ((h.y >> TAB_KIND) & 7u) == 2u;
       const uint8_t *rows = reinterpret_cast<const uint8_t *>(pool + h.x + nent);
-      const int most = single ? TAB_LISTS : 2;
+      const int most = min(want, single ? TAB_LISTS : 2);
       uint32_t words = 0u, off = 0u;
       int lists = 0;
       bool fits = false;

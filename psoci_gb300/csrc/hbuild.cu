@@ -2236,11 +2236,19 @@ psoci_status tab_prepare(psoci_ctx *c, const Params &P, int64_t npairs, bool own
   cudaError_t e = cudaSuccess;
   psoci_note_launch();
   k_cfg_rec<W><<<(int)std::min<int64_t>((n + 255) / 256, 152 * 16), 256, 0, st>>>(P, S.cfg);
-  // 2^18 key slots hold every space measured (up to 6 * 10^4 patterns); a full table grows, and a
-  // pool that was too small, whose keys and slots stay (the tables of 10 open shells go beyond 2^20
-  // words)
-  int64_t slots = 1 << 14, cap = std::max<int64_t>(hint + hint / 8, 1 << 20);
-  while (slots < 4 * npairs && slots < (1 << 18)) slots <<= 1;
+  // Key slots and pool words that hold the spaces measured, full CI of 2 to 8 electrons and reference
+  // spaces with singles and doubles: 0.56 patterns a pair at 32 pairs, 0.12 at 10^4, 5 * 10^4 at
+  // most; the density 10 to 800.  Words: up to 1.9 a pair (64 SEFs), the density 35,000 (16 SEFs), 180,000
+  // (64).  Few pairs take little: an allocation of a megabyte or more costs 30 to 70 us, and the first
+  // density of 1,001 SEFs took 490 us with 2^14 slots and 2^20 words.  A full table grows, and a
+  // pool that was too small, whose keys and slots stay.
+  const bool den = grad && !own;
+  const int64_t most = den ? 1 << 12 : 1 << 18, wide = std::max(2, c->max_nsef / 8);
+  int64_t slots = 1 << 11;
+  while (slots < npairs / 4 && slots < most) slots <<= 1;
+  int64_t cap = den ? std::max(1 << 14, c->max_nsef << 12)
+                    : std::min<int64_t>(std::max<int64_t>(1 << 12, wide * npairs), 1 << 20);
+  cap = std::max<int64_t>(cap, hint + hint / 8);
   bool keyed = false;
   for (int attempt = 0; attempt < 6 && e == cudaSuccess; ++attempt) {
     if ((!keyed && ((s = psoci_alloc(c, &S.t.keys, slots)) || (s = psoci_alloc(c, &S.t.hdr, 2 * slots)))) ||
@@ -2260,10 +2268,11 @@ psoci_status tab_prepare(psoci_ctx *c, const Params &P, int64_t npairs, bool own
     const TabBuildArgs B = {S.t.keys, slots, c->d_tmpl, c->d_tmpl_off, c->nelec, c->ksym & 1,
                             S.t.hdr, S.t.pool, S.t.counter, cap, S.t.err};
     psoci_note_launch();
-    k_tab_build<<<(unsigned)((slots / 32 + TABB_WARPS - 1) / TABB_WARPS), TABB_WARPS * 32, 0, st>>>(B);
+    k_tab_build<<<(unsigned)(slots / (TABB_SLOTS * TABB_WARPS)), TABB_WARPS * 32, 0, st>>>(B);
     if (grad) {
       psoci_note_launch();
-      k_tab_program<<<(unsigned)((slots / 32 + 3) / 4), 128, 0, st>>>(S.t.keys, slots, S.t.hdr, S.t.pool, S.t.counter, cap);
+      k_tab_program<<<(unsigned)(slots / (TABB_SLOTS * 4)), 128, 0, st>>>(S.t.keys, slots, den ? 1 : TAB_LISTS, S.t.hdr,
+                                                                          S.t.pool, S.t.counter, cap);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) break;
     unsigned long long back[2] = {0, 0};  // words used; error bits

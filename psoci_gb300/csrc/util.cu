@@ -268,6 +268,16 @@ psoci_status psoci_scan_i64(psoci_ctx *c, const int64_t *d_in, int64_t *d_out, i
     return PSOCI_OK;
   }
   int64_t nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
+  if (nb == 1) {  // one launch (the general way takes three, two allocations and a copy: 25 us more)
+    int64_t tot = 0;
+    psoci_note_launch();
+    k_scan_chunk<<<1, SCAN_T, 0, s>>>(d_in, d_out, n, d_out + n, nullptr);
+    PSOCI_CUDA(c, cudaGetLastError());
+    PSOCI_CUDA(c, cudaMemcpyAsync(&tot, d_out + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    PSOCI_CUDA(c, cudaStreamSynchronize(s));
+    if (total) *total = tot;
+    return PSOCI_OK;
+  }
   int64_t *d_bs = nullptr, *d_bo = nullptr;
   psoci_status st = psoci_alloc(c, &d_bs, nb + 1);
   if (st) return st;
@@ -277,13 +287,8 @@ psoci_status psoci_scan_i64(psoci_ctx *c, const int64_t *d_in, int64_t *d_out, i
   k_scan_chunk<<<(unsigned)nb, SCAN_T, 0, s>>>(d_in, nullptr, n, d_bs, nullptr);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) {
-    if (nb > 1) {
-      int64_t tb = 0;
-      st = psoci_scan_i64(c, d_bs, d_bo, nb, &tb);
-    } else {
-      int64_t z = 0;
-      e = cudaMemcpyAsync(d_bo, &z, sizeof(int64_t), cudaMemcpyHostToDevice, s);
-    }
+    int64_t tb = 0;
+    st = psoci_scan_i64(c, d_bs, d_bo, nb, &tb);
   }
   if (e == cudaSuccess && st == PSOCI_OK) {
     psoci_note_launch();
