@@ -62,7 +62,10 @@ struct BlockTab {
   uint4 *hdr = nullptr;      // [2 slots]
   uint32_t *pool = nullptr;
   unsigned long long *counter = nullptr;  // words of the pool in use
-  int *err = nullptr;        // bit 0: key table full, bit 1: a pattern outside the tables' form
+  // counter + 1: err, bit 0: key table full, bit 1: a pattern outside the tables' form; err + 1: the
+  // patterns, whose slots are in list
+  int *err = nullptr;
+  uint32_t *list = nullptr;  // [slots]
   int64_t slots = 0, cap = 0;
 };
 
@@ -163,14 +166,15 @@ __device__ __forceinline__ uint64_t tab_hash(uint64_t x) {
   return x ^ (x >> 32);
 }
 
-// slot of a key, inserted when new; TAB_NONE (and bit 0 of *err) when the table is full
-__device__ __forceinline__ uint32_t tab_insert(uint64_t *keys, uint32_t mask, uint64_t key, int *err) {
+// slot of a key, inserted (and listed) when new; TAB_NONE (and bit 0 of *err) when the table is full
+__device__ __forceinline__ uint32_t tab_insert(uint64_t *keys, uint32_t mask, uint64_t key, int *err, uint32_t *list) {
   uint32_t s = (uint32_t)tab_hash(key) & mask;
   for (int probe = 0; probe < 256; ++probe) {
     uint64_t cur = *(volatile uint64_t *)(keys + s);
     if (cur == key) return s;
     if (cur == 0ull) {
       cur = atomicCAS((unsigned long long *)(keys + s), 0ull, (unsigned long long)key);
+      if (cur == 0ull) list[atomicAdd(err + 1, 1)] = s;
       if (cur == 0ull || cur == key) return s;
     }
     s = (s + 1) & mask;
@@ -268,7 +272,6 @@ __device__ __forceinline__ uint32_t red_sum(uint32_t d0, uint32_t d1, bool m, ui
 }
 
 constexpr int TABB_WARPS = 4, TABB_LIST = 1024;
-constexpr int TABB_SLOTS = 8;  // key slots a warp looks through (up to one in eight is taken)
 struct TabBuildSmem {
   uint16_t aA[TAB_MAXDET], bA[TAB_MAXDET], aB[TAB_MAXDET], bB[TAB_MAXDET];
   uint32_t ent[TABB_LIST];  // the first entries and their rows
@@ -277,7 +280,7 @@ struct TabBuildSmem {
 
 struct TabBuildArgs {
   const uint64_t *keys;
-  int64_t slots;
+  const uint32_t *list;
   const uint32_t *tmpl;
   const int32_t *tmpl_off;
   int nelec, kodd;  // electrons; ksym odd
@@ -305,11 +308,13 @@ __device__ inline void tab_strings(uint32_t S, uint32_t D, int cls, int nop, con
   }
 }
 
-// Every occupied slot's table: lanes over its (row, column) elements, the entries found kept in shared
+// Every listed slot's table: lanes over its (row, column) elements, the entries found kept in shared
 // memory until their number, and so their place, is known; a table of more than TABB_LIST is
 // evaluated once more for its place.  Bound by integer issue; 2 * 10^4 patterns of up to 6 open
 // shells take about as long as reading the neighbour lists once.  (All tables evaluated twice: 0.77
-// ms for 8 electrons in 10 orbitals, up to 8 open shells; 0.42 ms now.)
+// ms for 8 electrons in 10 orbitals, up to 8 open shells; 0.42 ms now.  By the list, so that few large
+// tables go to as many warps: with a warp to 32 key slots a direct build of 200 configurations of up to 8
+// open shells took 2.5 ms, now 1.25.)
 __global__ void __launch_bounds__(TABB_WARPS * 32) k_tab_build(TabBuildArgs T) {
   __shared__ TabBuildSmem sm[TABB_WARPS];
   TabBuildSmem &S = sm[threadIdx.x >> 5];
@@ -317,152 +322,148 @@ __global__ void __launch_bounds__(TABB_WARPS * 32) k_tab_build(TabBuildArgs T) {
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const bool odd = T.nelec & 1;
-  for (int64_t s0 = warp * TABB_SLOTS; s0 < T.slots; s0 += nwarps * TABB_SLOTS) {
-    const uint64_t mykey = (lane < TABB_SLOTS && s0 + lane < T.slots) ? T.keys[s0 + lane] : 0ull;
-    unsigned todo = __ballot_sync(0xffffffffu, mykey != 0ull);
-    while (todo) {
-      const int src = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const uint64_t key = __shfl_sync(0xffffffffu, mykey, src);
-      // the pattern
-      uint32_t a1 = 0, a2 = 0, b1 = 0, b2 = 0;
-      for (int q = 0; q < TAB_SYMS; ++q) {
-        const uint32_t y = (uint32_t)(key >> (4 * q)) & 15u;
-        a1 |= (y & 1u) << q; a2 |= ((y >> 1) & 1u) << q; b1 |= ((y >> 2) & 1u) << q; b2 |= ((y >> 3) & 1u) << q;
-      }
-      const int kc = (int)(key >> 48) & 3;
-      const bool rowsB = (key >> 50) & 1ull;
-      RedPair R;
-      R.kind = kc == 1 ? 3 : kc == 2 ? 2 : 4;
-      R.jA = (int)(key >> 53) & 1;
-      R.jB = (int)(key >> 54) & 1;
-      R.SA = a1 & ~a2;
-      const uint32_t SB = b1 & ~b2;
-      R.nD = (T.nelec - __popc(a1) - __popc(a2)) / 2;
-      const uint32_t i1 = a1 & ~b1, i2 = a2 & ~b2, j1 = b1 & ~a1, j2 = b2 & ~a2;
-      R.ex0 = __ffs(i1 | i2) - 1;
-      R.ex1 = (i1 & i2) ? R.ex0 : __ffs((i1 | i2) & ((i1 | i2) - 1)) - 1;
-      R.jy0 = __ffs(j1 | j2) - 1;
-      R.jy1 = (j1 & j2) ? R.jy0 : __ffs((j1 | j2) & ((j1 | j2) - 1)) - 1;
-      R.ie = R.ex0;
-      R.je = R.jy0;
-      R.fold = R.kind == 3 && (R.ex0 == R.ex1 || R.jy0 == R.jy1);
-      const int opA = __popc(R.SA), opB = __popc(SB);
-      const int cls0 = odd ? CLS_FRAC_P : CLS_EVEN;
-      tab_strings(R.SA, a2, cls0 + ((int)(key >> 51) & 1), opA, T, S.aA, S.bA, lane);
-      tab_strings(SB, b2, cls0 + ((int)(key >> 52) & 1), opB, T, S.aB, S.bB, lane);
-      __syncwarp();
-      const bool oa = !odd && opA != 0, ob = !odd && opB != 0;
-      const bool mA = (R.jA != T.kodd), mB = (R.jB != T.kodd);  // -1 where true
-      const int lA = opA > 1 ? opA - 1 - (oa ? 1 : 0) : 0, lB = opB > 1 ? opB - 1 - (ob ? 1 : 0) : 0;  // log2 SEFs
-      const int lr = rowsB ? lB : lA, lc = rowsB ? lA : lB;
-      const int nrow = 1 << lr, tot = 1 << (lr + lc);
-      const bool counts = nrow <= 16;
-      uint32_t forms = 0u, ent0 = 0u;
-      bool bad = false, fits = false;
-      uint64_t nib[3] = {0ull, 0ull, 0ull};
-      int nent = 0;
-      for (int pass = 0; pass < 2; ++pass) {
-        int n = 0;
-        for (int e0 = 0; e0 < tot; e0 += 32) {
-          const int e = e0 + lane, r = e >> lc, t = e & ((1 << lc) - 1);
-          uint32_t ent = 0u;
-          bool have = false;
-          if (e < tot) {
-            const int a = rowsB ? t : r, b = rowsB ? r : t;
-            uint32_t d[2][2] = {{0u, 0u}, {0u, 0u}};
-#pragma unroll
-            for (int x = 0; x < 2; ++x)
-#pragma unroll
-              for (int y = 0; y < 2; ++y) {
-                if ((x && !oa) || (y && !ob)) continue;
-                const int da = oa ? 2 * a + x : (odd ? a : 0), db = ob ? 2 * b + y : (odd ? b : 0);
-                d[x][y] = red_code(R, S.aA[da], S.bA[da], S.aB[db], S.bB[db], bad);
-              }
-            uint32_t t1, u1;
-            const uint32_t t0 = red_sum(d[0][0], d[0][1], mB, t1);
-            have = t0 != 0u;
-            if (oa) {  // the second half, times mA: the same terms, or their negatives (sum zero)
-              uint32_t u0 = red_sum(d[1][0], d[1][1], mB, u1);
-              if (mA) { if (u0) u0 ^= RED_NEG; if (u1) u1 ^= RED_NEG; }
-              if ((u0 ^ t0) & ~RED_NEG || (u1 ^ t1) & ~RED_NEG) bad = true;
-              else if (t0 && u0 != t0) {
-                if (t1 && u1 == t1) bad = true;
-                have = false;
-              } else if (t1 && u1 != t1) bad = true;
-            }
-            if (have) {
-              if (R.kind == 2) {
-                ent = ((t0 & 0xfffu) << 8) | ((t1 ? (t1 & 0xfffu) : TAB_NOTERM) << 20);
-              } else {
-                const int f = t1 ? tab_form2((int)(t0 & 3u), (int)(t1 & 3u), (int)(((t0 ^ t1) & RED_NEG) != 0u))
-                                 : (int)(t0 & 3u);
-                forms |= 1u << f;
-                ent = ((uint32_t)f << 8) | ((uint32_t)r << 12) | ((t0 & RED_NEG) ? 0x80000000u : 0u);
-              }
-              ent |= (uint32_t)t;
-            }
-          }
-          const unsigned hb = __ballot_sync(0xffffffffu, have);
-          const int at = n + __popc(hb & ((1u << lane) - 1u));
-          if (pass == 0) {
-            if (have && at < TABB_LIST) {
-              S.ent[at] = ent;
-              S.row[at] = (uint8_t)r;
-            }
-            if (have && counts) {  // lanes' shares, summed below
-              nib[0] += 1ull << (4 * r);
-              const uint32_t f = (ent >> 8) & 15u;
-              if (R.kind == 3 && f == 1u) nib[1] += 1ull << (4 * r);
-              if (R.kind == 3 && f == 2u) nib[2] += 1ull << (4 * r);
-            }
-          } else if (fits) {
-            if (have) {
-              T.pool[ent0 + at] = ent;
-              reinterpret_cast<uint8_t *>(T.pool + ent0 + nent)[at] = (uint8_t)r;
-            }
-          }
-          n += __popc(hb);
-        }
-        if (pass == 0) {
-          nent = n;
-          const uint32_t words = (uint32_t)nent + (uint32_t)(nent + 3) / 4u;
-          unsigned long long o = 0;
-          if (lane == 0) o = atomicAdd(T.counter, (unsigned long long)words);
-          o = __shfl_sync(0xffffffffu, o, 0);
-          fits = (int64_t)(o + words) <= T.cap;
-          ent0 = (uint32_t)o;
-          // a row has at most 2 + one an open shell (of at most 6), so the 4-bit sums do not carry
-#pragma unroll
-          for (int o2 = 16; o2 > 0; o2 >>= 1)
-#pragma unroll
-            for (int u = 0; u < 3; ++u) nib[u] += __shfl_xor_sync(0xffffffffu, nib[u], o2);
-          __syncwarp();
-          if (nent <= TABB_LIST) {
-            if (fits)
-              for (int q = lane; q < nent; q += 32) {
-                T.pool[ent0 + q] = S.ent[q];
-                reinterpret_cast<uint8_t *>(T.pool + ent0 + nent)[q] = S.row[q];
-              }
-            break;
-          }
-        }
-      }
-      __syncwarp();
-      if (nent > TAB_ENTRIES) bad = true;
-#pragma unroll
-      for (int o2 = 16; o2 > 0; o2 >>= 1) forms |= __shfl_xor_sync(0xffffffffu, forms, o2);
-      if (__ballot_sync(0xffffffffu, bad) && lane == 0) atomicOr(T.err, 2);
-      if (lane == 0) {
-        const uint32_t fc = odd ? 0u : (oa && ob) ? 3u : ob ? 1u : oa ? 2u : 0u;
-        const uint32_t info = ((uint32_t)nent & TAB_ENTRIES) | (fc << TAB_FACTORS) | ((uint32_t)R.kind << TAB_KIND) |
-                              (counts ? 0u : TAB_NOCOUNTS) | (forms << TAB_FORMS);
-        T.hdr[2 * (s0 + src)] = make_uint4(ent0, info, (uint32_t)nib[0], (uint32_t)(nib[0] >> 32));
-        T.hdr[2 * (s0 + src) + 1] =
-            make_uint4((uint32_t)nib[1], (uint32_t)(nib[1] >> 32), (uint32_t)nib[2], (uint32_t)(nib[2] >> 32));
-      }
-      __syncwarp();
+  const int npat = T.err[1];
+  for (int64_t p = warp; p < npat; p += nwarps) {
+    const int64_t slot = T.list[p];
+    const uint64_t key = T.keys[slot];
+    // the pattern
+    uint32_t a1 = 0, a2 = 0, b1 = 0, b2 = 0;
+    for (int q = 0; q < TAB_SYMS; ++q) {
+      const uint32_t y = (uint32_t)(key >> (4 * q)) & 15u;
+      a1 |= (y & 1u) << q; a2 |= ((y >> 1) & 1u) << q; b1 |= ((y >> 2) & 1u) << q; b2 |= ((y >> 3) & 1u) << q;
     }
+    const int kc = (int)(key >> 48) & 3;
+    const bool rowsB = (key >> 50) & 1ull;
+    RedPair R;
+    R.kind = kc == 1 ? 3 : kc == 2 ? 2 : 4;
+    R.jA = (int)(key >> 53) & 1;
+    R.jB = (int)(key >> 54) & 1;
+    R.SA = a1 & ~a2;
+    const uint32_t SB = b1 & ~b2;
+    R.nD = (T.nelec - __popc(a1) - __popc(a2)) / 2;
+    const uint32_t i1 = a1 & ~b1, i2 = a2 & ~b2, j1 = b1 & ~a1, j2 = b2 & ~a2;
+    R.ex0 = __ffs(i1 | i2) - 1;
+    R.ex1 = (i1 & i2) ? R.ex0 : __ffs((i1 | i2) & ((i1 | i2) - 1)) - 1;
+    R.jy0 = __ffs(j1 | j2) - 1;
+    R.jy1 = (j1 & j2) ? R.jy0 : __ffs((j1 | j2) & ((j1 | j2) - 1)) - 1;
+    R.ie = R.ex0;
+    R.je = R.jy0;
+    R.fold = R.kind == 3 && (R.ex0 == R.ex1 || R.jy0 == R.jy1);
+    const int opA = __popc(R.SA), opB = __popc(SB);
+    const int cls0 = odd ? CLS_FRAC_P : CLS_EVEN;
+    tab_strings(R.SA, a2, cls0 + ((int)(key >> 51) & 1), opA, T, S.aA, S.bA, lane);
+    tab_strings(SB, b2, cls0 + ((int)(key >> 52) & 1), opB, T, S.aB, S.bB, lane);
+    __syncwarp();
+    const bool oa = !odd && opA != 0, ob = !odd && opB != 0;
+    const bool mA = (R.jA != T.kodd), mB = (R.jB != T.kodd);  // -1 where true
+    const int lA = opA > 1 ? opA - 1 - (oa ? 1 : 0) : 0, lB = opB > 1 ? opB - 1 - (ob ? 1 : 0) : 0;  // log2 SEFs
+    const int lr = rowsB ? lB : lA, lc = rowsB ? lA : lB;
+    const int nrow = 1 << lr, tot = 1 << (lr + lc);
+    const bool counts = nrow <= 16;
+    uint32_t forms = 0u, ent0 = 0u;
+    bool bad = false, fits = false;
+    uint64_t nib[3] = {0ull, 0ull, 0ull};
+    int nent = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+      int n = 0;
+      for (int e0 = 0; e0 < tot; e0 += 32) {
+        const int e = e0 + lane, r = e >> lc, t = e & ((1 << lc) - 1);
+        uint32_t ent = 0u;
+        bool have = false;
+        if (e < tot) {
+          const int a = rowsB ? t : r, b = rowsB ? r : t;
+          uint32_t d[2][2] = {{0u, 0u}, {0u, 0u}};
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+              if ((x && !oa) || (y && !ob)) continue;
+              const int da = oa ? 2 * a + x : (odd ? a : 0), db = ob ? 2 * b + y : (odd ? b : 0);
+              d[x][y] = red_code(R, S.aA[da], S.bA[da], S.aB[db], S.bB[db], bad);
+            }
+          uint32_t t1, u1;
+          const uint32_t t0 = red_sum(d[0][0], d[0][1], mB, t1);
+          have = t0 != 0u;
+          if (oa) {  // the second half, times mA: the same terms, or their negatives (sum zero)
+            uint32_t u0 = red_sum(d[1][0], d[1][1], mB, u1);
+            if (mA) { if (u0) u0 ^= RED_NEG; if (u1) u1 ^= RED_NEG; }
+            if ((u0 ^ t0) & ~RED_NEG || (u1 ^ t1) & ~RED_NEG) bad = true;
+            else if (t0 && u0 != t0) {
+              if (t1 && u1 == t1) bad = true;
+              have = false;
+            } else if (t1 && u1 != t1) bad = true;
+          }
+          if (have) {
+            if (R.kind == 2) {
+              ent = ((t0 & 0xfffu) << 8) | ((t1 ? (t1 & 0xfffu) : TAB_NOTERM) << 20);
+            } else {
+              const int f = t1 ? tab_form2((int)(t0 & 3u), (int)(t1 & 3u), (int)(((t0 ^ t1) & RED_NEG) != 0u))
+                               : (int)(t0 & 3u);
+              forms |= 1u << f;
+              ent = ((uint32_t)f << 8) | ((uint32_t)r << 12) | ((t0 & RED_NEG) ? 0x80000000u : 0u);
+            }
+            ent |= (uint32_t)t;
+          }
+        }
+        const unsigned hb = __ballot_sync(0xffffffffu, have);
+        const int at = n + __popc(hb & ((1u << lane) - 1u));
+        if (pass == 0) {
+          if (have && at < TABB_LIST) {
+            S.ent[at] = ent;
+            S.row[at] = (uint8_t)r;
+          }
+          if (have && counts) {  // lanes' shares, summed below
+            nib[0] += 1ull << (4 * r);
+            const uint32_t f = (ent >> 8) & 15u;
+            if (R.kind == 3 && f == 1u) nib[1] += 1ull << (4 * r);
+            if (R.kind == 3 && f == 2u) nib[2] += 1ull << (4 * r);
+          }
+        } else if (fits) {
+          if (have) {
+            T.pool[ent0 + at] = ent;
+            reinterpret_cast<uint8_t *>(T.pool + ent0 + nent)[at] = (uint8_t)r;
+          }
+        }
+        n += __popc(hb);
+      }
+      if (pass == 0) {
+        nent = n;
+        const uint32_t words = (uint32_t)nent + (uint32_t)(nent + 3) / 4u;
+        unsigned long long o = 0;
+        if (lane == 0) o = atomicAdd(T.counter, (unsigned long long)words);
+        o = __shfl_sync(0xffffffffu, o, 0);
+        fits = (int64_t)(o + words) <= T.cap;
+        ent0 = (uint32_t)o;
+        // a row has at most 2 + one an open shell (of at most 6), so the 4-bit sums do not carry
+#pragma unroll
+        for (int o2 = 16; o2 > 0; o2 >>= 1)
+#pragma unroll
+          for (int u = 0; u < 3; ++u) nib[u] += __shfl_xor_sync(0xffffffffu, nib[u], o2);
+        __syncwarp();
+        if (nent <= TABB_LIST) {
+          if (fits)
+            for (int q = lane; q < nent; q += 32) {
+              T.pool[ent0 + q] = S.ent[q];
+              reinterpret_cast<uint8_t *>(T.pool + ent0 + nent)[q] = S.row[q];
+            }
+          break;
+        }
+      }
+    }
+    __syncwarp();
+    if (nent > TAB_ENTRIES) bad = true;
+#pragma unroll
+    for (int o2 = 16; o2 > 0; o2 >>= 1) forms |= __shfl_xor_sync(0xffffffffu, forms, o2);
+    if (__ballot_sync(0xffffffffu, bad) && lane == 0) atomicOr(T.err, 2);
+    if (lane == 0) {
+      const uint32_t fc = odd ? 0u : (oa && ob) ? 3u : ob ? 1u : oa ? 2u : 0u;
+      const uint32_t info = ((uint32_t)nent & TAB_ENTRIES) | (fc << TAB_FACTORS) | ((uint32_t)R.kind << TAB_KIND) |
+                            (counts ? 0u : TAB_NOCOUNTS) | (forms << TAB_FORMS);
+      T.hdr[2 * slot] = make_uint4(ent0, info, (uint32_t)nib[0], (uint32_t)(nib[0] >> 32));
+      T.hdr[2 * slot + 1] =
+          make_uint4((uint32_t)nib[1], (uint32_t)(nib[1] >> 32), (uint32_t)nib[2], (uint32_t)(nib[2] >> 32));
+    }
+    __syncwarp();
   }
 }
 
@@ -542,63 +543,60 @@ __device__ __forceinline__ int tab_weight(uint32_t ent, bool single, int a) {
   return w;
 }
 
-// Programs of all occupied slots, from their entries (at most the first `want` lists); one warp a slot,
+// Programs of all listed slots, from their entries (at most the first `want` lists); one warp a slot,
 // lanes over the entries.
-__global__ void __launch_bounds__(128) k_tab_program(const uint64_t *__restrict__ keys, int64_t slots, int want,
-                                                     uint4 *hdr, uint32_t *pool, unsigned long long *counter,
+__global__ void __launch_bounds__(128) k_tab_program(const uint32_t *__restrict__ list, const int *__restrict__ err,
+                                                     int want, uint4 *hdr, uint32_t *pool, unsigned long long *counter,
                                                      int64_t cap) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t s0 = warp * TABB_SLOTS; s0 < slots; s0 += nwarps * TABB_SLOTS) {
-    unsigned todo = __ballot_sync(0xffffffffu, lane < TABB_SLOTS && s0 + lane < slots && keys[s0 + lane] != 0ull);
-    while (todo) {
-      const int64_t s = s0 + __ffs(todo) - 1;
-      todo &= todo - 1;
-      const uint4 h = hdr[2 * s];
-      const int nent = (int)(h.y & TAB_ENTRIES);
-      // entries that did not fit the pool were not written: the host, which sees the count, repeats
-      if ((int64_t)h.x + nent + (nent + 3) / 4 > cap) {
-        if (lane == 0) hdr[2 * s + 1] = make_uint4(0u, 0u, 0u, 0u);
-        continue;
-      }
-      const bool single = ((h.y >> TAB_KIND) & 7u) == 2u;
-      const uint8_t *rows = reinterpret_cast<const uint8_t *>(pool + h.x + nent);
-      const int most = min(want, single ? TAB_LISTS : 2);
-      uint32_t words = 0u, off = 0u;
-      int lists = 0;
-      bool fits = false;
-      for (int pass = 0; pass < 2; ++pass) {
-        int n = 0;
-        for (int a = 0; a < most; ++a) {
-          for (int e0 = 0; e0 < nent; e0 += 32) {
-            const int e = e0 + lane;
-            const uint32_t ent = e < nent ? pool[h.x + e] : 0u;
-            const int w = e < nent ? tab_weight(ent, single, a) : 0;
-            const unsigned b1 = __ballot_sync(0xffffffffu, w != 0), b2 = __ballot_sync(0xffffffffu, w == 2 || w == -2);
-            if (pass == 1 && fits && w != 0) {
-              const unsigned lt = (1u << lane) - 1u;
-              const uint32_t r = single ? rows[e] : (ent >> 12) & 0xffu;
-              const uint32_t x = (ent & 0xffu) | (r << 8) | (w < 0 ? 0x80000000u : 0u);
-              uint32_t *to = pool + off + (TAB_LISTS + 1) / 2 + n + __popc(b1 & lt) + __popc(b2 & lt);
-              to[0] = x;
-              if (w == 2 || w == -2) to[1] = x;
-            }
-            n += __popc(b1) + __popc(b2);
-            if (b1) lists = a + 1;
-          }
-          if (pass == 1 && fits && lane == 0) reinterpret_cast<uint16_t *>(pool + off)[a] = (uint16_t)n;
-        }
-        if (pass == 0) {
-          words = (uint32_t)(n + (TAB_LISTS + 1) / 2);
-          unsigned long long o = 0;
-          if (lane == 0) o = atomicAdd(counter, (unsigned long long)words);
-          o = __shfl_sync(0xffffffffu, o, 0);
-          fits = (int64_t)(o + words) <= cap;
-          off = (uint32_t)o;
-        }
-      }
-      if (lane == 0) hdr[2 * s + 1] = make_uint4(off, (uint32_t)lists, 0u, 0u);
+  const int npat = err[1];
+  for (int64_t p = warp; p < npat; p += nwarps) {
+    const int64_t s = list[p];
+    const uint4 h = hdr[2 * s];
+    const int nent = (int)(h.y & TAB_ENTRIES);
+    // entries that did not fit the pool were not written: the host, which sees the count, repeats
+    if ((int64_t)h.x + nent + (nent + 3) / 4 > cap) {
+      if (lane == 0) hdr[2 * s + 1] = make_uint4(0u, 0u, 0u, 0u);
+      continue;
     }
+    const bool single = ((h.y >> TAB_KIND) & 7u) == 2u;
+    const uint8_t *rows = reinterpret_cast<const uint8_t *>(pool + h.x + nent);
+    const int most = min(want, single ? TAB_LISTS : 2);
+    uint32_t words = 0u, off = 0u;
+    int lists = 0;
+    bool fits = false;
+    for (int pass = 0; pass < 2; ++pass) {
+      int n = 0;
+      for (int a = 0; a < most; ++a) {
+        for (int e0 = 0; e0 < nent; e0 += 32) {
+          const int e = e0 + lane;
+          const uint32_t ent = e < nent ? pool[h.x + e] : 0u;
+          const int w = e < nent ? tab_weight(ent, single, a) : 0;
+          const unsigned b1 = __ballot_sync(0xffffffffu, w != 0), b2 = __ballot_sync(0xffffffffu, w == 2 || w == -2);
+          if (pass == 1 && fits && w != 0) {
+            const unsigned lt = (1u << lane) - 1u;
+            const uint32_t r = single ? rows[e] : (ent >> 12) & 0xffu;
+            const uint32_t x = (ent & 0xffu) | (r << 8) | (w < 0 ? 0x80000000u : 0u);
+            uint32_t *to = pool + off + (TAB_LISTS + 1) / 2 + n + __popc(b1 & lt) + __popc(b2 & lt);
+            to[0] = x;
+            if (w == 2 || w == -2) to[1] = x;
+          }
+          n += __popc(b1) + __popc(b2);
+          if (b1) lists = a + 1;
+        }
+        if (pass == 1 && fits && lane == 0) reinterpret_cast<uint16_t *>(pool + off)[a] = (uint16_t)n;
+      }
+      if (pass == 0) {
+        words = (uint32_t)(n + (TAB_LISTS + 1) / 2);
+        unsigned long long o = 0;
+        if (lane == 0) o = atomicAdd(counter, (unsigned long long)words);
+        o = __shfl_sync(0xffffffffu, o, 0);
+        fits = (int64_t)(o + words) <= cap;
+        off = (uint32_t)o;
+      }
+    }
+    if (lane == 0) hdr[2 * s + 1] = make_uint4(off, (uint32_t)lists, 0u, 0u);
   }
 }

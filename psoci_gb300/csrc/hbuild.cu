@@ -1326,8 +1326,8 @@ __device__ __forceinline__ bool pair_values(const Params &P, const CfgRec<W> &A,
 template <int W, bool VALS, bool LOWER>
 __global__ void __launch_bounds__(256) k_pair_slots(Params P, const CfgRec<W> *__restrict__ cfg,
                                                     const int64_t *__restrict__ nbroff, const int32_t *__restrict__ nbr,
-                                                    uint64_t *keys, uint32_t mask, int *err, uint32_t *__restrict__ slot,
-                                                    double2 *__restrict__ vals) {
+                                                    uint64_t *keys, uint32_t mask, int *err, uint32_t *list,
+                                                    uint32_t *__restrict__ slot, double2 *__restrict__ vals) {
   __shared__ int64_t s_q[8][64];   // singles set aside: place in the lists ...
   __shared__ uint32_t s_m[8][64];  // ... ie | je << 8 | J > I << 16 | sign
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1394,7 +1394,7 @@ __global__ void __launch_bounds__(256) k_pair_slots(Params P, const CfgRec<W> *_
         meta = (uint32_t)s.ex0 | ((uint32_t)s.jy0 << 8) | ((uint32_t)up << 16) | s.sign;
         if (VALS && any && !single) any = pair_values<W>(P, A, B, s, v0, v1);
         if (any) {
-          sl = tab_insert(keys, mask, pair_key<W>(A, B, s.kind, up), err);
+          sl = tab_insert(keys, mask, pair_key<W>(A, B, s.kind, up), err, list);
           if (sl != TAB_NONE) sl |= s.sign;
           if (VALS && !single && sl != TAB_NONE) {
             const uint32_t oa = A.flags & 15u, ob = B.flags & 15u;
@@ -2195,7 +2195,7 @@ struct TabSet {
   double *D = nullptr;        // diagonal blocks, ldd columns
   int ldd = 0;
   void free() {
-    psoci_free(t.keys); psoci_free(t.hdr); psoci_free(t.pool); psoci_free(t.counter);
+    psoci_free(t.keys); psoci_free(t.list); psoci_free(t.hdr); psoci_free(t.pool); psoci_free(t.counter);
     psoci_free(cfg); psoci_free(slot); psoci_free(vals); psoci_free(D);
   }
 };
@@ -2238,12 +2238,13 @@ psoci_status tab_prepare(psoci_ctx *c, const Params &P, int64_t npairs, bool own
   k_cfg_rec<W><<<(int)std::min<int64_t>((n + 255) / 256, 152 * 16), 256, 0, st>>>(P, S.cfg);
   // Key slots and pool words that hold the spaces measured, full CI of 2 to 8 electrons and reference
   // spaces with singles and doubles: 0.56 patterns a pair at 32 pairs, 0.12 at 10^4, 5 * 10^4 at
-  // most; the density 10 to 800.  Words: up to 1.9 a pair (64 SEFs), the density 35,000 (16 SEFs), 180,000
-  // (64).  Few pairs take little: an allocation of a megabyte or more costs 30 to 70 us, and the first
-  // density of 1,001 SEFs took 490 us with 2^14 slots and 2^20 words.  A full table grows, and a
-  // pool that was too small, whose keys and slots stay.
+  // most; the density 10 to 800.  Words a pair: up to 1.5 with 16 SEFs; tables of more than 6 open shells take
+  // hundreds to thousands, and few configurations of them hardly share any; the density 35,000 words
+  // with 16 SEFs, 180,000 with 64.  Few pairs take little: an allocation of a megabyte or more costs 30 to
+  // 70 us, and the first density of 1,001 SEFs took 490 us with 2^14 slots and 2^20 words.  A full
+  // table grows, and a pool that was too small, whose keys and slots stay.
   const bool den = grad && !own;
-  const int64_t most = den ? 1 << 12 : 1 << 18, wide = std::max(2, c->max_nsef / 8);
+  const int64_t most = den ? 1 << 12 : 1 << 18, wide = c->max_nsef <= 16 ? 2 : 32 * c->max_nsef;
   int64_t slots = 1 << 11;
   while (slots < npairs / 4 && slots < most) slots <<= 1;
   int64_t cap = den ? std::max(1 << 14, c->max_nsef << 12)
@@ -2251,28 +2252,29 @@ psoci_status tab_prepare(psoci_ctx *c, const Params &P, int64_t npairs, bool own
   cap = std::max<int64_t>(cap, hint + hint / 8);
   bool keyed = false;
   for (int attempt = 0; attempt < 6 && e == cudaSuccess; ++attempt) {
-    if ((!keyed && ((s = psoci_alloc(c, &S.t.keys, slots)) || (s = psoci_alloc(c, &S.t.hdr, 2 * slots)))) ||
+    if ((!keyed && ((s = psoci_alloc(c, &S.t.keys, slots)) || (s = psoci_alloc(c, &S.t.list, slots)) ||
+                    (s = psoci_alloc(c, &S.t.hdr, 2 * slots)))) ||
         (s = psoci_alloc(c, &S.t.pool, cap))) {
       S.free();
       return s;
     }
     S.t.slots = slots;
     S.t.cap = cap;
-    e = cudaMemsetAsync(S.t.counter, 0, 2 * sizeof(unsigned long long), st);
+    e = cudaMemsetAsync(S.t.counter, 0, (keyed ? 1 : 2) * sizeof(unsigned long long), st);
     if (e == cudaSuccess && !keyed) e = cudaMemsetAsync(S.t.keys, 0, sizeof(uint64_t) * slots, st);
     if (e != cudaSuccess) break;
     if (!keyed) {
       psoci_note_launch();
       slots_of(S);
     }
-    const TabBuildArgs B = {S.t.keys, slots, c->d_tmpl, c->d_tmpl_off, c->nelec, c->ksym & 1,
+    const TabBuildArgs B = {S.t.keys, S.t.list, c->d_tmpl, c->d_tmpl_off, c->nelec, c->ksym & 1,
                             S.t.hdr, S.t.pool, S.t.counter, cap, S.t.err};
     psoci_note_launch();
-    k_tab_build<<<(unsigned)(slots / (TABB_SLOTS * TABB_WARPS)), TABB_WARPS * 32, 0, st>>>(B);
+    k_tab_build<<<(unsigned)std::min<int64_t>(slots / TABB_WARPS, 152 * 16), TABB_WARPS * 32, 0, st>>>(B);
     if (grad) {
       psoci_note_launch();
-      k_tab_program<<<(unsigned)(slots / (TABB_SLOTS * 4)), 128, 0, st>>>(S.t.keys, slots, den ? 1 : TAB_LISTS, S.t.hdr,
-                                                                          S.t.pool, S.t.counter, cap);
+      k_tab_program<<<(unsigned)std::min<int64_t>(slots / 4, 152 * 16), 128, 0, st>>>(
+          S.t.list, S.t.err, den ? 1 : TAB_LISTS, S.t.hdr, S.t.pool, S.t.counter, cap);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) break;
     unsigned long long back[2] = {0, 0};  // words used; error bits
@@ -2306,7 +2308,8 @@ psoci_status tab_prepare_lists(psoci_ctx *c, const Params &P, const int64_t *nbr
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)c->nconf * 32 + 255) / 256, 1 << 20));
   auto k = grad ? k_pair_slots<W, false, true> : vals ? k_pair_slots<W, true, false> : k_pair_slots<W, false, false>;
   return tab_prepare<W>(c, P, npairs, true, vals, grad, S, ok, [&](TabSet<W> &T) {
-    k<<<blocks, 256, 0, c->stream>>>(P, T.cfg, nbroff, nbr, T.t.keys, (uint32_t)(T.t.slots - 1), T.t.err, T.slot, T.vals);
+    k<<<blocks, 256, 0, c->stream>>>(P, T.cfg, nbroff, nbr, T.t.keys, (uint32_t)(T.t.slots - 1), T.t.err, T.t.list, T.slot,
+                                     T.vals);
   });
 }
 
@@ -4323,7 +4326,8 @@ template <int W>
 __global__ void __launch_bounds__(256) k_den_slots(Params P, const CfgRec<W> *__restrict__ cfg, int64_t ng, int64_t np,
                                                    const int64_t *__restrict__ geoff, const int64_t *__restrict__ gpoff,
                                                    const int32_t *__restrict__ gcfg, const uint8_t *__restrict__ gorb,
-                                                   uint64_t *keys, uint32_t mask, int *err, uint4 *__restrict__ recs) {
+                                                   uint64_t *keys, uint32_t mask, int *err, uint32_t *list,
+                                                   uint4 *__restrict__ recs) {
   const int64_t nchunk = (np + DEN_CHUNK - 1) / DEN_CHUNK;
   for (int64_t ch = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; ch < nchunk; ch += (int64_t)gridDim.x * blockDim.x) {
     const int64_t t0 = ch * DEN_CHUNK;
@@ -4347,7 +4351,7 @@ __global__ void __launch_bounds__(256) k_den_slots(Params P, const CfgRec<W> *__
       const PairShape s = pair_shape<W>(A, B);
       // members of a group share a hash, not always the occupation: only p -> q singles count
       if (s.kind == K_SINGLE && s.ex0 == p && s.jy0 == q) {
-        sl = tab_insert(keys, mask, pair_key<W>(A, B, s.kind, false), err);
+        sl = tab_insert(keys, mask, pair_key<W>(A, B, s.kind, false), err, list);
         if (sl != TAB_NONE) sl |= s.sign;
       }
       const int x = max(p, q), y = min(p, q);
@@ -4468,6 +4472,7 @@ template <int W>
 psoci_status den_plan(psoci_ctx *c) {
   const Params P = den_params(c);
   const int64_t np = c->den_npairs;
+  if (np == 0) return PSOCI_OK;
   size_t freeb = 0;
   PSOCI_CUDA(c, psoci_mem_free(c, &freeb));
   if ((double)np * sizeof(uint4) > 0.25 * ((double)freeb + (double)c->pool_bytes)) return PSOCI_OK;
@@ -4479,7 +4484,7 @@ psoci_status den_plan(psoci_ctx *c) {
     s = tab_prepare<W>(c, P, np, false, false, true, dir_set<W>(d), ok, [&](TabSet<W> &T) {
       k_den_slots<W><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((np + 1023) / 1024, 152 * 32)), 256, 0, c->stream>>>(
           P, T.cfg, c->den_ng, np, c->den_geoff, c->den_gpoff, c->den_gcfg, c->den_gorb, T.t.keys,
-          (uint32_t)(T.t.slots - 1), T.t.err, c->den_recs);
+          (uint32_t)(T.t.slots - 1), T.t.err, T.t.list, c->den_recs);
     });
   if (s != PSOCI_OK || !ok) {
     delete d;
@@ -4505,8 +4510,7 @@ cudaError_t den_pass(psoci_ctx *c, int k, const double *V, int64_t ldv, double *
   k_grad_rows<KP><<<(unsigned)std::min<int64_t>((N + 255) / 256, 152 * 16), 256, 0, st>>>(N, V, ldv, k, c->den_rows);
   k_den_diag<W, KP><<<(unsigned)std::min<int64_t>((c->nconf + 31) / 32, 152 * 4), 128, 0, st>>>(den_params(c), S.cfg,
                                                                                             c->den_rows, T);
-  if (np > 0)
-    k_den_pairs<KP><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((np * KP + 255) / 256, 152 * 32)), 256, 0, st>>>(
+  k_den_pairs<KP><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((np * KP + 255) / 256, 152 * 32)), 256, 0, st>>>(
         np, c->den_recs, S.t.hdr, S.t.pool, c->den_rows, T);
   k_den_out<KP><<<(ntri * k + 255) / 256, 256, 0, st>>>(ntri, k, T, D);
   return cudaGetLastError();
