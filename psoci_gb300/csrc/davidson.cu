@@ -897,6 +897,9 @@ struct SubBlock {
   const double *val;
 };
 
+// products of a basis of ld vectors and a new block, and the block's squared norms behind them
+size_t small_size(int ld) { return (size_t)ld * TN_MAXK + TN_MAXK * TN_MAXK; }
+
 struct Work {
   psoci_ctx *c = nullptr;
   int64_t N = 0;
@@ -1049,7 +1052,7 @@ psoci_status orthonormalize(Work &w, int m, int b, int *bk) {
   }
   // squared norms before the projection: a column that loses all but 1e-10 of its norm
   // against V (or the block's earlier columns) carries no new direction and is dropped
-  double *ref = w.small + (size_t)ld * ld / 2;
+  double *ref = w.small + small_size(ld) - TN_MAXK * TN_MAXK;
   if ((s = tn(w, w.T, tld, 0, b, w.T, tld, 0, b, ref, b, 0, true))) return s;
   for (int pass = 0; pass < 2 && m > 0; ++pass) {
     // C = V^T T (m x b) into w.small (ld = b), T -= V C
@@ -1251,7 +1254,7 @@ psoci_status davidson_run(psoci_ctx *c, int64_t N, const double *diag, const Sub
       (s = psoci_alloc(c, &w.R, (size_t)N * nr)) ||
       (s = psoci_alloc(c, &w.T, (size_t)N * nr)) || (s = psoci_alloc(c, &w.tmp, (size_t)N * std::max(nr, 2 * nr))) ||
       (s = psoci_alloc(c, &w.partial, (size_t)w.nblk * MAX_SUB * TN_MAXK)) ||
-      (s = psoci_alloc(c, &w.small, (size_t)ld * ld)) || (s = psoci_alloc(c, &w.F, 16 * 16)) ||
+      (s = psoci_alloc(c, &w.small, small_size(ld))) || (s = psoci_alloc(c, &w.F, 16 * 16)) ||
       (s = psoci_alloc(c, &w.norms, 16)) || (s = psoci_alloc(c, &w.sel, 16)) || (s = psoci_alloc(c, &w.ibuf, 4)) ||
       (s = psoci_alloc(c, &w.idx, 16)))
     return s;
@@ -1651,7 +1654,7 @@ psoci_status psoci_basis_create(psoci_ctx *c, int nroots, int max_vectors) {
       (s = psoci_alloc(c, &w.HX, (size_t)N * nroots)) || (s = psoci_alloc(c, &w.R, (size_t)N * nroots)) ||
       (s = psoci_alloc(c, &w.T, (size_t)N * nroots)) || (s = psoci_alloc(c, &w.tmp, (size_t)N * ld)) ||
       (s = psoci_alloc(c, &w.partial, (size_t)w.nblk * MAX_SUB * TN_MAXK)) ||
-      (s = psoci_alloc(c, &w.small, (size_t)ld * ld)) || (s = psoci_alloc(c, &w.F, 16 * 16)) ||
+      (s = psoci_alloc(c, &w.small, small_size(ld))) || (s = psoci_alloc(c, &w.F, 16 * 16)) ||
       (s = psoci_alloc(c, &w.norms, 16)) || (s = psoci_alloc(c, &w.sel, 16)) || (s = psoci_alloc(c, &w.ibuf, 4)) ||
       (s = psoci_alloc(c, &w.idx, 16)) || (s = psoci_alloc(c, &w.x32, (size_t)N * 16)) ||
       (s = psoci_alloc(c, &b->shift, 16))) {
