@@ -44,3 +44,21 @@ def test_dependent_vectors_are_dropped(kw, support, b, rank):
     assert lib.psoci_basis_vectors(c.ctx, rank, out.ctypes.data_as(ctypes.POINTER(ctypes.c_double))) == 0
     assert np.array_equal(out, ind / np.sqrt(support))
     c.close()
+
+
+@pytest.mark.parametrize("kw", [dict(nbf=6, nelec=4), dict(nbf=9, nelec=5)])
+@pytest.mark.parametrize("nroots,copies", [(3, 3), (9, 9), (16, 12)])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_restart_from_copies(kw, nroots, copies, mixed):
+    """Restart vectors that are copies of one: the roots are those of a solve without them."""
+    from psoci_gb300.inputs import make_problem
+
+    c = gpu_context(make_problem("fci", seed=5, ksym=2, **kw))
+    c.build_hamiltonian(mixed=mixed)
+    free = c.davidson(nroots, rtol=1e-8, mixed=mixed)
+    v = np.zeros((copies, c.nsef))
+    v[:, 7] = 1.0
+    c.set_guess(v)
+    r = c.davidson(nroots, rtol=1e-8, mixed=mixed)
+    assert np.abs(r.evals - free.evals).max() <= 1e-9
+    c.close()
