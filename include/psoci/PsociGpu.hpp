@@ -208,10 +208,17 @@ class PsociGAhamiltonian {
     check(dev_.get(), psoci_build_hamiltonian(dev_.get(), PSOCI_HMODE_DIRECT, &nnz_), "psoci_build_hamiltonian");
   }
   int64_t numberNonzeroElements() const { return nnz_; }
-  // the build's element evaluation in one launch (launches = 1: less memory, slower; the
-  // same matrix) or the automatic choice (0); no reference counterpart
+  // the build's pair integrals evaluated in the element launches (launches = 1: less memory,
+  // slower; the same matrix) or the automatic choice (0); no reference counterpart
   void setEvalLaunches(int launches) {
     check(dev_.get(), psoci_set_eval_launches(dev_.get(), launches), "psoci_set_eval_launches");
+  }
+  // device memory that the context may take (0: no limit); the bytes in use; stands in for the
+  // fixed memory of the Global Arrays processes
+  int64_t setMemoryLimit(int64_t bytes) {
+    int64_t held = 0;
+    check(dev_.get(), psoci_set_memory_limit(dev_.get(), bytes, &held), "psoci_set_memory_limit");
+    return held;
   }
   // constructCIdensityAltOrbMapChunkJmap (PsociGAhamiltonian.C:11570-11760): density[root] is
   // the packed nbf(nbf+1)/2 spin-free 1-particle density of root-major vectors vecs (k x N)

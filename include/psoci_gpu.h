@@ -133,9 +133,9 @@ typedef struct {
   int64_t nnz;           /* stored elements, both triangles                                  */
   int64_t nnz_lower;     /* the reference's lower-triangle count, (nnz + N) / 2              */
   int64_t slab_slots;    /* 0 (the build has no value slab)                                  */
-  int evaluations;       /* 1                                                                */
-  int fast;              /* 1: elements from coupling tables (at most 10 open shells);       */
-                         /* 0: generic path                                                  */
+  int evaluations;       /* 1; 0 in direct mode                                              */
+  int fast;              /* 1: a stored matrix from coupling tables (at most 10 open shells) */
+                         /* 0: from the generic kernels, or direct mode (tables or not)      */
   int lookup_screen;     /* 1: neighbours found by table lookup; 0: all-pairs test            */
   int eval_launches;     /* fast path: 2 pair integrals in a launch of their own, 1 in the   */
                          /* element launches; 0 otherwise                                    */

@@ -158,6 +158,7 @@ __device__ __forceinline__ uint64_t pair_key(const CfgRec<W> &A, const CfgRec<W>
          ((uint64_t)((B.flags >> 6) & 1u) << 54);
 }
 
+// the 64-bit mixer published by degski (invertible_hash_functions.hpp)
 __device__ __forceinline__ uint64_t tab_hash(uint64_t x) {
   x ^= x >> 32;
   x *= 0xd6e8feb86659fd93ull;
