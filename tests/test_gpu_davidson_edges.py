@@ -67,10 +67,10 @@ def test_orthonormal_set(rows, k):
     assert np.abs(v - (v @ q.T) @ q).max() <= 1e-11
 
 
-@pytest.mark.parametrize("nbf,nroots", [(5, 15), (6, 16)])
+@pytest.mark.parametrize("nbf,nroots", [(2, 3), (3, 6), (5, 15), (6, 16)])
 @pytest.mark.parametrize("mixed", [False, True])
 def test_many_roots_of_few_rows(nbf, nroots, mixed):
-    """15 of 15 and 16 of 21 roots, against a dense eigen-solve: residuals of 1e-8."""
+    """All of 3, 6 and 15 roots and 16 of 21, against a dense eigen-solve: residuals of 1e-8."""
     import scipy.sparse as sp
 
     from psoci_gb300.inputs import make_problem
